@@ -73,62 +73,13 @@ extern "C" int wahgpu_index_from_triple(wahgpu_ctx* ctx, int kind, uint64_t nrow
     return WAHGPU_OK;
 }
 
-// Per tile, the bitmaps holding a 1 bit in it (ascending), so a range term
-// visits only bitmaps with data in the tile: pairs (tile, bitmap) emitted in
-// bitmap order, stably sorted by tile, cut into CSR offsets.
-static int build_tile_lists(wahgpu_index* x) {
-    wahgpu_ctx* ctx = x->ctx;
-    const uint32_t nobs = x->nobs, nt = x->ntiles;
-    x->d_tl_off = static_cast<uint32_t*>(wg_alloc(ctx, ((size_t)nt + 1) * 4));
-    if (!x->d_tl_off) return wg_fail(ctx, WAHGPU_ENOMEM, "index allocation failed");
-    if (nobs == 0) {
-        CUDA_TRY(ctx, cudaMemsetAsync(x->d_tl_off, 0, ((size_t)nt + 1) * 4, ctx->stream));
-        x->d_tl_bm = static_cast<uint32_t*>(wg_alloc(ctx, 4));
-        return x->d_tl_bm ? WAHGPU_OK : wg_fail(ctx, WAHGPU_ENOMEM, "index allocation failed");
-    }
-    std::vector<void*> tmp;
-    auto get = [&](size_t bytes) { void* p = wg_alloc(ctx, std::max<size_t>(bytes, 16)); if (p) tmp.push_back(p); return p; };
-    auto release = [&]() { cudaStreamSynchronize(ctx->stream); for (void* p : tmp) wg_free(ctx, p); };
-    uint32_t* cnt = static_cast<uint32_t*>(get(((size_t)nobs + 1) * 4));
-    if (!cnt) { release(); return wg_fail(ctx, WAHGPU_ENOMEM, "index allocation failed"); }
-    const uint32_t threads = 256, blocks = (nobs * 32 + threads - 1) / threads;
-    CUDA_TRY(ctx, cudaMemsetAsync(cnt + nobs, 0, 4, ctx->stream));
-    k_tile_touch<<<blocks, threads, 0, ctx->stream>>>(x->d_words, x->d_bm, nobs, 0, cnt, nullptr, nullptr, nullptr);
-    size_t tb = 0;
-    CUDA_TRY(ctx, cub::DeviceScan::ExclusiveSum(nullptr, tb, cnt, cnt, nobs + 1, ctx->stream));
-    void* t1 = get(tb);
-    if (!t1) { release(); return wg_fail(ctx, WAHGPU_ENOMEM, "index allocation failed"); }
-    CUDA_TRY(ctx, cub::DeviceScan::ExclusiveSum(t1, tb, cnt, cnt, nobs + 1, ctx->stream));
-    uint32_t npairs = 0;
-    CUDA_TRY(ctx, cudaMemcpyAsync(&npairs, cnt + nobs, 4, cudaMemcpyDeviceToHost, ctx->stream));
-    CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-    uint32_t* pt = static_cast<uint32_t*>(get((size_t)npairs * 4));
-    uint32_t* pb = static_cast<uint32_t*>(get((size_t)npairs * 4));
-    uint32_t* st = static_cast<uint32_t*>(get((size_t)npairs * 4));
-    x->d_tl_bm = static_cast<uint32_t*>(wg_alloc(ctx, std::max<size_t>((size_t)npairs * 4, 16)));
-    if (!pt || !pb || !st || !x->d_tl_bm) { release(); return wg_fail(ctx, WAHGPU_ENOMEM, "index allocation failed"); }
-    k_tile_touch<<<blocks, threads, 0, ctx->stream>>>(x->d_words, x->d_bm, nobs, 1, nullptr, cnt, pt, pb);
-    int bits = 1;
-    while (bits < 32 && (1ull << bits) <= nt) ++bits;
-    tb = 0;
-    CUDA_TRY(ctx, cub::DeviceRadixSort::SortPairs(nullptr, tb, pt, st, pb, x->d_tl_bm, npairs, 0, bits, ctx->stream));
-    void* t2 = get(tb);
-    if (!t2) { release(); return wg_fail(ctx, WAHGPU_ENOMEM, "index allocation failed"); }
-    CUDA_TRY(ctx, cub::DeviceRadixSort::SortPairs(t2, tb, pt, st, pb, x->d_tl_bm, npairs, 0, bits, ctx->stream));
-    k_tile_offsets<<<(npairs + 1 + threads - 1) / threads, threads, 0, ctx->stream>>>(st, npairs, nt, x->d_tl_off);
-    ctx->launches += 5;
-    CUDA_TRY(ctx, cudaGetLastError());
-    release();
-    return WAHGPU_OK;
-}
-
 // Cumulative rows: for a stride S, dense row k-1 = OR of bitmaps [0, k*S)
 // (k = 1..K), so a range's wholly-inside span costs two dense reads per tile
 // plus at most 2S edge bitmaps.  S is the smallest stride >= 8 that keeps
 // the rows within CUM_BUDGET bytes (or the context's WAHGPU_TUNE_CUM_STRIDE);
 // indexes with fewer than two rows' worth of bitmaps keep none.
 static constexpr uint64_t CUM_BUDGET = 2ull << 30;
-static int build_cumulative(wahgpu_index* x) {
+static int cumulative_rows(wahgpu_index* x) {
     wahgpu_ctx* ctx = x->ctx;
     const uint32_t nobs = x->nobs;
     // rows are gx words rounded up to 4, so a tile's slice starts 16-byte aligned
@@ -142,56 +93,105 @@ static int build_cumulative(wahgpu_index* x) {
     x->d_cum = static_cast<uint32_t*>(wg_alloc(ctx, K * gx * 4));
     if (!x->d_cum) return WAHGPU_OK;  // no room: ranges use the bitmaps alone
     CUDA_TRY(ctx, cudaMemsetAsync(x->d_cum, 0, K * gx * 4, ctx->stream));
-    const uint32_t nb = (uint32_t)(K * stride), threads = 256;
-    const uint32_t blocks = (uint32_t)(((uint64_t)nb * 32 + threads - 1) / threads);
-    k_cum_blocks<<<blocks, threads, 0, ctx->stream>>>(x->d_words, x->d_bm, nb, (uint32_t)stride, (uint32_t)gx, x->d_cum);
-    k_cum_prefix<<<(uint32_t)((gx + 255) / 256), 256, 0, ctx->stream>>>(x->d_cum, (uint32_t)K, (uint32_t)gx);
-    ctx->launches += 2;
-    CUDA_TRY(ctx, cudaGetLastError());
     x->cum_k = (uint32_t)K;
     x->cum_stride = (uint32_t)stride;
     return WAHGPU_OK;
 }
 
+// Device blocks held for the duration of a call; they go back to the pool on
+// exit (whoever takes them next is ordered after this call on the stream).
+struct Temps {
+    wahgpu_ctx* ctx;
+    std::vector<void*> p;
+    explicit Temps(wahgpu_ctx* c) : ctx(c) {}
+    template <class T> T* get(size_t n) {
+        void* q = wg_alloc(ctx, std::max<size_t>(n * sizeof(T), 16));
+        if (q) p.push_back(q);
+        return static_cast<T*>(q);
+    }
+    ~Temps() { for (void* q : p) wg_free(ctx, q); }
+};
+
 // Second half of building an index, shared by the triple upload and the
-// device build: x->d_words / d_bm / bwords / keys are set; computes the
-// per-bitmap tile index and 1-bit counts and validates the words.
+// device build: x->d_words / d_bm / bwords / keys are set; validates the
+// words and computes the per-bitmap tile index and 1-bit counts, the tiles'
+// bitmap lists and the cumulative rows.
 int wg_index_attach(wahgpu_index* x) {
     wahgpu_ctx* ctx = x->ctx;
     const uint32_t nobs = x->nobs;
     x->ntiles = (x->groups + (x->anb ? 1 : 0) + RT - 1) / RT;
-    const size_t tiles_bytes = (size_t)nobs * (x->ntiles + 1) * 8;
-    x->d_tiles = static_cast<uint32_t*>(wg_alloc(ctx, std::max<size_t>(tiles_bytes, 8)));
-    uint32_t* d_ones = static_cast<uint32_t*>(wg_alloc(ctx, std::max<size_t>(nobs, 1) * 4));
-    DevMeta* d_st = static_cast<DevMeta*>(wg_alloc(ctx, sizeof(DevMeta)));
-    if (!x->d_tiles || !d_ones || !d_st) {
-        wg_free(ctx, d_ones);
-        wg_free(ctx, d_st);
+    const uint32_t nt = x->ntiles;
+    Temps tmp(ctx);
+    std::vector<uint32_t> choff(nobs + 1, 0);
+    uint64_t nch = 0;
+    for (uint32_t j = 0; j < nobs; ++j) {
+        nch += std::max<uint64_t>(1, (x->bwords[j] + ICHUNK - 1) / ICHUNK);
+        choff[j + 1] = (uint32_t)nch;
+    }
+    if (nch * 32 > 0xFFFFFFFFull) return wg_fail(ctx, WAHGPU_ERANGE, "index of %llu word chunks", (unsigned long long)nch);
+    const uint32_t nchunks = (uint32_t)nch;
+    x->d_tiles = static_cast<uint32_t*>(wg_alloc(ctx, std::max<size_t>((size_t)nobs * (nt + 1) * 8, 8)));
+    x->d_tl_off = static_cast<uint32_t*>(wg_alloc(ctx, ((size_t)nt + 1) * 4));
+    uint32_t* d_choff = tmp.get<uint32_t>((size_t)nobs + 1);
+    unsigned long long* d_cg = tmp.get<unsigned long long>(nchunks);
+    uint32_t* d_co = tmp.get<uint32_t>(nchunks);
+    uint32_t* d_ones = tmp.get<uint32_t>(nobs);
+    DevMeta* d_st = tmp.get<DevMeta>(1);
+    if (!x->d_tiles || !x->d_tl_off || !d_choff || !d_cg || !d_co || !d_ones || !d_st)
         return wg_fail(ctx, WAHGPU_ENOMEM, "index allocation failed");
-    }
-    int rc = WAHGPU_OK;
+    const uint32_t blocks = (uint32_t)(((uint64_t)nchunks * 32 + ITHREADS - 1) / ITHREADS);
     CUDA_TRY(ctx, cudaMemsetAsync(d_st, 0, sizeof(DevMeta), ctx->stream));
-    if (nobs) {
-        const uint32_t threads = 256, blocks = (nobs * 32 + threads - 1) / threads;
-        k_index_tiles<<<blocks, threads, 0, ctx->stream>>>(x->d_words, x->d_bm, nobs, x->ntiles, x->nrows,
-                                                           x->d_tiles, d_ones, d_st);
-        ctx->launches++;
-        CUDA_TRY(ctx, cudaGetLastError());
-    }
     DevMeta st{};
     x->bones.resize(nobs);
-    CUDA_TRY(ctx, cudaMemcpyAsync(&st, d_st, sizeof(DevMeta), cudaMemcpyDeviceToHost, ctx->stream));
-    if (nobs) CUDA_TRY(ctx, cudaMemcpyAsync(x->bones.data(), d_ones, nobs * 4, cudaMemcpyDeviceToHost, ctx->stream));
+    if (nobs) {
+        CUDA_TRY(ctx, cudaMemcpyAsync(d_choff, choff.data(), ((size_t)nobs + 1) * 4, cudaMemcpyHostToDevice, ctx->stream));
+        k_chunk_sums<<<blocks, ITHREADS, 0, ctx->stream>>>(x->d_words, x->d_bm, nobs, d_choff, nchunks, d_cg, d_co, d_st);
+        k_chunk_scan<<<(uint32_t)(((uint64_t)nobs * 32 + ITHREADS - 1) / ITHREADS), ITHREADS, 0, ctx->stream>>>(
+            x->d_bm, nobs, d_choff, x->nrows, d_cg, d_co, d_ones, d_st);
+        ctx->launches += 2;
+        CUDA_TRY(ctx, cudaGetLastError());
+        CUDA_TRY(ctx, cudaMemcpyAsync(&st, d_st, sizeof(DevMeta), cudaMemcpyDeviceToHost, ctx->stream));
+        CUDA_TRY(ctx, cudaMemcpyAsync(x->bones.data(), d_ones, (size_t)nobs * 4, cudaMemcpyDeviceToHost, ctx->stream));
+    }
     CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-    wg_free(ctx, d_ones);
-    wg_free(ctx, d_st);
-    if (st.status == DEV_ERR_FORMAT) rc = wg_fail(ctx, WAHGPU_EFORMAT, "a bitmap holds a fill word of length 0");
-    else if (st.status) rc = wg_fail(ctx, WAHGPU_ERANGE, "a bitmap holds more bits than the index has rows");
+    if (st.status == DEV_ERR_FORMAT) return wg_fail(ctx, WAHGPU_EFORMAT, "a bitmap holds a fill word of length 0");
+    if (st.status) return wg_fail(ctx, WAHGPU_ERANGE, "a bitmap holds more bits than the index has rows");
+    // the words are valid: every position below lies inside the index's rows
+    const uint32_t tw = (nobs + 31) / 32;
+    uint64_t most = 0;  // entries of the tile lists at most: a tile on a bitmap's list holds one of its 1 bits
+    for (uint32_t j = 0; j < nobs; ++j) most += std::min<uint64_t>(nt, x->bones[j]);
+    x->d_tl_bm = static_cast<uint32_t*>(wg_alloc(ctx, std::max<size_t>(most * 4, 16)));
+    if (!x->d_tl_bm) return wg_fail(ctx, WAHGPU_ENOMEM, "index allocation failed");
+    int rc = cumulative_rows(x);
     if (rc) return rc;
-    rc = build_tile_lists(x);
-    if (rc) return rc;
-    rc = build_cumulative(x);
-    if (rc) return rc;
+    if (nobs && nt) {
+        uint32_t* touch = tmp.get<uint32_t>((size_t)nt * tw);
+        if (!touch) return wg_fail(ctx, WAHGPU_ENOMEM, "index allocation failed");
+        CUDA_TRY(ctx, cudaMemsetAsync(touch, 0, (size_t)nt * tw * 4, ctx->stream));
+        PlaceArgs a;
+        a.words = x->d_words; a.bm = x->d_bm; a.nobs = nobs; a.choff = d_choff; a.nchunks = nchunks; a.cstart = d_cg;
+        a.ntiles = nt; a.tiles = x->d_tiles; a.touch = touch; a.tw = tw;
+        a.gx = (x->groups + (x->anb ? 1u : 0u) + 3u) & ~3u;
+        a.cum = x->cum_k ? x->d_cum : nullptr;
+        a.cum_nb = x->cum_k * x->cum_stride; a.cum_stride = x->cum_stride;
+        k_chunk_place<<<blocks, ITHREADS, 0, ctx->stream>>>(a);
+        const uint32_t nparts = (uint32_t)(((uint64_t)nt * tw + LTILE - 1) / LTILE);
+        TileRec* recs; LaunchSync* sync;
+        rc = wg_scratch(ctx, nparts, &recs, &sync);
+        if (rc) return rc;
+        k_tile_lists<<<nparts, ITHREADS, 0, ctx->stream>>>(touch, tw, nt, x->d_tl_off, x->d_tl_bm, d_st, recs, sync, nparts);
+        ctx->launches += 2;
+        if (x->cum_k) {
+            k_cum_prefix<<<(a.gx + 255) / 256, 256, 0, ctx->stream>>>(x->d_cum, x->cum_k, a.gx);
+            ctx->launches++;
+        }
+        CUDA_TRY(ctx, cudaGetLastError());
+        CUDA_TRY(ctx, cudaMemcpyAsync(&st, d_st, sizeof(DevMeta), cudaMemcpyDeviceToHost, ctx->stream));
+        CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+        if (st.status) return wg_fail(ctx, WAHGPU_ETIMEOUT, "a device-side look-back wait gave up");
+    } else {
+        CUDA_TRY(ctx, cudaMemsetAsync(x->d_tl_off, 0, ((size_t)nt + 1) * 4, ctx->stream));
+    }
     x->cum_words.assign(nobs + 1, 0);
     x->cum_ones.assign(nobs + 1, 0);
     for (uint32_t j = 0; j < nobs; ++j) {

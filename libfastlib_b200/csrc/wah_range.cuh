@@ -50,7 +50,7 @@ struct BitmapMeta {
     uint32_t n;       // m_vec words
     uint32_t anb;     // active bits
     uint32_t aval;    // active value
-    uint32_t groups;  // groups covered by m_vec (set by k_index_tiles)
+    uint32_t groups;  // groups covered by m_vec (set by k_chunk_scan)
 };
 
 struct DevIndex {
@@ -668,164 +668,253 @@ __global__ void __launch_bounds__(RTHREADS, 6) k_range(RangeArgs A) {
     if (tid == 0) finish_tile(A.sync, gridDim.x);
 }
 
-// Per-bitmap group-tile index of an attached index: one warp per bitmap
-// walks its words, records the word covering every multiple of RT, checks
-// the words and counts groups and ones.
-__global__ void k_index_tiles(const uint32_t* __restrict__ words, BitmapMeta* __restrict__ bm,
-                              uint32_t nobs, uint32_t ntiles, uint32_t nrows, uint32_t* __restrict__ tiles,
-                              uint32_t* __restrict__ bones, DevMeta* status) {
+// ---- attach: the passes over a new index's words
+// Every bitmap's words are cut into chunks of ICHUNK words, a warp each
+// (chunks choff[b] .. choff[b+1] are bitmap b's, at least one).  With a warp
+// per bitmap the few heavy bitmaps of a low-cardinality column set the time:
+// 100 bitmaps over 1M rows (3000 chunks) took 1430 us for the four passes
+// over the words there were, and take 51 us now (sums 6, scan 7, placement
+// 19, lists 9, prefix 9).  The passes are bound by their few dependent memory
+// round trips.  512 words: 16 rows of 32, four loaded per memory latency,
+// and still enough warps for a few bitmaps.
+constexpr uint32_t ICHUNK = 512;
+constexpr uint32_t ITHREADS = 256;  // threads per CTA of the attach kernels
+
+// Bitmap of chunk c: the last b with choff[b] <= c (whole warp).
+__device__ __forceinline__ uint32_t chunk_bitmap(const uint32_t* __restrict__ choff, uint32_t nobs, uint32_t c) {
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (b >= nobs) return;
-    const BitmapMeta m = bm[b];
-    const uint32_t* w = words + m.wstart;
-    uint32_t* tix = tiles + (size_t)b * (ntiles + 1) * 2;
-    uint32_t carry = 0, ones = 0, bad = 0;
-    for (uint32_t base = 0; base < m.n; base += 32) {
-        const uint32_t i = base + lane;
-        const bool in = i < m.n;
-        const uint32_t wd = in ? __ldg(w + i) : 0u;
-        const uint32_t c = in ? wgroups(wd) : 0u;
-        if (in && is_fill(wd) && c == 0) bad = 1;
-        if (in) ones += wd > ALLONES ? (wd >= HEADER1 ? c * 31u : 0u) : __popc(wd);
-        uint32_t x = c;
+    uint32_t lo = 0, hi = nobs;  // choff[lo] <= c < choff[hi]
+    while (hi - lo > 1u) {
+        const uint32_t step = (hi - lo + 31u) / 32u;
+        const uint32_t m = lo + lane * step;
+        const uint32_t k = __popc(__ballot_sync(0xffffffffu, m < hi && __ldg(choff + m) <= c));  // >= 1: lane 0
+        lo += (k - 1u) * step;
+        hi = min(hi, lo + step);
+    }
+    return lo;
+}
+
+// Groups and 1 bits of every chunk; a fill word of length 0 is a format error.
+__global__ void __launch_bounds__(ITHREADS)
+k_chunk_sums(const uint32_t* __restrict__ words, const BitmapMeta* __restrict__ bm, uint32_t nobs,
+             const uint32_t* __restrict__ choff, uint32_t nchunks, unsigned long long* __restrict__ cgroups,
+             uint32_t* __restrict__ cones, DevMeta* status) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t c = (blockIdx.x * ITHREADS + threadIdx.x) >> 5;
+    if (c >= nchunks) return;
+    const uint32_t b = chunk_bitmap(choff, nobs, c);
+    const uint32_t* w = words + bm[b].wstart;
+    const uint32_t i0 = (c - __ldg(choff + b)) * ICHUNK, i1 = min(i0 + ICHUNK, bm[b].n);
+    unsigned long long groups = 0;
+    uint32_t ones = 0, bad = 0;
+    for (uint32_t base = i0; base < i1; base += 128) {
+        uint32_t v[4];
 #pragma unroll
-        for (int d = 1; d < 32; d <<= 1) { uint32_t t = __shfl_up_sync(0xffffffffu, x, d); if (lane >= (uint32_t)d) x += t; }
-        const uint32_t p = carry + x - c;  // first group of word i
-        // word i covers boundaries t*RT in [p, p+c)
-        if (in && c > 0) {
-            uint32_t t = (p + RT - 1) / RT;
-            for (; (uint64_t)t * RT < (uint64_t)p + c && t <= ntiles; ++t) {
-                tix[2 * t] = i;
-                tix[2 * t + 1] = p;
-            }
+        for (int j = 0; j < 4; ++j) {
+            const uint32_t i = base + 32u * j + lane;
+            v[j] = i < i1 ? __ldg(w + i) : 0u;
         }
-        carry += __shfl_sync(0xffffffffu, x, 31);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (base + 32u * j + lane >= i1) break;
+            const uint32_t cnt = wgroups(v[j]);
+            groups += cnt;
+            ones += v[j] > ALLONES ? (v[j] >= HEADER1 ? cnt * 31u : 0u) : __popc(v[j]);
+            bad |= cnt == 0u ? 1u : 0u;
+        }
     }
-    // boundaries at or past the end of the words
-    for (uint32_t t = lane; t <= ntiles; t += 32) {
-        if ((uint64_t)t * RT >= carry) { tix[2 * t] = m.n; tix[2 * t + 1] = carry; }
-    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) groups += __shfl_xor_sync(0xffffffffu, groups, d);
     ones = __reduce_add_sync(0xffffffffu, ones);
     bad = __reduce_or_sync(0xffffffffu, bad);
     if (lane == 0) {
-        bm[b].groups = carry;
-        bones[b] = ones + __popc(m.anb ? (m.aval & ((1u << m.anb) - 1u)) : 0u);
+        cgroups[c] = groups;
+        cones[c] = ones;
         if (bad) atomicExch(&status->status, DEV_ERR_FORMAT);
-        else if ((uint64_t)carry * 31u + m.anb > nrows) atomicExch(&status->status, DEV_ERR_RANGE);
     }
 }
 
-// Tiles of RT groups in which bitmap b holds a 1 bit, each once and in
-// order (one warp per bitmap).  Pass 0 counts them into cnt[b]; pass 1
-// writes (tile, bitmap) pairs from pos[b].
-__global__ void k_tile_touch(const uint32_t* __restrict__ words, const BitmapMeta* __restrict__ bm,
-                             uint32_t nobs, int pass, uint32_t* __restrict__ cnt,
-                             const uint32_t* __restrict__ pos, uint32_t* __restrict__ out_tile,
-                             uint32_t* __restrict__ out_bm) {
+// A warp per bitmap: the first group of each of its chunks (in place of the
+// chunk's group count), the bitmap's groups and 1 bits; a bitmap of more bits
+// than the index has rows is a range error.
+__global__ void __launch_bounds__(ITHREADS)
+k_chunk_scan(BitmapMeta* __restrict__ bm, uint32_t nobs, const uint32_t* __restrict__ choff, uint32_t nrows,
+             unsigned long long* __restrict__ cgroups, const uint32_t* __restrict__ cones,
+             uint32_t* __restrict__ bones, DevMeta* status) {
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t b = (blockIdx.x * ITHREADS + threadIdx.x) >> 5;
     if (b >= nobs) return;
-    const BitmapMeta m = bm[b];
-    const uint32_t* w = words + m.wstart;
-    uint32_t carry = 0;        // first group of the next word
-    int64_t last = -1;         // last tile emitted
-    uint32_t n = 0;            // tiles emitted so far
-    const uint32_t o = pass ? pos[b] : 0u;
-    for (uint32_t base = 0; base < m.n; base += 32) {
-        const uint32_t i = base + lane;
-        const bool in = i < m.n;
-        const uint32_t wd = in ? __ldg(w + i) : 0u;
-        const uint32_t c = in ? wgroups(wd) : 0u;
-        uint32_t x = c;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) { uint32_t t = __shfl_up_sync(0xffffffffu, x, d); if (lane >= (uint32_t)d) x += t; }
-        const uint32_t p = carry + x - c;
-        const bool bits = in && c > 0 && (wd >= HEADER1 || (wd <= ALLONES && wd != 0u));
-        // tiles [k0, k1] of this word, minus those an earlier word emitted
-        int64_t k0 = bits ? (int64_t)(p / RT) : 0, k1 = bits ? (int64_t)((p + c - 1u) / RT) : -1;
-        int64_t prev = bits ? k1 : -1;  // highest tile of lanes up to this one
+    const uint32_t c0 = __ldg(choff + b), c1 = __ldg(choff + b + 1);
+    unsigned long long carry = 0;
+    uint32_t ones = 0;
+    for (uint32_t base = c0; base < c1; base += 32) {
+        const uint32_t c = base + lane;
+        const unsigned long long g = c < c1 ? cgroups[c] : 0ull;
+        if (c < c1) ones += __ldg(cones + c);
+        unsigned long long x = g;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
-            const int64_t t = __shfl_up_sync(0xffffffffu, prev, d);
-            if (lane >= (uint32_t)d) prev = max(prev, t);
+            const unsigned long long t = __shfl_up_sync(0xffffffffu, x, d);
+            if (lane >= (uint32_t)d) x += t;
         }
-        int64_t before = __shfl_up_sync(0xffffffffu, prev, 1);
-        if (lane == 0) before = -1;
-        before = max(before, last);
-        if (bits) k0 = max(k0, before + 1);
-        const uint32_t mine = (bits && k1 >= k0) ? (uint32_t)(k1 - k0 + 1) : 0u;
-        uint32_t ex = mine;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) { uint32_t t = __shfl_up_sync(0xffffffffu, ex, d); if (lane >= (uint32_t)d) ex += t; }
-        if (pass && mine) {
-            uint32_t q = o + n + ex - mine;
-            for (int64_t k = k0; k <= k1; ++k, ++q) { out_tile[q] = (uint32_t)k; out_bm[q] = b; }
-        }
-        n += __shfl_sync(0xffffffffu, ex, 31);
-        last = max(last, __shfl_sync(0xffffffffu, prev, 31));
+        if (c < c1) cgroups[c] = carry + x - g;
         carry += __shfl_sync(0xffffffffu, x, 31);
     }
-    // the active bits form the group after the whole words
+    ones = __reduce_add_sync(0xffffffffu, ones);
     if (lane == 0) {
-        if (m.anb > 0 && (m.aval & ((1u << m.anb) - 1u)) != 0u) {
-            const int64_t k = carry / RT;
-            if (k > last) {
-                if (pass) { out_tile[o + n] = (uint32_t)k; out_bm[o + n] = b; }
-                ++n;
+        const uint32_t anb = bm[b].anb, aval = bm[b].aval;
+        bm[b].groups = (uint32_t)carry;
+        bones[b] = ones + __popc(anb ? (aval & ((1u << anb) - 1u)) : 0u);
+        if (carry * 31ull + anb > nrows) atomicCAS(&status->status, 0u, DEV_ERR_RANGE);
+    }
+}
+
+struct PlaceArgs {
+    const uint32_t* words; const BitmapMeta* bm; uint32_t nobs;
+    const uint32_t* choff; uint32_t nchunks;
+    const unsigned long long* cstart;  // first group of every chunk
+    uint32_t ntiles;
+    uint32_t* tiles;      // per-bitmap tile index: nobs x (ntiles+1) x {word, its first group}
+    uint32_t* touch;      // ntiles x tw words, bit b of row k: bitmap b holds a 1 bit in tile k (zeroed)
+    uint32_t tw;
+    uint32_t* cum;        // block ORs for the cumulative rows (zeroed), or null
+    uint32_t cum_nb, cum_stride, gx;  // bitmaps b < cum_nb go into row b / cum_stride
+};
+
+// Second pass over the words, from every chunk's first group: the word
+// covering each multiple of RT groups, the tiles the bitmap touches, and its
+// bits OR'ed into its block's cumulative row (1-fills of more than 32 groups
+// by the whole warp).
+__global__ void __launch_bounds__(ITHREADS) k_chunk_place(PlaceArgs A) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t ch = (blockIdx.x * ITHREADS + threadIdx.x) >> 5;
+    if (ch >= A.nchunks) return;
+    const uint32_t b = chunk_bitmap(A.choff, A.nobs, ch);
+    const BitmapMeta m = A.bm[b];
+    const uint32_t* w = A.words + m.wstart;
+    const uint32_t i0 = (ch - __ldg(A.choff + b)) * ICHUNK, i1 = min(i0 + ICHUNK, m.n);
+    const bool last_chunk = ch + 1u == __ldg(A.choff + b + 1);
+    uint32_t* tix = A.tiles + (size_t)b * (A.ntiles + 1) * 2;
+    uint32_t* tcol = A.touch + (b >> 5);  // + tile * tw
+    const uint32_t tbit = 1u << (b & 31u);
+    uint32_t* row = A.cum && b < A.cum_nb ? A.cum + (size_t)(b / A.cum_stride) * A.gx : nullptr;
+    uint32_t carry = (uint32_t)A.cstart[ch];
+    uint32_t marked = 0xFFFFFFFFu;  // the last tile this chunk marked
+    for (uint32_t base0 = i0; base0 < i1; base0 += 128) {
+        uint32_t v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint32_t i = base0 + 32u * j + lane;
+            v[j] = i < i1 ? __ldg(w + i) : 0u;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint32_t base = base0 + 32u * j;
+            if (base >= i1) break;
+            const uint32_t i = base + lane;
+            const bool in = i < i1;
+            const uint32_t wd = v[j];
+            const uint32_t c = in ? wgroups(wd) : 0u;
+            uint32_t p;
+            if (__ballot_sync(0xffffffffu, in && is_fill(wd)) == 0u) {
+                p = carry + lane;
+                carry += min(32u, i1 - base);
+            } else {
+                uint32_t x = c;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const uint32_t t = __shfl_up_sync(0xffffffffu, x, d);
+                    if (lane >= (uint32_t)d) x += t;
+                }
+                p = carry + x - c;
+                carry += __shfl_sync(0xffffffffu, x, 31);
+            }
+            const uint32_t k0 = p / RT, k1 = c ? (p + c - 1u) / RT : k0;
+            // word i covers the boundaries t * RT in [p, p + c)
+            if (c) for (uint32_t t = k0 * RT == p ? k0 : k0 + 1u; t <= k1; ++t) { tix[2 * t] = i; tix[2 * t + 1] = p; }
+            const bool bits = c != 0u && (wd >= HEADER1 || (wd <= ALLONES && wd != 0u));
+            // positions ascend, so a tile that the nearest lane before this
+            // one with bits (or the row before) marked needs no second mark:
+            // few addresses, and an atomic per word would queue on them
+            const uint32_t hb = __ballot_sync(0xffffffffu, bits);
+            const uint32_t below = hb & ((1u << lane) - 1u);
+            const uint32_t near = __shfl_sync(0xffffffffu, k1, below ? 31u - __clz(below) : lane);
+            const uint32_t before = below ? near : marked;
+            if (bits)
+                for (uint32_t k = k0 == before ? k0 + 1u : k0; k <= k1; ++k) atomicOr(tcol + (size_t)k * A.tw, tbit);
+            if (hb) marked = __shfl_sync(0xffffffffu, k1, 31u - __clz(hb));
+            if (row) {
+                if (bits && wd <= ALLONES) atomicOr(row + p, wd);
+                else if (bits && c <= 32u) for (uint32_t g = 0; g < c; ++g) row[p + g] = ALLONES;
+                uint32_t f = __ballot_sync(0xffffffffu, bits && wd >= HEADER1 && c > 32u);
+                while (f) {
+                    const uint32_t src = __ffs(f) - 1u;
+                    f &= f - 1u;
+                    const uint32_t fp = __shfl_sync(0xffffffffu, p, src), fc = __shfl_sync(0xffffffffu, c, src);
+                    for (uint32_t g = lane; g < fc; g += 32u) row[fp + g] = ALLONES;
+                }
             }
         }
-        if (!pass) cnt[b] = n;
     }
-}
-
-// CSR offsets of the tile-sorted pairs: off[k] = first pair of tile k.
-__global__ void k_tile_offsets(const uint32_t* __restrict__ tile, uint32_t npairs, uint32_t ntiles,
-                               uint32_t* __restrict__ off) {
-    const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e > npairs) return;
-    const uint32_t k = e < npairs ? tile[e] : ntiles;
-    const uint32_t kp = e > 0 ? tile[e - 1] : 0u;
-    const uint32_t from = e > 0 ? kp + 1u : 0u;
-    for (uint32_t t = from; t <= k && t <= ntiles; ++t) off[t] = e;  // tiles kp+1 .. k start here
-}
-
-// Block ORs for the cumulative rows: bitmap b (< k*stride) is OR'ed into
-// row b / stride (one warp per bitmap; fills of more than 32 groups are
-// written by the whole warp).
-__global__ void k_cum_blocks(const uint32_t* __restrict__ words, const BitmapMeta* __restrict__ bm,
-                             uint32_t nb, uint32_t stride, uint32_t gx, uint32_t* __restrict__ rows) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (b >= nb) return;
-    const BitmapMeta m = bm[b];
-    const uint32_t* w = words + m.wstart;
-    uint32_t* row = rows + (size_t)(b / stride) * gx;
-    uint32_t carry = 0;
-    for (uint32_t base = 0; base < m.n; base += 32) {
-        const uint32_t i = base + lane;
-        const bool in = i < m.n;
-        const uint32_t wd = in ? __ldg(w + i) : 0u;
-        const uint32_t c = in ? wgroups(wd) : 0u;
-        uint32_t x = c;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) { uint32_t t = __shfl_up_sync(0xffffffffu, x, d); if (lane >= (uint32_t)d) x += t; }
-        const uint32_t p = carry + x - c;
-        if (in && wd <= ALLONES && wd != 0u) atomicOr(row + p, wd);
-        else if (in && wd >= HEADER1 && c <= 32u) for (uint32_t g = 0; g < c; ++g) row[p + g] = ALLONES;
-        uint32_t f = __ballot_sync(0xffffffffu, in && wd >= HEADER1 && c > 32u);
-        while (f) {
-            const uint32_t src = __ffs(f) - 1u;
-            f &= f - 1u;
-            const uint32_t fp = __shfl_sync(0xffffffffu, p, src), fc = __shfl_sync(0xffffffffu, c, src);
-            for (uint32_t g = lane; g < fc; g += 32u) row[fp + g] = ALLONES;
-        }
-        carry += __shfl_sync(0xffffffffu, x, 31);
-    }
+    if (!last_chunk) return;
+    // boundaries at or past the end of the words, and the active bits, which
+    // form the group after the whole words
+    for (uint32_t t = (carry + RT - 1u) / RT + lane; t <= A.ntiles; t += 32u) { tix[2 * t] = m.n; tix[2 * t + 1] = carry; }
     if (lane == 0 && m.anb > 0) {
         const uint32_t pat = (m.aval & ((1u << m.anb) - 1u)) << (31u - m.anb);
-        if (pat) atomicOr(row + m.groups, pat);
+        if (pat) {
+            atomicOr(tcol + (size_t)(carry / RT) * A.tw, tbit);
+            if (row) atomicOr(row + carry, pat);
+        }
     }
+}
+
+// Per tile the ascending list of the bitmaps holding a 1 bit in it: the set
+// bits of the touch matrix in order, one pass with a decoupled look-back for
+// the offsets (off[k] = the first entry of tile k, off[ntiles] = their number).
+constexpr uint32_t LWPT = 4;                        // matrix words per thread
+constexpr uint32_t LTILE = ITHREADS * LWPT;
+__global__ void __launch_bounds__(ITHREADS)
+k_tile_lists(const uint32_t* __restrict__ touch, uint32_t tw, uint32_t ntiles, uint32_t* __restrict__ off,
+             uint32_t* __restrict__ list, DevMeta* status, TileRec* recs, LaunchSync* sync, uint32_t nparts) {
+    __shared__ uint64_t sh[ITHREADS / 32 + 1];
+    __shared__ uint32_t hdr[2];
+    __shared__ uint64_t part_pre;
+    if (threadIdx.x == 0) { hdr[0] = claim_tile(sync); hdr[1] = ld_cg(&sync->epoch); }
+    __syncthreads();
+    const uint32_t t = hdr[0], epoch = hdr[1];
+    const uint32_t nw = ntiles * tw;
+    const uint32_t f0 = t * LTILE + threadIdx.x * LWPT;
+    uint32_t v[LWPT];
+    uint32_t cnt = 0;
+#pragma unroll
+    for (uint32_t j = 0; j < LWPT; ++j) {
+        v[j] = f0 + j < nw ? __ldg(touch + f0 + j) : 0u;
+        cnt += __popc(v[j]);
+    }
+    uint64_t total;
+    const uint64_t ex = block_exscan64(cnt, sh, total);
+    if (threadIdx.x < 32) {
+        uint64_t prefix; uint32_t pa, pb;
+        const bool ok = lookback64(recs, t, epoch, total, 0, 0, prefix, pa, pb);
+        if (threadIdx.x == 0) {
+            if (!ok) atomicExch(&status->status, DEV_ERR_TIMEOUT);
+            part_pre = prefix;
+            if (t == nparts - 1) off[ntiles] = (uint32_t)(prefix + total);
+        }
+    }
+    __syncthreads();
+    uint32_t o = (uint32_t)(part_pre + ex);
+#pragma unroll
+    for (uint32_t j = 0; j < LWPT; ++j) {
+        const uint32_t f = f0 + j;
+        if (f >= nw) break;
+        const uint32_t k = f / tw, wi = f - k * tw;
+        if (wi == 0u) off[k] = o;
+        for (uint32_t x = v[j]; x; x &= x - 1u) list[o++] = wi * 32u + (__ffs(x) - 1u);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) finish_tile(sync, nparts);
 }
 
 // Prefix OR down the rows: row k |= row k-1 for k = 1..nrows-1 (a thread per
