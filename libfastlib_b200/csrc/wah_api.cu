@@ -78,6 +78,15 @@ void* wg_alloc(wahgpu_ctx* ctx, size_t bytes) {
     ctx->bytes_allocated += c;
     return p;
 }
+// A cached block of the pool, or null: for buffers that a call can do without.
+static void* wg_alloc_cached(wahgpu_ctx* ctx, size_t bytes) {
+    std::lock_guard<std::mutex> g(ctx->mu);
+    auto it = ctx->pool.find(size_class(bytes));
+    if (it == ctx->pool.end() || it->second.empty()) return nullptr;
+    void* p = it->second.back();
+    it->second.pop_back();
+    return p;
+}
 void wg_free(wahgpu_ctx* ctx, void* p) {
     if (!p) return;
     std::lock_guard<std::mutex> g(ctx->mu);
@@ -274,6 +283,7 @@ static int bv_reserve(wahgpu_bv* b, uint64_t cap) {
     if (!b->words || !b->bpos) return wg_fail(ctx, WAHGPU_ENOMEM, "device allocation of %llu words failed", (unsigned long long)cap);
     b->cap = (uint32_t)cap;
     b->gt_valid = false;
+    b->rows_valid = false;
     return WAHGPU_OK;
 }
 
@@ -407,6 +417,7 @@ extern "C" int wahgpu_bv_free(wahgpu_bv* b) {
     wg_free(ctx, b->bpos);
     wg_free(ctx, b->meta);
     wg_free(ctx, b->gt);
+    wg_free(ctx, b->rows);
     delete b;
     return WAHGPU_OK;
 }
@@ -532,6 +543,8 @@ int wg_launch_merge(wahgpu_ctx* ctx, int op, bool fsm, bool unary, bool flip,
     CUDA_TRY(ctx, cudaGetLastError());
     res->h_valid = false;
     res->gt_valid = false;
+    res->rows_valid = false;
+    res->used = false;
     res->compressed_form = true;
     return WAHGPU_OK;
 }
@@ -605,72 +618,104 @@ int wg_launch_dense(wahgpu_ctx* ctx, int op, wahgpu_bv* x, wahgpu_bv* y, uint32_
     CUDA_TRY(ctx, cudaGetLastError());
     res->h_valid = false;
     res->gt_valid = false;
+    res->rows_valid = false;
+    res->used = false;
     res->compressed_form = true;
     return WAHGPU_OK;
 }
 
-// Two-pass group-space engine (wah_gop.cuh): expand + operate into dense
-// result patterns with per-tile head counts, then pack the words.
-int wg_launch_gop(wahgpu_ctx* ctx, int op, wahgpu_bv* x, wahgpu_bv* y, uint32_t groups,
-                  uint32_t anb, uint32_t aval, wahgpu_bv* res) {
-    int rc = bv_reserve(res, (uint64_t)x->h.n + y->h.n);
-    if (rc) return rc;
-    // the staging copies 16-byte chunks of the operands' word arrays (pool
-    // blocks, 256-byte aligned)
-    if ((reinterpret_cast<uintptr_t>(x->words) | reinterpret_cast<uintptr_t>(y->words)) & 15u)
-        return wg_fail(ctx, WAHGPU_EINVAL, "operand word arrays must be 16-byte aligned");
-    rc = wg_gtile(x);
-    if (rc) return rc;
-    rc = wg_gtile(y);
-    if (rc) return rc;
-    const uint32_t ntiles = (groups + GT - 1) / GT;
-    uint32_t* R = static_cast<uint32_t*>(wg_alloc(ctx, (size_t)ntiles * GT * 4));
-    const uint32_t nseg = (ntiles + GSEG - 1) / GSEG;
-    uint4* tiles = static_cast<uint4*>(wg_alloc(ctx, ((size_t)ntiles + nseg) * 16));
-    uint32_t* hmask = static_cast<uint32_t*>(wg_alloc(ctx, (size_t)ntiles * 32 * 4));
-    if (!R || !tiles || !hmask) {
-        wg_free(ctx, R); wg_free(ctx, tiles); wg_free(ctx, hmask);
-        return wg_fail(ctx, WAHGPU_ENOMEM, "allocation of %u tiles of result patterns failed", ntiles);
+// Room for the row index of b over `groups` groups.
+static bool rows_reserve(wahgpu_bv* b, uint32_t groups, void* (*alloc)(wahgpu_ctx*, size_t)) {
+    wahgpu_ctx* ctx = b->ctx;
+    const uint32_t need = (uint32_t)(((uint64_t)groups + PT - 1) / PT) * TROWS;
+    if (b->rows && b->rows_cap >= need) return true;
+    wg_free(ctx, b->rows);
+    b->rows_valid = false;
+    b->rows_cap = 0;
+    b->rows = static_cast<uint2*>(alloc(ctx, (size_t)need * sizeof(uint2)));
+    if (!b->rows) return false;
+    b->rows_cap = need;
+    return true;
+}
+// Row index of b (host metadata must be valid); built once.
+static int wg_rows(wahgpu_bv* b) {
+    if (b->rows_valid) return WAHGPU_OK;
+    wahgpu_ctx* ctx = b->ctx;
+    if (!rows_reserve(b, b->h.groups, wg_alloc)) return wg_fail(ctx, WAHGPU_ENOMEM, "allocation failed");
+    const uint32_t ntiles = (b->h.groups + PT - 1) / PT;
+    k_rows<<<(ntiles + GW - 1) / GW, GCTA, 0, ctx->stream>>>(b->words, b->bpos, b->h.n, b->h.groups, ntiles, b->rows);
+    ctx->launches++;
+    CUDA_TRY(ctx, cudaGetLastError());
+    b->rows_valid = true;
+    return WAHGPU_OK;
+}
+
+template <int OP, int KIND>
+static void launch_gop_op(const wahgpu_ctx* ctx, uint32_t ntiles, cudaStream_t s, const GopArgs& a) {
+    static PerDeviceSetup setup;
+    const size_t sm = GW * sizeof(GopWarp<(KIND >= GK_COPY)>);
+    const uint32_t per_sm = (uint32_t)wg_kernel_setup(setup, ctx->device, k_gop<OP, KIND>, GCTA, sm);
+    const uint32_t grid = std::min<uint32_t>((ntiles + GW - 1) / GW, per_sm * (uint32_t)ctx->sm_count);
+    wg_launch_pdl(k_gop<OP, KIND>, grid, GCTA, sm, s, a);
+}
+template <int KIND>
+static void launch_gop_kind(const wahgpu_ctx* ctx, int op, uint32_t ntiles, cudaStream_t s, const GopArgs& a) {
+    switch (op) {
+    case OP_AND: launch_gop_op<OP_AND, KIND>(ctx, ntiles, s, a); break;
+    case OP_OR: launch_gop_op<OP_OR, KIND>(ctx, ntiles, s, a); break;
+    case OP_XOR: launch_gop_op<OP_XOR, KIND>(ctx, ntiles, s, a); break;
+    default: launch_gop_op<OP_MINUS, KIND>(ctx, ntiles, s, a); break;
     }
+}
+
+// Two-pass group-space engine (wah_gop.cuh): the result patterns per group
+// with head masks and per-CTA totals, then the words.  kind: GopKind; y is
+// null for the copies.
+int wg_launch_gop(wahgpu_ctx* ctx, int kind, int op, wahgpu_bv* x, wahgpu_bv* y, uint32_t groups,
+                  uint32_t anb, uint32_t aval, wahgpu_bv* res) {
+    // positions are taken from the words: none that the upload scan refused
+    if (x->h.status || (y && y->h.status)) return wg_fail(ctx, WAHGPU_EFORMAT, "an operand's words are malformed");
+    int rc = bv_reserve(res, (uint64_t)x->h.n + (y ? y->h.n : 0));
+    if (!rc) rc = wg_rows(x);
+    if (!rc && y) rc = wg_rows(y);
+    if (rc) return rc;
+    const uint32_t ntiles = (uint32_t)(((uint64_t)groups + PT - 1) / PT);
+    // the result keeps its head masks as its row index where a block for it
+    // is at hand; else they are part of the scratch
+    const bool keep = rows_reserve(res, groups, wg_alloc_cached);
+    const size_t rb = (size_t)ntiles * PT * 4, hb = (size_t)ntiles * TROWS * sizeof(uint2);
+    unsigned char* scr = static_cast<unsigned char*>(wg_alloc(ctx, rb + hb + (size_t)ntiles * 12));
+    if (!scr) return wg_fail(ctx, WAHGPU_ENOMEM, "allocation of %u tiles of result patterns failed", ntiles);
+    uint32_t* tot = reinterpret_cast<uint32_t*>(scr + rb + hb);
     GopArgs a;
-    a.xw = x->words; a.xgt = x->gt; a.nx = x->h.n;
-    a.yw = y->words; a.ygt = y->gt; a.ny = y->h.n;
+    a.xw = x->words; a.xr = x->rows; a.xbp = x->bpos; a.nx = x->h.n;
+    a.yw = y ? y->words : nullptr; a.yr = y ? y->rows : nullptr; a.ybp = y ? y->bpos : nullptr; a.ny = y ? y->h.n : 0;
     a.groups = groups; a.ntiles = ntiles;
-    a.R = R; a.tiles = tiles; a.segs = tiles + ntiles; a.hmask = hmask;
+    a.R = reinterpret_cast<uint32_t*>(scr); a.heads = tot; a.first = tot + ntiles; a.ones = tot + 2 * (size_t)ntiles;
     a.out = res->words; a.obp = res->bpos; a.meta = res->meta;
+    a.orow = keep ? res->rows : reinterpret_cast<uint2*>(scr + rb);
     a.aval = aval; a.anb = anb;
     cudaStream_t s = ctx->stream;
-    rc = WAHGPU_OK;
-    if (cudaMemsetAsync(res->meta, 0, sizeof(DevMeta), s) != cudaSuccess ||
-        cudaMemsetAsync(a.segs, 0, (size_t)nseg * 16, s) != cudaSuccess)
-        rc = wg_fail(ctx, WAHGPU_ECUDA, "memset failed");
-    if (!rc) {
-        const uint32_t grid = (ntiles + GWARPS - 1) / GWARPS;
-        const size_t sm_op = GWARPS * sizeof(GopWarp);
-        static PerDeviceSetup setup[4];
-        wg_kernel_setup(setup[0], ctx->device, k_gop<OP_AND>, GTHREADS, sm_op);
-        wg_kernel_setup(setup[1], ctx->device, k_gop<OP_OR>, GTHREADS, sm_op);
-        wg_kernel_setup(setup[2], ctx->device, k_gop<OP_XOR>, GTHREADS, sm_op);
-        wg_kernel_setup(setup[3], ctx->device, k_gop<OP_MINUS>, GTHREADS, sm_op);
-        switch (op) {
-        case OP_AND: k_gop<OP_AND><<<grid, GTHREADS, sm_op, s>>>(a); break;
-        case OP_OR: k_gop<OP_OR><<<grid, GTHREADS, sm_op, s>>>(a); break;
-        case OP_XOR: k_gop<OP_XOR><<<grid, GTHREADS, sm_op, s>>>(a); break;
-        default: k_gop<OP_MINUS><<<grid, GTHREADS, sm_op, s>>>(a); break;
-        }
-        k_gpack<<<grid, GTHREADS, 0, s>>>(a);
-        ctx->launches += 2;
-        const cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) rc = wg_fail(ctx, WAHGPU_ECUDA, "launch failed: %s", cudaGetErrorString(e));
-    }
-    // stream-ordered: the next user of these blocks on this context's
-    // stream runs after the launches above
-    wg_free(ctx, R);
-    wg_free(ctx, tiles);
-    wg_free(ctx, hmask);
-    if (rc) return rc;
+    if (kind == GK_CANON) launch_gop_kind<GK_CANON>(ctx, op, ntiles, s, a);
+    else if (kind == GK_FSM) launch_gop_kind<GK_FSM>(ctx, op, ntiles, s, a);
+    else if (kind == GK_COPY) launch_gop_op<OP_AND, GK_COPY>(ctx, ntiles, s, a);
+    else launch_gop_op<OP_AND, GK_FLIP>(ctx, ntiles, s, a);
+    static PerDeviceSetup setup;
+    const size_t sm = GW * sizeof(PackWarp);
+    const uint32_t per_sm = (uint32_t)wg_kernel_setup(setup, ctx->device, k_gpack, GCTA, sm);
+    const uint32_t grid = std::max<uint32_t>(std::min<uint32_t>((ntiles + GW - 1) / GW, per_sm * (uint32_t)ctx->sm_count),
+                                             (ntiles + GRANGE - 1) / GRANGE);
+    wg_launch_pdl(k_gpack, grid, GCTA, sm, s, a);
+    ctx->launches += 2;
+    const cudaError_t e = cudaGetLastError();
+    // stream-ordered: the next user of the block on this context's stream
+    // runs after the launches above
+    wg_free(ctx, scr);
+    if (e != cudaSuccess) return wg_fail(ctx, WAHGPU_ECUDA, "launch failed: %s", cudaGetErrorString(e));
     res->h_valid = false;
     res->gt_valid = false;
+    res->rows_valid = keep;
+    res->used = false;
     res->compressed_form = true;
     return WAHGPU_OK;
 }
@@ -699,7 +744,7 @@ int wg_launch_fuse(wahgpu_ctx* ctx, int op, wahgpu_bv* x, wahgpu_bv* y, uint32_t
                    uint32_t anb, uint32_t aval, wahgpu_bv* res) {
     int rc = bv_reserve(res, (uint64_t)x->h.n + y->h.n);
     if (rc) return rc;
-    if (!fuse_applies(x, y, res, groups)) return wg_launch_gop(ctx, op, x, y, groups, anb, aval, res);
+    if (!fuse_applies(x, y, res, groups)) return wg_launch_gop(ctx, GK_CANON, op, x, y, groups, anb, aval, res);
     rc = wg_gtile(x);
     if (rc) return rc;
     rc = wg_gtile(y);
@@ -729,6 +774,8 @@ int wg_launch_fuse(wahgpu_ctx* ctx, int op, wahgpu_bv* x, wahgpu_bv* y, uint32_t
     CUDA_TRY(ctx, cudaGetLastError());
     res->h_valid = false;
     res->gt_valid = false;
+    res->rows_valid = false;
+    res->used = false;
     res->compressed_form = true;
     return WAHGPU_OK;
 }
@@ -739,7 +786,7 @@ int wg_launch_gone(wahgpu_ctx* ctx, int op, wahgpu_bv* x, wahgpu_bv* y, uint32_t
                    uint32_t anb, uint32_t aval, wahgpu_bv* res) {
     int rc = bv_reserve(res, (uint64_t)x->h.n + y->h.n);
     if (rc) return rc;
-    if (groups == 0) return wg_launch_gop(ctx, op, x, y, groups, anb, aval, res);
+    if (groups == 0) return wg_launch_gop(ctx, GK_CANON, op, x, y, groups, anb, aval, res);
     rc = wg_gtile(x);
     if (rc) return rc;
     rc = wg_gtile(y);
@@ -784,8 +831,37 @@ int wg_launch_gone(wahgpu_ctx* ctx, int op, wahgpu_bv* x, wahgpu_bv* y, uint32_t
     CUDA_TRY(ctx, cudaGetLastError());
     res->h_valid = false;
     res->gt_valid = false;
+    res->rows_valid = false;
+    res->used = false;
     res->compressed_form = true;
     return WAHGPU_OK;
+}
+
+// Group space or word space for an operator on the reference's _c2 path, and
+// for copies and complements (y null): group space costs by the groups, the
+// merge by the words.  Lines through measured calls, in us with g and n in
+// millions (group space: 8.8 at g = 0.03, 43 at 8.7; merge: 17 at n = 0.007,
+// 24 at 0.15, 58 at 1.4).  The row index an operand lacks is charged to its
+// first use; an operand that comes back is taken to come again.  A merge tile
+// set on the context asks for the merge.
+static bool in_group_space(const wahgpu_ctx* ctx, wahgpu_bv* x, wahgpu_bv* y, uint32_t groups) {
+    if (ctx->merge_tile) return false;
+    const double g = groups * 1e-6, n = ((double)x->h.n + (y ? y->h.n : 0)) * 1e-6;
+    double in_groups = y ? 8.0 + 3.8 * g : 7.0 + 3.0 * g;
+    for (wahgpu_bv* b : {x, y}) {
+        if (!b) continue;
+        if (!b->rows_valid && !b->used) in_groups += 3.0 + 1.2 * g;
+        b->used = true;
+    }
+    return in_groups < (y ? 15.5 + 29.5 * n : 14.0 + 15.0 * n);
+}
+
+// x, or its complement, as compress() leaves it.
+static int launch_copy(wahgpu_ctx* ctx, bool flip, wahgpu_bv* x, uint32_t groups, uint32_t anb, uint32_t aval,
+                       wahgpu_bv* res) {
+    if (groups > 0 && x->h.n > 0 && in_group_space(ctx, x, nullptr, groups))
+        return wg_launch_gop(ctx, flip ? GK_FLIP : GK_COPY, 0, x, nullptr, groups, anb, aval, res);
+    return wg_launch_merge(ctx, 0, false, true, flip, x, nullptr, groups, anb, aval, res);
 }
 
 // A one-word device bitvector holding the collapsed form of an all-zero
@@ -823,8 +899,8 @@ static OperandMeta opmeta(const wahgpu_bv* b) {
 
 // Engine for a canonical-result operator (WAHGPU_TUNE_DENSE_ENGINE): 1 the
 // pipelined group-space kernel, 2 the word-space merge, 3 the two-pass
-// group-space kernels, 4 the single-pass group-space kernel; 0 (default)
-// the single-pass kernel.
+// group-space kernels (0, the default, too), 4 / 5 the single-pass
+// group-space kernels over CTA / warp tiles.
 static bool dense_in_word_space(const wahgpu_ctx* ctx, const wahgpu_bv*, const wahgpu_bv*, uint32_t) {
     return ctx->dense_engine == 2;
 }
@@ -972,7 +1048,8 @@ extern "C" int wahgpu_bv_binop_into(wahgpu_ctx* ctx, int op, int inplace, wahgpu
     if (mb.n != b->h.n) { rc = collapsed_copy(ctx, b, &tmpb); if (rc) { if (tmpa) wahgpu_bv_free(tmpa); return rc; } cb = tmpb; }
     switch (p.kind) {
     case PK_MERGE_FSM:
-        rc = wg_launch_merge(ctx, op, true, false, false, ca, cb, G, anb, aval, res);
+        if (in_group_space(ctx, ca, cb, G)) rc = wg_launch_gop(ctx, GK_FSM, op, ca, cb, G, anb, aval, res);
+        else rc = wg_launch_merge(ctx, op, true, false, false, ca, cb, G, anb, aval, res);
         break;
     case PK_MERGE_CANON:
         // canonical result: the group-space kernel, or the word-space merge
@@ -984,13 +1061,13 @@ extern "C" int wahgpu_bv_binop_into(wahgpu_ctx* ctx, int op, int inplace, wahgpu
         else if (dense_fused(ctx))
             rc = wg_launch_fuse(ctx, op, ca, cb, G, anb, aval, res);
         else if (dense_two_pass(ctx))
-            rc = wg_launch_gop(ctx, op, ca, cb, G, anb, aval, res);
+            rc = wg_launch_gop(ctx, GK_CANON, op, ca, cb, G, anb, aval, res);
         else
             rc = wg_launch_dense(ctx, op, ca, cb, G, anb, aval, res);
         break;
     case PK_COPY:
     case PK_COPY_FLIP:
-        rc = wg_launch_merge(ctx, 0, false, true, p.kind == PK_COPY_FLIP, p.src ? cb : ca, nullptr, G, anb, aval, res);
+        rc = launch_copy(ctx, p.kind == PK_COPY_FLIP, p.src ? cb : ca, G, anb, aval, res);
         break;
     default: {
         rc = bv_reserve(res, 1);
@@ -1005,6 +1082,8 @@ extern "C" int wahgpu_bv_binop_into(wahgpu_ctx* ctx, int op, int inplace, wahgpu
         if (e != cudaSuccess) { rc = wg_fail(ctx, WAHGPU_ECUDA, "launch failed: %s", cudaGetErrorString(e)); break; }
         res->h_valid = false;
         res->gt_valid = false;
+        res->rows_valid = false;
+        res->used = false;
         res->compressed_form = true;
     }
     }
@@ -1038,6 +1117,10 @@ static void bv_take(wahgpu_bv* b, wahgpu_bv* tmp) {
     std::swap(b->h_valid, tmp->h_valid);
     std::swap(b->gt, tmp->gt);
     std::swap(b->gt_valid, tmp->gt_valid);
+    std::swap(b->rows, tmp->rows);
+    std::swap(b->rows_cap, tmp->rows_cap);
+    std::swap(b->rows_valid, tmp->rows_valid);
+    std::swap(b->used, tmp->used);
     b->compressed_form = tmp->compressed_form;
 }
 
@@ -1052,7 +1135,7 @@ static int unary_op(wahgpu_bv* b, bool flip) {
         rc = bv_reserve(r, 1);
         if (!rc) rc = wg_scan_meta(r, 0, b->h.anb, aval);
     } else {
-        rc = wg_launch_merge(ctx, 0, false, true, flip, b, nullptr, b->h.groups, b->h.anb, aval, r);
+        rc = launch_copy(ctx, flip, b, b->h.groups, b->h.anb, aval, r);
     }
     if (rc) { wahgpu_bv_free(r); return rc; }
     cudaStreamSynchronize(ctx->stream);

@@ -50,6 +50,10 @@ struct wahgpu_bv {
     bool h_valid = false;
     uint32_t* gt = nullptr;     // group-tile index (k_gtile), built on first use
     bool gt_valid = false;
+    uint2* rows = nullptr;      // row index (k_rows), built on first use or with the result
+    uint32_t rows_cap = 0;      // rows it has room for
+    bool rows_valid = false;
+    bool used = false;          // has been an operand where group and word space compete
     bool compressed_form = false;  // words are as compress() leaves them
 };
 
@@ -70,6 +74,18 @@ int wg_kernel_setup(PerDeviceSetup& s, int device, Kernel k, int threads, size_t
     if (v < 1) v = 1;
     s.per_sm[d].store(v, std::memory_order_relaxed);
     return v;
+}
+// Launches a kernel that calls pdl_wait() before it touches memory so that
+// its CTAs may be set up while the kernel before it on the stream drains.
+template <class... Args, class... Params>
+void wg_launch_pdl(void (*k)(Params...), uint32_t grid, uint32_t threads, size_t smem, cudaStream_t s, const Args&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid); cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k, args...);
 }
 int wg_fail(wahgpu_ctx* ctx, int code, const char* fmt, ...);
 void* wg_alloc(wahgpu_ctx* ctx, size_t bytes);

@@ -166,6 +166,60 @@ WAH_HD bool seg_fill_flag(uint32_t step, bool started, uint32_t xw, uint32_t yw)
     }
 }
 
+// ---- the count-1 flag without the walk
+// A run of exactly one uniform group at position p, operand words x and y
+// covering it: is its word a count-1 fill?  The step in progress at p depends
+// on the whole walk, but at such a run nearly all of it is fixed: a word
+// starts at p (the result changes there); a word of the other operand that
+// started before p is a fill whose value passes the first operand through
+// (else the result would not change at p); and a fill of two or more groups
+// starting at p must stick out past the other word's end at p + 1 (else the
+// run would be longer), which ends any copy step.  That leaves:
+//   both start at p: a new step, select_step decides;
+//   only x starts at p: a literal is copied as a literal; a fill of >= 2
+//     groups starts a new step; a count-1 fill is copied verbatim when the
+//     copy step over y's fill is already in progress, else it starts it;
+//   only y starts at p: the same with the operands' roles, and the tie rule
+//     (ry >= rx) of two fills ending together.
+// Only the count-1 fills can need words further back (SF_WALK_*).
+// xb / yb: the word starts at p; xe / ye: it ends at p + 1.
+enum SingleFlag : uint32_t {
+    SF_NO = 0,
+    SF_YES = 1,
+    // & |: true unless the x word ending at p is a fill of the absorbing value
+    // that began before y's word and a literal of y lies between their starts
+    SF_WALK_AND_X = 2,
+    // & |: true when a y literal lies in x's fill before p
+    SF_WALK_AND_Y = 3,
+    // -: true unless x's word ending at p is a 0-fill counted over the start of y's word
+    SF_WALK_MINUS_X = 4,
+    // -: true unless y's word ending at p is a 1-fill counted over the start of x's word
+    SF_WALK_MINUS_Y = 5
+};
+WAH_HD uint32_t single_flag(int op, uint32_t x, uint32_t y, bool xb, bool yb, bool xe, bool ye) {
+    const bool xf = is_fill(x), yf = is_fill(y);
+    const bool x1 = xf && wgroups(x) == 1u, y1 = yf && wgroups(y) == 1u;
+    if (xb && yb) {
+        const uint32_t s = select_step(op, x, wgroups(x), y, wgroups(y));
+        return s == S_CNT_X || s == S_CNT_Y ? SF_YES : SF_NO;
+    }
+    if (op == OP_XOR) return (xb ? x1 : y1) ? SF_YES : SF_NO;
+    if (xb) {
+        if (!xf) return SF_NO;
+        if (op == OP_MINUS) return x1 ? SF_WALK_MINUS_X : (fill_bit(x) == 0u ? SF_YES : SF_NO);
+        return x1 ? SF_WALK_AND_X : SF_YES;
+    }
+    if (!yf) return SF_NO;
+    if (op == OP_MINUS) {
+        if (!y1) return fill_bit(y) ? SF_YES : SF_NO;
+        return xe && fill_bit(y) ? SF_YES : SF_WALK_MINUS_Y;
+    }
+    const bool y0 = fill_bit(y) == (op == OP_AND ? 0u : 1u);  // y's fill absorbs x
+    if (y0) return SF_YES;
+    if (!y1) return SF_NO;
+    return xe ? SF_WALK_AND_Y : SF_YES;
+}
+
 // The word that represents a maximal run of class c with length len groups
 // starting at a segment whose literal value is v and count-1 flag is fflag.
 WAH_HD uint32_t run_word(uint32_t c, uint32_t len, uint32_t v, bool fflag) {

@@ -224,6 +224,13 @@ __device__ __forceinline__ bool lookback64(TileRec* recs, uint32_t t, uint32_t e
     return ok;
 }
 
+// Programmatic dependent launch: the kernel before this one on the stream is
+// done and its writes are visible (at once when the launch did not ask for
+// the overlap); and the kernel after this one may be scheduled as soon as
+// every CTA has got here.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- mbarriers and bulk copies (sm_90+ PTX), shared memory addressed by
 // its 32-bit shared-window offset
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {

@@ -1,86 +1,76 @@
-// Two-pass group-space engine for the operators whose result compress()
-// leaves canonical (the reference's _d2 / _d1 / _c1 / _c0 paths and the
-// all-literal loops, src/bitvector.cpp:2545-2830, 2981-3278, 3354-3619,
-// 3748-4079): after compress() the result words depend only on the result
-// bits, one word per maximal run of equal all-0 / all-1 groups (a fill when
-// the run holds two or more groups) and one literal per mixed group.
+// Two-pass group-space engine: operators, copies and complements over 31-bit
+// groups, whatever the operands' words look like, with the exact words the
+// reference holds after compress().
 //
-// Two launches, no look-back and no cross-CTA waits:
-//  * k_gop<OP>: one warp per tile of GT = 512 groups (the stride of the
-//    operands' group-tile index, which gives each tile's word range).  Both
-//    operands' words over the tile are staged in shared memory at once with
-//    cp.async and expanded to one 31-bit pattern per group (a word-start
-//    marker per word and a warp max-scan find the word of every group, so a
-//    fill costs one marker whatever its length; an operand with one word per
-//    group is read directly); the result patterns R = a OP b are stored
-//    densely (4 bytes per group) and the tile's run heads (a mixed group, or
-//    a class change) are counted, with the first head's position and the
-//    popcount.  Warps never wait for one another.
-//    Each tile's totals are also added into its segment of GSEG tiles.
-//  * k_gpack: one warp per tile with heads re-reads R, ranks the heads and
-//    writes the words in order: a mixed head's literal, or the run word
+// Canonical results (the reference's _d2 / _d1 / _c1 / _c0 paths and the
+// all-literal loops, src/bitvector.cpp:2545-2830, 2981-3278, 3354-3619,
+// 3748-4079): one word per maximal run of equal all-0 / all-1 groups (a fill
+// when the run holds two or more groups) and one literal per mixed group.
+// The _c2 walks (src/bitvector.cpp:2419-3745) differ from that only in runs
+// of one group, which may be count-1 fills; single_flag (wah_core.cuh) tells
+// those from the words meeting there, and copies keep the operand's.
+//
+// Every operand has a row index: for each 32 groups a mask of the groups
+// where a word starts and the word covering the group before them, so the
+// word of group 32 k + l is base + popc(mask & bits 0..l): no decode, no scan.
+// It is built once per bitvector (k_rows) and comes with every result of
+// this engine, whose head masks it is.
+//
+// Two launches, no look-back and no waits between CTAs, a warp per tile of
+// PT = 512 groups, every CTA a contiguous range of tiles:
+//  * k_gop: lane l of row r owns group 32 r + l.  The tile's words of both
+//    operands arrive in shared memory by bulk copies, issued one tile ahead
+//    (two buffers per warp, an mbarrier each); R = a OP b is stored densely,
+//    and a row's run heads come from two ballots (groups all 0, groups all 1)
+//    and a shift.  Per tile: heads, first head, 1 bits.
+//  * k_gpack: a tile's R arrives the same way; each head's lane writes its
+//    word at the number of heads before it: the literal, or the run word
 //    whose length reaches the next head.
-// Lanes own groups in NCH = 4 chunks of four consecutive groups (group
-// 128*j + 4*lane + e of the tile), so every global access of R is a
-// coalesced 16-byte vector and the chunk-major order is the group order.
+// Bound by instruction issue (the integer pipe first) and the few warps that
+// two buffers per warp leave room for.  At 2^28 bits, both operands of d =
+// 0.1 / 0.5: 39 / 44 us a call against 79 / 65 for the form before it (a
+// word-start marker per word and warp max-scans over 128 groups, operands
+// staged without prefetch, four neighbouring groups per lane; ~2370 + 1060
+// instructions per tile against 715 + 720); both of d = 0.01 through the _c2
+// path: 43 us against 58 for the word-space merge.  Tiles of 256 groups
+// double the resident warps and are slower (46 / 50 us: the per-tile work);
+// launching each kernel while the one before it drains saves 3 us a call.
 #ifndef WAH_GOP_CUH
 #define WAH_GOP_CUH
+#include <type_traits>
 #include "wah_dense.cuh"
 
 namespace wah {
 
-constexpr int GT = DT;                    // groups per tile: one warp's tile (the group-tile index stride)
-constexpr int GWARPS = 4;                 // warps (tiles) per CTA
+constexpr int GT = DT;                    // groups per tile of the single-pass warp-tile engine (wah_gone.cuh)
+constexpr int PT = 512;                   // groups per tile of this engine, a warp's
+constexpr int TROWS = PT / 32;            // rows of 32 groups per tile
+constexpr int GW = 8;                     // warps per CTA of this engine
+constexpr int GBUF = PT + 8;              // staged words of a tile: its own, the ones either side, 16-byte ends
+constexpr int GCTA = GW * 32;
+constexpr uint32_t GNONE = 0xFFFFFFFFu;   // no head
+// the single-pass warp-tile engine's shape (wah_gone.cuh)
+constexpr int GWARPS = 4;
 constexpr int GTHREADS = GWARPS * 32;
-constexpr int NCH = GT / 128;             // chunks of 128 groups (4 per lane) per tile
-constexpr int GWPL = (GT + 4 + 31) / 32;  // staged words per lane
-constexpr uint32_t GNONE = 0xFFFFFFFFu;   // no head in the tile
-constexpr uint32_t GSEG = 256;            // tiles per segment of the two-level prefix
-// staging holds a tile's <= GT words plus up to 3 before them and the
-// rest of the last 16-byte chunk
-static_assert(GT == NCH * 128 && NCH <= 8 && GWPL * 32 >= GT + 4 && (GWPL * 32 * 4) % 16 == 0, "tile shape");
+constexpr int NCH = GT / 128;
+static_assert(TROWS == 16, "a half warp holds a tile's rows");
+
+enum GopKind : int {
+    GK_CANON = 0,  // x OP y, canonical words
+    GK_FSM = 1,    // x OP y, the words of the reference's _c2 walk
+    GK_COPY = 2,   // x, as compress() leaves it
+    GK_FLIP = 3    // x complemented
+};
 
 struct GopArgs {
-    const uint32_t* xw; const uint32_t* xgt; uint32_t nx;
-    const uint32_t* yw; const uint32_t* ygt; uint32_t ny;
+    const uint32_t* xw; const uint2* xr; const uint32_t* xbp; uint32_t nx;  // words, row index, block positions, words
+    const uint32_t* yw; const uint2* yr; const uint32_t* ybp; uint32_t ny;
     uint32_t groups, ntiles;
-    uint32_t* R;          // ntiles * GT result patterns
-    uint4* tiles;         // per tile: {heads, first head (GNONE: none), popcount, -}
-    uint4* segs;          // per GSEG tiles (zeroed before k_gop): {heads, GNONE - first head (0: none), popcount, -}
-    uint32_t* hmask;      // per tile and lane: the lane's run heads (bit 4 j + e: group 128 j + 4 lane + e)
-    uint32_t* out; uint32_t* obp; DevMeta* meta;
+    uint32_t* R;          // ntiles * PT result patterns; bit 31: as a run of one group it is a count-1 fill
+    uint32_t* heads; uint32_t* first; uint32_t* ones;  // per tile: heads, first head (GNONE: none), 1 bits
+    uint32_t* out; uint32_t* obp; uint2* orow; DevMeta* meta;
     uint32_t aval, anb;
 };
-
-// per warp: both operands' words over its tile and the word-start markers
-struct GopWarp {
-    uint32_t ws[2][GWPL * 32];
-    uint16_t mk[GT];
-};
-
-__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(smem_u32(smem)), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_u32(smem)), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
-
-// Stages words [wi0, wi0 + nw) of an n-word array w (16-byte aligned) into
-// ws with both sides indexed from the 16-byte boundary a0 = wi0 & ~3:
-// ws[i] = w[a0 + i], so word wi0 + k lands at ws[k + (wi0 & 3)].  Whole
-// 16-byte chunks inside the array go as 16-byte copies (shared and global
-// addresses both 16-byte aligned: ws is, and a0 is a multiple of 4 words),
-// the at most 3 words of a chunk cut by the array's end as 4-byte ones.
-__device__ __forceinline__ void gop_stage(uint32_t* ws, const uint32_t* __restrict__ w, uint32_t wi0, uint32_t nw,
-                                          uint32_t n) {
-    const uint32_t lane = threadIdx.x & 31u;
-    if (nw == 0) return;
-    const uint32_t a0 = wi0 & ~3u, end = wi0 + nw;
-    const uint32_t nfull = min((end - a0 + 3u) / 4u, (n - a0) / 4u);
-    for (uint32_t c = lane; c < nfull; c += 32) cp_async16(ws + 4u * c, w + a0 + 4u * c);
-    for (uint32_t i = a0 + 4u * nfull + lane; i < end; i += 32) cp_async4(ws + (i - a0), w + i);
-}
 
 // Word range of one operand over the tile [g0, g1): words [wi0, wend), the
 // first starting at group s0.  gt: the operand's group-tile index (entry
@@ -99,319 +89,533 @@ __device__ __forceinline__ bool gop_range(const uint32_t* __restrict__ gt, uint3
     return ok;
 }
 
-// Places one operand's staged words: marks, at the first group of the tile
-// each word covers, the word's index + 1.  mk must be zero.  The words are
-// taken 32 at a time, one per lane; a row of literals needs no scan.
-__device__ __forceinline__ void gop_mark(const uint32_t* ws, uint16_t* mk, uint32_t nw, uint32_t s0, uint32_t g0,
-                                         uint32_t g1) {
+// The word covering group g < groups and its first group (whole warp): a
+// 32-way search of the block positions (bp[0] = 0, ascending), then a scan of
+// the block's words.
+__device__ __forceinline__ void word_of_group(const uint32_t* __restrict__ w, const uint32_t* __restrict__ bp, uint32_t n,
+                                              uint32_t g, uint32_t& wi, uint32_t& start) {
     const uint32_t lane = threadIdx.x & 31u;
-    uint32_t carry = s0;  // first group of the row's first word
-    for (uint32_t base = 0; base < nw; base += 32) {
-        const uint32_t k = base + lane;
-        const bool in = k < nw;
-        const uint32_t wd = in ? ws[k] : 0u;
-        uint32_t p, c = 1;
-        if (__ballot_sync(0xffffffffu, in && is_fill(wd)) == 0u) {
-            p = carry + lane;
-            carry += min(32u, nw - base);
-        } else {
-            c = in ? wgroups(wd) : 0u;
+    uint32_t lo = 0, hi = (n + 31u) / 32u;  // bp[lo] <= g < bp[hi]
+    while (hi - lo > 1u) {
+        const uint32_t step = (hi - lo + 31u) / 32u, m = lo + lane * step;
+        const uint32_t k = __popc(__ballot_sync(0xffffffffu, m < hi && __ldg(bp + m) <= g));  // >= 1: lane 0
+        lo += (k - 1u) * step;
+        hi = min(hi, lo + step);
+    }
+    const uint32_t i = 32u * lo + lane;
+    const uint32_t c = i < n ? wgroups(__ldg(w + i)) : 0u;
+    uint32_t x = c;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t u = __shfl_up_sync(0xffffffffu, x, d);
+        if (lane >= (uint32_t)d) x += u;
+    }
+    const uint32_t p = __ldg(bp + lo) + x - c;  // first group of the lane's word
+    const uint32_t in = __popc(__ballot_sync(0xffffffffu, i < n && p <= g));  // >= 1: lane 0
+    wi = 32u * lo + in - 1u;
+    start = __shfl_sync(0xffffffffu, p, in - 1u);
+}
+
+// The row index of a bitvector (ntiles * TROWS rows; rows past the last
+// group hold no start and the last word): a warp per tile finds the tile's
+// first word, takes its words 32 at a time, flags the group each one starts
+// at in shared memory (positions by a warp scan where a row holds a fill)
+// and ballots the flags.  Bound by latency (the search's round trips); a
+// launch of its own for the search (a binary search per thread) took 13 us
+// at 2^28 bits beside 10 us for the rows.
+__global__ void __launch_bounds__(GCTA) k_rows(const uint32_t* __restrict__ w, const uint32_t* __restrict__ bp,
+                                               uint32_t n, uint32_t groups, uint32_t ntiles, uint2* __restrict__ rows) {
+    __shared__ __align__(16) uint8_t mk_[GW][PT];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t t = blockIdx.x * GW + warp;
+    if (t >= ntiles) return;
+    uint8_t* mk = mk_[warp];
+    const uint32_t g0 = t * (uint32_t)PT, g1 = min(g0 + (uint32_t)PT, groups);
+    uint32_t wi0, s0;
+    word_of_group(w, bp, n, g0, wi0, s0);
+    reinterpret_cast<uint4*>(mk)[lane] = make_uint4(0u, 0u, 0u, 0u);
+    __syncwarp();
+    uint32_t carry = s0;  // first group of the next word
+    for (uint32_t base0 = wi0; base0 < n && carry < g1; base0 += 128) {
+        uint32_t v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint32_t k = base0 + 32u * j + lane;
+            v[j] = k < n ? __ldg(w + k) : 0u;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint32_t base = base0 + 32u * j;
+            if (base >= n || carry >= g1) break;
+            const bool in = base + lane < n;
+            uint32_t p;
+            if (__ballot_sync(0xffffffffu, in && is_fill(v[j])) == 0u) {
+                p = carry + lane;
+                carry += min(32u, n - base);
+            } else {
+                const uint32_t c = in ? wgroups(v[j]) : 0u;
+                uint32_t x = c;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const uint32_t u = __shfl_up_sync(0xffffffffu, x, d);
+                    if (lane >= (uint32_t)d) x += u;
+                }
+                p = carry + x - c;
+                carry += __shfl_sync(0xffffffffu, x, 31);
+            }
+            if (in && p >= g0 && p < g1) mk[p - g0] = 1u;
+        }
+    }
+    __syncwarp();
+    uint32_t m = 0;
+#pragma unroll
+    for (int r = 0; r < TROWS; ++r) {
+        const uint32_t b = __ballot_sync(0xffffffffu, mk[32 * r + lane] != 0u);
+        if (lane == (uint32_t)r) m = b;
+    }
+    // words before each row: those before the tile, then the rows' starts
+    uint32_t x = __popc(m);
+#pragma unroll
+    for (int d = 1; d < TROWS; d <<= 1) {
+        const uint32_t u = __shfl_up_sync(0xffffffffu, x, d);
+        if (lane >= (uint32_t)d) x += u;
+    }
+    const uint32_t w0 = s0 == g0 ? wi0 : wi0 + 1u;  // the first word starting in the tile
+    if (lane < (uint32_t)TROWS) rows[(size_t)t * TROWS + lane] = make_uint2(m, w0 + x - __popc(m) - 1u);
+}
+
+// ---- words further back, for the count-1 flags that need them (whole warp,
+// uniform arguments).  Rare: only one-group runs over count-1 fill words.
+// First group of word j.
+__device__ __forceinline__ uint32_t word_start(const uint32_t* __restrict__ w, const uint32_t* __restrict__ bp, uint32_t j) {
+    const uint32_t lane = threadIdx.x & 31u, k = j >> 5;
+    const uint32_t c = lane < (j & 31u) ? wgroups(__ldg(w + 32u * k + lane)) : 0u;
+    return __ldg(bp + k) + __reduce_add_sync(0xffffffffu, c);
+}
+// Is one of the words before word j that start at or after group a a literal?
+__device__ __forceinline__ bool literal_since(const uint32_t* __restrict__ w, const uint32_t* __restrict__ bp, uint32_t j,
+                                              uint32_t a) {
+    if (j == 0u) return false;
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t k = (j - 1u) >> 5;; --k) {
+        const uint32_t i = 32u * k + lane;
+        const uint32_t v = i < j ? __ldg(w + i) : HEADER0;
+        const uint32_t lit = __ballot_sync(0xffffffffu, !is_fill(v));
+        if (lit) {  // the last one starts latest
+            const uint32_t top = 31u - __clz(lit);
+            return __ldg(bp + k) + __reduce_add_sync(0xffffffffu, lane < top ? wgroups(v) : 0u) >= a;
+        }
+        if (__ldg(bp + k) <= a) return false;
+    }
+}
+// "-": is the 0-fill word i of x, which began before group q where y's word j
+// starts and ends later, being counted (S_CNT_X) at q?  It is unless y's word
+// before j is a 1-fill begun before it and itself being counted there; two
+// neighbouring fills of one value take the question one word back in both.
+__device__ __forceinline__ bool minus_counted(const GopArgs& A, uint32_t i, uint32_t q, uint32_t j) {
+    uint32_t a = word_start(A.xw, A.xbp, i);
+    while (true) {
+        if (j == 0u) return true;
+        const uint32_t v = __ldg(A.yw + j - 1u);
+        if (!(is_fill(v) && fill_bit(v))) return true;
+        const uint32_t c = q - wgroups(v);
+        if (c >= a) return true;
+        if (i == 0u) return false;
+        const uint32_t u = __ldg(A.xw + i - 1u);
+        if (!is_fill(u) || fill_bit(u)) return false;
+        const uint32_t a2 = a - wgroups(u);
+        if (a2 >= c) return false;
+        --i; --j;
+        q = c; a = a2;
+    }
+}
+// The flag of the one-group run at p, words xi / yi covering it.
+template <int OP>
+__device__ __noinline__ bool walk_flag(const GopArgs& A, uint32_t code, uint32_t p, uint32_t xi, uint32_t yi) {
+    const uint32_t absorb = OP == OP_OR ? 1u : 0u;
+    if (code == SF_WALK_AND_Y) {
+        return literal_since(A.yw, A.ybp, yi, p + 1u - wgroups(__ldg(A.xw + xi)));  // x's fill ends at p + 1
+    } else if (code == SF_WALK_AND_X) {
+        if (xi == 0u) return true;
+        const uint32_t v = __ldg(A.xw + xi - 1u);
+        if (!is_fill(v) || fill_bit(v) != absorb) return true;
+        const uint32_t a = p - wgroups(v);
+        return !(a < word_start(A.yw, A.ybp, yi) && literal_since(A.yw, A.ybp, yi, a));
+    } else if (code == SF_WALK_MINUS_X) {
+        if (xi == 0u) return true;
+        const uint32_t v = __ldg(A.xw + xi - 1u);
+        if (!is_fill(v) || fill_bit(v)) return true;
+        const uint32_t q = word_start(A.yw, A.ybp, yi);
+        return !(p - wgroups(v) < q && minus_counted(A, xi - 1u, q, yi));
+    }
+    if (yi == 0u) return true;
+    const uint32_t v = __ldg(A.yw + yi - 1u);  // ends at p
+    if (!is_fill(v) || !fill_bit(v)) return true;
+    const uint32_t c = p - wgroups(v), a = word_start(A.xw, A.xbp, xi);
+    if (c >= a) return true;
+    if (xi == 0u) return false;
+    const uint32_t u = __ldg(A.xw + xi - 1u);
+    return is_fill(u) && !fill_bit(u) && a - wgroups(u) < c && minus_counted(A, xi - 1u, c, yi - 1u);
+}
+
+// Pattern of one group of word w in bits 0..30 (bit 31 is not part of it).
+__device__ __forceinline__ uint32_t gop_pattern(uint32_t w) {
+    return (int32_t)w < 0 ? (uint32_t)((int32_t)(w << 1) >> 31) : w;
+}
+// Result pattern of one group from its words (bit 31: a fill word of x, for
+// the kinds that keep count-1 fills).
+template <int OP, int KIND>
+__device__ __forceinline__ uint32_t gop_value(uint32_t x, uint32_t y) {
+    if (KIND == GK_COPY) return (gop_pattern(x) & ALLONES) | (x & HEADER0);
+    if (KIND == GK_FLIP) return (~gop_pattern(x) & ALLONES) | (x & HEADER0);
+    return op2<OP>(gop_pattern(x), gop_pattern(y)) & ALLONES;
+}
+
+__device__ __forceinline__ uint32_t lds32(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+    return v;
+}
+
+// Tiles of CTA `cta` of `n`: [lo, hi).
+__device__ __forceinline__ void gop_range_of(uint32_t ntiles, uint32_t cta, uint32_t n, uint32_t& lo, uint32_t& hi) {
+    const uint32_t q = (ntiles + n - 1u) / n;
+    lo = min(cta * q, ntiles);
+    hi = min(lo + q, ntiles);
+}
+
+template <bool UNARY>
+struct GopWarp {
+    uint32_t w[UNARY ? 1 : 2][2][GBUF];  // operand, buffer
+    uint2 row[2][32];                    // per buffer: lanes 0-15 x's rows, 16-31 y's: mask, shared address of the word before
+    uint2 hu[TROWS];                     // heads and uniform groups of each row
+    uint64_t bar[2];
+};
+
+template <int OP, int KIND>
+__global__ void __launch_bounds__(GCTA, 3) k_gop(const __grid_constant__ GopArgs A) {
+    constexpr bool UNARY = KIND >= GK_COPY;
+    extern __shared__ __align__(16) unsigned char gsm[];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    GopWarp<UNARY>& W = reinterpret_cast<GopWarp<UNARY>*>(gsm)[warp];
+    if (lane == 0) { mbar_init(&W.bar[0], 1); mbar_init(&W.bar[1], 1); mbar_init_fence(); }
+    uint32_t t, tend;
+    gop_range_of(A.ntiles, blockIdx.x, gridDim.x, t, tend);
+    t += warp;
+    __syncwarp();
+    pdl_wait();
+    pdl_launch();
+    if (blockIdx.x == 0 && threadIdx.x == 0) { A.meta->nfill = 0; A.meta->status = 0; }
+    if (t >= tend) return;
+    const uint32_t le = (2u << lane) - 1u;  // lanes up to this one (lane 31: all)
+    const uint32_t* __restrict__ xw = A.xw;
+    const uint32_t* __restrict__ yw = A.yw;
+
+    // rows of tile u, one per lane
+    auto load_rows = [&](uint32_t u) {
+        const uint2* p = lane < 16u || UNARY ? A.xr : A.yr;
+        return __ldg(p + (size_t)u * TROWS + (lane & 15u));
+    };
+    // issues the copies of a tile's words: from the one covering the group
+    // before it to the one after its last, 16-byte ends rounded outwards (the
+    // word arrays are pool blocks: aligned and padded to 256 bytes)
+    auto stage = [&](uint2 row, uint32_t b) {
+        const uint32_t half = lane & 16u, n = half ? A.ny : A.nx;
+        const uint32_t fst = __shfl_sync(0xffffffffu, row.y, half);
+        const uint32_t lst = __shfl_sync(0xffffffffu, row.y + __popc(row.x), half + TROWS - 1u);
+        const uint32_t lo = (fst == GNONE ? 0u : fst) & ~3u, hi = min(lst + 2u, n);
+        const uint32_t bytes = ((hi - lo + 3u) & ~3u) * 4u;
+        uint32_t* buf = W.w[UNARY ? 0 : half >> 4][b];
+        row.y = smem_u32(buf) + (row.y - lo) * 4u;
+        W.row[b][lane] = row;
+        __syncwarp();
+        const uint32_t both = bytes + (UNARY ? 0u : __shfl_xor_sync(0xffffffffu, bytes, 16));
+        if (lane == 0) mbar_arrive_tx(&W.bar[b], both);
+        __syncwarp();
+        if ((lane & 15u) == 0u && (lane == 0u || !UNARY)) bulk_g2s(buf, (half ? yw : xw) + lo, bytes, &W.bar[b]);
+    };
+
+    uint2 nrow = load_rows(t);
+    stage(nrow, 0);
+    if (t + GW < tend) nrow = load_rows(t + GW);
+    for (uint32_t k = 0; t < tend; t += GW, ++k) {
+        const uint32_t b = k & 1u;
+        if (t + GW < tend) {
+            stage(nrow, b ^ 1u);
+            if (t + 2 * GW < tend) nrow = load_rows(t + 2 * GW);
+        }
+        if (!__all_sync(0xffffffffu, mbar_wait(&W.bar[b], (k >> 1) & 1u))) {
+            // gave up: nothing of the tile is written; leave once the copies
+            // in flight are done or have been waited for as long again
+            if (lane == 0) atomicExch(&A.meta->status, DEV_ERR_TIMEOUT);
+            if (t + GW < tend) mbar_wait(&W.bar[b ^ 1u], ((k + 1u) >> 1) & 1u);
+            return;
+        }
+        const uint32_t g0 = t * (uint32_t)PT;
+        const uint32_t left = A.groups - g0;  // valid groups from g0 on
+        const uint4* rows = reinterpret_cast<const uint4*>(W.row[b]);
+        uint32_t* R = A.R + g0 + lane;
+        uint32_t ones = 0;
+        // bit 31: was the group before all 0 / all 1
+        uint32_t zp = 0, op = 0;
+        if (g0) {
+            const uint32_t pv = gop_value<OP, KIND>(lds32(W.row[b][0].y), UNARY ? 0u : lds32(W.row[b][16].y)) & ALLONES;
+            zp = pv == 0u ? 0x80000000u : 0u;
+            op = pv == ALLONES ? 0x80000000u : 0u;
+        }
+        // FULL: every group of the tile is valid
+        auto rows_of = [&](auto full_tile) {
+            constexpr bool FULL = decltype(full_tile)::value;
+#pragma unroll 2
+            for (int r0 = 0; r0 < TROWS; r0 += 4) {
+                uint32_t xv[4], yv[4];
+#pragma unroll
+                for (int j = 0; j < 4; j += 2) {
+                    const uint4 m = rows[(r0 + j) / 2];
+                    xv[j] = lds32(m.y + 4u * __popc(m.x & le));
+                    xv[j + 1] = lds32(m.w + 4u * __popc(m.z & le));
+                    if (!UNARY) {
+                        const uint4 q = rows[(TROWS + r0 + j) / 2];
+                        yv[j] = lds32(q.y + 4u * __popc(q.x & le));
+                        yv[j + 1] = lds32(q.w + 4u * __popc(q.z & le));
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const uint32_t r = r0 + j;
+                    uint32_t v = gop_value<OP, KIND>(xv[j], UNARY ? 0u : yv[j]);
+                    R[32u * r] = v;
+                    if (UNARY) v &= ALLONES;
+                    uint32_t vm = 0xFFFFFFFFu;
+                    if (!FULL) {
+                        const uint32_t c = left > 32u * r ? left - 32u * r : 0u;
+                        vm = c >= 32u ? 0xFFFFFFFFu : (1u << c) - 1u;
+                        if (!((vm >> lane) & 1u)) v = 0u;
+                    }
+                    const uint32_t z = __ballot_sync(0xffffffffu, v == 0u), o = __ballot_sync(0xffffffffu, v == ALLONES);
+                    // a head: mixed, or of another class than the group before
+                    const uint32_t h = ~((z & __funnelshift_l(zp, z, 1)) | (o & __funnelshift_l(op, o, 1))) & vm;
+                    zp = z;
+                    op = o;
+                    ones += __popc(v);
+                    if (lane == 0) W.hu[r] = make_uint2(h, z | o);
+                }
+            }
+        };
+        if (left >= (uint32_t)PT) rows_of(std::true_type());
+        else rows_of(std::false_type());
+        __syncwarp();
+        uint32_t H = 0, U = 0, heads = 0, first = GNONE;
+        if (lane < (uint32_t)TROWS) {
+            const uint2 hu = W.hu[lane];
+            H = hu.x; U = hu.y;
+            A.orow[(size_t)t * TROWS + lane] = hu;  // k_gpack puts the words before the row in U's place
+            heads = __popc(H);
+            if (H) first = g0 + 32u * lane + (__ffs(H) - 1u);
+        }
+        if (KIND == GK_FSM) {
+            // runs of one group: a uniform head followed by a head (or the end)
+            uint32_t nb = __shfl_down_sync(0xffffffffu, H, 1) & 1u;
+            if (left > (uint32_t)PT) {  // the head test of the group after the tile
+                const uint2* xr = A.xr + (size_t)(t + 1) * TROWS;
+                const uint2* yr = A.yr + (size_t)(t + 1) * TROWS;
+                const uint2 mx = __ldg(xr), my = __ldg(yr);
+                const uint32_t pv = gop_value<OP, KIND>(__ldg(xw + (mx.y + (mx.x & 1u))), __ldg(yw + (my.y + (my.x & 1u))));
+                if (lane == TROWS - 1u) nb = !((pv == 0u && zp >> 31) || (pv == ALLONES && op >> 31));
+            } else if (left == 32u * lane + 32u) {
+                nb = 1u;
+            }
+            uint32_t S = H >> 1 | nb << 31;
+            if (left > 32u * lane && left < 32u * lane + 32u) S |= 1u << (left - 32u * lane - 1u);
+            S &= H & U;
+            uint32_t todo = __ballot_sync(0xffffffffu, lane < (uint32_t)TROWS && S != 0u);
+            while (todo) {
+                const uint32_t r = __ffs(todo) - 1u;
+                todo &= todo - 1u;
+                const uint32_t s = __shfl_sync(0xffffffffu, S, r);
+                const uint2* xr = A.xr + (size_t)t * TROWS + r;
+                const uint2* yr = A.yr + (size_t)t * TROWS + r;
+                const uint2 mx = __ldg(xr), my = __ldg(yr);
+                const uint32_t p = g0 + 32u * r + lane;
+                const uint32_t xi = mx.y + __popc(mx.x & le), yi = my.y + __popc(my.x & le);
+                uint32_t code = SF_NO;
+                if ((s >> lane) & 1u) {
+                    // do the words end at p + 1 (the next row's first start, past a row's end)
+                    bool xe = true, ye = true;
+                    if (p + 1u < A.groups) {
+                        xe = lane < 31u ? (mx.x >> (lane + 1u)) & 1u : __ldg(&xr[1].x) & 1u;
+                        ye = lane < 31u ? (my.x >> (lane + 1u)) & 1u : __ldg(&yr[1].x) & 1u;
+                    }
+                    code = single_flag(OP, __ldg(xw + xi), __ldg(yw + yi), (mx.x >> lane) & 1u, (my.x >> lane) & 1u, xe, ye);
+                }
+                uint32_t walk = __ballot_sync(0xffffffffu, code > SF_YES);
+                while (walk) {
+                    const uint32_t l = __ffs(walk) - 1u;
+                    walk &= walk - 1u;
+                    const bool f = walk_flag<OP>(A, __shfl_sync(0xffffffffu, code, l), __shfl_sync(0xffffffffu, p, l),
+                                                 __shfl_sync(0xffffffffu, xi, l), __shfl_sync(0xffffffffu, yi, l));
+                    if (lane == l) code = f ? SF_YES : SF_NO;
+                }
+                if (code == SF_YES) R[32u * r] |= HEADER0;  // this lane's own store above
+            }
+        }
+        ones = __reduce_add_sync(0xffffffffu, ones);
+        heads = __reduce_add_sync(0xffffffffu, heads);
+        first = __reduce_min_sync(0xffffffffu, first);
+        if (lane == 0) { A.heads[t] = heads; A.first[t] = first; A.ones[t] = ones; }
+        __syncwarp();  // the buffer, the rows and the head masks are free again
+    }
+}
+
+// Position of the k-th set bit (from 0) of h.
+__device__ __forceinline__ uint32_t nth_bit(uint32_t h, uint32_t k) {
+    uint32_t pos = 0;
+#pragma unroll
+    for (int w = 16; w > 0; w >>= 1) {
+        const uint32_t c = __popc((h >> pos) & ((1u << w) - 1u));
+        if (k >= c) { k -= c; pos += w; }
+    }
+    return pos;
+}
+
+struct PackWarp {
+    uint32_t r[2][PT];  // result patterns
+    uint2 hu[2][TROWS];
+    uint4 row[TROWS];   // heads; index of the row's first head; groups from the row's end to the head after it; heads of runs
+    uint64_t bar[2];
+};
+constexpr uint32_t GRANGE = 1024;  // tiles of a CTA at most
+
+// The words of one tile per warp.  The last CTA writes the metadata.
+__global__ void __launch_bounds__(GCTA) k_gpack(const __grid_constant__ GopArgs A) {
+    extern __shared__ __align__(16) unsigned char gsm[];
+    __shared__ uint32_t sh[2][GW];
+    __shared__ uint32_t pre[GRANGE];  // heads before each tile of the range, from its start
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    PackWarp& W = reinterpret_cast<PackWarp*>(gsm)[warp];
+    uint32_t tb, tend;
+    gop_range_of(A.ntiles, blockIdx.x, gridDim.x, tb, tend);
+    if (lane == 0) { mbar_init(&W.bar[0], 1); mbar_init(&W.bar[1], 1); mbar_init_fence(); }
+    __syncwarp();
+    pdl_wait();
+    pdl_launch();
+    if (tb >= tend) return;
+    auto stage = [&](uint32_t u, uint32_t b) {
+        if (lane == 0) {
+            mbar_arrive_tx(&W.bar[b], sizeof W.r[0] + sizeof W.hu[0]);
+            bulk_g2s(W.r[b], A.R + (size_t)u * PT, sizeof W.r[0], &W.bar[b]);
+            bulk_g2s(W.hu[b], A.orow + (size_t)u * TROWS, sizeof W.hu[0], &W.bar[b]);
+        }
+    };
+    uint32_t t = tb + warp;
+    if (t < tend) stage(t, 0);
+    // heads before the range; the last CTA also sums the 1 bits
+    const bool last = tend == A.ntiles;
+    uint32_t part = 0, ones = 0;
+    for (uint32_t i = threadIdx.x; i < tb; i += GCTA) part += A.heads[i];
+    if (last) for (uint32_t i = threadIdx.x; i < A.ntiles; i += GCTA) ones += A.ones[i];
+    part = __reduce_add_sync(0xffffffffu, part);
+    ones = __reduce_add_sync(0xffffffffu, ones);
+    if (lane == 0) { sh[0][warp] = part; sh[1][warp] = ones; }
+    if (warp == 0) {  // scan of the range's tiles
+        uint32_t carry = 0;
+        for (uint32_t i = tb; i < tend; i += 32u) {
+            const uint32_t c = i + lane < tend ? A.heads[i + lane] : 0u;
             uint32_t x = c;
 #pragma unroll
             for (int d = 1; d < 32; d <<= 1) {
-                const uint32_t t = __shfl_up_sync(0xffffffffu, x, d);
-                if (lane >= (uint32_t)d) x += t;
+                const uint32_t u = __shfl_up_sync(0xffffffffu, x, d);
+                if (lane >= (uint32_t)d) x += u;
             }
-            p = carry + x - c;
+            if (i + lane < tend) pre[i + lane - tb] = carry + x - c;
             carry += __shfl_sync(0xffffffffu, x, 31);
         }
-        if (in && p < g1 && p + c > g0) mk[max(p, g0) - g0] = (uint16_t)(k + 1u);
+        part = carry;  // warp 0: the range's heads
     }
-}
-
-// Patterns of chunk j (groups 128*j + 4*lane + e of the tile) of an impure
-// operand; carry = the last word index + 1 seen before the chunk (markers,
-// word index + 1 at a word's first group, grow with the group).
-__device__ __forceinline__ uint4 gop_chunk(const uint32_t* ws, const uint16_t* mk, uint32_t j, uint32_t& carry) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint2 m = reinterpret_cast<const uint2*>(mk)[32 * j + lane];
-    const uint32_t r0 = m.x & 0xFFFFu, r1 = max(r0, m.x >> 16), r2 = max(r1, m.y & 0xFFFFu), r3 = max(r2, m.y >> 16);
-    // markers grow with the group, so the largest one before this lane is
-    // the last one of the nearest lower lane holding any
-    const uint32_t nz = __ballot_sync(0xffffffffu, r3 != 0u);
-    const uint32_t below = nz & ((1u << lane) - 1u);
-    const uint32_t lo = __shfl_sync(0xffffffffu, r3, below ? 31u - __clz(below) : lane);
-    const uint32_t hi = __shfl_sync(0xffffffffu, r3, nz ? 31u - __clz(nz) : 0u);
-    const uint32_t ex = below ? lo : carry;
-    if (nz) carry = hi;
-    const uint32_t i0 = max(ex, r0), i1 = max(ex, r1), i2 = max(ex, r2), i3 = max(ex, r3);  // >= 1 inside the tile
-    return make_uint4(wpattern(ws[i0 ? i0 - 1u : 0u]), wpattern(ws[i1 ? i1 - 1u : 0u]),
-                      wpattern(ws[i2 ? i2 - 1u : 0u]), wpattern(ws[i3 ? i3 - 1u : 0u]));
-}
-
-// Staged words 4 q .. 4 q + 3: one 16-byte read when the base is 16-byte
-// aligned (al, warp-uniform), else four.
-__device__ __forceinline__ uint4 gop_ld4(const uint32_t* ws, uint32_t q, bool al) {
-    if (al) return reinterpret_cast<const uint4*>(ws)[q];
-    return make_uint4(ws[4u * q], ws[4u * q + 1u], ws[4u * q + 2u], ws[4u * q + 3u]);
-}
-
-// Result patterns of one warp's tile [g0, g1) of x OP y: both operands'
-// words over the tile are staged in shared memory at once with cp.async and
-// expanded to one 31-bit pattern per group (a word-start marker per word
-// and a warp max-scan find the word of every group, so a fill costs one
-// marker whatever its length; an operand with one word per group is read
-// directly).  Calls f(j, r) for the chunks j = 0..7 in order, r holding the
-// results of groups 128 j + 4 lane + e of the tile (e = 0..3; groups past
-// g1 hold whatever the zero-padded words give and must be ignored).  prev
-// is set to the result of group g0 - 1 (0 for g0 = 0).  Returns false for a
-// word range the metadata scan would have rejected (the patterns are then
-// meaningless).
-template <int OP, class F>
-__device__ __forceinline__ bool gop_tile(const uint32_t* __restrict__ xw, const uint32_t* __restrict__ xgt,
-                                         uint32_t nx, const uint32_t* __restrict__ yw,
-                                         const uint32_t* __restrict__ ygt, uint32_t ny, GopWarp& W, uint32_t g0,
-                                         uint32_t g1, uint32_t& prev, F&& f) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t ng = g1 - g0;
-    uint32_t xi0, xs0, xn, yi0, ys0, yn;
-    const bool ok = gop_range(xgt, nx, g0, g1, xi0, xs0, xn) & gop_range(ygt, ny, g0, g1, yi0, ys0, yn);
-    // both operands' words in flight at once; word k of the tile at wsx[k]
-    gop_stage(W.ws[0], xw, xi0, xn, nx);
-    gop_stage(W.ws[1], yw, yi0, yn, ny);
-    const uint32_t* wsx = W.ws[0] + (xi0 & 3u);
-    const uint32_t* wsy = W.ws[1] + (yi0 & 3u);
-    const bool xpure = xs0 == g0 && xn == ng, ypure = ys0 == g0 && yn == ng;
-    // the result before the tile (the words covering g0 - 1)
-    prev = 0;
-    if (g0 > 0 && ok) {
-        const uint32_t xp = __ldg(xw + (xs0 < g0 ? xi0 : xi0 - 1u));
-        const uint32_t yp = __ldg(yw + (ys0 < g0 ? yi0 : yi0 - 1u));
-        prev = op2<OP>(wpattern(xp), wpattern(yp));
-    }
-    cp_async_wait_all();
-    __syncwarp();
-    uint32_t xc = 0, yc = 0;
-    // an impure operand is placed first (its markers then its patterns);
-    // two impure operands share the marker array one after the other, so
-    // the second one's patterns are read in a second sweep
-    const bool both = !xpure && !ypure;
-    uint4 xb[NCH];
-    if (!xpure) {
-        reinterpret_cast<uint2*>(W.mk)[lane] = make_uint2(0u, 0u);
+    __syncthreads();
+    uint32_t base = 0;
 #pragma unroll
-        for (int j = 1; j < NCH; ++j) reinterpret_cast<uint2*>(W.mk)[32 * j + lane] = make_uint2(0u, 0u);
+    for (uint32_t k = 0; k < (uint32_t)GW; ++k) base += sh[0][k];
+    if (last && threadIdx.x == 0) {
+        uint32_t sum = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < (uint32_t)GW; ++k) sum += sh[1][k];
+        const uint32_t n = base + part;
+        A.obp[(n + 31u) / 32u] = A.groups;
+        A.meta->n = n;
+        A.meta->groups = A.groups;
+        A.meta->nset = sum;
+        A.meta->anb = A.anb;
+        A.meta->aval = A.aval;
+    }
+    const uint32_t bit = 1u << lane, lt = bit - 1u, gt = ~(lt | bit);
+    uint32_t any = 0;  // the words written, OR'ed
+    for (uint32_t k = 0; t < tend; t += GW, ++k) {
+        const uint32_t b = k & 1u;
+        if (t + GW < tend) stage(t + GW, b ^ 1u);
+        // the first head after the tile: of the tiles after it, 32 at a time
+        uint32_t later = GNONE;
+        for (uint32_t i = t + 1u; later == GNONE; i += 32u) {
+            const uint32_t v = i + lane < A.ntiles ? A.first[i + lane] : (i + lane == A.ntiles ? A.groups : GNONE);
+            later = __reduce_min_sync(0xffffffffu, v);
+        }
+        if (!__all_sync(0xffffffffu, mbar_wait(&W.bar[b], (k >> 1) & 1u))) {
+            if (lane == 0) atomicExch(&A.meta->status, DEV_ERR_TIMEOUT);
+            if (t + GW < tend) mbar_wait(&W.bar[b ^ 1u], ((k + 1u) >> 1) & 1u);
+            return;
+        }
+        const uint32_t g0 = t * (uint32_t)PT;
+        const uint2 hu = lane < (uint32_t)TROWS ? W.hu[b][lane] : make_uint2(0u, 0u);
+        const uint32_t H = hu.x, c = __popc(H);
+        uint32_t x = c;
+#pragma unroll
+        for (int d = 1; d < TROWS; d <<= 1) {
+            const uint32_t u = __shfl_up_sync(0xffffffffu, x, d);
+            if (lane >= (uint32_t)d) x += u;
+        }
+        x += base + pre[t - tb] - c;  // lane r: index of row r's first head
+        const uint32_t fh = H ? g0 + 32u * lane + (__ffs(H) - 1u) : GNONE;
+        uint32_t nx = __shfl_down_sync(0xffffffffu, fh, 1);
+        if (lane >= TROWS - 1u) nx = later;
+#pragma unroll
+        for (int d = 1; d < TROWS; d <<= 1) nx = min(nx, __shfl_down_sync(0xffffffffu, nx, d));
+        if (lane < (uint32_t)TROWS) {
+            W.row[lane] = make_uint4(H, x, nx - (g0 + 32u * lane + 32u), hu.y & H);
+            A.orow[(size_t)t * TROWS + lane].y = x - 1u;
+            // block positions: a row holds at most one head of index 32 j
+            const uint32_t m = (x + 31u) & ~31u;
+            if (m < x + c) A.obp[m >> 5] = g0 + 32u * lane + nth_bit(H, m - x);
+        }
         __syncwarp();
-        gop_mark(wsx, W.mk, xn, xs0, g0, g1);
-        __syncwarp();
-        if (both) {
+        const uint32_t* rl = W.r[b] + lane;
+#pragma unroll 1
+        for (int r0 = 0; r0 < TROWS; r0 += 4) {
+            uint4 q[4];
 #pragma unroll
-            for (int j = 0; j < NCH; ++j) xb[j] = gop_chunk(wsx, W.mk, j, xc);
-            __syncwarp();
+            for (int j = 0; j < 4; ++j) q[j] = W.row[r0 + j];
+            if ((q[0].x | q[1].x | q[2].x | q[3].x) == 0u) continue;  // inside a run
 #pragma unroll
-            for (int j = 0; j < NCH; ++j) reinterpret_cast<uint2*>(W.mk)[32 * j + lane] = make_uint2(0u, 0u);
-            __syncwarp();
-        }
-    }
-    if (!ypure) {
-        if (xpure) {
-#pragma unroll
-            for (int j = 0; j < NCH; ++j) reinterpret_cast<uint2*>(W.mk)[32 * j + lane] = make_uint2(0u, 0u);
-            __syncwarp();
-        }
-        if (xpure || both) {
-            gop_mark(wsy, W.mk, yn, ys0, g0, g1);
-            __syncwarp();
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < NCH; ++j) {
-        uint4 a, b;
-        if (xpure) a = pattern4(gop_ld4(wsx, 32 * j + lane, (xi0 & 3u) == 0u));
-        else if (both) a = xb[j];
-        else a = gop_chunk(wsx, W.mk, j, xc);
-        if (ypure) b = pattern4(gop_ld4(wsy, 32 * j + lane, (yi0 & 3u) == 0u));
-        else b = gop_chunk(wsy, W.mk, j, yc);
-        f(j, make_uint4(op2<OP>(a.x, b.x), op2<OP>(a.y, b.y), op2<OP>(a.z, b.z), op2<OP>(a.w, b.w)));
-    }
-    return ok;
-}
-
-template <int OP>
-__global__ void __launch_bounds__(GTHREADS, 10) k_gop(GopArgs A) {
-    extern __shared__ __align__(16) unsigned char gsm[];
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint32_t t = blockIdx.x * GWARPS + warp;
-    if (t >= A.ntiles) return;
-    GopWarp& W = reinterpret_cast<GopWarp*>(gsm)[warp];
-    const uint32_t G = A.groups;
-    const uint32_t g0 = t * (uint32_t)GT, g1 = min(g0 + (uint32_t)GT, G);
-    const uint32_t ng = g1 - g0;
-    uint32_t* R = A.R + g0;
-    uint32_t heads = 0, first = GNONE, popc = 0, hm = 0;
-    uint32_t before;  // the result of the group before the current chunk
-    const bool ok = gop_tile<OP>(A.xw, A.xgt, A.nx, A.yw, A.ygt, A.ny, W, g0, g1, before, [&](int j, uint4 r) {
-        reinterpret_cast<uint4*>(R)[32 * j + lane] = r;
-        uint32_t pb = __shfl_up_sync(0xffffffffu, r.w, 1);
-        if (lane == 0) pb = before;
-        before = __shfl_sync(0xffffffffu, r.w, 31);
-        const uint32_t rv[4] = {r.x, r.y, r.z, r.w};
-        uint32_t pc = cls_of(pb);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const uint32_t pos = 128u * j + 4u * lane + e;
-            const uint32_t c = cls_of(rv[e]);
-            if (pos < ng) {
-                if ((g0 + pos == 0u) || c == C_MIXED || c != pc) {
-                    ++heads;
-                    first = min(first, g0 + pos);
-                    hm |= 1u << (4 * j + e);
+            for (int j = 0; j < 4; ++j) {
+                const uint32_t rv = rl[32 * (r0 + j)];
+                const uint32_t above = q[j].x & gt;  // the row's heads after this lane
+                // groups to the next head: in the row (its lowest bit above
+                // this lane), else past the row's end
+                const uint32_t low = 31u - __clz(above & (0u - above));  // -1: none
+                uint32_t len = low - lane;
+                if (above == 0u) len = q[j].z + (32u - lane);
+                const bool f = (q[j].w & bit) && (len >= 2u || rv >= HEADER0);
+                uint32_t wd = rv & ALLONES;
+                if (f) wd = (rv & FILLBIT) | len | HEADER0;
+                if (q[j].x & bit) {
+                    A.out[q[j].y + __popc(q[j].x & lt)] = wd;
+                    any |= wd;
                 }
-                popc += __popc(rv[e]);
             }
-            pc = c;
         }
-    });
-    A.hmask[(size_t)t * 32u + lane] = hm;
-    if (!ok && lane == 0) atomicExch(&A.meta->status, DEV_ERR_FORMAT);
-    heads = __reduce_add_sync(0xffffffffu, heads);
-    popc = __reduce_add_sync(0xffffffffu, popc);
-    first = __reduce_min_sync(0xffffffffu, first);
-    if (lane == 0) {
-        A.tiles[t] = make_uint4(heads, first, popc, 0u);
-        uint4* sg = A.segs + t / GSEG;
-        if (heads) atomicAdd(&sg->x, heads);
-        if (first != GNONE) atomicMax(&sg->y, GNONE - first);
-        if (popc) atomicAdd(&sg->z, popc);
+        if (t == 0 && lane == 0) A.meta->w0 = A.out[0];  // this lane's own store: group 0 is a head
+        __syncwarp();  // the rows and the buffer are free again
     }
-}
-
-// The words of one tile per warp, in order (tiles without heads have none).
-// The tile's first output index is the heads of the segments before its own
-// plus those of the tiles before it in its segment; the head after the tile
-// is the first head of the later tiles of its segment, else of the first
-// later segment holding one.  A head's word needs the next head's position:
-// the lanes find it with a suffix minimum over the lanes after them, chunks
-// taken last to first.  The warp of the last tile writes the metadata.
-__global__ void __launch_bounds__(GTHREADS) k_gpack(GopArgs A) {
-    // this tile's words, from the 16-byte boundary at or below its first
-    // output index (a tile holds at most GT heads, so GT + 3 slots)
-    __shared__ __align__(16) uint32_t sout[GWARPS][GT + 4];
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint32_t t = blockIdx.x * GWARPS + warp;
-    const uint32_t T = A.ntiles;
-    if (t >= T) return;
-    const uint32_t G = A.groups;
-    // the tile's result patterns and head masks, loaded first so their
-    // round trip overlaps the prefix and next-head loads below
-    const uint32_t g0 = t * (uint32_t)GT;
-    const uint4* R4 = reinterpret_cast<const uint4*>(A.R + g0);
-    const uint32_t hm = A.hmask[(size_t)t * 32u + lane];
-    uint4 rqs[NCH];
-#pragma unroll
-    for (int j = 0; j < NCH; ++j) rqs[j] = R4[32 * j + lane];
-    const uint32_t sg = t / GSEG, nseg = (T + GSEG - 1) / GSEG;
-    uint32_t off = 0;
-    for (uint32_t i = lane; i < sg; i += 32) off += A.segs[i].x;
-    // the tiles before this one in its segment: at most GSEG / 32 per lane,
-    // loaded together
-#pragma unroll
-    for (uint32_t k = 0; k < GSEG / 32u; ++k) {
-        const uint32_t i = sg * GSEG + lane + 32u * k;
-        if (i < t) off += A.tiles[i].x;
-    }
-    off = __reduce_add_sync(0xffffffffu, off);
-    const uint32_t cnt = A.tiles[t].x;
-    if (t == T - 1) {
-        uint32_t ones = 0;
-        for (uint32_t i = lane; i < nseg; i += 32) ones += A.segs[i].z;
-        ones = __reduce_add_sync(0xffffffffu, ones);
-        if (lane == 0) {
-            const uint32_t n = off + cnt;
-            A.obp[(n + 31u) / 32u] = G;
-            A.meta->n = n;
-            A.meta->groups = G;
-            A.meta->nset = ones;
-            A.meta->anb = A.anb;
-            A.meta->aval = A.aval;
-            if (n == 0) A.meta->w0 = 0;
-        }
-    }
-    if (cnt == 0) return;
-    uint32_t nxt = GNONE;
-    for (uint32_t i0 = t + 1; i0 < min(T, (sg + 1) * GSEG) && nxt == GNONE; i0 += 32) {
-        const uint32_t i = i0 + lane;
-        const uint32_t v = i < min(T, (sg + 1) * GSEG) ? A.tiles[i].y : GNONE;
-        nxt = __reduce_min_sync(0xffffffffu, v);
-    }
-    for (uint32_t i0 = sg + 1; i0 < nseg && nxt == GNONE; i0 += 32) {
-        const uint32_t i = i0 + lane;
-        const uint32_t v = i < nseg ? A.segs[i].y : 0u;
-        const uint32_t f = __reduce_max_sync(0xffffffffu, v);
-        if (f) nxt = GNONE - f;
-    }
-    if (nxt == GNONE) nxt = G;
-    // hm: the lane's heads as k_gop found them (bit 4 j + e for group 128 j + 4 lane + e)
-    uint32_t* so = sout[warp];
-    const uint32_t oal = off & ~3u;
-    const uint32_t gt = (2u << lane) - 1u;  // lanes up to this one (lane 31: all)
-    uint32_t later = nxt;  // the first head after the chunk
-    uint32_t rest = cnt;   // heads in the chunks before and at the current one
-    bool fill = false;
-#pragma unroll
-    for (int j = NCH - 1; j >= 0; --j) {
-        const uint32_t m = (hm >> (4 * j)) & 15u;
-        const uint32_t hl = __ballot_sync(0xffffffffu, m != 0u);
-        if (hl == 0u) continue;  // a chunk inside a run
-        // heads of the lanes before this one, from the bits of each lane's
-        // count (0..4); the chunk's own count
-        const uint32_t nh = __popc(m);
-        const uint32_t c0 = __ballot_sync(0xffffffffu, nh & 1u);
-        const uint32_t c1 = __ballot_sync(0xffffffffu, nh & 2u);
-        const uint32_t c2 = __ballot_sync(0xffffffffu, nh & 4u);
-        rest -= __popc(c0) + 2u * __popc(c1) + 4u * __popc(c2);
-        const uint32_t lt = gt >> 1;  // lanes before this one
-        uint32_t o = off + rest + __popc(c0 & lt) + 2u * __popc(c1 & lt) + 4u * __popc(c2 & lt);
-        // the head after this lane's last one: the first head of the
-        // nearest higher lane holding one, else the first after the chunk
-        const uint32_t g = g0 + 128u * j + 4u * lane;
-        const uint32_t mine = m ? g + (__ffs(m) - 1u) : GNONE;
-        const uint32_t above = hl & ~gt;
-        const uint32_t nl = __shfl_sync(0xffffffffu, mine, above ? __ffs(above) - 1u : lane);
-        const uint32_t after = above ? nl : later;
-        later = __shfl_sync(0xffffffffu, mine, __ffs(hl) - 1u);
-        if (m) {
-            const uint4 rq = rqs[j];
-            const uint32_t r[4] = {rq.x, rq.y, rq.z, rq.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-                if ((m >> e) & 1u) {
-                    const uint32_t more = m >> (e + 1);
-                    const uint32_t next = more ? g + e + __ffs(more) : after;
-                    const uint32_t wd = run_word(cls_of(r[e]), next - (g + e), r[e], false);
-                    so[o - oal] = wd;
-                    if ((o & 31u) == 0u) A.obp[o >> 5] = g + e;
-                    if (o == 0u) A.meta->w0 = wd;
-                    fill |= is_fill(wd);
-                    ++o;
-                }
-        }
-    }
-    if (__any_sync(0xffffffffu, fill) && lane == 0) atomicOr(&A.meta->nfill, 1u);
-    // the tile's words leave as 16-byte stores (the output array is a pool
-    // block, 16-byte aligned), the ragged ends word by word
-    __syncwarp();
-    const uint32_t end = off + cnt;
-    for (uint32_t v = lane; 4u * v < end - oal; v += 32u) {
-        const uint32_t gi = oal + 4u * v;
-        if (gi >= off && gi + 4u <= end) {
-            *reinterpret_cast<uint4*>(A.out + gi) = *reinterpret_cast<const uint4*>(so + 4u * v);
-        } else {
-#pragma unroll
-            for (uint32_t e = 0; e < 4u; ++e)
-                if (gi + e >= off && gi + e < end) A.out[gi + e] = so[4u * v + e];
-        }
-    }
+    if (__any_sync(0xffffffffu, any >= HEADER0) && lane == 0) A.meta->nfill = 1u;
 }
 
 }  // namespace wah
