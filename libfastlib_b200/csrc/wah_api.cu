@@ -637,10 +637,20 @@ static bool rows_reserve(wahgpu_bv* b, uint32_t groups, void* (*alloc)(wahgpu_ct
     b->rows_cap = need;
     return true;
 }
+// Room for a result's row index: a cached block, or, once the context has
+// made a few such results, a new one (a fresh context's first calls do not
+// pay for blocks that may never be read).
+static bool result_rows(wahgpu_bv* res, uint32_t groups) {
+    const bool fresh = res->ctx->row_results < 8;
+    if (fresh) res->ctx->row_results++;
+    return rows_reserve(res, groups, fresh ? wg_alloc_cached : wg_alloc);
+}
 // Row index of b (host metadata must be valid); built once.
 static int wg_rows(wahgpu_bv* b) {
-    if (b->rows_valid) return WAHGPU_OK;
     wahgpu_ctx* ctx = b->ctx;
+    // positions are taken from the words: none that the upload scan refused
+    if (b->h.status) return wg_fail(ctx, WAHGPU_EFORMAT, "the bitvector's words are malformed");
+    if (b->rows_valid) return WAHGPU_OK;
     if (!rows_reserve(b, b->h.groups, wg_alloc)) return wg_fail(ctx, WAHGPU_ENOMEM, "allocation failed");
     const uint32_t ntiles = (b->h.groups + PT - 1) / PT;
     k_rows<<<(ntiles + GW - 1) / GW, GCTA, 0, ctx->stream>>>(b->words, b->bpos, b->h.n, b->h.groups, ntiles, b->rows);
@@ -673,8 +683,6 @@ static void launch_gop_kind(const wahgpu_ctx* ctx, int op, uint32_t ntiles, cuda
 // null for the copies.
 int wg_launch_gop(wahgpu_ctx* ctx, int kind, int op, wahgpu_bv* x, wahgpu_bv* y, uint32_t groups,
                   uint32_t anb, uint32_t aval, wahgpu_bv* res) {
-    // positions are taken from the words: none that the upload scan refused
-    if (x->h.status || (y && y->h.status)) return wg_fail(ctx, WAHGPU_EFORMAT, "an operand's words are malformed");
     int rc = bv_reserve(res, (uint64_t)x->h.n + (y ? y->h.n : 0));
     if (!rc) rc = wg_rows(x);
     if (!rc && y) rc = wg_rows(y);
@@ -682,7 +690,7 @@ int wg_launch_gop(wahgpu_ctx* ctx, int kind, int op, wahgpu_bv* x, wahgpu_bv* y,
     const uint32_t ntiles = (uint32_t)(((uint64_t)groups + PT - 1) / PT);
     // the result keeps its head masks as its row index where a block for it
     // is at hand; else they are part of the scratch
-    const bool keep = rows_reserve(res, groups, wg_alloc_cached);
+    const bool keep = result_rows(res, groups);
     const size_t rb = (size_t)ntiles * PT * 4, hb = (size_t)ntiles * TROWS * sizeof(uint2);
     unsigned char* scr = static_cast<unsigned char*>(wg_alloc(ctx, rb + hb + (size_t)ntiles * 12));
     if (!scr) return wg_fail(ctx, WAHGPU_ENOMEM, "allocation of %u tiles of result patterns failed", ntiles);
@@ -1162,14 +1170,24 @@ extern "C" int wahgpu_bv_decompress(wahgpu_bv* b) {
     wahgpu_bv* r = wg_bv_new(ctx);
     if (!r) return wg_fail(ctx, WAHGPU_ENOMEM, "allocation failed");
     rc = bv_reserve(r, G);
+    if (!rc && b->h.n) rc = wg_rows(b);
     if (!rc && b->h.n) {
-        uint32_t nt = (b->h.n + SCAN_TILE - 1) / SCAN_TILE;
-        k_decompress<<<nt, SCAN_THREADS, 0, ctx->stream>>>(b->words, b->h.n, b->bpos, r->words);
+        // the groups are b's: only the words and their number change
+        r->h = b->h;
+        r->h.n = G;
+        r->h.w0 = wpattern(b->h.w0);
+        r->h.nfill = 0;
+        r->h_valid = true;
+        r->rows_valid = result_rows(r, G);
+        const uint32_t ntiles = (uint32_t)(((uint64_t)G + PT - 1) / PT);
+        k_expand<<<(ntiles + GW - 1) / GW, GCTA, 0, ctx->stream>>>(b->words, b->rows, ntiles, r->words, r->bpos,
+                                                                   r->rows_valid ? r->rows : nullptr, r->meta, r->h);
         ctx->launches++;
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) rc = wg_fail(ctx, WAHGPU_ECUDA, "launch failed: %s", cudaGetErrorString(e));
+    } else if (!rc) {
+        rc = wg_scan_meta(r, G, b->h.anb, b->h.aval);
     }
-    if (!rc) rc = wg_scan_meta(r, G, b->h.anb, b->h.aval);
     if (rc) { wahgpu_bv_free(r); return rc; }
     cudaStreamSynchronize(ctx->stream);
     bv_take(b, r);
@@ -1186,7 +1204,7 @@ int64_t wg_rids_device(wahgpu_bv* b, uint32_t* dev_out, uint64_t cap, uint64_t* 
     *total = cnt;
     if (cap < cnt) return wg_fail(ctx, WAHGPU_ESIZE, "need room for %llu row ids", (unsigned long long)cnt);
     const uint32_t n = b->h.n;
-    const uint32_t ntiles = n ? (n + SCAN_TILE - 1) / SCAN_TILE : 1;
+    const uint32_t ntiles = n ? (n + RIDS_TILE - 1) / RIDS_TILE : 1;
     TileRec* recs; LaunchSync* sync;
     rc = wg_scratch(ctx, ntiles, &recs, &sync);
     if (rc) return rc;

@@ -27,6 +27,7 @@ struct wahgpu_ctx {
     uint32_t scratch_tiles = 0;
     void* h_meta_stage = nullptr;  // pinned staging for metadata reads
     uint64_t launches = 0;
+    uint32_t row_results = 0;           // results that could have kept a row index so far
     uint32_t dense_tile = 2048;         // WAHGPU_TUNE_DENSE_TILE
     uint32_t dense_engine = 0;          // WAHGPU_TUNE_DENSE_ENGINE
     uint32_t range_order = 1;           // WAHGPU_TUNE_RANGE_ORDER

@@ -184,6 +184,45 @@ __global__ void __launch_bounds__(GCTA) k_rows(const uint32_t* __restrict__ w, c
     if (lane < (uint32_t)TROWS) rows[(size_t)t * TROWS + lane] = make_uint2(m, w0 + x - __popc(m) - 1u);
 }
 
+// decompress(): every group of a bitvector as a literal word, with the
+// result's block positions, row index (when orow is given) and metadata, all
+// of which are known beforehand.  A warp per tile; bound by the stores.  (A
+// thread per 16 words with the fills listed and written one after the other
+// by the CTA took 244 us at 2^27 bits, d = 0.05, and the metadata another 23;
+// this takes 12 and k_rows, where the index is not there yet, 12.)
+__global__ void __launch_bounds__(GCTA) k_expand(const uint32_t* __restrict__ w, const uint2* __restrict__ rows,
+                                                 uint32_t ntiles, uint32_t* __restrict__ out, uint32_t* __restrict__ obp,
+                                                 uint2* __restrict__ orow, DevMeta* meta, DevMeta m) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t t = blockIdx.x * GW + (threadIdx.x >> 5);
+    const uint32_t le = (2u << lane) - 1u;
+    if (blockIdx.x == 0 && threadIdx.x == 0) { *meta = m; obp[(m.groups + 31u) / 32u] = m.groups; }
+    if (t >= ntiles) return;
+    const uint32_t g0 = t * (uint32_t)PT;
+    const uint2* xr = rows + (size_t)t * TROWS;
+#pragma unroll
+    for (int r0 = 0; r0 < TROWS; r0 += 8) {
+        uint32_t v[8];
+#pragma unroll
+        for (int j = 0; j < 8; j += 2) {
+            const uint4 q = __ldg(reinterpret_cast<const uint4*>(xr + r0 + j));
+            v[j] = __ldg(w + (q.y + __popc(q.x & le)));
+            v[j + 1] = __ldg(w + (q.w + __popc(q.z & le)));
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const uint32_t g = g0 + 32u * (r0 + j) + lane;
+            if (g < m.groups) out[g] = wpattern(v[j]);
+        }
+    }
+    if (lane < (uint32_t)TROWS) {
+        const uint32_t g = g0 + 32u * lane;
+        const uint32_t k = m.groups > g ? m.groups - g : 0u;  // groups from the row on
+        if (k) obp[g >> 5] = g;
+        if (orow) orow[(size_t)t * TROWS + lane] = make_uint2(k >= 32u ? 0xFFFFFFFFu : (1u << k) - 1u, min(g, m.groups) - 1u);
+    }
+}
+
 // ---- words further back, for the count-1 flags that need them (whole warp,
 // uniform arguments).  Rare: only one-group runs over count-1 fill words.
 // First group of word j.

@@ -144,6 +144,15 @@ __global__ void k_small(int mode, int op, const uint32_t* xw, const uint32_t* yw
 // Row ids of the 1 bits: ascending positions (the reference's indexSet walk,
 // src/bitvector.cpp:4524-4590).  Literal bit 30-k of the word at group g is
 // row 31g+k; the active word's bits follow, most significant first.
+//
+// A CTA takes RIDS_TILE words, four neighbouring words per thread: a small
+// vector spreads over many CTAs (100 K words over 108; tiles of 4096 words
+// left 27 CTAs and took 25 us, this takes 15).  Every warp then writes its
+// 128 words' ids row by row of 32 words: a row without 1-fills through
+// shared memory, so that neighbouring lanes store neighbouring ids; 1-fills
+// of up to RIDS_FILL groups by the warp, longer ones by the CTA.
+constexpr uint32_t RIDS_TILE = SCAN_THREADS * 4;
+constexpr uint32_t RIDS_FILL = 32;
 __global__ void __launch_bounds__(SCAN_THREADS)
 k_rids(const uint32_t* __restrict__ w, uint32_t n, const uint32_t* __restrict__ bpos,
        uint32_t groups, uint32_t anb, uint32_t aval, uint32_t* __restrict__ out, uint64_t cap,
@@ -152,124 +161,114 @@ k_rids(const uint32_t* __restrict__ w, uint32_t n, const uint32_t* __restrict__ 
     __shared__ uint32_t hdr[2];
     __shared__ uint64_t tile_pre;
     __shared__ uint32_t fq_n;
-    __shared__ uint64_t fq_off[SCAN_TILE / 2];
-    __shared__ uint32_t fq_row[SCAN_TILE / 2];
-    __shared__ uint32_t fq_len[SCAN_TILE / 2];
+    __shared__ uint64_t fq_off[RIDS_TILE];
+    __shared__ uint32_t fq_row[RIDS_TILE], fq_len[RIDS_TILE];
+    __shared__ uint32_t stage[SCAN_THREADS / 32][32 * 31];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) { hdr[0] = claim_tile(sync); hdr[1] = ld_cg(&sync->epoch); fq_n = 0; }
     __syncthreads();
     const uint32_t t = hdr[0], epoch = hdr[1];
-    const uint32_t base = t * SCAN_TILE + threadIdx.x * SCAN_WPT;
-    uint32_t v[SCAN_WPT];
-    uint64_t cnt = 0;
-    uint32_t gpos = 0;
-    if (base < n) {
-        // group position of this thread's first word: block position + scan within the block
-        const uint32_t blk = base / 32u;
-        gpos = __ldg(bpos + blk);
-        for (uint32_t k = blk * 32u; k < base; ++k) gpos += wgroups(__ldg(w + k));
+    // the warp's 128 words: word 32 r + lane of row r
+    const uint32_t base = t * RIDS_TILE + warp * 128u;
+    uint32_t v[4], p[4];
+    uint64_t cnt = 0;  // 1 bits of the lane's words
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const uint32_t i = base + 32u * r + lane;
+        v[r] = i < n ? __ldg(w + i) : 0u;
+        p[r] = base + 32u * r < n ? __ldg(bpos + (base >> 5) + r) : 0u;
     }
 #pragma unroll
-    for (int q = 0; q < SCAN_WPT; ++q) {
-        v[q] = (base + q < n) ? __ldg(w + base + q) : 0u;
-        const uint32_t x = v[q];
-        if (base + q < n) cnt += (x > ALLONES) ? ((x >= HEADER1) ? (uint64_t)(x & MAXCNT) * 31u : 0u) : __popc(x);
+    for (int r = 0; r < 4; ++r) {
+        const bool in = base + 32u * r + lane < n;
+        const uint32_t x = v[r];
+        const uint32_t c = in ? wgroups(x) : 0u;
+        if (in) cnt += x > ALLONES ? (x >= HEADER1 ? (uint64_t)c * 31u : 0u) : __popc(x);
+        uint32_t s = c;  // first group of the word
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t u = __shfl_up_sync(0xffffffffu, s, d);
+            if (lane >= (uint32_t)d) s += u;
+        }
+        p[r] += s - c;
     }
     uint64_t total;
-    const uint64_t ex = block_exscan64(cnt, sh, total);
+    uint64_t off = block_exscan64(cnt, sh, total);
     if (threadIdx.x < 32) {
         uint64_t prefix; uint32_t pa, pb;
         bool ok = lookback64(recs, t, epoch, total, 0, 0, prefix, pa, pb);
         if (threadIdx.x == 0 && !ok) atomicExch(&meta->status, DEV_ERR_TIMEOUT);
         if (threadIdx.x == 0) tile_pre = prefix;
         if (threadIdx.x == 0 && t == ntiles - 1) {
-            uint64_t off = prefix + total;
+            uint64_t o = prefix + total;
             const uint32_t rbase = groups * 31u;
             for (uint32_t b = 0; b < anb; ++b)
-                if ((aval >> (anb - 1u - b)) & 1u) { if (off < cap) out[off] = rbase + b; ++off; }
-            *total_out = off;
+                if ((aval >> (anb - 1u - b)) & 1u) { if (o < cap) out[o] = rbase + b; ++o; }
+            *total_out = o;
         }
     }
     __syncthreads();
-    uint64_t off = tile_pre + ex;
-    uint32_t g = gpos;
+    // the warp's first id: the lanes' words interleave, so from lane 0's place
+    uint64_t o0 = tile_pre + __shfl_sync(0xffffffffu, off, 0);
+    uint32_t* st = stage[warp];
 #pragma unroll
-    for (int q = 0; q < SCAN_WPT; ++q) {
-        if (base + q < n) {
-            const uint32_t x = v[q];
-            if (x > ALLONES) {
-                const uint32_t c = x & MAXCNT;
-                if (x >= HEADER1) {
-                    const uint32_t slot = atomicAdd(&fq_n, 1u);
-                    if (slot < (uint32_t)(SCAN_TILE / 2)) {
-                        fq_off[slot] = off; fq_row[slot] = g * 31u; fq_len[slot] = c * 31u;
-                    } else {  // list full: this thread writes the fill
-                        for (uint32_t r = 0; r < c * 31u; ++r) if (off + r < cap) out[off + r] = g * 31u + r;
-                    }
-                    off += (uint64_t)c * 31u;
-                }
-                g += c;
-            } else {
-                uint32_t bits = x;
-                while (bits) {
-                    const uint32_t b = 31u - __clz(bits);  // highest set bit
-                    if (off < cap) out[off] = g * 31u + (30u - b);
-                    ++off;
-                    bits &= ~(1u << b);
-                }
-                g += 1;
+    for (int r = 0; r < 4; ++r) {
+        const uint32_t x = v[r], row = p[r] * 31u;
+        const bool fill1 = x >= HEADER1;
+        const uint32_t ones = fill1 ? (x & MAXCNT) * 31u : (x > ALLONES ? 0u : __popc(x));
+        uint64_t q = ones;  // ids of the row's words up to this one
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint64_t u = __shfl_up_sync(0xffffffffu, q, d);
+            if (lane >= (uint32_t)d) q += u;
+        }
+        const uint64_t rt = __shfl_sync(0xffffffffu, q, 31);
+        q -= ones;
+        uint32_t fills = __ballot_sync(0xffffffffu, fill1);
+        if (fills == 0u) {
+            uint32_t k = (uint32_t)q;
+            for (uint32_t bits = x > ALLONES ? 0u : x; bits;) {
+                const uint32_t b = 31u - __clz(bits);  // highest set bit
+                st[k++] = row + (30u - b);
+                bits &= ~(1u << b);
+            }
+            __syncwarp();
+            for (uint32_t i = lane; i < (uint32_t)rt; i += 32u)
+                if (o0 + i < cap) out[o0 + i] = st[i];
+            __syncwarp();
+        } else {
+            uint64_t k = o0 + q;
+            for (uint32_t bits = x > ALLONES ? 0u : x; bits;) {
+                const uint32_t b = 31u - __clz(bits);
+                if (k < cap) out[k] = row + (30u - b);
+                ++k;
+                bits &= ~(1u << b);
+            }
+            if (fill1 && (x & MAXCNT) > RIDS_FILL) {
+                const uint32_t slot = atomicAdd(&fq_n, 1u);  // a slot per word of the tile
+                fq_off[slot] = o0 + q; fq_row[slot] = row; fq_len[slot] = ones;
+            }
+            fills = __ballot_sync(0xffffffffu, fill1 && (x & MAXCNT) <= RIDS_FILL);
+            while (fills) {
+                const uint32_t l = __ffs(fills) - 1u;
+                fills &= fills - 1u;
+                const uint64_t fo = o0 + __shfl_sync(0xffffffffu, q, l);
+                const uint32_t fr = __shfl_sync(0xffffffffu, row, l), fl = __shfl_sync(0xffffffffu, ones, l);
+                for (uint32_t i = lane; i < fl; i += 32u)
+                    if (fo + i < cap) out[fo + i] = fr + i;
             }
         }
+        o0 += rt;
     }
     __syncthreads();
     // the CTA writes every listed 1-fill of the tile cooperatively
-    const uint32_t nfq = min(fq_n, (uint32_t)(SCAN_TILE / 2));
-    for (uint32_t k = 0; k < nfq; ++k) {
+    for (uint32_t k = 0; k < fq_n; ++k) {
         const uint64_t o = fq_off[k];
         const uint32_t r0 = fq_row[k], len = fq_len[k];
         for (uint32_t r = threadIdx.x; r < len; r += SCAN_THREADS)
             if (o + r < cap) out[o + r] = r0 + r;
     }
-    __syncthreads();
     if (threadIdx.x == 0) finish_tile(sync, ntiles);
-}
-
-// decompress(): every word expanded to its groups as literal words.
-__global__ void __launch_bounds__(SCAN_THREADS)
-k_decompress(const uint32_t* __restrict__ w, uint32_t n, const uint32_t* __restrict__ bpos,
-             uint32_t* __restrict__ out) {
-    __shared__ uint32_t fq_n;
-    __shared__ uint32_t fq_pos[SCAN_TILE / 2], fq_len[SCAN_TILE / 2], fq_val[SCAN_TILE / 2];
-    if (threadIdx.x == 0) fq_n = 0;
-    __syncthreads();
-    const uint32_t base = blockIdx.x * SCAN_TILE + threadIdx.x * SCAN_WPT;
-    if (base < n) {
-        const uint32_t blk = base / 32u;
-        uint32_t g = __ldg(bpos + blk);
-        for (uint32_t k = blk * 32u; k < base; ++k) g += wgroups(__ldg(w + k));
-        for (int q = 0; q < SCAN_WPT && base + q < n; ++q) {
-            const uint32_t x = __ldg(w + base + q);
-            if (x > ALLONES) {
-                const uint32_t c = x & MAXCNT;
-                const uint32_t val = (x >= HEADER1) ? ALLONES : 0u;
-                const uint32_t slot = atomicAdd(&fq_n, 1u);
-                if (slot < (uint32_t)(SCAN_TILE / 2)) {
-                    fq_pos[slot] = g; fq_len[slot] = c; fq_val[slot] = val;
-                } else {  // list full: this thread writes the fill
-                    for (uint32_t r = 0; r < c; ++r) out[g + r] = val;
-                }
-                g += c;
-            } else {
-                out[g] = x;
-                g += 1;
-            }
-        }
-    }
-    __syncthreads();
-    const uint32_t nfq = min(fq_n, (uint32_t)(SCAN_TILE / 2));
-    for (uint32_t k = 0; k < nfq; ++k) {
-        const uint32_t p = fq_pos[k], len = fq_len[k], val = fq_val[k];
-        for (uint32_t r = threadIdx.x; r < len; r += SCAN_THREADS) out[p + r] = val;
-    }
 }
 
 }  // namespace wah
