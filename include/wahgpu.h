@@ -80,12 +80,12 @@ int64_t wahgpu_ctx_launches(wahgpu_ctx* ctx);
                                       2 word-space merge, 3 two-pass group-space kernels, \
                                       4 single-pass group-space kernel over CTA tiles, \
                                       5 single-pass group-space kernel over warp tiles */
-#define WAHGPU_TUNE_RANGE_ORDER 2 /* batch work order: 0 query by query; 1 (default) tile by tile for count-only \
-                                     batches, else query by query; 2 tile by tile, row ids of several queries \
-                                     placed by a count pass and a scan (capped batches: the id pass revisits \
-                                     only the tiles holding ids under each query's limit) */
+#define WAHGPU_TUNE_RANGE_ORDER 2 /* batch work order: 0 query by query; 1 (default) tile by tile, row ids in one \
+                                     pass (query by query) for small batches, else as 2; 2 tile by tile, row ids \
+                                     of several queries placed by a count pass and a scan (capped batches: the id \
+                                     pass revisits only the tiles holding ids under each query's limit) */
 #define WAHGPU_TUNE_RANGE_CTAS 3  /* resident CTAs per SM of the persistent range launch: 0 (all that fit) .. 32 */
-#define WAHGPU_TUNE_CUM_STRIDE 5  /* bitmaps per cumulative row of indexes built or attached later: 0 auto, 1 none, >= 2 that stride */
+#define WAHGPU_TUNE_CUM_STRIDE 5  /* bitmaps per cumulative row of indexes built or attached later: 0 auto (a row per bitmap where that fits), 1 none, >= 2 that stride */
 #define WAHGPU_TUNE_MERGE_TILE 6  /* block-index entries per tile of the word-space merge: 0 auto (by operand size), 16 | 32 | 64 */
 /* Failure-path test hooks (no counterpart in the reference; never needed in
  * normal use).  WAHGPU_TEST_WITHHOLD_TILE = t: in the next operator call on
@@ -284,8 +284,9 @@ int64_t wahgpu_evaluate(wahgpu_ctx* ctx, const wahgpu_term* terms, uint32_t nter
 
 /* Batches: nq conjunctive queries, query q being terms
  * [query_offsets[q], query_offsets[q+1]); all indexes of a batch share one
- * row count.  The whole batch runs as one kernel launch (wahgpu_batch_run,
- * capturable in a CUDA graph); rid_cap > 0 keeps the row ids of all queries
+ * row count.  The whole batch runs at once (wahgpu_batch_run: one or two
+ * kernel launches, three with the row ids of a large batch; capturable in a
+ * CUDA graph after a first run); rid_cap > 0 keeps the row ids of all queries
  * back to back in device memory, rid_cap == 0 counts only. */
 int wahgpu_batch_create(wahgpu_ctx* ctx, const wahgpu_term* terms, const uint32_t* query_offsets,
                         uint32_t nq, uint64_t rid_cap, int dense_first, wahgpu_batch** out);
@@ -294,8 +295,7 @@ int wahgpu_batch_create(wahgpu_ctx* ctx, const wahgpu_term* terms, const uint32_
  * region of its own, so one query with many hits cannot crowd out the
  * others (no counterpart in the reference, whose getHitRows returns all
  * rows, src/countQuery.cpp:387-410).  Counts are always complete;
- * wahgpu_batch_rids returns min(count, rid_caps[q]) ids.  Runs query by
- * query. */
+ * wahgpu_batch_rids returns min(count, rid_caps[q]) ids. */
 int wahgpu_batch_create_capped(wahgpu_ctx* ctx, const wahgpu_term* terms, const uint32_t* query_offsets,
                                uint32_t nq, const uint64_t* rid_caps, wahgpu_batch** out);
 int wahgpu_batch_run(wahgpu_batch* batch);

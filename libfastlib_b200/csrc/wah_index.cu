@@ -75,9 +75,11 @@ extern "C" int wahgpu_index_from_triple(wahgpu_ctx* ctx, int kind, uint64_t nrow
 
 // Cumulative rows: for a stride S, dense row k-1 = OR of bitmaps [0, k*S)
 // (k = 1..K), so a range's wholly-inside span costs two dense reads per tile
-// plus at most 2S edge bitmaps.  S is the smallest stride >= 8 that keeps
-// the rows within CUM_BUDGET bytes (or the context's WAHGPU_TUNE_CUM_STRIDE);
-// indexes with fewer than two rows' worth of bitmaps keep none.
+// plus at most 2S edge bitmaps.  S is the smallest stride that keeps the rows
+// within CUM_BUDGET bytes (or the context's WAHGPU_TUNE_CUM_STRIDE): 1, a row
+// per bitmap, where that fits (a range is then its rows alone: no word of a
+// bitmap is read), else at least 8.  Indexes with fewer than two rows' worth
+// of bitmaps keep none.
 static constexpr uint64_t CUM_BUDGET = 2ull << 30;
 static int cumulative_rows(wahgpu_index* x) {
     wahgpu_ctx* ctx = x->ctx;
@@ -86,10 +88,11 @@ static int cumulative_rows(wahgpu_index* x) {
     const uint64_t gx = ((uint64_t)x->groups + (x->anb ? 1 : 0) + 3) & ~3ull;
     x->cum_k = 0; x->cum_stride = 0;
     if (ctx->cum_stride == 1 || gx == 0) return WAHGPU_OK;
-    const uint64_t stride = ctx->cum_stride ? ctx->cum_stride
-                                            : std::max<uint64_t>(8, (nobs * gx * 4 + CUM_BUDGET - 1) / CUM_BUDGET);
+    const uint64_t fit = (nobs * gx * 4 + CUM_BUDGET - 1) / CUM_BUDGET;
+    const uint64_t stride = ctx->cum_stride ? ctx->cum_stride : fit <= 1 ? 1 : std::max<uint64_t>(8, fit);
     const uint64_t K = nobs / stride;
-    if (K < 2) return WAHGPU_OK;
+    if (K < 2 && stride > 1) return WAHGPU_OK;
+    if (K == 0) return WAHGPU_OK;
     x->d_cum = static_cast<uint32_t*>(wg_alloc(ctx, K * gx * 4));
     if (!x->d_cum) return WAHGPU_OK;  // no room: ranges use the bitmaps alone
     CUDA_TRY(ctx, cudaMemsetAsync(x->d_cum, 0, K * gx * 4, ctx->stream));
@@ -136,11 +139,11 @@ int wg_index_attach(wahgpu_index* x) {
     unsigned long long* d_cg = tmp.get<unsigned long long>(nchunks);
     uint32_t* d_co = tmp.get<uint32_t>(nchunks);
     uint32_t* d_ones = tmp.get<uint32_t>(nobs);
-    DevMeta* d_st = tmp.get<DevMeta>(1);
+    DevMeta* d_st = tmp.get<DevMeta>(2);
     if (!x->d_tiles || !x->d_tl_off || !d_choff || !d_cg || !d_co || !d_ones || !d_st)
         return wg_fail(ctx, WAHGPU_ENOMEM, "index allocation failed");
     const uint32_t blocks = (uint32_t)(((uint64_t)nchunks * 32 + ITHREADS - 1) / ITHREADS);
-    CUDA_TRY(ctx, cudaMemsetAsync(d_st, 0, sizeof(DevMeta), ctx->stream));
+    CUDA_TRY(ctx, cudaMemsetAsync(d_st, 0, 2 * sizeof(DevMeta), ctx->stream));
     DevMeta st{};
     x->bones.resize(nobs);
     if (nobs) {
@@ -181,14 +184,26 @@ int wg_index_attach(wahgpu_index* x) {
         if (rc) return rc;
         k_tile_lists<<<nparts, ITHREADS, 0, ctx->stream>>>(touch, tw, nt, x->d_tl_off, x->d_tl_bm, d_st, recs, sync, nparts);
         ctx->launches += 2;
+        unsigned long long* d_or = reinterpret_cast<unsigned long long*>(d_st + 1);  // 1 bits of all bitmaps OR'ed
+        unsigned long long h_or = 0;
         if (x->cum_k) {
             k_cum_prefix<<<(a.gx + 255) / 256, 256, 0, ctx->stream>>>(x->d_cum, x->cum_k, a.gx);
             ctx->launches++;
+            if (x->cum_stride == 1) {
+                k_row_ones<<<std::min<uint32_t>((a.gx + 255) / 256, 2u * (uint32_t)ctx->sm_count), 256, 0, ctx->stream>>>(
+                    x->d_cum + (size_t)(x->cum_k - 1) * a.gx, a.gx, d_or);
+                ctx->launches++;
+            }
         }
         CUDA_TRY(ctx, cudaGetLastError());
         CUDA_TRY(ctx, cudaMemcpyAsync(&st, d_st, sizeof(DevMeta), cudaMemcpyDeviceToHost, ctx->stream));
+        CUDA_TRY(ctx, cudaMemcpyAsync(&h_or, d_or, sizeof h_or, cudaMemcpyDeviceToHost, ctx->stream));
         CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
         if (st.status) return wg_fail(ctx, WAHGPU_ETIMEOUT, "a device-side look-back wait gave up");
+        // no row in two bitmaps: the OR holds as many 1 bits as all of them
+        uint64_t ones = 0;
+        for (uint32_t j = 0; j < nobs; ++j) ones += x->bones[j];
+        x->disjoint = x->cum_stride == 1 && h_or == ones;
     } else {
         CUDA_TRY(ctx, cudaMemsetAsync(x->d_tl_off, 0, ((size_t)nt + 1) * 4, ctx->stream));
     }
@@ -359,6 +374,13 @@ static int locate(wahgpu_ctx* ctx, const wahgpu_index* x, const wahgpu_term* t, 
     if (nc > 0 && !x->d_values)
         return wg_fail(ctx, WAHGPU_EINVAL, "range needs row checks but the index has no raw values attached");
     out.h0 = h0; out.h1 = h1; out.ncand = nc;
+    if (x->cum_k && x->cum_stride == 1) {
+        // a row per bitmap: the span and the edge bitmaps by rows
+        out.dense = 1; out.cum = x->d_cum;
+        out.c0 = h1 > h0 ? h0 : 0; out.c1 = h1 > h0 ? h1 : 0;
+        out.e0 = h0; out.e1 = h1;
+        return WAHGPU_OK;
+    }
     if (x->cum_k && h1 > h0) {
         // C(k1) & ~C(k0) covers [k0*S, k1*S); the rest are edge bitmaps
         const uint32_t S = x->cum_stride;
@@ -431,14 +453,17 @@ static int batch_create(wahgpu_ctx* ctx, const wahgpu_term* terms, const uint32_
         // bytes the term reads: the OR'ed bitmaps' words, the edge bitmaps'
         // words and the raw value of each of their rows
         const uint64_t in = x->cum_words[dt[i].h1] - x->cum_words[dt[i].h0];
-        if (dt[i].c1)
+        const uint64_t rowb = 4 * ((uint64_t)x->groups + (x->anb ? 1 : 0));
+        if (dt[i].dense) bytes += rowb * ((dt[i].c1 ? 1 : 0) + (dt[i].c0 ? 1 : 0));
+        else if (dt[i].c1)
             bytes += 4 * ((dt[i].c0 ? 2 : 1) * ((uint64_t)x->groups + (x->anb ? 1 : 0)) +
                           (x->cum_words[dt[i].e0] - x->cum_words[dt[i].h0]) +
                           (x->cum_words[dt[i].h1] - x->cum_words[dt[i].e1]));
         else
             bytes += 4 * (dt[i].flip ? x->cum_words[x->nobs] - in : in);
         for (uint32_t c = 0; c < dt[i].ncand; ++c)
-            bytes += 4 * (x->bwords[dt[i].cand[c]] + x->bones[dt[i].cand[c]]);
+            bytes += 4 * (uint64_t)x->bones[dt[i].cand[c]] +
+                     (dt[i].dense ? rowb * (dt[i].cand[c] ? 2 : 1) : 4 * x->bwords[dt[i].cand[c]]);
         // what sumBins itself must read: the covered bitmaps or, when they
         // hold more than half the words, their complement
         // (src/index.cpp:6490), plus the edge bitmaps and their rows
@@ -446,16 +471,41 @@ static int batch_create(wahgpu_ctx* ctx, const wahgpu_term* terms, const uint32_
         for (uint32_t c = 0; c < dt[i].ncand; ++c)
             min_bytes += 4 * (x->bwords[dt[i].cand[c]] + x->bones[dt[i].cand[c]]);
     }
-    std::vector<DevQuery> dq(nq);
+    std::vector<DevQuery> dq;  // the queries k_range evaluates
+    std::vector<uint64_t> base(nq, 0);  // counts known beforehand
+    std::vector<uint32_t> edge_term, edge_q;  // {term, bitmap} and query of the edges counted alone
+    const bool count_only = !rid_cap && !dense_first;
+    uint64_t rid_base = 0;
+    bool general = false;
     for (uint32_t q = 0; q < nq; ++q) {
         if (query_offsets[q + 1] <= query_offsets[q] || query_offsets[q + 1] > nt)
             return wg_fail(ctx, WAHGPU_EINVAL, "query %u has no term", q);
-        dq[q].t0 = query_offsets[q]; dq[q].t1 = query_offsets[q + 1];
-        dq[q].rid_base = q ? dq[q - 1].rid_base + (caps ? caps[q - 1] : 0) : 0;
-        dq[q].rid_lim = caps ? caps[q] : 0;
-        std::stable_sort(dt.begin() + dq[q].t0, dt.begin() + dq[q].t1, [&](const DevTerm& a, const DevTerm& b) {
+        const uint32_t t0 = query_offsets[q];
+        if (count_only && query_offsets[q + 1] == t0 + 1 && dt[t0].dense && terms[t0].idx->disjoint) {
+            // one term over disjoint bitmaps: the wholly-inside bitmaps' 1
+            // bits add up, only the edge bins' rows are left to count
+            const wahgpu_index* x = terms[t0].idx;
+            base[q] = x->cum_ones[dt[t0].h1] - x->cum_ones[dt[t0].h0];
+            for (uint32_t c = 0; c < dt[t0].ncand; ++c) {
+                edge_term.push_back(t0); edge_term.push_back(dt[t0].cand[c]);
+                edge_q.push_back(q);
+            }
+            continue;
+        }
+        dq.push_back(DevQuery{});
+        DevQuery& d = dq.back();
+        d.q = q;
+        d.t0 = t0; d.t1 = query_offsets[q + 1];
+        d.rid_base = rid_base;
+        d.rid_lim = caps ? caps[q] : 0;
+        rid_base += caps ? caps[q] : 0;
+        std::stable_sort(dt.begin() + d.t0, dt.begin() + d.t1, [&](const DevTerm& a, const DevTerm& b) {
+            if (a.dense != b.dense) return a.dense > b.dense;
             return term_estimate(idx[a.index], a) < term_estimate(idx[b.index], b);
         });
+        d.td = d.t0;
+        while (d.td < d.t1 && dt[d.td].dense) ++d.td;
+        general |= d.td < d.t1;
     }
     std::vector<DevIndex> di;
     for (auto* x : idx) di.push_back(x->dev);
@@ -464,10 +514,20 @@ static int batch_create(wahgpu_ctx* ctx, const wahgpu_term* terms, const uint32_
     B->bytes = bytes + 8ull * nq;
     B->min_bytes = min_bytes + 8ull * nq;
     B->groups = x0->groups; B->anb = x0->anb; B->ntiles = x0->ntiles;
+    B->general = general;
+    B->nrange = (uint32_t)dq.size();
+    B->nedges = (uint32_t)edge_q.size();
+    B->etiles = x0->ntiles;
+    // few items and dense terms only: smaller tiles, so that they spread
+    if (!general && (uint64_t)B->nrange * B->ntiles < 2ull * (uint64_t)ctx->sm_count) {
+        B->small = true;
+        B->ntiles = (B->groups + (B->anb ? 1 : 0) + RT_SMALL - 1) / RT_SMALL;
+    }
     B->d_idx = static_cast<DevIndex*>(wg_alloc(ctx, di.size() * sizeof(DevIndex)));
     B->d_terms = static_cast<DevTerm*>(wg_alloc(ctx, nt * sizeof(DevTerm)));
-    B->d_queries = static_cast<DevQuery*>(wg_alloc(ctx, nq * sizeof(DevQuery)));
+    B->d_queries = static_cast<DevQuery*>(wg_alloc(ctx, std::max<size_t>(dq.size(), 1) * sizeof(DevQuery)));
     B->d_counts = static_cast<unsigned long long*>(wg_alloc(ctx, nq * 8));
+    B->d_base = static_cast<unsigned char*>(wg_alloc(ctx, nq * 8 + edge_q.size() * 12));
     B->d_start = static_cast<unsigned long long*>(wg_alloc(ctx, nq * 8));
     B->d_status = static_cast<DevMeta*>(wg_alloc(ctx, sizeof(DevMeta)));
     B->rid_cap = rid_cap;
@@ -475,57 +535,97 @@ static int batch_create(wahgpu_ctx* ctx, const wahgpu_term* terms, const uint32_
     if (caps) {
         B->h_lim.assign(caps, caps + nq);
         B->h_base.resize(nq);
-        for (uint32_t q = 0; q < nq; ++q) B->h_base[q] = dq[q].rid_base;
+        for (uint32_t q = 1; q < nq; ++q) B->h_base[q] = B->h_base[q - 1] + caps[q - 1];
     }
     if (rid_cap) B->d_rids = static_cast<uint32_t*>(wg_alloc(ctx, rid_cap * 4));
     if (dense_first) B->d_dense = static_cast<uint32_t*>(wg_alloc(ctx, ((size_t)x0->groups + 1) * 4));
-    if (!B->d_idx || !B->d_terms || !B->d_queries || !B->d_counts || !B->d_start || !B->d_status ||
+    if (!B->d_idx || !B->d_terms || !B->d_queries || !B->d_counts || !B->d_base || !B->d_start || !B->d_status ||
         (rid_cap && !B->d_rids) || (dense_first && !B->d_dense)) {
         wahgpu_batch_free(B);
         return wg_fail(ctx, WAHGPU_ENOMEM, "batch allocation failed");
     }
     // the tables leave from pinned staging the batch keeps until it is
     // freed, so the host does not wait for the copies
-    const size_t bi = di.size() * sizeof(DevIndex), bt = (size_t)nt * sizeof(DevTerm), bq = (size_t)nq * sizeof(DevQuery);
-    B->h_stage = static_cast<unsigned char*>(wg_host_alloc(ctx, bi + bt + bq));
+    const size_t bi = di.size() * sizeof(DevIndex), bt = (size_t)nt * sizeof(DevTerm), bq = dq.size() * sizeof(DevQuery);
+    const size_t be = nq * 8ull, bd = edge_term.size() * 4, bg = edge_q.size() * 4;  // counts known beforehand, edges
+    B->h_stage = static_cast<unsigned char*>(wg_host_alloc(ctx, bi + bt + bq + be + bd + bg));
     if (!B->h_stage) {
         wahgpu_batch_free(B);
         return wg_fail(ctx, WAHGPU_ENOMEM, "batch staging allocation failed");
     }
     memcpy(B->h_stage, di.data(), bi);
     memcpy(B->h_stage + bi, dt.data(), bt);
-    memcpy(B->h_stage + bi + bt, dq.data(), bq);
+    if (bq) memcpy(B->h_stage + bi + bt, dq.data(), bq);
+    unsigned char* hb = B->h_stage + bi + bt + bq;
+    memcpy(hb, base.data(), be);
+    if (bd) { memcpy(hb + be, edge_term.data(), bd); memcpy(hb + be + bd, edge_q.data(), bg); }
     CUDA_TRY(ctx, cudaMemcpyAsync(B->d_idx, B->h_stage, bi, cudaMemcpyHostToDevice, ctx->stream));
     CUDA_TRY(ctx, cudaMemcpyAsync(B->d_terms, B->h_stage + bi, bt, cudaMemcpyHostToDevice, ctx->stream));
-    CUDA_TRY(ctx, cudaMemcpyAsync(B->d_queries, B->h_stage + bi + bt, bq, cudaMemcpyHostToDevice, ctx->stream));
+    if (bq) CUDA_TRY(ctx, cudaMemcpyAsync(B->d_queries, B->h_stage + bi + bt, bq, cudaMemcpyHostToDevice, ctx->stream));
+    CUDA_TRY(ctx, cudaMemcpyAsync(B->d_base, hb, be + bd + bg, cudaMemcpyHostToDevice, ctx->stream));
     *out = B;
     return WAHGPU_OK;
+}
+
+template <int Q, int MODE, bool GEN>
+static void launch_range(const wahgpu_ctx* ctx, const RangeArgs& a) {
+    static PerDeviceSetup setup;
+    constexpr size_t sm = range_smem(GEN, MODE >= RM_IDS);
+    const int per_sm = wg_kernel_setup(setup, ctx->device, k_range<Q, MODE, GEN>, RTHREADS, sm);
+    const uint32_t ctas = ctx->range_ctas ? std::min<uint32_t>(ctx->range_ctas, (uint32_t)per_sm) : (uint32_t)per_sm;
+    // the look-back takes a CTA per item
+    const uint32_t grid = MODE == RM_LOOK ? a.nitems : std::min<uint32_t>(a.nitems, ctas * (uint32_t)ctx->sm_count);
+    k_range<Q, MODE, GEN><<<grid, RTHREADS, sm, ctx->stream>>>(a);
+}
+template <int MODE>
+static void launch_range_mode(const wahgpu_batch* B, const RangeArgs& a) {
+    if (B->general) launch_range<RQUADS, MODE, true>(B->ctx, a);
+    else if (B->small) launch_range<1, MODE, false>(B->ctx, a);
+    else launch_range<RQUADS, MODE, false>(B->ctx, a);
 }
 
 extern "C" int wahgpu_batch_run(wahgpu_batch* B) {
     if (!B) return WAHGPU_EINVAL;
     wahgpu_ctx* ctx = B->ctx;
-    const uint32_t nitems = B->nq * B->ntiles;
-    if (nitems == 0) return WAHGPU_OK;
-    TileRec* recs; LaunchSync* sync;
-    int rc = wg_scratch(ctx, nitems, &recs, &sync);
-    if (rc) return rc;
-    CUDA_TRY(ctx, cudaMemsetAsync(B->d_counts, 0, B->nq * 8, ctx->stream));
+    if (B->etiles == 0) return WAHGPU_OK;
+    // the counts start from those known beforehand (0 for most queries)
+    CUDA_TRY(ctx, cudaMemcpyAsync(B->d_counts, B->d_base, B->nq * 8ull, cudaMemcpyDeviceToDevice, ctx->stream));
     CUDA_TRY(ctx, cudaMemsetAsync(B->d_status, 0, sizeof(DevMeta), ctx->stream));
+    if (B->nedges) {
+        EdgeArgs e;
+        e.idx = B->d_idx; e.terms = B->d_terms;
+        e.edges = reinterpret_cast<const uint2*>(B->d_base + B->nq * 8ull);
+        e.edge_q = reinterpret_cast<const uint32_t*>(B->d_base + B->nq * 8ull + B->nedges * 8ull);
+        e.nedges = B->nedges; e.ntiles = B->etiles; e.GX = B->groups + (B->anb ? 1u : 0u);
+        e.counts = B->d_counts;
+        static PerDeviceSetup setup;
+        const uint32_t per_sm = (uint32_t)wg_kernel_setup(setup, ctx->device, k_edge_counts, RTHREADS, 0);
+        const uint64_t ctas = ((uint64_t)B->nedges * B->etiles + RWARPS - 1) / RWARPS;
+        k_edge_counts<<<(uint32_t)std::min<uint64_t>(ctas, per_sm * (uint64_t)ctx->sm_count), RTHREADS, 0, ctx->stream>>>(e);
+        ctx->launches++;
+        CUDA_TRY(ctx, cudaGetLastError());
+    }
+    B->h_valid = false;
+    const uint32_t nitems = B->nrange * B->ntiles;
+    if (nitems == 0) return WAHGPU_OK;
     RangeArgs a;
-    a.idx = B->d_idx; a.terms = B->d_terms; a.queries = B->d_queries; a.nq = B->nq;
+    a.idx = B->d_idx; a.terms = B->d_terms; a.queries = B->d_queries; a.nq = B->nrange;
     a.groups = B->groups; a.anb = B->anb; a.ntiles = B->ntiles;
     a.counts = B->d_counts; a.rids = B->d_rids; a.rid_cap = B->rid_cap; a.rid_start = B->d_start;
     a.dense = B->d_dense;
-    a.recs = recs; a.sync = sync; a.nitems = nitems; a.status = B->d_status;
-    // tile by tile when only counts are wanted (orders 1 and 2); with row ids
-    // order 2 runs two tile-by-tile passes around a scan of the items' hits,
-    // order 1 (and a single query) goes query by query with the look-back
-    const bool ids = B->d_rids || B->d_dense;
-    const bool two_pass = ctx->range_order == 2 && ids && B->nq > 1;
-    a.tile_major = ((ctx->range_order != 0 && !ids) || two_pass) ? 1u : 0u;
-    a.pass = 0; a.item_cnt = nullptr; a.item_off = nullptr;
+    a.recs = nullptr; a.sync = nullptr; a.nitems = nitems; a.status = B->d_status;
+    a.gx = (B->groups + (B->anb ? 1u : 0u) + 3u) & ~3u;
+    a.item_cnt = nullptr; a.item_off = nullptr;
     a.capped = B->capped && B->d_rids ? 1u : 0u;
+    // Row ids: order 0 asks for the look-back, order 2 for two passes (of
+    // several queries); order 1 takes the look-back while every item has a
+    // CTA of its own at once.  Past that a CTA would sit waiting for the
+    // slowest of the items before its own: 1024 conjunctions over 10M rows,
+    // 256 ids each, took 7.7 ms so and take 3.6 ms in two passes.
+    const bool ids = B->d_rids || B->d_dense;
+    const bool two_pass = ids && ((ctx->range_order == 2 && B->nq > 1) ||
+                                  (ctx->range_order == 1 && nitems > 4u * (uint32_t)ctx->sm_count));
+    a.tile_major = ((ctx->range_order != 0 && !ids) || two_pass) ? 1u : 0u;
     if (two_pass) {
         if (!B->d_items) {
             B->d_items = static_cast<unsigned long long*>(wg_alloc(ctx, (size_t)nitems * 16));
@@ -539,22 +639,21 @@ extern "C" int wahgpu_batch_run(wahgpu_batch* B) {
             }
         }
         if (B->d_dense) CUDA_TRY(ctx, cudaMemsetAsync(B->d_dense, 0, ((size_t)B->groups + 1) * 4, ctx->stream));
-    }
-    static PerDeviceSetup setup;
-    const size_t sm = sizeof(RangeShared);
-    const int per_sm = wg_kernel_setup(setup, ctx->device, k_range, RTHREADS, sm);
-    const uint32_t ctas = ctx->range_ctas ? std::min<uint32_t>(ctx->range_ctas, (uint32_t)per_sm) : (uint32_t)per_sm;
-    const uint32_t grid = std::min<uint32_t>(nitems, ctas * (uint32_t)ctx->sm_count);
-    if (two_pass) {
-        a.pass = 1; a.item_cnt = B->d_items;
-        k_range<<<grid, RTHREADS, sm, ctx->stream>>>(a);
+        a.item_cnt = B->d_items;
+        launch_range_mode<RM_ITEMS>(B, a);
         CUDA_TRY(ctx, cudaGetLastError());
         CUDA_TRY(ctx, cub::DeviceScan::ExclusiveSum(B->d_scan_tmp, B->scan_tmp_bytes, B->d_items, B->d_items + nitems,
                                                     (int)nitems, ctx->stream));
-        a.pass = 2; a.item_off = B->d_items + nitems;
+        a.item_off = B->d_items + nitems;
+        launch_range_mode<RM_IDS>(B, a);
         ctx->launches += 2;  // the count pass and the scan
+    } else if (ids) {
+        int rc = wg_scratch(ctx, nitems, &a.recs, &a.sync);
+        if (rc) return rc;
+        launch_range_mode<RM_LOOK>(B, a);
+    } else {
+        launch_range_mode<RM_COUNT>(B, a);
     }
-    k_range<<<grid, RTHREADS, sm, ctx->stream>>>(a);
     ctx->launches++;
     CUDA_TRY(ctx, cudaGetLastError());
     B->h_valid = false;
@@ -637,7 +736,7 @@ extern "C" int wahgpu_batch_free(wahgpu_batch* B) {
     wahgpu_ctx* ctx = B->ctx;
     cudaStreamSynchronize(ctx->stream);
     wg_free(ctx, B->d_idx); wg_free(ctx, B->d_terms); wg_free(ctx, B->d_queries);
-    wg_free(ctx, B->d_counts); wg_free(ctx, B->d_start); wg_free(ctx, B->d_status);
+    wg_free(ctx, B->d_counts); wg_free(ctx, B->d_base); wg_free(ctx, B->d_start); wg_free(ctx, B->d_status);
     wg_free(ctx, B->d_rids); wg_free(ctx, B->d_dense);
     wg_free(ctx, B->d_items); wg_free(ctx, B->d_scan_tmp);
     wg_host_free(ctx, B->h_stage);

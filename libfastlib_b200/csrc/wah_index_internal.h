@@ -26,6 +26,7 @@ struct wahgpu_index {
     uint32_t* d_tl_bm = nullptr;
     uint32_t* d_cum = nullptr;        // cumulative dense rows (range spans in two reads)
     uint32_t cum_stride = 0, cum_k = 0;
+    bool disjoint = false;            // no row in two bitmaps (known with a cumulative row per bitmap)
     void* d_values = nullptr;
     uint32_t vtype = 0;
     wah::DevIndex dev{};
@@ -34,11 +35,18 @@ struct wahgpu_index {
 struct wahgpu_batch {
     wahgpu_ctx* ctx = nullptr;
     uint32_t nq = 0, nterms = 0, nidx = 0;
-    uint32_t groups = 0, anb = 0, ntiles = 0;
+    uint32_t groups = 0, anb = 0, ntiles = 0;  // tiles per query
+    bool general = false;             // some term is not dense
+    bool small = false;               // tiles of RT_SMALL groups
     wah::DevIndex* d_idx = nullptr;
     wah::DevTerm* d_terms = nullptr;
     wah::DevQuery* d_queries = nullptr;
     unsigned long long* d_counts = nullptr;
+    // one-term count queries over disjoint bitmaps: their wholly-inside 1
+    // bits (0 for the other queries), then the edges to count
+    unsigned char* d_base = nullptr;
+    uint32_t nrange = 0;              // queries k_range evaluates
+    uint32_t nedges = 0, etiles = 0;  // edges to count, RT tiles per column
     unsigned long long* d_start = nullptr;
     uint32_t* d_rids = nullptr;
     uint64_t rid_cap = 0;

@@ -15,20 +15,30 @@
 // OR order (a heap ordered by pointer values) changes only the words of its
 // intermediate results, never the bits.
 //
-// Work item = (query, tile of RT groups), claimed in query-major order
-// (row ids by a decoupled look-back in claim order, so each query's ids are
-// contiguous and ascending), tile-major order (the queries of a batch share
-// each tile's words in L2; counts only, or two passes around a scan of the
-// items' hits for row ids).  For each term, warp 0 stages the term and its
-// index in shared memory; a span covering whole blocks of the index's
-// cumulative rows starts as C(k1) & ~C(k0) read as 16-byte vectors, and the
-// remaining bitmaps (the edges of such a span, a short span, or the tile's
-// list of bitmaps holding a 1 bit in it) are OR'ed into a shared-memory
-// accumulator: a bitmap with a few words over the tile by one lane (32 such
-// bitmaps per warp at once), a longer one and each edge bin's row check by a
-// whole warp walking its words 128 at a time (positions by ballot / scan).  The
-// term result is AND'ed into the query result; a tile whose AND is empty
-// skips the query's remaining terms.
+// Work item = (query, tile of groups).  Every thread owns whole quads of
+// groups and keeps the query's AND over them in registers.
+//
+// Dense terms.  Where the index keeps a cumulative row per bitmap (stride 1),
+// a range's span is C(h1) & ~C(h0), two rows read as 16-byte vectors, and an
+// edge bin's bitmap is C(j+1) & ~C(j): its set rows' raw values are compared
+// right there.  No word is decoded, nothing is shared between threads and a
+// count needs no block barrier.
+//
+// Other terms (rows kept for every few bitmaps, or none): warp 0 stages the
+// term and its index in shared memory; a span covering whole blocks of the
+// cumulative rows starts as C(k1) & ~C(k0), and the remaining bitmaps (the
+// edges of such a span, a short span, or the tile's list of bitmaps holding a
+// 1 bit in it) are OR'ed into a shared-memory accumulator: a bitmap with a
+// few words over the tile by one lane (32 such bitmaps per warp at once), a
+// longer one and each edge bin's row check by a whole warp walking its words
+// 128 at a time (positions by ballot / scan).
+//
+// A query's dense terms go first; an empty AND skips the rest.
+//
+// Counts run tile by tile (the queries of a batch share a tile's rows and
+// words in L2), items dealt to the CTAs in turn.  Row ids take two such
+// passes around a scan of the items' hits, or, when the items are few, one
+// pass with a decoupled look-back in query order.
 #ifndef WAH_RANGE_CUH
 #define WAH_RANGE_CUH
 #include "wah_dev.cuh"
@@ -38,11 +48,13 @@ namespace wah {
 constexpr int RT = 4096;             // groups per tile
 constexpr int RTHREADS = 256;
 constexpr int RWARPS = RTHREADS / 32;
-constexpr int RGPT = RT / RTHREADS;  // groups per thread in the epilogue
 constexpr uint32_t RDIRECT = 32;     // spans of at most this many bitmaps skip the tile lists
 constexpr int RCHK = 2;              // raw values in flight per lane in an edge-bin row check
-// the row-id epilogue stages 16 groups' ids (<= 496) in each warp's RT / RWARPS words of S.tmp
-static_assert(RGPT * RTHREADS == RT && 16 * 31 <= RT / RWARPS, "row-id staging");
+constexpr int RQUADS = RT / 4 / RTHREADS;  // quads of groups per thread over an RT tile
+static_assert(RQUADS * 4 * RTHREADS == RT, "quads");
+// Tile of a batch of few items and dense terms only: a quad per thread, so
+// one query over a million rows spreads over 32 CTAs instead of 8.
+constexpr int RT_SMALL = 4 * RTHREADS;
 
 // per-bitmap metadata of an attached index
 struct BitmapMeta {
@@ -79,11 +91,14 @@ struct DevTerm {
     uint32_t ncand;       // edge bitmaps to check row by row (0..2)
     uint32_t cand[2];
     uint32_t lop, rop;    // lo lop x rop hi
+    uint32_t dense;       // the index keeps a row per bitmap: span C(c1) & ~C(c0) (c1 == 0: empty), edges by rows
+    const uint32_t* cum;  // dense: the index's rows
     double lo, hi;
 };
 
 struct DevQuery {
-    uint32_t t0, t1;      // terms [t0, t1)
+    uint32_t t0, t1;      // terms [t0, t1): dense ones up to td, then the others
+    uint32_t td, q;       // q: the query's place in the counts
     uint64_t rid_base;    // capped batches: the query's row-id region
     uint64_t rid_lim;     // capped batches: at most this many row ids (the first ones)
 };
@@ -103,17 +118,17 @@ struct RangeArgs {
     uint32_t* dense;          // dense hit words of query 0 (or null)
     TileRec* recs; LaunchSync* sync; uint32_t nitems;
     DevMeta* status;
-    uint32_t tile_major;      // 1: items ordered tile by tile (no look-back)
-    // two-pass order (tile by tile, row ids placed without a look-back):
-    // pass 1 writes each item's hits to item_cnt, the host scans them into
-    // item_off, pass 2 writes the row ids; items are indexed q*ntiles + k
-    uint32_t pass;            // 0 one pass, 1 counts, 2 row ids
+    uint32_t gx;              // words per cumulative row
+    uint32_t tile_major;      // 1: items ordered tile by tile, else query by query
+    // two passes: the first writes each item's hits to item_cnt, a scan turns
+    // them into item_off, the second writes the row ids; items are indexed
+    // q*ntiles + k
     unsigned long long* item_cnt;
     const unsigned long long* item_off;
     // 1: every query writes at most rid_lim row ids into its own region at
-    // rid_base (query-major order: offsets within the query by a segmented
-    // look-back; two-pass order: by the items' scan, pass 2 skipping the
-    // items whose ids lie past the limit)
+    // rid_base (one pass: offsets within the query by a segmented look-back;
+    // two: by the items' scan, the second skipping the items whose ids lie
+    // past the limit)
     uint32_t capped;
 };
 
@@ -128,15 +143,27 @@ struct SegSum64Comb {
     }
 };
 
-struct RangeShared {
-    uint32_t acc[RT];
-    uint32_t tmp[RT];
-    uint64_t scan[RWARPS + 1];
-    uint32_t hdr[8];
-    unsigned long long base;
-    DevTerm term;    // the term being evaluated and its index
-    DevIndex index;
+enum RangeMode : int {
+    RM_COUNT = 0,   // the queries' counts
+    RM_ITEMS = 1,   // two passes, first: counts per item too
+    RM_IDS = 2,     // two passes, second: row ids at the items' offsets
+    RM_LOOK = 3     // one pass: counts and row ids, offsets by a look-back
 };
+constexpr uint32_t RSTAGE = 32 * 31;  // row ids of 32 groups at most
+struct RangeShared {
+    uint32_t hdr[8];
+    uint64_t base;
+    uint32_t sums[2][RWARPS];
+    DevTerm term;    // the term being evaluated and its index (terms that are not dense)
+    DevIndex index;
+    // the accumulator of a term that is not dense (RT words), then the
+    // row-id staging (RWARPS * RSTAGE)
+    alignas(16) uint32_t tmp[1];
+};
+constexpr size_t range_smem(bool general, bool ids) {
+    return sizeof(RangeShared) + 4 * (size_t)(ids ? RWARPS * RSTAGE : general ? RT : 0);
+}
+static_assert(RT <= RWARPS * (int)RSTAGE, "the staging covers the accumulator");
 constexpr uint32_t TERM_WORDS = sizeof(DevTerm) / 4, INDEX_WORDS = sizeof(DevIndex) / 4;
 static_assert(sizeof(DevTerm) % 4 == 0 && TERM_WORDS <= 32, "a warp stages a term");
 static_assert(sizeof(DevIndex) % 4 == 0 && INDEX_WORDS <= 32, "a warp stages an index");
@@ -408,264 +435,480 @@ __device__ __forceinline__ uint32_t group16_lower_bound(const uint32_t* __restri
     return lo;
 }
 
-// Persistent: every CTA claims items until none is left.
-__global__ void __launch_bounds__(RTHREADS, 6) k_range(RangeArgs A) {
+// A general term over the tile [g0, g1) of RT groups, left in S.tmp (whole
+// CTA; ends with a block barrier).
+__device__ __forceinline__ void range_term(RangeShared& S, const RangeArgs& A, uint32_t t, uint32_t k, uint32_t g0,
+                                           uint32_t g1, uint32_t G, uint32_t anb, uint32_t lastmask) {
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const uint32_t ng = g1 - g0;
+    // the term and its index, staged in shared memory by warp 0
+    if (warp == 0) {
+        const uint32_t v = lane < TERM_WORDS ? __ldg(reinterpret_cast<const uint32_t*>(A.terms + t) + lane) : 0u;
+        const uint32_t ix = __shfl_sync(0xffffffffu, v, 0);  // DevTerm::index
+        if (lane < TERM_WORDS) reinterpret_cast<uint32_t*>(&S.term)[lane] = v;
+        if (lane < INDEX_WORDS)
+            reinterpret_cast<uint32_t*>(&S.index)[lane] = __ldg(reinterpret_cast<const uint32_t*>(A.idx + ix) + lane);
+    }
+    __syncthreads();
+    const DevTerm& T = S.term;
+    const DevIndex& I = S.index;
+    uint4* t4 = reinterpret_cast<uint4*>(S.tmp);
+    if (T.c1) {
+        // the wholly-inside span from two cumulative rows
+        // (16-byte slices: g0 is a multiple of RT and the rows'
+        // padding past the last group is zero)
+        const uint4* hi = reinterpret_cast<const uint4*>(I.cum + (size_t)(T.c1 - 1u) * I.gx + g0);
+        const uint4* lo = reinterpret_cast<const uint4*>(T.c0 ? I.cum + (size_t)(T.c0 - 1u) * I.gx + g0 : I.cum);
+        const uint32_t n4 = (ng + 3u) >> 2;
+        const bool two = T.c0 != 0u;
+#pragma unroll
+        for (uint32_t l = tid; l < RT / 4; l += RTHREADS) {
+            uint4 v = make_uint4(0u, 0u, 0u, 0u);
+            if (l < n4) {
+                const uint4 a = __ldg(hi + l);
+                const uint4 b = two ? __ldg(lo + l) : v;
+                v = make_uint4(a.x & ~b.x, a.y & ~b.y, a.z & ~b.z, a.w & ~b.w);
+            }
+            t4[rsw4(l)] = v;
+        }
+    } else {
+#pragma unroll
+        for (uint32_t l = tid; l < RT / 4; l += RTHREADS) t4[l] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    // the bitmaps to OR, as two ranges: with cumulative rows the
+    // edge spans [h0, e0) and [e1, h1), else the span [h0, h1) or
+    // the complement [0, h0) and [h1, nobs).  Ranges of at most
+    // RDIRECT bitmaps in all are walked directly (one that misses
+    // the tile costs its tile-index lookup); wider ones take the
+    // entries of the tile's list of bitmaps holding a 1 bit in it
+    // that fall in the ranges (lower bounds by 16-lane searches)
+    const bool flip = T.flip != 0u;
+    uint32_t ra0, ra1, rb0, rb1;  // bitmap ids [ra0, ra1) u [rb0, rb1)
+    if (T.c1) { ra0 = T.h0; ra1 = T.e0; rb0 = T.e1; rb1 = T.h1; }
+    else if (flip) { ra0 = 0u; ra1 = T.h0; rb0 = T.h1; rb1 = I.nobs; }
+    else { ra0 = T.h0; ra1 = T.h1; rb0 = rb1 = T.h1; }
+    const bool direct = !flip && (ra1 - ra0) + (rb1 - rb0) <= RDIRECT;
+    if (!direct && warp < 2) {
+        const uint32_t o0 = __ldg(I.tl_off + k), o1 = __ldg(I.tl_off + k + 1);
+        const uint32_t gbase = lane & 16u;
+        const uint32_t v = warp == 0 ? (gbase ? ra1 : ra0) : (gbase ? rb1 : rb0);
+        const uint32_t r = group16_lower_bound(I.tl_bm + o0, o1 - o0, v, gbase, lane & 15u);
+        if ((lane & 15u) == 0) S.hdr[2 + 2 * warp + (gbase >> 4)] = o0 + r;
+    }
+    __syncthreads();
+    // one job list per term: the edge bitmaps' row checks first
+    // (the longest jobs), then the bitmaps to OR; a complement is
+    // flipped before the checked rows join it
+    const uint32_t nc = flip ? 0u : T.ncand;
+    uint32_t sa = ra0, sb = rb0, na = ra1 - ra0, nb = rb1 - rb0;  // the two ranges' starts and sizes
+    if (!direct) {  // as entries of the tile list
+        sa = S.hdr[2]; na = S.hdr[3] - sa;
+        sb = S.hdr[4]; nb = S.hdr[5] - sb;
+    }
+    const uint32_t nsel = na + nb;
+    // row checks (the longest jobs) one per warp from warp 0; the
+    // bitmaps to OR in batches of up to 32 per warp (one per lane),
+    // spread over the warps from the one after the checks, so the
+    // warps holding a check get an OR batch last
+    for (uint32_t c = warp; c < nc; c += RWARPS) warp_check_bitmap(S, I, T.cand[c], k, g0, g1, T);
+    const uint32_t nfree = RWARPS - min(nc, (uint32_t)RWARPS - 1u);  // warps without a check
+    const uint32_t per = min(32u, (nsel + nfree - 1) / nfree);
+    const uint32_t wr = (warp + RWARPS - nc % RWARPS) % RWARPS;      // the warp's place in the OR order
+    for (uint32_t j0 = wr * per; j0 < nsel; j0 += RWARPS * per) {
+        const uint32_t jj = j0 + lane;
+        const bool have = lane < per && jj < nsel;
+        uint32_t b = 0;
+        if (have) {
+            const uint32_t e = jj < na ? sa + jj : sb + (jj - na);
+            b = direct ? e : __ldg(I.tl_bm + e);
+        }
+        lanes_or_bitmaps(S, I, have, b, k, g0, g1, G, anb);
+    }
+    if (flip) {
+        __syncthreads();
+        for (uint32_t l = tid; l < ng; l += RTHREADS) {
+            const uint32_t msk = (g0 + l == G && anb > 0) ? lastmask : ALLONES;
+            S.tmp[rsw(l)] ^= msk;
+        }
+        __syncthreads();
+        // edge bitmaps: rows checked against the raw values
+        for (uint32_t c = warp; c < T.ncand; c += RWARPS)
+            warp_check_bitmap(S, I, T.cand[c], k, g0, g1, T);
+    }
+    __syncthreads();
+}
+
+__device__ __forceinline__ uint4 andn4(uint4 a, uint4 b) { return make_uint4(a.x & ~b.x, a.y & ~b.y, a.z & ~b.z, a.w & ~b.w); }
+__device__ __forceinline__ uint4 and4(uint4 a, uint4 b) { return make_uint4(a.x & b.x, a.y & b.y, a.z & b.z, a.w & b.w); }
+__device__ __forceinline__ uint4 or4(uint4 a, uint4 b) { return make_uint4(a.x | b.x, a.y | b.y, a.z | b.z, a.w | b.w); }
+__device__ __forceinline__ bool any4(uint4 a) { return (a.x | a.y | a.z | a.w) != 0u; }
+
+// The set rows of a quad's edge bits whose raw values pass the term (groups
+// g .. g + 3).  Edge bits are few and scattered (a bin of 1000 holds one row
+// in 32 groups), so a lane takes one row at a time, whichever group it is in:
+// the warp runs as long as its fullest lane.
+__device__ __forceinline__ uint4 check_quad(uint4 e, uint32_t g, const uint32_t* __restrict__ raw, uint32_t vtype,
+                                            const DevTerm& T) {
+    uint4 r = make_uint4(0u, 0u, 0u, 0u);
+    while (any4(e)) {
+        const uint32_t j = e.x ? 0u : e.y ? 1u : e.z ? 2u : 3u;
+        const uint32_t b = e.x ? e.x : e.y ? e.y : e.z ? e.z : e.w;
+        const uint32_t hb = 31u - __clz(b), bit = 1u << hb;  // highest set bit
+        const uint32_t v = __ldg(raw + (g + j) * 31u + (30u - hb));
+        const uint32_t keep = pass_cmp(raw_value(v, vtype), T.lop, T.lo, T.rop, T.hi) ? bit : 0u;
+        if (j == 0u) { e.x ^= bit; r.x |= keep; }
+        else if (j == 1u) { e.y ^= bit; r.y |= keep; }
+        else if (j == 2u) { e.z ^= bit; r.z |= keep; }
+        else { e.w ^= bit; r.w |= keep; }
+    }
+    return r;
+}
+// Q quads of groups per thread: tiles of 4 * Q * RTHREADS groups.  GEN: the
+// batch holds terms that are not dense (tiles of RT groups).  Dense terms are
+// bound by the rows' loads (16 KB per row and tile, shared in L2) and the
+// edge rows' gathers, the others by the block barriers between their steps.
+// One range over 1M rows of 100 values with its row ids: 17 us on 32 CTAs,
+// 93 us when 8 CTAs walked the edge bitmaps' words; 1024 conjunctions over
+// 10M rows: 3.6 ms against 7.7 ms.
+template <int Q, int MODE, bool GEN>
+__global__ void __launch_bounds__(RTHREADS, MODE >= RM_IDS || GEN ? 3 : 4) k_range(RangeArgs A) {
+    static_assert(!GEN || Q == RQUADS, "the tile index is over RT groups");
+    constexpr uint32_t TG = 4u * Q * RTHREADS;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     RangeShared& S = *reinterpret_cast<RangeShared*>(smem_raw);
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    if (tid == 0) S.hdr[1] = ld_cg(&A.sync->epoch);
     const uint32_t G = A.groups, anb = A.anb;
     const uint32_t GX = G + (anb > 0 ? 1u : 0u);  // groups incl. the active one
     const uint32_t lastmask = anb > 0 ? (((1u << anb) - 1u) << (31u - anb)) : ALLONES;
-    // tile-major items are claimed one item ahead, so the ticket's round
-    // trip overlaps the current item (not with the look-back: an item held
-    // back behind a long one would stall every later item waiting on it)
-    const bool ahead = A.tile_major != 0u;
-    uint32_t next = 0;
-    if (tid == 0 && ahead) next = claim_tile(A.sync);
-    while (true) {
-        if (tid == 0) {
-            if (ahead) {
-                S.hdr[0] = next;
-                if (next < A.nitems) next = claim_tile(A.sync);
-            } else {
-                S.hdr[0] = claim_tile(A.sync);
-            }
-        }
+    uint32_t first = blockIdx.x, epoch = 0;
+    if (MODE == RM_LOOK) {
+        // items in claim order: an item's predecessors are running or done
+        if (tid == 0) { S.hdr[0] = claim_tile(A.sync); S.hdr[1] = ld_cg(&A.sync->epoch); }
         __syncthreads();
-        const uint32_t item = S.hdr[0], epoch = S.hdr[1];
-        if (item >= A.nitems) break;
-        // query-major items keep a query's row ids contiguous (look-back in
-        // claim order); tile-major items let the queries of one batch share
-        // each tile's bitmap words in L2
+        first = S.hdr[0];
+        epoch = S.hdr[1];
+    }
+    uint32_t par = 0;
+    for (uint32_t item = first; item < A.nitems; item += MODE == RM_LOOK ? A.nitems : gridDim.x) {
         const uint32_t q = A.tile_major ? item % A.nq : item / A.ntiles;
         const uint32_t k = A.tile_major ? item / A.nq : item % A.ntiles;
-        const uint32_t g0 = k * (uint32_t)RT, g1 = min(g0 + (uint32_t)RT, GX);
+        const uint32_t g0 = k * TG, g1 = min(g0 + TG, GX);
         const uint32_t ng = g1 > g0 ? g1 - g0 : 0u;
-        const uint32_t qi = q * A.ntiles + k;  // the item's place in query-major order
-        const DevQuery Q = A.queries[q];
-        if (A.pass == 2u) {
-            // row ids of the two-pass order: items without hits are done, and
-            // so (capped) are items whose ids all lie past the query's limit
-            // (offsets within the query: the scan runs in query-major order)
-            if (tid == 0 && k == 0) A.rid_start[q] = A.capped ? Q.rid_base : A.item_off[qi];
-            const bool past = A.capped && A.item_off[qi] - A.item_off[q * A.ntiles] >= Q.rid_lim;
-            if (A.item_cnt[qi] == 0ull || past) { __syncthreads(); continue; }
+        const uint32_t qi = q * A.ntiles + k;  // the item's place in query order
+        const DevQuery DQ = A.queries[q];
+        if (MODE == RM_IDS) {
+            // items without hits are done, and so (capped) are items whose
+            // ids all lie past the query's limit
+            if (tid == 0 && k == 0) A.rid_start[q] = A.capped ? DQ.rid_base : A.item_off[qi];
+            if (A.item_cnt[qi] == 0ull || (A.capped && A.item_off[qi] - A.item_off[q * A.ntiles] >= DQ.rid_lim)) continue;
         }
-
-        for (uint32_t l = tid; l < RT; l += RTHREADS) S.acc[l] = ALLONES;
-        for (uint32_t t = Q.t0; t < Q.t1; ++t) {
-            // the term and its index, staged in shared memory by warp 0
-            if (warp == 0) {
-                const uint32_t v = lane < TERM_WORDS ? __ldg(reinterpret_cast<const uint32_t*>(A.terms + t) + lane) : 0u;
-                const uint32_t ix = __shfl_sync(0xffffffffu, v, 0);  // DevTerm::index
-                if (lane < TERM_WORDS) reinterpret_cast<uint32_t*>(&S.term)[lane] = v;
-                if (lane < INDEX_WORDS)
-                    reinterpret_cast<uint32_t*>(&S.index)[lane] = __ldg(reinterpret_cast<const uint32_t*>(A.idx + ix) + lane);
-            }
-            __syncthreads();
-            const DevTerm& T = S.term;
-            const DevIndex& I = S.index;
-            uint4* t4 = reinterpret_cast<uint4*>(S.tmp);
-            if (T.c1) {
-                // the wholly-inside span from two cumulative rows
-                // (16-byte slices: g0 is a multiple of RT and the rows'
-                // padding past the last group is zero)
-                const uint4* hi = reinterpret_cast<const uint4*>(I.cum + (size_t)(T.c1 - 1u) * I.gx + g0);
-                const uint4* lo = reinterpret_cast<const uint4*>(T.c0 ? I.cum + (size_t)(T.c0 - 1u) * I.gx + g0 : I.cum);
-                const uint32_t n4 = (ng + 3u) >> 2;
-                const bool two = T.c0 != 0u;
+        // the thread's quads: 32 Q consecutive ones per warp, neighbouring lanes on neighbouring quads
+        const uint32_t ql = warp * (32u * Q) + lane;  // + 32 i
+        uint4 acc[Q];
 #pragma unroll
-                for (uint32_t l = tid; l < RT / 4; l += RTHREADS) {
-                    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-                    if (l < n4) {
-                        const uint4 a = __ldg(hi + l);
-                        const uint4 b = two ? __ldg(lo + l) : v;
-                        v = make_uint4(a.x & ~b.x, a.y & ~b.y, a.z & ~b.z, a.w & ~b.w);
-                    }
-                    t4[rsw4(l)] = v;
+        for (int i = 0; i < Q; ++i) {
+            acc[i] = make_uint4(ALLONES, ALLONES, ALLONES, ALLONES);
+            const uint32_t l = 4u * (ql + 32u * i);
+            if (l + 4u > ng || (anb > 0 && g0 + l + 4u > G)) {  // the column's end
+                uint32_t m[4];
+#pragma unroll
+                for (uint32_t e = 0; e < 4u; ++e) m[e] = l + e >= ng ? 0u : (g0 + l + e == G ? lastmask : ALLONES);
+                acc[i] = make_uint4(m[0], m[1], m[2], m[3]);
+            }
+        }
+        bool live = true;  // the AND is not empty (dense terms: the warp's part of it)
+        for (uint32_t t = DQ.t0; t < DQ.td && live; ++t) {
+            const DevTerm& T = A.terms[t];
+            const uint32_t c0 = T.c0, c1 = T.c1, nc = T.ncand;
+            // rows are GX words rounded up to 4 and the quads past them masked
+            const uint4* cum = reinterpret_cast<const uint4*>(T.cum) + (g0 >> 2);
+            const uint32_t gx4 = A.gx >> 2, n4 = gx4 - (g0 >> 2);  // quads of a row from g0 on
+            const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+            const uint4* hi = cum + (size_t)(c1 - 1u) * gx4 + ql;
+            const uint4* lo = cum + (size_t)(c0 - 1u) * gx4 + ql;
+            bool any = false;
+            if (nc == 0u) {
+                uint4 v[Q];
+#pragma unroll
+                for (int i = 0; i < Q; ++i) {
+                    const bool in = ql + 32u * i < n4;
+                    v[i] = in && c1 ? __ldg(hi + 32 * i) : zero;
+                    if (in && c0) v[i] = andn4(v[i], __ldg(lo + 32 * i));
+                }
+#pragma unroll
+                for (int i = 0; i < Q; ++i) {
+                    acc[i] = and4(acc[i], v[i]);
+                    any |= any4(acc[i]);
                 }
             } else {
+                const DevIndex& I = A.idx[T.index];
+                const uint32_t* raw = reinterpret_cast<const uint32_t*>(I.values);
+                const uint32_t vtype = I.vtype;
+                // the edge bitmaps' rows; one edge: the same twice
+                const uint32_t j0 = T.cand[0], j1 = nc > 1u ? T.cand[1] : j0;
+                const uint4* h0 = cum + (size_t)j0 * gx4 + ql;
+                const uint4* h1 = cum + (size_t)j1 * gx4 + ql;
 #pragma unroll
-                for (uint32_t l = tid; l < RT / 4; l += RTHREADS) t4[l] = make_uint4(0u, 0u, 0u, 0u);
-            }
-            // the bitmaps to OR, as two ranges: with cumulative rows the
-            // edge spans [h0, e0) and [e1, h1), else the span [h0, h1) or
-            // the complement [0, h0) and [h1, nobs).  Ranges of at most
-            // RDIRECT bitmaps in all are walked directly (one that misses
-            // the tile costs its tile-index lookup); wider ones take the
-            // entries of the tile's list of bitmaps holding a 1 bit in it
-            // that fall in the ranges (lower bounds by 16-lane searches)
-            const bool flip = T.flip != 0u;
-            uint32_t ra0, ra1, rb0, rb1;  // bitmap ids [ra0, ra1) u [rb0, rb1)
-            if (T.c1) { ra0 = T.h0; ra1 = T.e0; rb0 = T.e1; rb1 = T.h1; }
-            else if (flip) { ra0 = 0u; ra1 = T.h0; rb0 = T.h1; rb1 = I.nobs; }
-            else { ra0 = T.h0; ra1 = T.h1; rb0 = rb1 = T.h1; }
-            const bool direct = !flip && (ra1 - ra0) + (rb1 - rb0) <= RDIRECT;
-            if (!direct && warp < 2) {
-                const uint32_t o0 = __ldg(I.tl_off + k), o1 = __ldg(I.tl_off + k + 1);
-                const uint32_t gbase = lane & 16u;
-                const uint32_t v = warp == 0 ? (gbase ? ra1 : ra0) : (gbase ? rb1 : rb0);
-                const uint32_t r = group16_lower_bound(I.tl_bm + o0, o1 - o0, v, gbase, lane & 15u);
-                if ((lane & 15u) == 0) S.hdr[2 + 2 * warp + (gbase >> 4)] = o0 + r;
-            }
-            __syncthreads();
-            // one job list per term: the edge bitmaps' row checks first
-            // (the longest jobs), then the bitmaps to OR; a complement is
-            // flipped before the checked rows join it
-            const uint32_t nc = flip ? 0u : T.ncand;
-            uint32_t sa = ra0, sb = rb0, na = ra1 - ra0, nb = rb1 - rb0;  // the two ranges' starts and sizes
-            if (!direct) {  // as entries of the tile list
-                sa = S.hdr[2]; na = S.hdr[3] - sa;
-                sb = S.hdr[4]; nb = S.hdr[5] - sb;
-            }
-            const uint32_t nsel = na + nb;
-            // row checks (the longest jobs) one per warp from warp 0; the
-            // bitmaps to OR in batches of up to 32 per warp (one per lane),
-            // spread over the warps from the one after the checks, so the
-            // warps holding a check get an OR batch last
-            for (uint32_t c = warp; c < nc; c += RWARPS) warp_check_bitmap(S, I, T.cand[c], k, g0, g1, T);
-            const uint32_t nfree = RWARPS - min(nc, (uint32_t)RWARPS - 1u);  // warps without a check
-            const uint32_t per = min(32u, (nsel + nfree - 1) / nfree);
-            const uint32_t wr = (warp + RWARPS - nc % RWARPS) % RWARPS;      // the warp's place in the OR order
-            for (uint32_t j0 = wr * per; j0 < nsel; j0 += RWARPS * per) {
-                const uint32_t jj = j0 + lane;
-                const bool have = lane < per && jj < nsel;
-                uint32_t b = 0;
-                if (have) {
-                    const uint32_t e = jj < na ? sa + jj : sb + (jj - na);
-                    b = direct ? e : __ldg(I.tl_bm + e);
+                for (int i = 0; i < Q; ++i) {
+                    if (ql + 32u * i >= n4) { acc[i] = zero; continue; }
+                    uint4 v = c1 ? __ldg(hi + 32 * i) : zero;
+                    uint4 e = __ldg(h0 + 32 * i), f = __ldg(h1 + 32 * i);
+                    if (c0) v = andn4(v, __ldg(lo + 32 * i));
+                    if (j0) e = andn4(e, __ldg(h0 + 32 * i - gx4));
+                    if (j1) f = andn4(f, __ldg(h1 + 32 * i - gx4));
+                    e = and4(or4(e, f), acc[i]);  // only the rows still in the AND
+                    if (any4(e)) v = or4(v, check_quad(e, g0 + 4u * (ql + 32u * i), raw, vtype, T));
+                    acc[i] = and4(acc[i], v);
+                    any |= any4(acc[i]);
                 }
-                lanes_or_bitmaps(S, I, have, b, k, g0, g1, G, anb);
             }
-            if (flip) {
-                __syncthreads();
-                for (uint32_t l = tid; l < ng; l += RTHREADS) {
-                    const uint32_t msk = (g0 + l == G && anb > 0) ? lastmask : ALLONES;
-                    S.tmp[rsw(l)] ^= msk;
+            live = __any_sync(0xffffffffu, any);
+        }
+        if (GEN && DQ.td < DQ.t1) {
+            bool on = DQ.td == DQ.t0 || __syncthreads_or(live);
+            for (uint32_t t = DQ.td; t < DQ.t1 && on; ++t) {
+                range_term(S, A, t, k, g0, g1, G, anb, lastmask);
+                bool any = false;
+#pragma unroll
+                for (int i = 0; i < Q; ++i) {
+                    const uint4 v = reinterpret_cast<const uint4*>(S.tmp)[rsw4(ql + 32u * i)];
+                    acc[i] = and4(acc[i], v);
+                    any |= any4(acc[i]);
                 }
-                __syncthreads();
-                // edge bitmaps: rows checked against the raw values
-                for (uint32_t c = warp; c < T.ncand; c += RWARPS)
-                    warp_check_bitmap(S, I, T.cand[c], k, g0, g1, T);
+                // an empty AND ends the query's work on this tile (and S.tmp is read)
+                on = __syncthreads_or(any);
             }
-            __syncthreads();
-            uint32_t any = 0;
-            for (uint32_t l = tid; l < RT; l += RTHREADS) { const uint32_t v = S.acc[l] & S.tmp[l]; S.acc[l] = v; any |= v; }
-            // an empty AND ends the query's work on this tile
-            if (!__syncthreads_or(any != 0u)) break;
         }
         // ---- counts and row ids
-        const uint32_t l0 = tid * RGPT;
         uint32_t cnt = 0;
 #pragma unroll
-        for (int j = 0; j < RGPT; ++j) {
-            const uint32_t l = l0 + j;
-            if (l < ng) {
-                uint32_t v = S.acc[rsw(l)];
-                if (g0 + l == G && anb > 0) v &= lastmask;
-                S.acc[rsw(l)] = v;
-                cnt += __popc(v);
-            } else if (l < RT) {
-                S.acc[rsw(l)] = 0u;
-            }
+        for (int i = 0; i < Q; ++i) cnt += __popc(acc[i].x) + __popc(acc[i].y) + __popc(acc[i].z) + __popc(acc[i].w);
+        cnt = __reduce_add_sync(0xffffffffu, cnt);  // the warp's hits
+        if (MODE == RM_COUNT) {
+            if (lane == 0 && cnt) atomicAdd(&A.counts[DQ.q], (unsigned long long)cnt);
+            continue;
         }
-        if (A.tile_major && A.pass == 1u) {
-            uint64_t total;
-            block_exscan64(cnt, S.scan, total);
+        if (lane == 0) S.sums[par][warp] = cnt;
+        __syncthreads();
+        uint32_t before = 0, total = 0;
+#pragma unroll
+        for (uint32_t w = 0; w < (uint32_t)RWARPS; ++w) {
+            const uint32_t c = S.sums[par][w];
+            total += c;
+            before += w < warp ? c : 0u;
+        }
+        par ^= 1u;
+        if (MODE == RM_ITEMS) {
             if (tid == 0) {
                 A.item_cnt[qi] = total;
                 if (total) atomicAdd(&A.counts[q], (unsigned long long)total);
             }
-            __syncthreads();
             continue;
         }
-        if (A.tile_major && A.pass == 0u) {
-            cnt = __reduce_add_sync(0xffffffffu, cnt);
-            if (lane == 0 && cnt) atomicAdd(&A.counts[q], (unsigned long long)cnt);
+        uint64_t base;
+        if (MODE == RM_IDS) {
+            base = A.capped ? A.item_off[qi] - A.item_off[q * A.ntiles] : A.item_off[qi];
+        } else {
+            if (warp == 0 && A.capped) {
+                // the row ids before this tile within its own query
+                const uint4 mine = make_uint4(total, 0u, 0u, k == 0 ? 1u : 0u);
+                uint4 pre = make_uint4(0u, 0u, 0u, 0u);
+                bool ok = true;
+                if (item == 0) {
+                    if (lane == 0) publish(&A.recs[0], epoch, REC_INCL, mine);
+                } else {
+                    if (lane == 0) publish(&A.recs[item], epoch, REC_AGG, mine);
+                    pre = warp_lookback(A.recs, item, epoch, make_uint4(0u, 0u, 0u, 0u), SegSum64Comb(), &ok);
+                    if (lane == 0) publish(&A.recs[item], epoch, REC_INCL, SegSum64Comb()(pre, mine));
+                }
+                if (lane == 0) {
+                    if (!ok) atomicExch(&A.status->status, DEV_ERR_TIMEOUT);
+                    S.base = k == 0 ? 0ull : ((uint64_t)pre.y << 32 | pre.x);
+                    if (total) atomicAdd(&A.counts[q], (unsigned long long)total);
+                    if (k == 0) A.rid_start[q] = DQ.rid_base;
+                }
+            } else if (warp == 0) {
+                uint64_t prefix; uint32_t pa, pb;
+                const bool ok = lookback64(A.recs, item, epoch, total, 0, 0, prefix, pa, pb);
+                if (lane == 0) {
+                    if (!ok) atomicExch(&A.status->status, DEV_ERR_TIMEOUT);
+                    S.base = prefix;
+                    if (total) atomicAdd(&A.counts[q], (unsigned long long)total);
+                    if (k == 0) A.rid_start[q] = prefix;
+                }
+            }
             __syncthreads();
-            continue;
+            base = S.base;
         }
-        uint64_t total;
-        const uint64_t ex = block_exscan64(cnt, S.scan, total);
-        if (A.pass == 2u) {
-            if (tid == 0) S.base = A.capped ? A.item_off[qi] - A.item_off[q * A.ntiles] : A.item_off[qi];
-        } else if (warp == 0 && A.capped) {
-            // the row ids before this tile within its own query
-            const uint4 mine = make_uint4((uint32_t)total, (uint32_t)(total >> 32), 0u, k == 0 ? 1u : 0u);
-            uint4 pre = make_uint4(0u, 0u, 0u, 0u);
-            bool ok = true;
-            if (item == 0) {
-                if (lane == 0) publish(&A.recs[0], epoch, REC_INCL, mine);
-            } else {
-                if (lane == 0) publish(&A.recs[item], epoch, REC_AGG, mine);
-                pre = warp_lookback(A.recs, item, epoch, make_uint4(0u, 0u, 0u, 0u), SegSum64Comb(), &ok);
-                if (lane == 0) publish(&A.recs[item], epoch, REC_INCL, SegSum64Comb()(pre, mine));
-            }
-            if (lane == 0) {
-                if (!ok) atomicExch(&A.status->status, DEV_ERR_TIMEOUT);
-                S.base = k == 0 ? 0ull : ((uint64_t)pre.y << 32 | pre.x);
-                if (total) atomicAdd(&A.counts[q], (unsigned long long)total);
-                if (k == 0) A.rid_start[q] = Q.rid_base;
-            }
-        } else if (warp == 0) {
-            uint64_t prefix; uint32_t pa, pb;
-            const bool ok = lookback64(A.recs, item, epoch, total, 0, 0, prefix, pa, pb);
-            if (lane == 0) {
-                if (!ok) atomicExch(&A.status->status, DEV_ERR_TIMEOUT);
-                S.base = prefix;
-                if (total) atomicAdd(&A.counts[q], (unsigned long long)total);
-                if (k == 0) A.rid_start[q] = prefix;
-            }
-        }
-        __syncthreads();
-        if (A.rids) {
+        if (A.rids && cnt) {
             // capped: offsets are within the query; ids past its limit are
             // dropped and the rest land in its region
-            const uint64_t lim = A.capped ? Q.rid_lim : A.rid_cap;
-            const uint64_t rbase0 = A.capped ? Q.rid_base : 0ull;
-            // each warp owns RGPT * 32 consecutive groups (its threads' in
-            // the count above) and writes their ids 16 groups at a time:
-            // lanes 0-15 expand a group each into the warp's part of S.tmp
-            // (free once the terms are done), then the warp stores the run
-            // of ids with consecutive lanes on consecutive slots
-            constexpr uint32_t WG = RGPT * 32;      // groups per warp
-            uint32_t* st = S.tmp + warp * WG;       // <= 16 * 31 ids per round
-            uint64_t off = S.base + __shfl_sync(0xffffffffu, ex, 0);
-            for (uint32_t r = 0; r < WG / 16u && off < lim; ++r) {
-                const uint32_t l = warp * WG + r * 16u + (lane & 15u);
-                uint32_t bits = (lane < 16u && l < ng) ? S.acc[rsw(l)] : 0u;
-                const uint32_t c = __popc(bits);
+            const uint64_t lim = A.capped ? DQ.rid_lim : A.rid_cap;
+            const uint64_t rbase0 = A.capped ? DQ.rid_base : 0ull;
+            // 32 groups at a time: lane l takes group 32 r + l from the lane
+            // owning its quad and expands it into the warp's staging, then
+            // the warp stores the run of ids with neighbouring lanes on
+            // neighbouring slots
+            uint32_t* st = S.tmp + warp * RSTAGE;
+            uint64_t off = base + before;
+#pragma unroll
+            for (int i = 0; i < Q; ++i) {
+                if (!__any_sync(0xffffffffu, any4(acc[i]))) continue;
+#pragma unroll 1
+                for (uint32_t r = 0; r < 4u && off < lim; ++r) {
+                    const uint32_t src = 8u * r + (lane >> 2);
+                    const uint32_t x = __shfl_sync(0xffffffffu, acc[i].x, src), y = __shfl_sync(0xffffffffu, acc[i].y, src);
+                    const uint32_t z = __shfl_sync(0xffffffffu, acc[i].z, src), w = __shfl_sync(0xffffffffu, acc[i].w, src);
+                    uint32_t bits = lane & 2u ? (lane & 1u ? w : z) : (lane & 1u ? y : x);
+                    const uint32_t c = __popc(bits);
+                    uint32_t s = c;
+#pragma unroll
+                    for (int d = 1; d < 32; d <<= 1) {
+                        const uint32_t u = __shfl_up_sync(0xffffffffu, s, d);
+                        if (lane >= (uint32_t)d) s += u;
+                    }
+                    const uint32_t rt = __shfl_sync(0xffffffffu, s, 31);
+                    uint32_t p = s - c;
+                    const uint32_t row = (g0 + 4u * (warp * (32u * Q) + 32u * i + 8u * r) + lane) * 31u;
+                    while (bits) {
+                        const uint32_t hb = 31u - __clz(bits);
+                        st[p++] = row + (30u - hb);
+                        bits &= ~(1u << hb);
+                    }
+                    __syncwarp();
+                    for (uint32_t j = lane; j < rt; j += 32u) {
+                        const uint64_t o = off + j;
+                        if (o < lim && rbase0 + o < A.rid_cap) A.rids[rbase0 + o] = st[j];
+                    }
+                    __syncwarp();
+                    off += rt;
+                }
+            }
+        }
+        if (A.dense && q == 0) {
+#pragma unroll
+            for (int i = 0; i < Q; ++i) {
+                const uint32_t l = 4u * (ql + 32u * i);
+                const uint32_t v[4] = {acc[i].x, acc[i].y, acc[i].z, acc[i].w};
+#pragma unroll
+                for (uint32_t e = 0; e < 4u; ++e)
+                    if (l + e < ng) A.dense[g0 + l + e] = v[e];
+            }
+        }
+        // the staging is free before the next item's terms use it
+        if (GEN) __syncthreads();
+    }
+    if (MODE == RM_LOOK) {
+        __syncthreads();
+        if (tid == 0) finish_tile(A.sync, gridDim.x);
+    }
+}
+
+// Counts of one-term queries over disjoint bitmaps: the host has added up
+// the wholly-inside bitmaps' 1 bits; what is left are the edge bins' rows that
+// pass the comparison.  A warp per (edge, tile of RT groups), tile by tile so
+// that the queries share a tile's raw values in L2: the bin's words of the
+// tile 128 at a time, the first set row of every literal loaded before any is
+// compared (few literals of an edge bin hold more).  Bound by those loads'
+// latency.  1000 ranges over 10M rows, 1000 bins: 0.18 ms; 1.1 ms reading the
+// spans and the edges from the cumulative rows, 1.9 ms from a row per 8
+// bitmaps and the other bitmaps' words.
+struct EdgeArgs {
+    const DevIndex* idx;
+    const DevTerm* terms;
+    const uint2* edges;        // {term, bitmap}
+    const uint32_t* edge_q;    // the query of each edge
+    uint32_t nedges, ntiles, GX;
+    unsigned long long* counts;
+};
+__global__ void __launch_bounds__(RTHREADS) k_edge_counts(EdgeArgs A) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t nw = gridDim.x * RWARPS;
+    const uint64_t items = (uint64_t)A.nedges * A.ntiles;
+    for (uint64_t it = (uint64_t)blockIdx.x * RWARPS + (threadIdx.x >> 5); it < items; it += nw) {
+        const uint32_t k = (uint32_t)(it / A.nedges), ei = (uint32_t)(it - (uint64_t)k * A.nedges);
+        const uint32_t g0 = k * (uint32_t)RT, g1 = min(g0 + (uint32_t)RT, A.GX);
+        const uint2 ed = __ldg(A.edges + ei);
+        const DevTerm& T = A.terms[ed.x];
+        const DevIndex& I = A.idx[T.index];
+        const BitmapMeta m = I.bm[ed.y];
+        const uint32_t* tix = I.tiles + ((size_t)ed.y * (I.ntiles + 1) + k) * 2;
+        const uint32_t i0 = __ldg(tix), s0 = __ldg(tix + 1);
+        const uint32_t in1 = __ldg(tix + 2), sn1 = __ldg(tix + 3);
+        const uint32_t i1 = min(sn1 < g1 ? in1 + 1u : in1, m.n);
+        const uint32_t* w = I.words + m.wstart;
+        const uint32_t* raw = reinterpret_cast<const uint32_t*>(I.values);
+        const uint32_t vtype = I.vtype;
+        const uint32_t lop = T.lop, rop = T.rop;
+        const double lo = T.lo, hi = T.hi;
+        uint32_t carry = s0, cnt = 0;
+        for (uint32_t base0 = i0; base0 < i1; base0 += 128) {
+            uint32_t wv[4], pv[4], v0[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const uint32_t i = base0 + 32u * j + lane;
+                wv[j] = i < i1 ? __ldg(w + i) : 0u;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const uint32_t base = base0 + 32u * j;
+                pv[j] = 0;
+                if (base >= i1) continue;
+                const uint32_t c = base + lane < i1 ? wgroups(wv[j]) : 0u;
                 uint32_t x = c;
 #pragma unroll
                 for (int d = 1; d < 32; d <<= 1) {
                     const uint32_t u = __shfl_up_sync(0xffffffffu, x, d);
                     if (lane >= (uint32_t)d) x += u;
                 }
-                const uint32_t rt = __shfl_sync(0xffffffffu, x, 31);
-                if (rt == 0u) continue;
-                uint32_t p = x - c;
-                const uint32_t rbase = (g0 + l) * 31u;
-                while (bits) {
-                    const uint32_t hb = 31u - __clz(bits);
-                    st[p++] = rbase + (30u - hb);
-                    bits &= ~(1u << hb);
+                pv[j] = carry + x - c;
+                carry += __shfl_sync(0xffffffffu, x, 31);
+            }
+            // words past i1 are 0 and hold nothing
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const bool lit = wv[j] - 1u < ALLONES && pv[j] >= g0 && pv[j] < g1;
+                v0[j] = lit ? __ldg(raw + pv[j] * 31u + (__clz(wv[j]) - 1u)) : 0u;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const uint32_t wd = wv[j], p = pv[j];
+                if (wd - 1u < ALLONES) {
+                    if (p >= g0 && p < g1) {
+                        cnt += pass_cmp(raw_value(v0[j], vtype), lop, lo, rop, hi);
+                        for (uint32_t bits = wd & ~(0x80000000u >> __clz(wd)); bits;) {
+                            const uint32_t hb = 31u - __clz(bits);
+                            bits &= ~(1u << hb);
+                            cnt += pass_cmp(raw_value(__ldg(raw + p * 31u + (30u - hb)), vtype), lop, lo, rop, hi);
+                        }
+                    }
                 }
-                __syncwarp();
-                for (uint32_t i = lane; i < rt; i += 32u) {
-                    const uint64_t o = off + i;
-                    if (o < lim && rbase0 + o < A.rid_cap) A.rids[rbase0 + o] = st[i];
+            }
+            // 1-fills: the rows of their groups in the tile, by the warp
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                uint32_t fills = __ballot_sync(0xffffffffu, wv[j] >= HEADER1);
+                while (fills) {
+                    const uint32_t l = __ffs(fills) - 1u;
+                    fills &= fills - 1u;
+                    const uint32_t p = __shfl_sync(0xffffffffu, pv[j], l);
+                    const uint32_t c = __shfl_sync(0xffffffffu, wv[j], l) & MAXCNT;
+                    const uint32_t a = max(p, g0) * 31u, e = min(p + c, g1) * 31u;
+                    for (uint32_t r = a + lane; r < e; r += 32u)
+                        cnt += pass_cmp(raw_value(__ldg(raw + r), vtype), lop, lo, rop, hi);
                 }
-                __syncwarp();
-                off += rt;
             }
         }
-        if (A.dense && q == 0) {
-            for (uint32_t l = tid; l < ng; l += RTHREADS) A.dense[g0 + l] = S.acc[rsw(l)];
-        }
-        __syncthreads();
+        // the bitmap's active bits form the group after its whole words
+        if (lane == 0 && m.anb > 0 && m.groups >= g0 && m.groups < g1)
+            for (uint32_t bits = (m.aval & ((1u << m.anb) - 1u)) << (31u - m.anb); bits;) {
+                const uint32_t hb = 31u - __clz(bits);
+                bits &= ~(1u << hb);
+                cnt += pass_cmp(raw_value(__ldg(raw + m.groups * 31u + (30u - hb)), vtype), lop, lo, rop, hi);
+            }
+        cnt = __reduce_add_sync(0xffffffffu, cnt);
+        if (lane == 0 && cnt) atomicAdd(&A.counts[__ldg(A.edge_q + ei)], (unsigned long long)cnt);
     }
-    if (tid == 0) finish_tile(A.sync, gridDim.x);
 }
 
 // ---- attach: the passes over a new index's words
@@ -918,16 +1161,30 @@ k_tile_lists(const uint32_t* __restrict__ touch, uint32_t tw, uint32_t ntiles, u
 }
 
 // Prefix OR down the rows: row k |= row k-1 for k = 1..nrows-1 (a thread per
-// word column; neighbouring threads read neighbouring words of each row).
+// word column; neighbouring threads read neighbouring words of each row, 16
+// rows loaded before any is stored).
 __global__ void k_cum_prefix(uint32_t* __restrict__ rows, uint32_t nrows, uint32_t gx) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= gx) return;
     uint32_t acc = 0;
-    for (uint32_t k = 0; k < nrows; ++k) {
-        uint32_t* p = rows + (size_t)k * gx + i;
-        acc |= *p;
-        *p = acc;
+    for (uint32_t k0 = 0; k0 < nrows; k0 += 16) {
+        uint32_t v[16];
+#pragma unroll
+        for (uint32_t j = 0; j < 16; ++j) v[j] = k0 + j < nrows ? rows[(size_t)(k0 + j) * gx + i] : 0u;
+#pragma unroll
+        for (uint32_t j = 0; j < 16; ++j) {
+            acc |= v[j];
+            if (k0 + j < nrows) rows[(size_t)(k0 + j) * gx + i] = acc;
+        }
     }
+}
+
+// 1 bits of one cumulative row (into *total, zeroed).
+__global__ void k_row_ones(const uint32_t* __restrict__ row, uint32_t gx, unsigned long long* total) {
+    uint32_t c = 0;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < gx; i += gridDim.x * blockDim.x) c += __popc(row[i]);
+    c = __reduce_add_sync(0xffffffffu, c);
+    if ((threadIdx.x & 31u) == 0 && c) atomicAdd(total, (unsigned long long)c);
 }
 
 #endif  // WAH_RANGE_TYPES_ONLY
