@@ -493,6 +493,16 @@ def parse_index_file(data: bytes):
 
 def evaluate(ctx: Context, terms, want_rids: bool = True, want_hits: bool = False):
     """AND of the terms: (count, row ids or None, hit Bitvector or None)."""
+    if want_rids and not want_hits:
+        # the ids stay on the device until their number is known, so their
+        # array is made at its size
+        b = Batch(ctx, [terms], rid_cap=int(ctx.lib.wahgpu_index_nrows(terms[0].idx)))
+        try:
+            b.run()
+            n = int(b.counts()[0])
+            return n, b.rids(0, n), None
+        finally:
+            b.close()
     arr = (_Term * len(terms))(*terms)
     nrows = None
     cap = 0

@@ -180,7 +180,7 @@ extern "C" int wahgpu_ctx_create(int device, wahgpu_ctx** out) {
         return wg_fail(nullptr, WAHGPU_ECUDA, "stream creation failed");
     }
     c->stream = c->own_stream;
-    if (cudaMallocHost(&c->h_meta_stage, sizeof(DevMeta) * 4) != cudaSuccess) {
+    if (cudaMallocHost(&c->h_meta_stage, sizeof(DevMeta) * (META_SLOTS + 4)) != cudaSuccess) {
         cudaStreamDestroy(c->own_stream);
         delete c;
         return wg_fail(nullptr, WAHGPU_ENOMEM, "pinned staging allocation failed");
@@ -287,23 +287,88 @@ static int bv_reserve(wahgpu_bv* b, uint64_t cap) {
     return WAHGPU_OK;
 }
 
+// Metadata slot of a bitvector, from blocks of META_SLOTS.
+static DevMeta* meta_get(wahgpu_ctx* ctx) {
+    DevMeta* blk = nullptr;
+    {
+        std::lock_guard<std::mutex> g(ctx->mu);
+        if (!ctx->meta_free.empty()) {
+            DevMeta* m = ctx->meta_free.back();
+            ctx->meta_free.pop_back();
+            return m;
+        }
+    }
+    blk = static_cast<DevMeta*>(wg_alloc(ctx, META_SLOTS * sizeof(DevMeta)));
+    if (!blk) return nullptr;
+    std::lock_guard<std::mutex> g(ctx->mu);
+    ctx->meta_blocks.push_back(blk);
+    for (uint32_t i = META_SLOTS; i > 1; --i) ctx->meta_free.push_back(blk + i - 1);
+    return blk;
+}
 wahgpu_bv* wg_bv_new(wahgpu_ctx* ctx) {
     wahgpu_bv* b = new wahgpu_bv();
     b->ctx = ctx;
-    b->meta = static_cast<DevMeta*>(wg_alloc(ctx, sizeof(DevMeta)));
+    b->meta = meta_get(ctx);
     if (!b->meta) { delete b; return nullptr; }
     return b;
 }
 
-// Waits for the producer of b and copies its metadata to the host.
-int wg_bv_meta(wahgpu_bv* b) {
-    if (b->h_valid) return WAHGPU_OK;
+static void bv_unpend(wahgpu_bv* b) {  // ctx->mu held
+    if (b->pend < 0) return;
+    std::vector<wahgpu_bv*>& p = b->ctx->pending;
+    p[b->pend] = p.back();
+    p[b->pend]->pend = b->pend;
+    p.pop_back();
+    b->pend = -1;
+}
+// b's metadata have been launched on the context's stream: the host copy is
+// stale.  Work that is only being captured runs at some later time, so such a
+// result is read when it is asked for and not along with another one.
+static void bv_launched(wahgpu_bv* b) {
     wahgpu_ctx* ctx = b->ctx;
-    DevMeta* st = reinterpret_cast<DevMeta*>(ctx->h_meta_stage);
-    CUDA_TRY(ctx, cudaMemcpyAsync(st, b->meta, sizeof(DevMeta), cudaMemcpyDeviceToHost, ctx->stream));
-    CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-    b->h = *st;
-    b->h_valid = true;
+    b->h_valid = false;
+    b->told = false;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &cs) != cudaSuccess) { cudaGetLastError(); cs = cudaStreamCaptureStatusActive; }
+    std::lock_guard<std::mutex> g(ctx->mu);
+    if (cs != cudaStreamCaptureStatusNone) { bv_unpend(b); return; }
+    b->pend_stream = ctx->stream;
+    if (b->pend < 0) {
+        b->pend = (int32_t)ctx->pending.size();
+        ctx->pending.push_back(b);
+    }
+}
+
+// Waits for the producer of b and copies its metadata to the host, and with
+// it, in the same copy, those of the other results launched on this stream
+// since (a program that runs several operators and then asks for their counts
+// waits once).
+int wg_bv_meta(wahgpu_bv* b) {
+    wahgpu_ctx* ctx = b->ctx;
+    if (!b->h_valid) {
+        const DevMeta* blk = nullptr;
+        {
+            std::lock_guard<std::mutex> g(ctx->mu);
+            for (const DevMeta* m : ctx->meta_blocks)
+                if (b->meta >= m && b->meta < m + META_SLOTS) blk = m;
+        }
+        DevMeta* st = reinterpret_cast<DevMeta*>(ctx->h_meta_stage);
+        CUDA_TRY(ctx, cudaMemcpyAsync(st, blk, META_SLOTS * sizeof(DevMeta), cudaMemcpyDeviceToHost, ctx->stream));
+        CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+        std::lock_guard<std::mutex> g(ctx->mu);
+        b->h = st[b->meta - blk];
+        b->h_valid = true;
+        bv_unpend(b);
+        for (size_t i = ctx->pending.size(); i > 0; --i) {
+            wahgpu_bv* o = ctx->pending[i - 1];
+            if (o->pend_stream != ctx->stream || o->meta < blk || o->meta >= blk + META_SLOTS) continue;
+            o->h = st[o->meta - blk];
+            o->h_valid = true;
+            bv_unpend(o);
+        }
+    }
+    if (b->told) return WAHGPU_OK;
+    b->told = true;
     switch (b->h.status) {
     case 0: return WAHGPU_OK;
     case DEV_ERR_TIMEOUT: return wg_fail(ctx, WAHGPU_ETIMEOUT, "a device-side look-back wait gave up");
@@ -328,7 +393,7 @@ int wg_scan_meta(wahgpu_bv* b, uint32_t n, uint32_t anb, uint32_t aval) {
     }
     ctx->launches++;
     CUDA_TRY(ctx, cudaGetLastError());
-    b->h_valid = false;
+    bv_launched(b);
     return WAHGPU_OK;
 }
 
@@ -415,7 +480,11 @@ extern "C" int wahgpu_bv_free(wahgpu_bv* b) {
     // to later work before earlier work on the same stream has used it
     wg_free(ctx, b->words);
     wg_free(ctx, b->bpos);
-    wg_free(ctx, b->meta);
+    {
+        std::lock_guard<std::mutex> g(ctx->mu);
+        bv_unpend(b);
+        if (b->meta) ctx->meta_free.push_back(b->meta);
+    }
     wg_free(ctx, b->gt);
     wg_free(ctx, b->rows);
     delete b;
@@ -541,7 +610,7 @@ int wg_launch_merge(wahgpu_ctx* ctx, int op, bool fsm, bool unary, bool flip,
     else launch_merge_tb<64>(ctx, op, fsm, unary, flip, g, ctx->stream, a);
     ctx->launches++;
     CUDA_TRY(ctx, cudaGetLastError());
-    res->h_valid = false;
+    bv_launched(res);
     res->gt_valid = false;
     res->rows_valid = false;
     res->used = false;
@@ -616,7 +685,7 @@ int wg_launch_dense(wahgpu_ctx* ctx, int op, wahgpu_bv* x, wahgpu_bv* y, uint32_
     }
     ctx->launches++;
     CUDA_TRY(ctx, cudaGetLastError());
-    res->h_valid = false;
+    bv_launched(res);
     res->gt_valid = false;
     res->rows_valid = false;
     res->used = false;
@@ -720,7 +789,7 @@ int wg_launch_gop(wahgpu_ctx* ctx, int kind, int op, wahgpu_bv* x, wahgpu_bv* y,
     // runs after the launches above
     wg_free(ctx, scr);
     if (e != cudaSuccess) return wg_fail(ctx, WAHGPU_ECUDA, "launch failed: %s", cudaGetErrorString(e));
-    res->h_valid = false;
+    bv_launched(res);
     res->gt_valid = false;
     res->rows_valid = keep;
     res->used = false;
@@ -780,7 +849,7 @@ int wg_launch_fuse(wahgpu_ctx* ctx, int op, wahgpu_bv* x, wahgpu_bv* y, uint32_t
     }
     ctx->launches++;
     CUDA_TRY(ctx, cudaGetLastError());
-    res->h_valid = false;
+    bv_launched(res);
     res->gt_valid = false;
     res->rows_valid = false;
     res->used = false;
@@ -837,7 +906,7 @@ int wg_launch_gone(wahgpu_ctx* ctx, int op, wahgpu_bv* x, wahgpu_bv* y, uint32_t
     }
     ctx->launches++;
     CUDA_TRY(ctx, cudaGetLastError());
-    res->h_valid = false;
+    bv_launched(res);
     res->gt_valid = false;
     res->rows_valid = false;
     res->used = false;
@@ -879,7 +948,7 @@ static int collapsed_copy(wahgpu_ctx* ctx, const wahgpu_bv* src, wahgpu_bv** out
     if (!b) return wg_fail(ctx, WAHGPU_ENOMEM, "allocation failed");
     int rc = bv_reserve(b, 1);
     if (rc) { wahgpu_bv_free(b); return rc; }
-    uint32_t* st = reinterpret_cast<uint32_t*>(ctx->h_meta_stage) + 16;
+    uint32_t* st = reinterpret_cast<uint32_t*>(reinterpret_cast<DevMeta*>(ctx->h_meta_stage) + META_SLOTS);
     st[0] = HEADER0 | src->h.groups;
     st[1] = 0;
     st[2] = src->h.groups;
@@ -891,6 +960,7 @@ static int collapsed_copy(wahgpu_ctx* ctx, const wahgpu_bv* src, wahgpu_bv** out
     b->h.w0 = st[0];
     b->h.nfill = 1;
     b->h_valid = true;
+    b->told = true;
     // device meta mirrors the host copy
     CUDA_TRY(ctx, cudaMemcpyAsync(b->meta, &b->h, sizeof(DevMeta), cudaMemcpyHostToDevice, ctx->stream));
     CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
@@ -1088,7 +1158,7 @@ extern "C" int wahgpu_bv_binop_into(wahgpu_ctx* ctx, int op, int inplace, wahgpu
         ctx->launches++;
         e = cudaGetLastError();
         if (e != cudaSuccess) { rc = wg_fail(ctx, WAHGPU_ECUDA, "launch failed: %s", cudaGetErrorString(e)); break; }
-        res->h_valid = false;
+        bv_launched(res);
         res->gt_valid = false;
         res->rows_valid = false;
         res->used = false;
@@ -1123,6 +1193,7 @@ static void bv_take(wahgpu_bv* b, wahgpu_bv* tmp) {
     std::swap(b->cap, tmp->cap);
     std::swap(b->h, tmp->h);
     std::swap(b->h_valid, tmp->h_valid);
+    std::swap(b->told, tmp->told);
     std::swap(b->gt, tmp->gt);
     std::swap(b->gt_valid, tmp->gt_valid);
     std::swap(b->rows, tmp->rows);
@@ -1145,8 +1216,9 @@ static int unary_op(wahgpu_bv* b, bool flip) {
     } else {
         rc = launch_copy(ctx, flip, b, b->h.groups, b->h.anb, aval, r);
     }
+    // the wait for the result brings its metadata along
+    if (!rc) rc = wg_bv_meta(r);
     if (rc) { wahgpu_bv_free(r); return rc; }
-    cudaStreamSynchronize(ctx->stream);
     bv_take(b, r);
     wahgpu_bv_free(r);
     return WAHGPU_OK;
@@ -1178,6 +1250,7 @@ extern "C" int wahgpu_bv_decompress(wahgpu_bv* b) {
         r->h.w0 = wpattern(b->h.w0);
         r->h.nfill = 0;
         r->h_valid = true;
+        r->told = true;
         r->rows_valid = result_rows(r, G);
         const uint32_t ntiles = (uint32_t)(((uint64_t)G + PT - 1) / PT);
         k_expand<<<(ntiles + GW - 1) / GW, GCTA, 0, ctx->stream>>>(b->words, b->rows, ntiles, r->words, r->bpos,

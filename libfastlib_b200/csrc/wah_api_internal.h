@@ -26,6 +26,10 @@ struct wahgpu_ctx {
     void* scratch = nullptr;
     uint32_t scratch_tiles = 0;
     void* h_meta_stage = nullptr;  // pinned staging for metadata reads
+    // the bitvectors' metadata live in blocks of META_SLOTS, so that one copy
+    // reads those of every result launched since the last read
+    std::vector<wah::DevMeta*> meta_blocks, meta_free;
+    std::vector<struct wahgpu_bv*> pending;  // launched, metadata not read yet
     uint64_t launches = 0;
     uint32_t row_results = 0;           // results that could have kept a row index so far
     uint32_t dense_tile = 2048;         // WAHGPU_TUNE_DENSE_TILE
@@ -41,6 +45,8 @@ struct wahgpu_ctx {
     int64_t test_fail_alloc = 0;
 };
 
+constexpr uint32_t META_SLOTS = 128;
+
 struct wahgpu_bv {
     wahgpu_ctx* ctx = nullptr;
     uint32_t* words = nullptr;  // m_vec
@@ -49,6 +55,9 @@ struct wahgpu_bv {
     uint32_t cap = 0;           // capacity in words
     wah::DevMeta h{};           // host copy of *meta
     bool h_valid = false;
+    bool told = false;          // the device status in h has been reported
+    int32_t pend = -1;          // its place in ctx->pending
+    cudaStream_t pend_stream = nullptr;  // where it was launched
     uint32_t* gt = nullptr;     // group-tile index (k_gtile), built on first use
     bool gt_valid = false;
     uint2* rows = nullptr;      // row index (k_rows), built on first use or with the result

@@ -38,20 +38,28 @@ struct wahgpu_batch {
     uint32_t groups = 0, anb = 0, ntiles = 0;  // tiles per query
     bool general = false;             // some term is not dense
     bool small = false;               // tiles of RT_SMALL groups
+    // one device block of tables: indexes, terms, queries, then what a run
+    // starts from (counts known beforehand: one-term count queries over
+    // disjoint bitmaps, 0 for the others; row-id starts; status), then the
+    // edges to count
+    unsigned char* d_tab = nullptr;
     wah::DevIndex* d_idx = nullptr;
     wah::DevTerm* d_terms = nullptr;
     wah::DevQuery* d_queries = nullptr;
+    unsigned char* d_init = nullptr;
+    unsigned char* d_edges = nullptr;
+    // one device block of results, copied back at once: counts, row-id
+    // starts, status
     unsigned long long* d_counts = nullptr;
-    // one-term count queries over disjoint bitmaps: their wholly-inside 1
-    // bits (0 for the other queries), then the edges to count
-    unsigned char* d_base = nullptr;
+    unsigned long long* d_start = nullptr;
+    wah::DevMeta* d_status = nullptr;
+    size_t out_bytes = 0;
+    unsigned char* h_out = nullptr;    // pinned
     uint32_t nrange = 0;              // queries k_range evaluates
     uint32_t nedges = 0, etiles = 0;  // edges to count, RT tiles per column
-    unsigned long long* d_start = nullptr;
     uint32_t* d_rids = nullptr;
     uint64_t rid_cap = 0;
     uint32_t* d_dense = nullptr;
-    wah::DevMeta* d_status = nullptr;
     // two-pass order: per-item hits and first row-id slots (2 x nq*ntiles)
     // and the scan's temporary storage, allocated at the first such run
     unsigned long long* d_items = nullptr;
