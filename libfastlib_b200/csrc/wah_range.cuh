@@ -120,15 +120,15 @@ struct RangeArgs {
     DevMeta* status;
     uint32_t gx;              // words per cumulative row
     uint32_t tile_major;      // 1: items ordered tile by tile, else query by query
-    // two passes: the first writes each item's hits to item_cnt, a scan turns
+    // two passes: the first adds each item's hits to item_cnt (zeroed), a scan turns
     // them into item_off, the second writes the row ids; items are indexed
     // q*ntiles + k
     unsigned long long* item_cnt;
     const unsigned long long* item_off;
+    const uint2* item_list;      // capped: {item, ids before it within its query}, status->n of them
     // 1: every query writes at most rid_lim row ids into its own region at
     // rid_base (one pass: offsets within the query by a segmented look-back;
-    // two: by the items' scan, the second skipping the items whose ids lie
-    // past the limit)
+    // two: a list of the items holding ids under their query's limit)
     uint32_t capped;
 };
 
@@ -546,7 +546,8 @@ __device__ __forceinline__ bool any4(uint4 a) { return (a.x | a.y | a.z | a.w) !
 // The set rows of a quad's edge bits whose raw values pass the term (groups
 // g .. g + 3).  Edge bits are few and scattered (a bin of 1000 holds one row
 // in 32 groups), so a lane takes one row at a time, whichever group it is in:
-// the warp runs as long as its fullest lane.
+// the warp runs as long as its fullest lane.  (Lining the warp's rows up in
+// shared memory to load 32 at once took 18 % longer.)
 __device__ __forceinline__ uint4 check_quad(uint4 e, uint32_t g, const uint32_t* __restrict__ raw, uint32_t vtype,
                                             const DevTerm& T) {
     uint4 r = make_uint4(0u, 0u, 0u, 0u);
@@ -563,15 +564,51 @@ __device__ __forceinline__ uint4 check_quad(uint4 e, uint32_t g, const uint32_t*
     }
     return r;
 }
+
+// The AND of a query's dense terms over one quad per lane (quad o of the tile
+// at g0), starting from acc (whole warp).
+__device__ __forceinline__ uint4 dense_terms(const RangeArgs& A, const DevQuery& DQ, uint4 acc, uint32_t g0,
+                                             uint32_t o) {
+    const uint32_t gx4 = A.gx >> 2;
+    const bool in = o < gx4 - (g0 >> 2);  // rows are the groups rounded up to 4
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    for (uint32_t t = DQ.t0; t < DQ.td; ++t) {
+        const DevTerm& T = A.terms[t];
+        const uint32_t c0 = T.c0, c1 = T.c1, nc = T.ncand;
+        const uint4* row = reinterpret_cast<const uint4*>(T.cum) + (g0 >> 2) + o;  // + k * gx4: C(k + 1)
+        uint4 v = in && c1 ? __ldg(row + (size_t)(c1 - 1u) * gx4) : zero;
+        const uint4 z = in && c0 ? __ldg(row + (size_t)(c0 - 1u) * gx4) : zero;
+        if (nc) {
+            // an edge bitmap j is C(j + 1) & ~C(j)
+            const uint32_t j0 = T.cand[0], j1 = nc > 1u ? T.cand[1] : j0;
+            uint4 e = in ? __ldg(row + (size_t)j0 * gx4) : zero;
+            const uint4 e0 = in && j0 ? __ldg(row + (size_t)(j0 - 1u) * gx4) : zero;
+            uint4 f = in ? __ldg(row + (size_t)j1 * gx4) : zero;
+            const uint4 f0 = in && j1 ? __ldg(row + (size_t)(j1 - 1u) * gx4) : zero;
+            e = and4(or4(andn4(e, e0), andn4(f, f0)), acc);  // only the rows still in the AND
+            v = andn4(v, z);
+            if (any4(e)) {
+                const DevIndex& I = A.idx[T.index];
+                v = or4(v, check_quad(e, g0 + 4u * o, reinterpret_cast<const uint32_t*>(I.values), I.vtype, T));
+            }
+        } else {
+            v = andn4(v, z);
+        }
+        acc = and4(acc, v);
+        if (!__any_sync(0xffffffffu, any4(acc))) break;
+    }
+    return acc;
+}
+
 // Q quads of groups per thread: tiles of 4 * Q * RTHREADS groups.  GEN: the
 // batch holds terms that are not dense (tiles of RT groups).  Dense terms are
 // bound by the rows' loads (16 KB per row and tile, shared in L2) and the
 // edge rows' gathers, the others by the block barriers between their steps.
 // One range over 1M rows of 100 values with its row ids: 17 us on 32 CTAs,
 // 93 us when 8 CTAs walked the edge bitmaps' words; 1024 conjunctions over
-// 10M rows: 3.6 ms against 7.7 ms.
+// 10M rows: 3.1 ms against 7.7 ms (9 GB of rows from DRAM at 3.6 TB/s).
 template <int Q, int MODE, bool GEN>
-__global__ void __launch_bounds__(RTHREADS, MODE >= RM_IDS || GEN ? 3 : 4) k_range(RangeArgs A) {
+__global__ void __launch_bounds__(RTHREADS, 6) k_range(RangeArgs A) {
     static_assert(!GEN || Q == RQUADS, "the tile index is over RT groups");
     constexpr uint32_t TG = 4u * Q * RTHREADS;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -589,18 +626,20 @@ __global__ void __launch_bounds__(RTHREADS, MODE >= RM_IDS || GEN ? 3 : 4) k_ran
         epoch = S.hdr[1];
     }
     uint32_t par = 0;
-    for (uint32_t item = first; item < A.nitems; item += MODE == RM_LOOK ? A.nitems : gridDim.x) {
-        const uint32_t q = A.tile_major ? item % A.nq : item / A.ntiles;
-        const uint32_t k = A.tile_major ? item / A.nq : item % A.ntiles;
+    const bool listed = MODE == RM_IDS && A.capped;  // the items holding ids under their query's limit
+    const uint32_t nitems = listed ? A.status->n : A.nitems;
+    for (uint32_t at = first; at < nitems; at += MODE == RM_LOOK ? nitems : gridDim.x) {
+        const uint2 li = listed ? A.item_list[at] : make_uint2(at, 0u);
+        const uint32_t item = li.x;
+        const uint32_t q = A.tile_major && !listed ? item % A.nq : item / A.ntiles;
+        const uint32_t k = A.tile_major && !listed ? item / A.nq : item % A.ntiles;
         const uint32_t g0 = k * TG, g1 = min(g0 + TG, GX);
         const uint32_t ng = g1 > g0 ? g1 - g0 : 0u;
         const uint32_t qi = q * A.ntiles + k;  // the item's place in query order
         const DevQuery DQ = A.queries[q];
-        if (MODE == RM_IDS) {
-            // items without hits are done, and so (capped) are items whose
-            // ids all lie past the query's limit
-            if (tid == 0 && k == 0) A.rid_start[q] = A.capped ? DQ.rid_base : A.item_off[qi];
-            if (A.item_cnt[qi] == 0ull || (A.capped && A.item_off[qi] - A.item_off[q * A.ntiles] >= DQ.rid_lim)) continue;
+        if (MODE == RM_IDS && !listed) {
+            if (tid == 0 && k == 0) A.rid_start[q] = A.item_off[qi];
+            if (A.item_cnt[qi] == 0ull) continue;  // no hits
         }
         // the thread's quads: 32 Q consecutive ones per warp, neighbouring lanes on neighbouring quads
         const uint32_t ql = warp * (32u * Q) + lane;  // + 32 i
@@ -616,56 +655,18 @@ __global__ void __launch_bounds__(RTHREADS, MODE >= RM_IDS || GEN ? 3 : 4) k_ran
                 acc[i] = make_uint4(m[0], m[1], m[2], m[3]);
             }
         }
-        bool live = true;  // the AND is not empty (dense terms: the warp's part of it)
-        for (uint32_t t = DQ.t0; t < DQ.td && live; ++t) {
-            const DevTerm& T = A.terms[t];
-            const uint32_t c0 = T.c0, c1 = T.c1, nc = T.ncand;
-            // rows are GX words rounded up to 4 and the quads past them masked
-            const uint4* cum = reinterpret_cast<const uint4*>(T.cum) + (g0 >> 2);
-            const uint32_t gx4 = A.gx >> 2, n4 = gx4 - (g0 >> 2);  // quads of a row from g0 on
-            const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-            const uint4* hi = cum + (size_t)(c1 - 1u) * gx4 + ql;
-            const uint4* lo = cum + (size_t)(c0 - 1u) * gx4 + ql;
-            bool any = false;
-            if (nc == 0u) {
-                uint4 v[Q];
+        // a quad at a time through all its dense terms: few registers, so that
+        // many warps' loads are in flight (all quads of a term at once on 3
+        // CTAs per SM: 4.0 ms for the conjunctions that take 3.1 ms so; 4 / 5 /
+        // 6 CTAs of this form, spilling a little at 6: 4.0 / 3.6 / 3.3)
+        bool live = false;  // the AND is not empty
 #pragma unroll
-                for (int i = 0; i < Q; ++i) {
-                    const bool in = ql + 32u * i < n4;
-                    v[i] = in && c1 ? __ldg(hi + 32 * i) : zero;
-                    if (in && c0) v[i] = andn4(v[i], __ldg(lo + 32 * i));
-                }
-#pragma unroll
-                for (int i = 0; i < Q; ++i) {
-                    acc[i] = and4(acc[i], v[i]);
-                    any |= any4(acc[i]);
-                }
-            } else {
-                const DevIndex& I = A.idx[T.index];
-                const uint32_t* raw = reinterpret_cast<const uint32_t*>(I.values);
-                const uint32_t vtype = I.vtype;
-                // the edge bitmaps' rows; one edge: the same twice
-                const uint32_t j0 = T.cand[0], j1 = nc > 1u ? T.cand[1] : j0;
-                const uint4* h0 = cum + (size_t)j0 * gx4 + ql;
-                const uint4* h1 = cum + (size_t)j1 * gx4 + ql;
-#pragma unroll
-                for (int i = 0; i < Q; ++i) {
-                    if (ql + 32u * i >= n4) { acc[i] = zero; continue; }
-                    uint4 v = c1 ? __ldg(hi + 32 * i) : zero;
-                    uint4 e = __ldg(h0 + 32 * i), f = __ldg(h1 + 32 * i);
-                    if (c0) v = andn4(v, __ldg(lo + 32 * i));
-                    if (j0) e = andn4(e, __ldg(h0 + 32 * i - gx4));
-                    if (j1) f = andn4(f, __ldg(h1 + 32 * i - gx4));
-                    e = and4(or4(e, f), acc[i]);  // only the rows still in the AND
-                    if (any4(e)) v = or4(v, check_quad(e, g0 + 4u * (ql + 32u * i), raw, vtype, T));
-                    acc[i] = and4(acc[i], v);
-                    any |= any4(acc[i]);
-                }
-            }
-            live = __any_sync(0xffffffffu, any);
+        for (int i = 0; i < Q; ++i) {
+            acc[i] = dense_terms(A, DQ, acc[i], g0, ql + 32u * i);
+            live |= any4(acc[i]);
         }
         if (GEN && DQ.td < DQ.t1) {
-            bool on = DQ.td == DQ.t0 || __syncthreads_or(live);
+            bool on = __syncthreads_or(live);
             for (uint32_t t = DQ.td; t < DQ.t1 && on; ++t) {
                 range_term(S, A, t, k, g0, g1, G, anb, lastmask);
                 bool any = false;
@@ -684,8 +685,11 @@ __global__ void __launch_bounds__(RTHREADS, MODE >= RM_IDS || GEN ? 3 : 4) k_ran
 #pragma unroll
         for (int i = 0; i < Q; ++i) cnt += __popc(acc[i].x) + __popc(acc[i].y) + __popc(acc[i].z) + __popc(acc[i].w);
         cnt = __reduce_add_sync(0xffffffffu, cnt);  // the warp's hits
-        if (MODE == RM_COUNT) {
-            if (lane == 0 && cnt) atomicAdd(&A.counts[DQ.q], (unsigned long long)cnt);
+        if (MODE <= RM_ITEMS) {
+            if (lane == 0 && cnt) {
+                atomicAdd(&A.counts[DQ.q], (unsigned long long)cnt);
+                if (MODE == RM_ITEMS) atomicAdd(&A.item_cnt[qi], (unsigned long long)cnt);
+            }
             continue;
         }
         if (lane == 0) S.sums[par][warp] = cnt;
@@ -698,16 +702,9 @@ __global__ void __launch_bounds__(RTHREADS, MODE >= RM_IDS || GEN ? 3 : 4) k_ran
             before += w < warp ? c : 0u;
         }
         par ^= 1u;
-        if (MODE == RM_ITEMS) {
-            if (tid == 0) {
-                A.item_cnt[qi] = total;
-                if (total) atomicAdd(&A.counts[q], (unsigned long long)total);
-            }
-            continue;
-        }
         uint64_t base;
         if (MODE == RM_IDS) {
-            base = A.capped ? A.item_off[qi] - A.item_off[q * A.ntiles] : A.item_off[qi];
+            base = listed ? li.y : A.item_off[qi];
         } else {
             if (warp == 0 && A.capped) {
                 // the row ids before this tile within its own query
@@ -801,6 +798,36 @@ __global__ void __launch_bounds__(RTHREADS, MODE >= RM_IDS || GEN ? 3 : 4) k_ran
     if (MODE == RM_LOOK) {
         __syncthreads();
         if (tid == 0) finish_tile(A.sync, gridDim.x);
+    }
+}
+
+// Capped queries, between the passes: a warp per query scans its items' hits
+// and lists those holding ids under the limit (in any order) with the ids
+// before them, so that the second pass visits no item only to skip it (0.9
+// ms without the list, 0.6 with it, of 81 K items).
+__global__ void __launch_bounds__(RTHREADS) k_cap_items(RangeArgs A, uint2* __restrict__ list) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t q = (blockIdx.x * RTHREADS + threadIdx.x) >> 5;
+    if (q >= A.nq) return;
+    const uint64_t lim = A.queries[q].rid_lim;
+    if (lane == 0) A.rid_start[q] = A.queries[q].rid_base;
+    uint64_t before = 0;
+    for (uint32_t k0 = 0; k0 < A.ntiles && before < lim; k0 += 32u) {
+        const uint32_t k = k0 + lane;
+        const uint32_t c = k < A.ntiles ? (uint32_t)A.item_cnt[(size_t)q * A.ntiles + k] : 0u;
+        uint32_t s = c;  // a tile holds at most RT * 31 hits
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t u = __shfl_up_sync(0xffffffffu, s, d);
+            if (lane >= (uint32_t)d) s += u;
+        }
+        const bool on = c != 0u && before + (s - c) < lim;
+        const uint32_t m = __ballot_sync(0xffffffffu, on);
+        uint32_t at = 0;
+        if (lane == 0 && m) at = atomicAdd(&A.status->n, __popc(m));
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
+        if (on) list[at] = make_uint2(q * A.ntiles + k, (uint32_t)before + (s - c));
+        before += __shfl_sync(0xffffffffu, s, 31);
     }
 }
 
