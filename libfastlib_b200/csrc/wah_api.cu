@@ -11,6 +11,7 @@
 
 #include <cuda_runtime.h>
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstdarg>
 #include <cstring>
@@ -548,7 +549,7 @@ static void launch_k(const wahgpu_ctx* ctx, dim3 g, cudaStream_t s, const MergeA
     static PerDeviceSetup setup;
     const size_t sm = sizeof(TileShared<TB>);
     wg_kernel_setup(setup, ctx->device, k_merge<OP, FSM, UNARY, FLIP, TB>, MERGE_THREADS, sm);
-    k_merge<OP, FSM, UNARY, FLIP, TB><<<g, MERGE_THREADS, sm, s>>>(a);
+    wg_launch_pdl(k_merge<OP, FSM, UNARY, FLIP, TB>, g.x, MERGE_THREADS, sm, s, a);
 }
 template <int TB>
 static void launch_merge_tb(const wahgpu_ctx* ctx, int op, bool fsm, bool unary, bool flip, dim3 g, cudaStream_t s,
@@ -570,13 +571,15 @@ static void launch_merge_tb(const wahgpu_ctx* ctx, int op, bool fsm, bool unary,
 #undef WG_MERGE_OP
 }
 // Block-index entries per merge tile: the context's setting, else by the
-// operands' size: the largest of 64 / 32 / 16 that still gives about two
-// tiles per SM, so small operands spread over the GPU in short tiles.
+// operands' size.  Small operands spread over the GPU in short tiles; long
+// tiles share their fixed steps among more words (2^28 bits, us at 16 / 32 /
+// 64 entries: 4.6 K blocks 14.5 / 13.3 / 14.7, 14 K 25.7 / 17.6 / 17.1, 45 K
+// 63 / 42 / 34).
 static uint32_t merge_tile_blocks(const wahgpu_ctx* ctx, uint32_t nblocks) {
     if (ctx->merge_tile) return ctx->merge_tile;
-    const uint64_t want = 2ull * (uint64_t)ctx->sm_count;
-    if ((uint64_t)nblocks >= want * 64u) return 64;
-    if ((uint64_t)nblocks >= want * 32u) return 32;
+    const uint64_t sms = (uint64_t)ctx->sm_count;
+    if (nblocks >= sms * 88u) return 64;
+    if (nblocks >= sms * 30u) return 32;
     return 16;
 }
 
@@ -603,7 +606,6 @@ int wg_launch_merge(wahgpu_ctx* ctx, int op, bool fsm, bool unary, bool flip,
     a.out = res->words; a.obp = res->bpos; a.meta = res->meta;
     a.recs = recs; a.sync = sync; a.ntiles = ntiles;
     a.aval = aval; a.anb = anb;
-    CUDA_TRY(ctx, cudaMemsetAsync(res->meta, 0, sizeof(DevMeta), ctx->stream));
     dim3 g(ntiles);
     if (tb == 16) launch_merge_tb<16>(ctx, op, fsm, unary, flip, g, ctx->stream, a);
     else if (tb == 32) launch_merge_tb<32>(ctx, op, fsm, unary, flip, g, ctx->stream, a);
@@ -916,21 +918,23 @@ int wg_launch_gone(wahgpu_ctx* ctx, int op, wahgpu_bv* x, wahgpu_bv* y, uint32_t
 
 // Group space or word space for an operator on the reference's _c2 path, and
 // for copies and complements (y null): group space costs by the groups, the
-// merge by the words.  Lines through measured calls, in us with g and n in
-// millions (group space: 8.8 at g = 0.03, 43 at 8.7; merge: 17 at n = 0.007,
-// 24 at 0.15, 58 at 1.4).  The row index an operand lacks is charged to its
-// first use; an operand that comes back is taken to come again.  A merge tile
-// set on the context asks for the merge.
+// merge by the words, each at least its chain of steps.  Curves through
+// measured calls of & | - at 2^16 .. 2^28 bits, d = 1e-4 .. 0.06, in us:
+// group space 7.3 at 0.13M groups, 15 at 2.2M, 41 at 8.7M; merge 7.7 at 400
+// words of both operands, 9.8 at 7 K, 12.3 at 63 K, 17 at 0.4M, 37 at 1.4M,
+// 87 at 4M.  The row index an operand lacks is charged to its first use; an
+// operand that comes back is taken to come again.  A merge tile set on the
+// context asks for the merge.
 static bool in_group_space(const wahgpu_ctx* ctx, wahgpu_bv* x, wahgpu_bv* y, uint32_t groups) {
     if (ctx->merge_tile) return false;
-    const double g = groups * 1e-6, n = ((double)x->h.n + (y ? y->h.n : 0)) * 1e-6;
-    double in_groups = y ? 8.0 + 3.8 * g : 7.0 + 3.0 * g;
+    const double g = groups * 1e-6, n = (double)x->h.n + (y ? y->h.n : 0);
+    double in_groups = 6.6 + (y ? 4.0 : 3.1) * g;
     for (wahgpu_bv* b : {x, y}) {
         if (!b) continue;
-        if (!b->rows_valid && !b->used) in_groups += 3.0 + 1.2 * g;
+        if (!b->rows_valid && !b->used) in_groups += 3.0 + 1.5 * g;
         b->used = true;
     }
-    return in_groups < (y ? 15.5 + 29.5 * n : 14.0 + 15.0 * n);
+    return in_groups < 7.0 + 0.5 * std::log2(1.0 + n / 200.0) + (y ? 17e-6 : 12e-6) * n;
 }
 
 // x, or its complement, as compress() leaves it.

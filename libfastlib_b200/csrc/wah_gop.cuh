@@ -223,80 +223,6 @@ __global__ void __launch_bounds__(GCTA) k_expand(const uint32_t* __restrict__ w,
     }
 }
 
-// ---- words further back, for the count-1 flags that need them (whole warp,
-// uniform arguments).  Rare: only one-group runs over count-1 fill words.
-// First group of word j.
-__device__ __forceinline__ uint32_t word_start(const uint32_t* __restrict__ w, const uint32_t* __restrict__ bp, uint32_t j) {
-    const uint32_t lane = threadIdx.x & 31u, k = j >> 5;
-    const uint32_t c = lane < (j & 31u) ? wgroups(__ldg(w + 32u * k + lane)) : 0u;
-    return __ldg(bp + k) + __reduce_add_sync(0xffffffffu, c);
-}
-// Is one of the words before word j that start at or after group a a literal?
-__device__ __forceinline__ bool literal_since(const uint32_t* __restrict__ w, const uint32_t* __restrict__ bp, uint32_t j,
-                                              uint32_t a) {
-    if (j == 0u) return false;
-    const uint32_t lane = threadIdx.x & 31u;
-    for (uint32_t k = (j - 1u) >> 5;; --k) {
-        const uint32_t i = 32u * k + lane;
-        const uint32_t v = i < j ? __ldg(w + i) : HEADER0;
-        const uint32_t lit = __ballot_sync(0xffffffffu, !is_fill(v));
-        if (lit) {  // the last one starts latest
-            const uint32_t top = 31u - __clz(lit);
-            return __ldg(bp + k) + __reduce_add_sync(0xffffffffu, lane < top ? wgroups(v) : 0u) >= a;
-        }
-        if (__ldg(bp + k) <= a) return false;
-    }
-}
-// "-": is the 0-fill word i of x, which began before group q where y's word j
-// starts and ends later, being counted (S_CNT_X) at q?  It is unless y's word
-// before j is a 1-fill begun before it and itself being counted there; two
-// neighbouring fills of one value take the question one word back in both.
-__device__ __forceinline__ bool minus_counted(const GopArgs& A, uint32_t i, uint32_t q, uint32_t j) {
-    uint32_t a = word_start(A.xw, A.xbp, i);
-    while (true) {
-        if (j == 0u) return true;
-        const uint32_t v = __ldg(A.yw + j - 1u);
-        if (!(is_fill(v) && fill_bit(v))) return true;
-        const uint32_t c = q - wgroups(v);
-        if (c >= a) return true;
-        if (i == 0u) return false;
-        const uint32_t u = __ldg(A.xw + i - 1u);
-        if (!is_fill(u) || fill_bit(u)) return false;
-        const uint32_t a2 = a - wgroups(u);
-        if (a2 >= c) return false;
-        --i; --j;
-        q = c; a = a2;
-    }
-}
-// The flag of the one-group run at p, words xi / yi covering it.
-template <int OP>
-__device__ __noinline__ bool walk_flag(const GopArgs& A, uint32_t code, uint32_t p, uint32_t xi, uint32_t yi) {
-    const uint32_t absorb = OP == OP_OR ? 1u : 0u;
-    if (code == SF_WALK_AND_Y) {
-        return literal_since(A.yw, A.ybp, yi, p + 1u - wgroups(__ldg(A.xw + xi)));  // x's fill ends at p + 1
-    } else if (code == SF_WALK_AND_X) {
-        if (xi == 0u) return true;
-        const uint32_t v = __ldg(A.xw + xi - 1u);
-        if (!is_fill(v) || fill_bit(v) != absorb) return true;
-        const uint32_t a = p - wgroups(v);
-        return !(a < word_start(A.yw, A.ybp, yi) && literal_since(A.yw, A.ybp, yi, a));
-    } else if (code == SF_WALK_MINUS_X) {
-        if (xi == 0u) return true;
-        const uint32_t v = __ldg(A.xw + xi - 1u);
-        if (!is_fill(v) || fill_bit(v)) return true;
-        const uint32_t q = word_start(A.yw, A.ybp, yi);
-        return !(p - wgroups(v) < q && minus_counted(A, xi - 1u, q, yi));
-    }
-    if (yi == 0u) return true;
-    const uint32_t v = __ldg(A.yw + yi - 1u);  // ends at p
-    if (!is_fill(v) || !fill_bit(v)) return true;
-    const uint32_t c = p - wgroups(v), a = word_start(A.xw, A.xbp, xi);
-    if (c >= a) return true;
-    if (xi == 0u) return false;
-    const uint32_t u = __ldg(A.xw + xi - 1u);
-    return is_fill(u) && !fill_bit(u) && a - wgroups(u) < c && minus_counted(A, xi - 1u, c, yi - 1u);
-}
-
 // Pattern of one group of word w in bits 0..30 (bit 31 is not part of it).
 __device__ __forceinline__ uint32_t gop_pattern(uint32_t w) {
     return (int32_t)w < 0 ? (uint32_t)((int32_t)(w << 1) >> 31) : w;
@@ -321,6 +247,17 @@ __device__ __forceinline__ void gop_range_of(uint32_t ntiles, uint32_t cta, uint
     const uint32_t q = (ntiles + n - 1u) / n;
     lo = min(cta * q, ntiles);
     hi = min(lo + q, ntiles);
+}
+
+// Position of the k-th set bit (from 0) of h.
+__device__ __forceinline__ uint32_t nth_bit(uint32_t h, uint32_t k) {
+    uint32_t pos = 0;
+#pragma unroll
+    for (int w = 16; w > 0; w >>= 1) {
+        const uint32_t c = __popc((h >> pos) & ((1u << w) - 1u));
+        if (k >= c) { k -= c; pos += w; }
+    }
+    return pos;
 }
 
 template <bool UNARY>
@@ -455,10 +392,12 @@ __global__ void __launch_bounds__(GCTA, 3) k_gop(const __grid_constant__ GopArgs
         if (KIND == GK_FSM) {
             // runs of one group: a uniform head followed by a head (or the end)
             uint32_t nb = __shfl_down_sync(0xffffffffu, H, 1) & 1u;
+            uint32_t xnext = 0, ynext = 0;  // starts of the row after the tile
             if (left > (uint32_t)PT) {  // the head test of the group after the tile
                 const uint2* xr = A.xr + (size_t)(t + 1) * TROWS;
                 const uint2* yr = A.yr + (size_t)(t + 1) * TROWS;
                 const uint2 mx = __ldg(xr), my = __ldg(yr);
+                xnext = mx.x; ynext = my.x;
                 const uint32_t pv = gop_value<OP, KIND>(__ldg(xw + (mx.y + (mx.x & 1u))), __ldg(yw + (my.y + (my.x & 1u))));
                 if (lane == TROWS - 1u) nb = !((pv == 0u && zp >> 31) || (pv == ALLONES && op >> 31));
             } else if (left == 32u * lane + 32u) {
@@ -467,35 +406,50 @@ __global__ void __launch_bounds__(GCTA, 3) k_gop(const __grid_constant__ GopArgs
             uint32_t S = H >> 1 | nb << 31;
             if (left > 32u * lane && left < 32u * lane + 32u) S |= 1u << (left - 32u * lane - 1u);
             S &= H & U;
-            uint32_t todo = __ballot_sync(0xffffffffu, lane < (uint32_t)TROWS && S != 0u);
-            while (todo) {
-                const uint32_t r = __ffs(todo) - 1u;
-                todo &= todo - 1u;
-                const uint32_t s = __shfl_sync(0xffffffffu, S, r);
-                const uint2* xr = A.xr + (size_t)t * TROWS + r;
-                const uint2* yr = A.yr + (size_t)t * TROWS + r;
-                const uint2 mx = __ldg(xr), my = __ldg(yr);
-                const uint32_t p = g0 + 32u * r + lane;
-                const uint32_t xi = mx.y + __popc(mx.x & le), yi = my.y + __popc(my.x & le);
-                uint32_t code = SF_NO;
-                if ((s >> lane) & 1u) {
-                    // do the words end at p + 1 (the next row's first start, past a row's end)
-                    bool xe = true, ye = true;
-                    if (p + 1u < A.groups) {
-                        xe = lane < 31u ? (mx.x >> (lane + 1u)) & 1u : __ldg(&xr[1].x) & 1u;
-                        ye = lane < 31u ? (my.x >> (lane + 1u)) & 1u : __ldg(&yr[1].x) & 1u;
-                    }
-                    code = single_flag(OP, __ldg(xw + xi), __ldg(yw + yi), (mx.x >> lane) & 1u, (my.x >> lane) & 1u, xe, ye);
+            if (lane >= (uint32_t)TROWS) S = 0u;
+            // the tile's one-group runs, 32 at a time whatever rows they are in
+            const uint32_t ns = __popc(S);
+            uint32_t before = ns;  // lane r: those before row r
+#pragma unroll
+            for (int d = 1; d < TROWS; d <<= 1) {
+                const uint32_t u = __shfl_up_sync(0xffffffffu, before, d);
+                if (lane >= (uint32_t)d) before += u;
+            }
+            const uint32_t nsingle = __shfl_sync(0xffffffffu, before, TROWS - 1);
+            before -= ns;
+            for (uint32_t k0 = 0; k0 < nsingle; k0 += 32u) {
+                const uint32_t k = min(k0 + lane, nsingle - 1u);
+                uint32_t r = 0;  // the last row with at most k before it
+#pragma unroll
+                for (uint32_t d = TROWS / 2; d > 0; d >>= 1)
+                    if (__shfl_sync(0xffffffffu, before, r + d) <= k) r += d;
+                const uint32_t bit = nth_bit(__shfl_sync(0xffffffffu, S, r), k - __shfl_sync(0xffffffffu, before, r));
+                const uint32_t p = g0 + 32u * r + bit;
+                // its words, as staged
+                const uint2 mx = W.row[b][r], my = W.row[b][TROWS + r];
+                const uint32_t upto = (2u << bit) - 1u;
+                const uint32_t x = lds32(mx.y + 4u * __popc(mx.x & upto)), y = lds32(my.y + 4u * __popc(my.x & upto));
+                // do they end at p + 1 (does the next one start there)
+                bool xe = true, ye = true;
+                if (p + 1u < A.groups) {
+                    const uint32_t nbit = (bit + 1u) & 31u, nr = r + (bit == 31u ? 1u : 0u);
+                    xe = ((nr < (uint32_t)TROWS ? W.row[b][nr].x : xnext) >> nbit) & 1u;
+                    ye = ((nr < (uint32_t)TROWS ? W.row[b][TROWS + nr].x : ynext) >> nbit) & 1u;
                 }
+                uint32_t code = k0 + lane < nsingle
+                                    ? single_flag(OP, x, y, (mx.x >> bit) & 1u, (my.x >> bit) & 1u, xe, ye) : SF_NO;
                 uint32_t walk = __ballot_sync(0xffffffffu, code > SF_YES);
                 while (walk) {
                     const uint32_t l = __ffs(walk) - 1u;
                     walk &= walk - 1u;
-                    const bool f = walk_flag<OP>(A, __shfl_sync(0xffffffffu, code, l), __shfl_sync(0xffffffffu, p, l),
-                                                 __shfl_sync(0xffffffffu, xi, l), __shfl_sync(0xffffffffu, yi, l));
+                    const uint32_t wp = __shfl_sync(0xffffffffu, p, l), wm = (2u << (wp & 31u)) - 1u;
+                    const uint2 rx = __ldg(A.xr + (wp >> 5)), ry = __ldg(A.yr + (wp >> 5));
+                    const bool f = walk_flag<OP>(Operands{A.xw, A.xbp, A.yw, A.ybp}, __shfl_sync(0xffffffffu, code, l), wp,
+                                                 rx.y + __popc(rx.x & wm), ry.y + __popc(ry.x & wm));
                     if (lane == l) code = f ? SF_YES : SF_NO;
                 }
-                if (code == SF_YES) R[32u * r] |= HEADER0;  // this lane's own store above
+                // over the pattern another lane stored (the warp has synchronised since)
+                if (code == SF_YES) A.R[p] = gop_value<OP, KIND>(x, y) | HEADER0;
             }
         }
         ones = __reduce_add_sync(0xffffffffu, ones);
@@ -504,17 +458,6 @@ __global__ void __launch_bounds__(GCTA, 3) k_gop(const __grid_constant__ GopArgs
         if (lane == 0) { A.heads[t] = heads; A.first[t] = first; A.ones[t] = ones; }
         __syncwarp();  // the buffer, the rows and the head masks are free again
     }
-}
-
-// Position of the k-th set bit (from 0) of h.
-__device__ __forceinline__ uint32_t nth_bit(uint32_t h, uint32_t k) {
-    uint32_t pos = 0;
-#pragma unroll
-    for (int w = 16; w > 0; w >>= 1) {
-        const uint32_t c = __popc((h >> pos) & ((1u << w) - 1u));
-        if (k >= c) { k -= c; pos += w; }
-    }
-    return pos;
 }
 
 struct PackWarp {

@@ -19,8 +19,16 @@
 // Encoding.  Result words are maximal runs (wah_core.cuh).  A run's word is
 // written by the thread that meets the next run head (its length is only
 // known then); mixed literals are written at once.  Head counts, the last
-// head, popcounts and the step-state transfer function are carried across
-// tiles by a single-pass decoupled look-back over TileRec records.
+// head and popcounts are carried across tiles by a single-pass decoupled
+// look-back over TileRec records, in block order.  The walk's count-1 fills
+// are told from the words meeting at a one-group run (single_flag), so no
+// state is carried for them.
+//
+// Bound by the chain of dependent steps of a tile (search, loads, scans,
+// look-back).  2^28 bits, d = 1e-3 / 1e-2: 14 / 37 us a call.  The form
+// that carried the walk's five step states as transfer functions through the
+// scans, claimed its tile by an atomic and had its metadata cleared by a
+// memset took 23.5 / 58.
 #ifndef WAH_MERGE_CUH
 #define WAH_MERGE_CUH
 #include "wah_dev.cuh"
@@ -57,60 +65,39 @@ struct MergeArgs {
     uint32_t aval, anb;   // result active word (already combined)
 };
 
-// Look-back aggregate: heads, last head (position, class, count-1 flag for
-// each of the 5 possible incoming step states), popcount, transfer function.
+// Look-back aggregate: heads, last head (position, class, count-1 flag), popcount.
 struct Agg {
     uint32_t nheads, pos, info, popc;
 };
 __device__ __forceinline__ uint32_t agg_cls(uint32_t info) { return info & 3u; }
 __device__ __forceinline__ bool agg_has(uint32_t info) { return (info >> 2) & 1u; }
-__device__ __forceinline__ uint32_t agg_fmask(uint32_t info) { return (info >> 3) & 31u; }
-__device__ __forceinline__ uint32_t agg_fsm(uint32_t info) { return (info >> 8) & 0x7FFFu; }
-__device__ __forceinline__ uint32_t mk_info(uint32_t cls, bool has, uint32_t fmask, uint32_t fsm) {
-    return cls | (has ? 4u : 0u) | (fmask << 3) | (fsm << 8);
+__device__ __forceinline__ bool agg_flag(uint32_t info) { return (info >> 3) & 1u; }
+__device__ __forceinline__ uint32_t mk_info(uint32_t cls, bool has, bool flag) {
+    return cls | (has ? 4u : 0u) | (flag ? 8u : 0u);
 }
 __device__ __forceinline__ Agg agg_identity() {
-    Agg a; a.nheads = 0; a.pos = 0; a.popc = 0; a.info = mk_info(0, false, 0, FSM_IDENTITY);
+    Agg a; a.nheads = 0; a.pos = 0; a.popc = 0; a.info = 0;
     return a;
 }
 // a followed by b
-template <bool FSM>
 __device__ __forceinline__ Agg agg_combine(const Agg& a, const Agg& b) {
+    const bool h = agg_has(b.info);
     Agg r;
     r.nheads = a.nheads + b.nheads;
     r.popc = a.popc + b.popc;
-    uint32_t fa = agg_fsm(a.info), fb = agg_fsm(b.info);
-    uint32_t f = FSM ? fsm_compose(fa, fb) : FSM_IDENTITY;
-    if (agg_has(b.info)) {
-        r.pos = b.pos;
-        // the last head's flags are indexed by the state entering b; seen
-        // from the start of a they are re-indexed through a's transfer.
-        // Without step states (copy / canonical modes) they do not depend
-        // on the state.
-        uint32_t bm = agg_fmask(b.info), m = bm;
-        if (FSM) {
-            m = 0;
-#pragma unroll
-            for (uint32_t s = 0; s < 5; ++s) m |= ((bm >> fsm_apply(fa, s)) & 1u) << s;
-        }
-        r.info = mk_info(agg_cls(b.info), true, m, f);
-    } else {
-        r.pos = a.pos;
-        r.info = mk_info(agg_cls(a.info), agg_has(a.info), agg_fmask(a.info), f);
-    }
+    r.pos = h ? b.pos : a.pos;
+    r.info = h ? b.info : a.info;
     return r;
 }
 __device__ __forceinline__ uint4 agg_pack(const Agg& a) { return make_uint4(a.nheads, a.pos, a.info, a.popc); }
 __device__ __forceinline__ Agg agg_unpack(uint4 v) { Agg a; a.nheads = v.x; a.pos = v.y; a.info = v.z; a.popc = v.w; return a; }
 
-template <bool FSM>
 struct AggComb {
     __device__ __forceinline__ uint4 operator()(uint4 a, uint4 b) const {
-        return agg_pack(agg_combine<FSM>(agg_unpack(a), agg_unpack(b)));
+        return agg_pack(agg_combine(agg_unpack(a), agg_unpack(b)));
     }
 };
 
-template <bool FSM>
 __device__ __forceinline__ Agg agg_shfl_up(const Agg& a, int d) {
     Agg r;
     r.nheads = __shfl_up_sync(0xffffffffu, a.nheads, d);
@@ -118,6 +105,84 @@ __device__ __forceinline__ Agg agg_shfl_up(const Agg& a, int d) {
     r.info = __shfl_up_sync(0xffffffffu, a.info, d);
     r.popc = __shfl_up_sync(0xffffffffu, a.popc, d);
     return r;
+}
+
+// ---- words further back, for the count-1 flags that need them (whole warp,
+// uniform arguments).  Rare: only one-group runs over count-1 fill words.
+struct Operands {  // words and block positions
+    const uint32_t* __restrict__ xw; const uint32_t* __restrict__ xbp;
+    const uint32_t* __restrict__ yw; const uint32_t* __restrict__ ybp;
+};
+// First group of word j.
+__device__ __forceinline__ uint32_t word_start(const uint32_t* __restrict__ w, const uint32_t* __restrict__ bp, uint32_t j) {
+    const uint32_t lane = threadIdx.x & 31u, k = j >> 5;
+    const uint32_t c = lane < (j & 31u) ? wgroups(__ldg(w + 32u * k + lane)) : 0u;
+    return __ldg(bp + k) + __reduce_add_sync(0xffffffffu, c);
+}
+// Is one of the words before word j that start at or after group a a literal?
+__device__ __forceinline__ bool literal_since(const uint32_t* __restrict__ w, const uint32_t* __restrict__ bp, uint32_t j,
+                                              uint32_t a) {
+    if (j == 0u) return false;
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t k = (j - 1u) >> 5;; --k) {
+        const uint32_t i = 32u * k + lane;
+        const uint32_t v = i < j ? __ldg(w + i) : HEADER0;
+        const uint32_t lit = __ballot_sync(0xffffffffu, !is_fill(v));
+        if (lit) {  // the last one starts latest
+            const uint32_t top = 31u - __clz(lit);
+            return __ldg(bp + k) + __reduce_add_sync(0xffffffffu, lane < top ? wgroups(v) : 0u) >= a;
+        }
+        if (__ldg(bp + k) <= a) return false;
+    }
+}
+// "-": is the 0-fill word i of x, which began before group q where y's word j
+// starts and ends later, being counted (S_CNT_X) at q?  It is unless y's word
+// before j is a 1-fill begun before it and itself being counted there; two
+// neighbouring fills of one value take the question one word back in both.
+__device__ __forceinline__ bool minus_counted(const Operands& A, uint32_t i, uint32_t q, uint32_t j) {
+    uint32_t a = word_start(A.xw, A.xbp, i);
+    while (true) {
+        if (j == 0u) return true;
+        const uint32_t v = __ldg(A.yw + j - 1u);
+        if (!(is_fill(v) && fill_bit(v))) return true;
+        const uint32_t c = q - wgroups(v);
+        if (c >= a) return true;
+        if (i == 0u) return false;
+        const uint32_t u = __ldg(A.xw + i - 1u);
+        if (!is_fill(u) || fill_bit(u)) return false;
+        const uint32_t a2 = a - wgroups(u);
+        if (a2 >= c) return false;
+        --i; --j;
+        q = c; a = a2;
+    }
+}
+// The flag of the one-group run at p, words xi / yi covering it.
+template <int OP>
+__device__ __noinline__ bool walk_flag(const Operands A, uint32_t code, uint32_t p, uint32_t xi, uint32_t yi) {
+    const uint32_t absorb = OP == OP_OR ? 1u : 0u;
+    if (code == SF_WALK_AND_Y) {
+        return literal_since(A.yw, A.ybp, yi, p + 1u - wgroups(__ldg(A.xw + xi)));  // x's fill ends at p + 1
+    } else if (code == SF_WALK_AND_X) {
+        if (xi == 0u) return true;
+        const uint32_t v = __ldg(A.xw + xi - 1u);
+        if (!is_fill(v) || fill_bit(v) != absorb) return true;
+        const uint32_t a = p - wgroups(v);
+        return !(a < word_start(A.yw, A.ybp, yi) && literal_since(A.yw, A.ybp, yi, a));
+    } else if (code == SF_WALK_MINUS_X) {
+        if (xi == 0u) return true;
+        const uint32_t v = __ldg(A.xw + xi - 1u);
+        if (!is_fill(v) || fill_bit(v)) return true;
+        const uint32_t q = word_start(A.yw, A.ybp, yi);
+        return !(p - wgroups(v) < q && minus_counted(A, xi - 1u, q, yi));
+    }
+    if (yi == 0u) return true;
+    const uint32_t v = __ldg(A.yw + yi - 1u);  // ends at p
+    if (!is_fill(v) || !fill_bit(v)) return true;
+    const uint32_t c = p - wgroups(v), a = word_start(A.xw, A.xbp, xi);
+    if (c >= a) return true;
+    if (xi == 0u) return false;
+    const uint32_t u = __ldg(A.xw + xi - 1u);
+    return is_fill(u) && !fill_bit(u) && a - wgroups(u) < c && minus_counted(A, xi - 1u, c, yi - 1u);
 }
 
 // Smallest m in [lo, hi] with !(a[m] <= b[d-1-m]) : the number of entries
@@ -154,9 +219,6 @@ struct TileShared {
     uint32_t warp_agg[MERGE_THREADS / 32][4];
     uint32_t tile_prefix[4];
     uint32_t hdr[16];  // tile geometry broadcast
-    // seg_transfer for every (step, xb, yb, fits_x, fits_y): entry
-    // 16 * step + 8 xb + 4 yb + 2 fits_x + fits_y
-    uint32_t trans_tab[80];
 };
 
 // Starts copying words [g0, g1) of an operand into shared memory (128-bit
@@ -216,7 +278,7 @@ __device__ __forceinline__ uint32_t first_end_after(const uint32_t* se, uint32_t
 
 // Segment record kept in registers between the two passes.
 struct SegRec {
-    uint32_t pos, val, bits;  // bits: trans(20) | cls<<20 | head<<22 | xfill<<23 | yfill<<24
+    uint32_t pos, val, bits;  // bits: cls | head << 2 | flag << 3
 };
 
 template <int OP, bool FSM, bool UNARY, bool FLIP, int TB>
@@ -227,19 +289,15 @@ __global__ void __launch_bounds__(MERGE_THREADS, 2) k_merge(MergeArgs A) {
     TileShared& S = *reinterpret_cast<TileShared*>(smem_raw);
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
 
-    // ---- claim a tile and read the launch epoch (two threads, so the two
-    // round trips overlap; the epoch only changes after the last CTA of the
-    // previous launch on this stream finished)
-    if (tid == 0) S.hdr[0] = claim_tile(A.sync);
-    if (tid == 32) S.hdr[1] = ld_cg(&A.sync->epoch);
-    if (FSM && tid >= 64 && tid < 64 + 80) {
-        const uint32_t e = tid - 64;
-        S.trans_tab[e] = seg_transfer(e >> 4, (e >> 3) & 1u, (e >> 2) & 1u, (e >> 1) & 1u, e & 1u);
-    }
-    __syncthreads();
-    const uint32_t t = S.hdr[0];
-    const uint32_t epoch = S.hdr[1];
+    // tile = block: blocks are dispatched in order, so a tile's predecessors
+    // are running or done (and every wait is bounded)
+    const uint32_t t = blockIdx.x;
     const uint32_t G = A.groups;
+    pdl_wait();
+    pdl_launch();
+    // the launch epoch, read while the tile is found (it only changes after
+    // the last CTA of the previous launch on this stream finished)
+    if (tid == MERGE_THREADS - 1) S.hdr[1] = ld_cg(&A.sync->epoch);
 
     // ---- tile geometry
     if (UNARY) {
@@ -339,9 +397,8 @@ __global__ void __launch_bounds__(MERGE_THREADS, 2) k_merge(MergeArgs A) {
     // ---- pass 1: one record per event, the thread aggregate
     SegRec seg[SEG_PER_THREAD];
     Agg agg = agg_identity();
-    uint32_t fsm_run = FSM_IDENTITY;
-    bool has_head = false;
-    uint32_t h_pre = FSM_IDENTITY, h_bits = 0;  // transfer before the last head, its bits
+    uint32_t last = 0;  // the record of the last head (when agg.nheads > 0)
+    bool walks = false; // a flag needs words further back
     {
         uint32_t pos = 0;
         uint32_t prevcls = C_NONE;
@@ -387,67 +444,72 @@ __global__ void __launch_bounds__(MERGE_THREADS, 2) k_merge(MergeArgs A) {
                 if (segend > pos) {
                     const uint32_t cls = cls_of(val);
                     const bool head = (cls == C_MIXED) || (cls != prevcls);
-                    uint32_t trans = 0;
-                    if (FSM) {
-                        const uint32_t xe2 = xendk(kx), ye2 = yendk(ky);
-                        const bool xb = (pos == xstart(kx)), yb = (pos == ystart(ky));
-                        const uint32_t sel = select_step(OP, xw_, xe2 - pos, yw_, ye2 - pos);
-                        trans = S.trans_tab[16u * sel + (xb ? 8u : 0u) + (yb ? 4u : 0u) +
-                                            (xe2 <= ye2 ? 2u : 0u) + (ye2 <= xe2 ? 1u : 0u)];
-                    }
                     const uint32_t len = segend - pos;
                     agg.popc += (cls == C_MIXED) ? __popc(val) : (cls == C_ONE ? len * 31u : 0u);
-                    const uint32_t bits = trans | (cls << 20) | ((head ? 1u : 0u) << 22) |
-                                          ((is_fill(xw_) ? 1u : 0u) << 23) | ((is_fill(yw_) ? 1u : 0u) << 24);
-                    if (head) {
-                        ++agg.nheads;
-                        agg.pos = pos;
-                        has_head = true;
-                        h_pre = fsm_run;
-                        h_bits = bits;
+                    uint32_t code = SF_NO;  // count-1 flag, should the run be this one group
+                    if (UNARY) {
+                        code = is_fill(xw_) ? SF_YES : SF_NO;
+                    } else if (FSM && head && cls != C_MIXED && len == 1u) {
+                        code = single_flag(OP, xw_, yw_, pos == xstart(kx), pos == ystart(ky), xendk(kx) == pos + 1u,
+                                           yendk(ky) == pos + 1u);
+                        walks |= code > SF_YES;
                     }
                     seg[q].pos = pos;
                     seg[q].val = val;
-                    seg[q].bits = bits;
-                    if (FSM) fsm_run = fsm_compose(fsm_run, trans);
+                    seg[q].bits = cls | (head ? 4u : 0u) | (code << 3);
+                    if (head) {
+                        ++agg.nheads;
+                        agg.pos = pos;
+                        last = q;
+                    }
                     prevcls = cls;
                     pos = segend;
                 }
                 if (UNARY || take_x) ++i; else ++j;
             }
         }
-        // last head: class and count-1 flag for every incoming step state
-        uint32_t fmask = 0;
-        if (has_head) {
-            if (FSM) {
-                const uint32_t tr = h_bits & 0xFFFFFu;
+    }
+    if (FSM && __any_sync(0xffffffffu, walks)) {
 #pragma unroll
-                for (uint32_t s = 0; s < 5; ++s) {
-                    const uint32_t sp = fsm_apply(h_pre, s);
-                    const bool st = fsm_started(tr, sp);
-                    const uint32_t sn = fsm_apply(tr, sp);
-                    const bool f = seg_fill_flag(sn, st, (h_bits >> 23) & 1u ? HEADER0 | 1u : 0u,
-                                                 (h_bits >> 24) & 1u ? HEADER0 | 1u : 0u);
-                    fmask |= (f ? 1u : 0u) << s;
-                }
-            } else if (UNARY) {
-                fmask = ((h_bits >> 23) & 1u) ? 31u : 0u;
+        for (int q = 0; q < SEG_PER_THREAD; ++q) {
+            uint32_t code = seg[q].bits == 0xFFFFFFFFu ? SF_NO : seg[q].bits >> 3;
+            const uint32_t p = seg[q].pos;
+            uint32_t todo = __ballot_sync(0xffffffffu, code > SF_YES);
+            uint32_t xi = 0, yi = 0;  // the words covering p
+            if (code > SF_YES) {
+                xi = gx0 + first_end_after(S.ex, hx, p);
+                yi = gy0 + first_end_after(S.ey, hy, p);
             }
+            while (todo) {
+                const uint32_t l = __ffs(todo) - 1u;
+                todo &= todo - 1u;
+                const bool f = walk_flag<OP>(Operands{A.xw, A.xbp, A.yw, A.ybp}, __shfl_sync(0xffffffffu, code, l),
+                                             __shfl_sync(0xffffffffu, p, l), __shfl_sync(0xffffffffu, xi, l),
+                                             __shfl_sync(0xffffffffu, yi, l));
+                if (lane == l) code = f ? SF_YES : SF_NO;
+            }
+            if (seg[q].bits != 0xFFFFFFFFu) seg[q].bits = (seg[q].bits & 7u) | (code << 3);
         }
-        agg.info = mk_info(has_head ? (h_bits >> 20) & 3u : 0u, has_head, fmask, fsm_run & 0x7FFFu);
+    }
+    if (agg.nheads) {
+        uint32_t lb = 0;
+#pragma unroll
+        for (int q = 0; q < SEG_PER_THREAD; ++q)
+            if (last == (uint32_t)q) lb = seg[q].bits;
+        agg.info = mk_info(lb & 3u, true, (lb >> 3) & 1u);
     }
     // ---- block-wide exclusive scan of the aggregates
     Agg incl = agg;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
-        Agg o = agg_shfl_up<FSM>(incl, d);
-        if (lane >= (uint32_t)d) incl = agg_combine<FSM>(o, incl);
+        Agg o = agg_shfl_up(incl, d);
+        if (lane >= (uint32_t)d) incl = agg_combine(o, incl);
     }
     if (lane == 31) {
         uint4 v = agg_pack(incl);
         S.warp_agg[warp][0] = v.x; S.warp_agg[warp][1] = v.y; S.warp_agg[warp][2] = v.z; S.warp_agg[warp][3] = v.w;
     }
-    Agg excl_in_warp = agg_shfl_up<FSM>(incl, 1);
+    Agg excl_in_warp = agg_shfl_up(incl, 1);
     if (lane == 0) excl_in_warp = agg_identity();
     __syncthreads();
     if (warp == 0) {
@@ -459,10 +521,10 @@ __global__ void __launch_bounds__(MERGE_THREADS, 2) k_merge(MergeArgs A) {
         Agg wi = w;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
-            Agg o = agg_shfl_up<FSM>(wi, d);
-            if (lane >= (uint32_t)d) wi = agg_combine<FSM>(o, wi);
+            Agg o = agg_shfl_up(wi, d);
+            if (lane >= (uint32_t)d) wi = agg_combine(o, wi);
         }
-        Agg wx = agg_shfl_up<FSM>(wi, 1);
+        Agg wx = agg_shfl_up(wi, 1);
         if (lane == 0) wx = agg_identity();
         const Agg tot = agg_unpack(make_uint4(__shfl_sync(0xffffffffu, wi.nheads, NW - 1),
                                               __shfl_sync(0xffffffffu, wi.pos, NW - 1),
@@ -473,16 +535,23 @@ __global__ void __launch_bounds__(MERGE_THREADS, 2) k_merge(MergeArgs A) {
             S.warp_agg[lane][0] = pv.x; S.warp_agg[lane][1] = pv.y; S.warp_agg[lane][2] = pv.z; S.warp_agg[lane][3] = pv.w;
         }
         // ---- decoupled look-back over the preceding tiles
+        const uint32_t epoch = S.hdr[1];
         Agg prefix = agg_identity();
         if (t == 0) {
-            if (lane == 0) publish(&A.recs[0], epoch, REC_INCL, agg_pack(tot));
+            if (lane == 0) {
+                // every other tile writes its metadata after this record has
+                // reached it
+                A.meta->nfill = 0;
+                A.meta->status = 0;
+                publish(&A.recs[0], epoch, REC_INCL, agg_pack(tot));
+            }
         } else {
             if (lane == 0) publish(&A.recs[t], epoch, REC_AGG, agg_pack(tot));
             bool ok;
-            prefix = agg_unpack(warp_lookback(A.recs, t, epoch, agg_pack(agg_identity()), AggComb<FSM>(), &ok));
+            prefix = agg_unpack(warp_lookback(A.recs, t, epoch, agg_pack(agg_identity()), AggComb(), &ok));
             if (lane == 0) {
                 if (!ok) atomicExch(&A.meta->status, DEV_ERR_TIMEOUT);
-                publish(&A.recs[t], epoch, REC_INCL, agg_pack(agg_combine<FSM>(prefix, tot)));
+                publish(&A.recs[t], epoch, REC_INCL, agg_pack(agg_combine(prefix, tot)));
             }
         }
         if (lane == 0) {
@@ -490,10 +559,10 @@ __global__ void __launch_bounds__(MERGE_THREADS, 2) k_merge(MergeArgs A) {
             S.tile_prefix[0] = pv.x; S.tile_prefix[1] = pv.y; S.tile_prefix[2] = pv.z; S.tile_prefix[3] = pv.w;
             // the last tile finishes the result
             if (t == A.ntiles - 1) {
-                Agg all = agg_combine<FSM>(prefix, tot);
+                Agg all = agg_combine(prefix, tot);
                 const uint32_t n = all.nheads;
                 if (agg_has(all.info) && agg_cls(all.info) != C_MIXED) {
-                    const bool f = (agg_fmask(all.info) & 1u) != 0;
+                    const bool f = agg_flag(all.info);
                     const uint32_t w = run_word(agg_cls(all.info), G - all.pos, 0, f);
                     A.out[n - 1] = w;
                     if (n - 1 == 0) A.meta->w0 = w;
@@ -513,29 +582,18 @@ __global__ void __launch_bounds__(MERGE_THREADS, 2) k_merge(MergeArgs A) {
     // ---- pass 2: emit words
     Agg tp = agg_unpack(make_uint4(S.tile_prefix[0], S.tile_prefix[1], S.tile_prefix[2], S.tile_prefix[3]));
     Agg wp = agg_unpack(make_uint4(S.warp_agg[warp][0], S.warp_agg[warp][1], S.warp_agg[warp][2], S.warp_agg[warp][3]));
-    Agg pre = agg_combine<FSM>(agg_combine<FSM>(tp, wp), excl_in_warp);
+    Agg pre = agg_combine(agg_combine(tp, wp), excl_in_warp);
     uint32_t idx = pre.nheads;
     bool lhas = agg_has(pre.info);
     uint32_t lcls = agg_cls(pre.info), lpos = pre.pos;
-    bool lf = (agg_fmask(pre.info) & 1u) != 0;
-    uint32_t state = fsm_apply(agg_fsm(pre.info), 0u);
+    bool lf = agg_flag(pre.info);
     bool wrote_fill = false;
 #pragma unroll
     for (int k = 0; k < SEG_PER_THREAD; ++k) {
         const SegRec& s = seg[k];
         if (s.bits == 0xFFFFFFFFu) continue;
-        const uint32_t tr = s.bits & 0xFFFFFu;
-        bool f = false;
-        if (FSM) {
-            const bool st = fsm_started(tr, state);
-            state = fsm_apply(tr, state);
-            f = seg_fill_flag(state, st, (s.bits >> 23) & 1u ? HEADER0 | 1u : 0u,
-                              (s.bits >> 24) & 1u ? HEADER0 | 1u : 0u);
-        } else if (UNARY) {
-            f = (s.bits >> 23) & 1u;
-        }
-        if ((s.bits >> 22) & 1u) {  // head
-            const uint32_t cls = (s.bits >> 20) & 3u;
+        if ((s.bits >> 2) & 1u) {  // head
+            const uint32_t cls = s.bits & 3u;
             if (lhas && lcls != C_MIXED) {
                 const uint32_t w = run_word(lcls, s.pos - lpos, 0, lf);
                 A.out[idx - 1] = w;
@@ -548,7 +606,7 @@ __global__ void __launch_bounds__(MERGE_THREADS, 2) k_merge(MergeArgs A) {
             }
             if ((idx & 31u) == 0) A.obp[idx >> 5] = s.pos;
             ++idx;
-            lhas = true; lcls = cls; lpos = s.pos; lf = f;
+            lhas = true; lcls = cls; lpos = s.pos; lf = (s.bits >> 3) & 1u;
         }
     }
     if (wrote_fill) atomicOr(&A.meta->nfill, 1u);
