@@ -28,13 +28,14 @@
 //    whose length reaches the next head.
 // Bound by instruction issue (the integer pipe first) and the few warps that
 // two buffers per warp leave room for.  At 2^28 bits, both operands of d =
-// 0.1 / 0.5: 39 / 44 us a call against 79 / 65 for the form before it (a
+// 0.1 / 0.5: 39 / 40 us a call against 79 / 65 for the form before it (a
 // word-start marker per word and warp max-scans over 128 groups, operands
 // staged without prefetch, four neighbouring groups per lane; ~2370 + 1060
-// instructions per tile against 715 + 720); both of d = 0.01 through the _c2
-// path: 43 us against 58 for the word-space merge.  Tiles of 256 groups
-// double the resident warps and are slower (46 / 50 us: the per-tile work);
-// launching each kernel while the one before it drains saves 3 us a call.
+// instructions per tile against 715 + 720).  Tiles of 256 groups double the
+// resident warps and are slower (46 / 50 us: the per-tile work), and so is
+// packing a tile's words in k_gop with k_gpack a copy (45 / 48: the integer
+// pipe is busy 69 % of the time there); launching each kernel while the one
+// before it drains saves 3 us a call.
 #ifndef WAH_GOP_CUH
 #define WAH_GOP_CUH
 #include <type_traits>
@@ -579,15 +580,17 @@ __global__ void __launch_bounds__(GCTA) k_gpack(const __grid_constant__ GopArgs 
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const uint32_t rv = rl[32 * (r0 + j)];
-                const uint32_t above = q[j].x & gt;  // the row's heads after this lane
-                // groups to the next head: in the row (its lowest bit above
-                // this lane), else past the row's end
-                const uint32_t low = 31u - __clz(above & (0u - above));  // -1: none
-                uint32_t len = low - lane;
-                if (above == 0u) len = q[j].z + (32u - lane);
-                const bool f = (q[j].w & bit) && (len >= 2u || rv >= HEADER0);
                 uint32_t wd = rv & ALLONES;
-                if (f) wd = (rv & FILLBIT) | len | HEADER0;
+                if (q[j].w) {  // heads of runs among them
+                    const uint32_t above = q[j].x & gt;  // the row's heads after this lane
+                    // groups to the next head: in the row (its lowest bit
+                    // above this lane), else past the row's end
+                    const uint32_t low = 31u - __clz(above & (0u - above));  // -1: none
+                    uint32_t len = low - lane;
+                    if (above == 0u) len = q[j].z + (32u - lane);
+                    const bool f = (q[j].w & bit) && (len >= 2u || rv >= HEADER0);
+                    if (f) wd = (rv & FILLBIT) | len | HEADER0;
+                }
                 if (q[j].x & bit) {
                     A.out[q[j].y + __popc(q[j].x & lt)] = wd;
                     any |= wd;
@@ -595,6 +598,9 @@ __global__ void __launch_bounds__(GCTA) k_gpack(const __grid_constant__ GopArgs 
             }
         }
         if (t == 0 && lane == 0) A.meta->w0 = A.out[0];  // this lane's own store: group 0 is a head
+        // R is read once: its lines need not be written back to memory when
+        // operands, R and words outgrow L2 (2^28 bits of d = 0.5: 44 -> 40 us)
+        if (lane < PT / 32u) asm volatile("discard.global.L2 [%0], 128;" ::"l"(A.R + g0 + 32u * lane) : "memory");
         __syncwarp();  // the rows and the buffer are free again
     }
     if (__any_sync(0xffffffffu, any >= HEADER0) && lane == 0) A.meta->nfill = 1u;
