@@ -573,12 +573,12 @@ static void launch_merge_tb(const wahgpu_ctx* ctx, int op, bool fsm, bool unary,
 // Block-index entries per merge tile: the context's setting, else by the
 // operands' size.  Small operands spread over the GPU in short tiles; long
 // tiles share their fixed steps among more words (2^28 bits, us at 16 / 32 /
-// 64 entries: 4.6 K blocks 14.5 / 13.3 / 14.7, 14 K 25.7 / 17.6 / 17.1, 45 K
-// 63 / 42 / 34).
+// 64 entries: 4.6 K blocks 14.8 / 13.3 / 15.4, 14 K 25.7 / 17.7 / 18.1, 45 K
+// 63 / 42 / 26).
 static uint32_t merge_tile_blocks(const wahgpu_ctx* ctx, uint32_t nblocks) {
     if (ctx->merge_tile) return ctx->merge_tile;
     const uint64_t sms = (uint64_t)ctx->sm_count;
-    if (nblocks >= sms * 88u) return 64;
+    if (nblocks >= sms * 128u) return 64;
     if (nblocks >= sms * 30u) return 32;
     return 16;
 }
@@ -921,8 +921,8 @@ int wg_launch_gone(wahgpu_ctx* ctx, int op, wahgpu_bv* x, wahgpu_bv* y, uint32_t
 // merge by the words, each at least its chain of steps.  Curves through
 // measured calls of & | - at 2^16 .. 2^28 bits, d = 1e-4 .. 0.06, in us:
 // group space 7.3 at 0.13M groups, 15 at 2.2M, 41 at 8.7M; merge 7.7 at 400
-// words of both operands, 9.8 at 7 K, 12.3 at 63 K, 17 at 0.4M, 37 at 1.4M,
-// 87 at 4M.  The row index an operand lacks is charged to its first use; an
+// words of both operands, 9.8 at 7 K, 12.3 at 63 K, 17 at 0.4M, 29 at 1.4M,
+// 72 at 4M.  The row index an operand lacks is charged to its first use; an
 // operand that comes back is taken to come again.  A merge tile set on the
 // context asks for the merge.
 static bool in_group_space(const wahgpu_ctx* ctx, wahgpu_bv* x, wahgpu_bv* y, uint32_t groups) {
@@ -934,7 +934,7 @@ static bool in_group_space(const wahgpu_ctx* ctx, wahgpu_bv* x, wahgpu_bv* y, ui
         if (!b->rows_valid && !b->used) in_groups += 3.0 + 1.5 * g;
         b->used = true;
     }
-    return in_groups < 7.0 + 0.5 * std::log2(1.0 + n / 200.0) + (y ? 17e-6 : 12e-6) * n;
+    return in_groups < 7.0 + 0.5 * std::log2(1.0 + n / 200.0) + (y ? 13e-6 : 10e-6) * n;
 }
 
 // x, or its complement, as compress() leaves it.

@@ -25,7 +25,7 @@
 // state is carried for them.
 //
 // Bound by the chain of dependent steps of a tile (search, loads, scans,
-// look-back).  2^28 bits, d = 1e-3 / 1e-2: 14 / 37 us a call.  The form
+// look-back).  2^28 bits, d = 1e-3 / 1e-2: 14 / 29 us a call.  The form
 // that carried the walk's five step states as transfer functions through the
 // scans, claimed its tile by an atomic and had its metadata cleared by a
 // memset took 23.5 / 58.
@@ -281,8 +281,11 @@ struct SegRec {
     uint32_t pos, val, bits;  // bits: cls | head << 2 | flag << 3
 };
 
+// Many tiles in flight hide the chain of steps in each: at 1.4M words 5 CTAs
+// per SM take 29 us, 4 take 35, 2 or 3 take 37 (tiles of 64 entries, which
+// only such sizes use; fewer, shorter tiles do not fill the SMs anyway).
 template <int OP, bool FSM, bool UNARY, bool FLIP, int TB>
-__global__ void __launch_bounds__(MERGE_THREADS, 2) k_merge(MergeArgs A) {
+__global__ void __launch_bounds__(MERGE_THREADS, TB == 64 ? 5 : 4) k_merge(MergeArgs A) {
     constexpr int TILE_BLOCKS = TB, SEG_PER_THREAD = MCfg<TB>::SEG_PER_THREAD;
     using TileShared = wah::TileShared<TB>;
     extern __shared__ __align__(16) unsigned char smem_raw[];

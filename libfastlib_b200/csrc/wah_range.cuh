@@ -149,7 +149,7 @@ enum RangeMode : int {
     RM_IDS = 2,     // two passes, second: row ids at the items' offsets
     RM_LOOK = 3     // one pass: counts and row ids, offsets by a look-back
 };
-constexpr uint32_t RSTAGE = 32 * 31;  // row ids of 32 groups at most
+constexpr uint32_t RSTAGE = 32 * 31 + 4;  // row ids of 32 groups at most, from the output's place in 16 bytes on
 struct RangeShared {
     uint32_t hdr[8];
     uint64_t base;
@@ -740,12 +740,13 @@ __global__ void __launch_bounds__(RTHREADS, 6) k_range(RangeArgs A) {
         if (A.rids && cnt) {
             // capped: offsets are within the query; ids past its limit are
             // dropped and the rest land in its region
-            const uint64_t lim = A.capped ? DQ.rid_lim : A.rid_cap;
             const uint64_t rbase0 = A.capped ? DQ.rid_base : 0ull;
+            const uint64_t room = A.rid_cap > rbase0 ? A.rid_cap - rbase0 : 0ull;
+            const uint64_t lim = A.capped ? min(DQ.rid_lim, room) : room;
             // 32 groups at a time: lane l takes group 32 r + l from the lane
-            // owning its quad and expands it into the warp's staging, then
-            // the warp stores the run of ids with neighbouring lanes on
-            // neighbouring slots
+            // owning its quad and expands it into the warp's staging, then the
+            // warp stores the run of ids, neighbouring lanes on neighbouring
+            // 16 bytes of the output (single ids at its ragged ends)
             uint32_t* st = S.tmp + warp * RSTAGE;
             uint64_t off = base + before;
 #pragma unroll
@@ -756,7 +757,7 @@ __global__ void __launch_bounds__(RTHREADS, 6) k_range(RangeArgs A) {
                     const uint32_t src = 8u * r + (lane >> 2);
                     const uint32_t x = __shfl_sync(0xffffffffu, acc[i].x, src), y = __shfl_sync(0xffffffffu, acc[i].y, src);
                     const uint32_t z = __shfl_sync(0xffffffffu, acc[i].z, src), w = __shfl_sync(0xffffffffu, acc[i].w, src);
-                    uint32_t bits = lane & 2u ? (lane & 1u ? w : z) : (lane & 1u ? y : x);
+                    uint32_t bits = (lane & 2u ? (lane & 1u ? w : z) : (lane & 1u ? y : x)) << 1;  // row 0 at bit 31
                     const uint32_t c = __popc(bits);
                     uint32_t s = c;
 #pragma unroll
@@ -765,17 +766,25 @@ __global__ void __launch_bounds__(RTHREADS, 6) k_range(RangeArgs A) {
                         if (lane >= (uint32_t)d) s += u;
                     }
                     const uint32_t rt = __shfl_sync(0xffffffffu, s, 31);
-                    uint32_t p = s - c;
+                    const uint32_t sh = (uint32_t)(rbase0 + off) & 3u;
+                    uint32_t* p = st + (sh + s - c);
                     const uint32_t row = (g0 + 4u * (warp * (32u * Q) + 32u * i + 8u * r) + lane) * 31u;
                     while (bits) {
-                        const uint32_t hb = 31u - __clz(bits);
-                        st[p++] = row + (30u - hb);
-                        bits &= ~(1u << hb);
+                        const uint32_t k = __clz(bits);
+                        *p++ = row + k;
+                        bits &= ~(0x80000000u >> k);
                     }
                     __syncwarp();
-                    for (uint32_t j = lane; j < rt; j += 32u) {
-                        const uint64_t o = off + j;
-                        if (o < lim && rbase0 + o < A.rid_cap) A.rids[rbase0 + o] = st[j];
+                    const uint32_t end = sh + (uint32_t)min((uint64_t)rt, lim - off);
+                    uint32_t* out = A.rids + (rbase0 + off - sh);  // 16-byte aligned
+                    for (uint32_t j = 4u * lane; j < end; j += 128u) {
+                        if (j >= sh && j + 4u <= end) {
+                            *reinterpret_cast<uint4*>(out + j) = *reinterpret_cast<const uint4*>(st + j);
+                        } else {
+#pragma unroll
+                            for (uint32_t e = 0; e < 4u; ++e)
+                                if (j + e >= sh && j + e < end) out[j + e] = st[j + e];
+                        }
                     }
                     __syncwarp();
                     off += rt;
