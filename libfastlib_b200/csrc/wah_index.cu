@@ -227,8 +227,8 @@ int wg_index_attach(wahgpu_index* x) {
     x->dev.tl_off = x->d_tl_off; x->dev.tl_bm = x->d_tl_bm;
     x->dev.cum = x->d_cum; x->dev.cum_stride = x->cum_stride; x->dev.cum_k = x->cum_k;
     x->dev.gx = (x->groups + (x->anb ? 1u : 0u) + 3u) & ~3u;
-    x->dev.values = nullptr; x->dev.nobs = nobs; x->dev.vtype = 0; x->dev.ntiles = x->ntiles;
-    if (x->d_values) { x->dev.values = x->d_values; x->dev.vtype = x->vtype; }
+    x->dev.values = nullptr; x->dev.nobs = nobs; x->dev.ntiles = x->ntiles;
+    if (x->d_values) x->dev.values = x->d_values;
     return WAHGPU_OK;
 }
 
@@ -242,7 +242,6 @@ extern "C" int wahgpu_index_set_values(wahgpu_index* x, int vtype, const void* v
     CUDA_TRY(ctx, cudaMemcpyAsync(x->d_values, values, n * 4, cudaMemcpyHostToDevice, ctx->stream));
     x->vtype = (uint32_t)vtype;
     x->dev.values = x->d_values;
-    x->dev.vtype = x->vtype;
     return WAHGPU_OK;
 }
 
@@ -295,7 +294,6 @@ enum LocMode { LOC_HITS = 0, LOC_LOWER = 1, LOC_UPPER = 2 };
 static int locate(wahgpu_ctx* ctx, const wahgpu_index* x, const wahgpu_term* t, DevTerm& out,
                   int mode = LOC_HITS) {
     out = DevTerm{};
-    out.lop = (uint32_t)t->lop; out.rop = (uint32_t)t->rop; out.lo = t->lo; out.hi = t->hi;
     uint32_t h0 = 0, h1 = 0, nc = 0;
     if (x->kind == WAHGPU_RELIC) {
         // keys ascending: the passing keys are one interval, found by the
@@ -373,6 +371,12 @@ static int locate(wahgpu_ctx* ctx, const wahgpu_index* x, const wahgpu_term* t, 
     }
     if (nc > 0 && !x->d_values)
         return wg_fail(ctx, WAHGPU_EINVAL, "range needs row checks but the index has no raw values attached");
+    if (nc > 0) {
+        // the edge rows' comparison in the column's value keys
+        const KeyMap m = key_map(x->vtype);
+        out.kflip = m.flip; out.ksign = m.sign;
+        if (!key_range(x->vtype, (uint32_t)t->lop, t->lo, (uint32_t)t->rop, t->hi, out.klo, out.kspan)) nc = 0;
+    }
     out.h0 = h0; out.h1 = h1; out.ncand = nc;
     if (x->cum_k && x->cum_stride == 1) {
         // a row per bitmap: the span and the edge bitmaps by rows

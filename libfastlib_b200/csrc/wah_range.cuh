@@ -42,6 +42,7 @@
 #ifndef WAH_RANGE_CUH
 #define WAH_RANGE_CUH
 #include "wah_dev.cuh"
+#include "wah_keys.h"
 
 namespace wah {
 
@@ -75,12 +76,9 @@ struct DevIndex {
     uint32_t cum_stride, cum_k, gx, pad2;  // gx: groups incl. the active one, rounded up to 4
     const void* values;        // raw column (nrows), or null
     uint32_t nobs;
-    uint32_t vtype;            // 0 uint32, 1 float32, 2 int32
     uint32_t ntiles;
-    uint32_t pad;
 };
 
-// comparison ops (qExpr::COMPARE): 0 none, 1 <, 2 <=
 struct DevTerm {
     uint32_t index;       // into the DevIndex table
     uint32_t h0, h1;      // bitmaps wholly inside: [h0, h1)
@@ -90,10 +88,11 @@ struct DevTerm {
     uint32_t c0, c1, e0, e1;
     uint32_t ncand;       // edge bitmaps to check row by row (0..2)
     uint32_t cand[2];
-    uint32_t lop, rop;    // lo lop x rop hi
+    uint32_t klo, kspan;  // the range in value keys
+    uint32_t kflip, ksign;  // the column's KeyMap
     uint32_t dense;       // the index keeps a row per bitmap: span C(c1) & ~C(c0) (c1 == 0: empty), edges by rows
+    uint32_t pad;
     const uint32_t* cum;  // dense: the index's rows
-    double lo, hi;
 };
 
 struct DevQuery {
@@ -175,21 +174,9 @@ static_assert(sizeof(DevIndex) % 4 == 0 && INDEX_WORDS <= 32, "a warp stages an 
 // 16-byte vector in order.  rsw4: the same for quad index l (groups 4l..).
 __device__ __forceinline__ uint32_t rsw(uint32_t l) { return l ^ (((l >> 5) & 7u) << 2); }
 __device__ __forceinline__ uint32_t rsw4(uint32_t l) { return l ^ ((l >> 3) & 7u); }
-__device__ __forceinline__ bool pass_cmp(double v, uint32_t lop, double lo, uint32_t rop, double hi) {
-    const bool a = lop == 0 ? true : (lop == 1 ? lo < v : lo <= v);
-    const bool b = rop == 0 ? true : (rop == 1 ? v < hi : v <= hi);
-    return a && b;
-}
-// a column value from its 4 raw bytes (0 uint32, 1 float32, 2 int32)
-__device__ __forceinline__ double raw_value(uint32_t v, uint32_t vtype) {
-    if (vtype == 1) return (double)__uint_as_float(v);
-    if (vtype == 2) return (double)(int32_t)v;
-    return (double)v;
-}
-__device__ __forceinline__ double col_value(const void* vals, uint32_t vtype, uint32_t row) {
-    if (vtype == 1) return (double)__ldg(reinterpret_cast<const float*>(vals) + row);
-    if (vtype == 2) return (double)__ldg(reinterpret_cast<const int32_t*>(vals) + row);
-    return (double)__ldg(reinterpret_cast<const uint32_t*>(vals) + row);
+// Does a raw value (4 bytes of the column) pass the term's comparison?
+__device__ __forceinline__ bool pass_key(uint32_t v, const DevTerm& T) {
+    return value_key(v, KeyMap{T.kflip, T.ksign}) - T.klo <= T.kspan;
 }
 
 // One warp ORs bitmap b's words for the tile [g0, g1) into S.tmp (the
@@ -315,7 +302,7 @@ __device__ __forceinline__ void warp_check_bitmap(RangeShared& S, const DevIndex
                 uint32_t bits = wpattern(wd), set = 0;
                 if (lit) {
                     const uint32_t hb = 31u - __clz(bits);
-                    if (pass_cmp(raw_value(v0[j], I.vtype), T.lop, T.lo, T.rop, T.hi)) set |= 1u << hb;
+                    if (pass_key(v0[j], T)) set |= 1u << hb;
                     bits &= ~(1u << hb);
                 }
                 while (bits) {
@@ -330,7 +317,7 @@ __device__ __forceinline__ void warp_check_bitmap(RangeShared& S, const DevIndex
                         v[q] = hb[q] < 32u ? __ldg(raw + g * 31u + (30u - hb[q])) : 0u;
 #pragma unroll
                     for (int q = 0; q < RCHK; ++q)
-                        if (hb[q] < 32u && pass_cmp(raw_value(v[q], I.vtype), T.lop, T.lo, T.rop, T.hi))
+                        if (hb[q] < 32u && pass_key(v[q], T))
                             set |= 1u << hb[q];
                 }
                 if (set) atomicOr(&S.tmp[rsw(g - g0)], set);
@@ -344,7 +331,7 @@ __device__ __forceinline__ void warp_check_bitmap(RangeShared& S, const DevIndex
         while (bits) {
             const uint32_t hb = 31u - __clz(bits);
             const uint32_t row = Gb * 31u + (30u - hb);
-            if (pass_cmp(col_value(I.values, I.vtype, row), T.lop, T.lo, T.rop, T.hi)) set |= 1u << hb;
+            if (pass_key(__ldg(raw + row), T)) set |= 1u << hb;
             bits &= ~(1u << hb);
         }
         if (set) atomicOr(&S.tmp[rsw(Gb - g0)], set);
@@ -548,15 +535,14 @@ __device__ __forceinline__ bool any4(uint4 a) { return (a.x | a.y | a.z | a.w) !
 // in 32 groups), so a lane takes one row at a time, whichever group it is in:
 // the warp runs as long as its fullest lane.  (Lining the warp's rows up in
 // shared memory to load 32 at once took 18 % longer.)
-__device__ __forceinline__ uint4 check_quad(uint4 e, uint32_t g, const uint32_t* __restrict__ raw, uint32_t vtype,
-                                            const DevTerm& T) {
+__device__ __forceinline__ uint4 check_quad(uint4 e, uint32_t g, const uint32_t* __restrict__ raw, const DevTerm& T) {
     uint4 r = make_uint4(0u, 0u, 0u, 0u);
     while (any4(e)) {
         const uint32_t j = e.x ? 0u : e.y ? 1u : e.z ? 2u : 3u;
         const uint32_t b = e.x ? e.x : e.y ? e.y : e.z ? e.z : e.w;
         const uint32_t hb = 31u - __clz(b), bit = 1u << hb;  // highest set bit
         const uint32_t v = __ldg(raw + (g + j) * 31u + (30u - hb));
-        const uint32_t keep = pass_cmp(raw_value(v, vtype), T.lop, T.lo, T.rop, T.hi) ? bit : 0u;
+        const uint32_t keep = pass_key(v, T) ? bit : 0u;
         if (j == 0u) { e.x ^= bit; r.x |= keep; }
         else if (j == 1u) { e.y ^= bit; r.y |= keep; }
         else if (j == 2u) { e.z ^= bit; r.z |= keep; }
@@ -589,7 +575,7 @@ __device__ __forceinline__ uint4 dense_terms(const RangeArgs& A, const DevQuery&
             v = andn4(v, z);
             if (any4(e)) {
                 const DevIndex& I = A.idx[T.index];
-                v = or4(v, check_quad(e, g0 + 4u * o, reinterpret_cast<const uint32_t*>(I.values), I.vtype, T));
+                v = or4(v, check_quad(e, g0 + 4u * o, reinterpret_cast<const uint32_t*>(I.values), T));
             }
         } else {
             v = andn4(v, z);
@@ -846,8 +832,8 @@ __global__ void __launch_bounds__(RTHREADS) k_cap_items(RangeArgs A, uint2* __re
 // that the queries share a tile's raw values in L2: the bin's words of the
 // tile 128 at a time, the first set row of every literal loaded before any is
 // compared (few literals of an edge bin hold more).  Bound by those loads'
-// latency.  1000 ranges over 10M rows, 1000 bins: 0.18 ms; 1.1 ms reading the
-// spans and the edges from the cumulative rows, 1.9 ms from a row per 8
+// latency.  1000 ranges over 10M rows, 1000 bins: 0.16 ms (0.18 ms comparing in
+// double: two conversions and comparisons a row); 1.1 ms reading the spans and the edges from the cumulative rows, 1.9 ms from a row per 8
 // bitmaps and the other bitmaps' words.
 struct EdgeArgs {
     const DevIndex* idx;
@@ -874,9 +860,9 @@ __global__ void __launch_bounds__(RTHREADS) k_edge_counts(EdgeArgs A) {
         const uint32_t i1 = min(sn1 < g1 ? in1 + 1u : in1, m.n);
         const uint32_t* w = I.words + m.wstart;
         const uint32_t* raw = reinterpret_cast<const uint32_t*>(I.values);
-        const uint32_t vtype = I.vtype;
-        const uint32_t lop = T.lop, rop = T.rop;
-        const double lo = T.lo, hi = T.hi;
+        const KeyMap km{T.kflip, T.ksign};
+        const uint32_t klo = T.klo, kspan = T.kspan;
+        auto pass = [&](uint32_t v) { return value_key(v, km) - klo <= kspan ? 1u : 0u; };
         uint32_t carry = s0, cnt = 0;
         for (uint32_t base0 = i0; base0 < i1; base0 += 128) {
             uint32_t wv[4], pv[4], v0[4];
@@ -911,11 +897,11 @@ __global__ void __launch_bounds__(RTHREADS) k_edge_counts(EdgeArgs A) {
                 const uint32_t wd = wv[j], p = pv[j];
                 if (wd - 1u < ALLONES) {
                     if (p >= g0 && p < g1) {
-                        cnt += pass_cmp(raw_value(v0[j], vtype), lop, lo, rop, hi);
+                        cnt += pass(v0[j]);
                         for (uint32_t bits = wd & ~(0x80000000u >> __clz(wd)); bits;) {
                             const uint32_t hb = 31u - __clz(bits);
                             bits &= ~(1u << hb);
-                            cnt += pass_cmp(raw_value(__ldg(raw + p * 31u + (30u - hb)), vtype), lop, lo, rop, hi);
+                            cnt += pass(__ldg(raw + p * 31u + (30u - hb)));
                         }
                     }
                 }
@@ -931,7 +917,7 @@ __global__ void __launch_bounds__(RTHREADS) k_edge_counts(EdgeArgs A) {
                     const uint32_t c = __shfl_sync(0xffffffffu, wv[j], l) & MAXCNT;
                     const uint32_t a = max(p, g0) * 31u, e = min(p + c, g1) * 31u;
                     for (uint32_t r = a + lane; r < e; r += 32u)
-                        cnt += pass_cmp(raw_value(__ldg(raw + r), vtype), lop, lo, rop, hi);
+                        cnt += pass(__ldg(raw + r));
                 }
             }
         }
@@ -940,7 +926,7 @@ __global__ void __launch_bounds__(RTHREADS) k_edge_counts(EdgeArgs A) {
             for (uint32_t bits = (m.aval & ((1u << m.anb) - 1u)) << (31u - m.anb); bits;) {
                 const uint32_t hb = 31u - __clz(bits);
                 bits &= ~(1u << hb);
-                cnt += pass_cmp(raw_value(__ldg(raw + m.groups * 31u + (30u - hb)), vtype), lop, lo, rop, hi);
+                cnt += pass(__ldg(raw + m.groups * 31u + (30u - hb)));
             }
         cnt = __reduce_add_sync(0xffffffffu, cnt);
         if (lane == 0 && cnt) atomicAdd(&A.counts[__ldg(A.edge_q + ei)], (unsigned long long)cnt);
