@@ -71,6 +71,13 @@ void* wg_alloc(wahgpu_ctx* ctx, size_t bytes) {
                 ctx->bytes_allocated -= kv.first;
             }
         ctx->pool.clear();
+        if (ctx->gop_scratch && !ctx->gop_captured) {
+            cudaFree(ctx->gop_scratch);
+            ctx->bytes_allocated -= ctx->gop_bytes;
+            ctx->sizes.erase(ctx->gop_scratch);
+            ctx->gop_scratch = nullptr;
+            ctx->gop_bytes = 0;
+        }
         cudaGetLastError();
         if (cudaMalloc(&p, c) != cudaSuccess) { cudaGetLastError(); return nullptr; }
     }
@@ -146,6 +153,32 @@ int wg_scratch(wahgpu_ctx* ctx, uint32_t ntiles, TileRec** recs, LaunchSync** sy
     *sync = reinterpret_cast<LaunchSync*>(ctx->scratch);
     *recs = reinterpret_cast<TileRec*>(reinterpret_cast<char*>(ctx->scratch) + 2 * sizeof(LaunchSync));
     return WAHGPU_OK;
+}
+// The stream's calls are being captured: they run later, and perhaps often.
+bool wg_capturing(const wahgpu_ctx* ctx) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &cs) != cudaSuccess) { cudaGetLastError(); return true; }
+    return cs != cudaStreamCaptureStatusNone;
+}
+// Result patterns of the two-pass engine: one block of the context that grows
+// with its calls and is never handed to anything else, so a captured call's
+// replays write into no other object.  A block that captured calls hold is
+// kept beside the larger one that follows it (at least twice its size, so
+// these come to less than the last) until the context ends.
+static unsigned char* gop_scratch(wahgpu_ctx* ctx, size_t bytes, bool captured) {
+    if (ctx->gop_bytes < bytes) {
+        const size_t want = ctx->gop_captured ? std::max(bytes, 2 * ctx->gop_bytes) : bytes;
+        if (!ctx->gop_captured) wg_free(ctx, ctx->gop_scratch);
+        ctx->gop_scratch = nullptr;
+        ctx->gop_bytes = 0;
+        ctx->gop_captured = false;
+        ctx->gop_scratch = wg_alloc(ctx, want);
+        if (!ctx->gop_scratch) return nullptr;
+        std::lock_guard<std::mutex> g(ctx->mu);
+        ctx->gop_bytes = ctx->sizes[ctx->gop_scratch];
+    }
+    ctx->gop_captured |= captured;
+    return static_cast<unsigned char*>(ctx->gop_scratch);
 }
 // The dense kernel's records, after the TileRec array of the scratch block.
 static uint4* wg_dense_recs(wahgpu_ctx* ctx, TileRec* recs) {
@@ -329,10 +362,9 @@ static void bv_launched(wahgpu_bv* b) {
     wahgpu_ctx* ctx = b->ctx;
     b->h_valid = false;
     b->told = false;
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(ctx->stream, &cs) != cudaSuccess) { cudaGetLastError(); cs = cudaStreamCaptureStatusActive; }
+    const bool later = wg_capturing(ctx);
     std::lock_guard<std::mutex> g(ctx->mu);
-    if (cs != cudaStreamCaptureStatusNone) { bv_unpend(b); return; }
+    if (later) { bv_unpend(b); return; }
     b->pend_stream = ctx->stream;
     if (b->pend < 0) {
         b->pend = (int32_t)ctx->pending.size();
@@ -710,13 +742,16 @@ static bool rows_reserve(wahgpu_bv* b, uint32_t groups, void* (*alloc)(wahgpu_ct
 }
 // Room for a result's row index: a cached block, or, once the context has
 // made a few such results, a new one (a fresh context's first calls do not
-// pay for blocks that may never be read).
+// pay for blocks that may never be read).  A captured call keeps none: until
+// its replay the index would not be that of the words.
 static bool result_rows(wahgpu_bv* res, uint32_t groups) {
+    if (wg_capturing(res->ctx)) return false;
     const bool fresh = res->ctx->row_results < 8;
     if (fresh) res->ctx->row_results++;
     return rows_reserve(res, groups, fresh ? wg_alloc_cached : wg_alloc);
 }
-// Row index of b (host metadata must be valid); built once.
+// Row index of b (host metadata must be valid); built once, and by a captured
+// call on each of its replays.
 static int wg_rows(wahgpu_bv* b) {
     wahgpu_ctx* ctx = b->ctx;
     // positions are taken from the words: none that the upload scan refused
@@ -727,7 +762,7 @@ static int wg_rows(wahgpu_bv* b) {
     k_rows<<<(ntiles + GW - 1) / GW, GCTA, 0, ctx->stream>>>(b->words, b->bpos, b->h.n, b->h.groups, ntiles, b->rows);
     ctx->launches++;
     CUDA_TRY(ctx, cudaGetLastError());
-    b->rows_valid = true;
+    b->rows_valid = !wg_capturing(ctx);
     return WAHGPU_OK;
 }
 
@@ -749,6 +784,11 @@ static void launch_gop_kind(const wahgpu_ctx* ctx, int op, uint32_t ntiles, cuda
     }
 }
 
+static size_t gop_bytes(uint32_t groups) {
+    const size_t ntiles = ((uint64_t)groups + PT - 1) / PT;
+    return ntiles * (PT * 4 + TROWS * sizeof(uint2) + 12);
+}
+
 // Two-pass group-space engine (wah_gop.cuh): the result patterns per group
 // with head masks and per-CTA totals, then the words.  kind: GopKind; y is
 // null for the copies.
@@ -763,7 +803,7 @@ int wg_launch_gop(wahgpu_ctx* ctx, int kind, int op, wahgpu_bv* x, wahgpu_bv* y,
     // is at hand; else they are part of the scratch
     const bool keep = result_rows(res, groups);
     const size_t rb = (size_t)ntiles * PT * 4, hb = (size_t)ntiles * TROWS * sizeof(uint2);
-    unsigned char* scr = static_cast<unsigned char*>(wg_alloc(ctx, rb + hb + (size_t)ntiles * 12));
+    unsigned char* scr = gop_scratch(ctx, gop_bytes(groups), wg_capturing(ctx));
     if (!scr) return wg_fail(ctx, WAHGPU_ENOMEM, "allocation of %u tiles of result patterns failed", ntiles);
     uint32_t* tot = reinterpret_cast<uint32_t*>(scr + rb + hb);
     GopArgs a;
@@ -787,9 +827,6 @@ int wg_launch_gop(wahgpu_ctx* ctx, int kind, int op, wahgpu_bv* x, wahgpu_bv* y,
     wg_launch_pdl(k_gpack, grid, GCTA, sm, s, a);
     ctx->launches += 2;
     const cudaError_t e = cudaGetLastError();
-    // stream-ordered: the next user of the block on this context's stream
-    // runs after the launches above
-    wg_free(ctx, scr);
     if (e != cudaSuccess) return wg_fail(ctx, WAHGPU_ECUDA, "launch failed: %s", cudaGetErrorString(e));
     bv_launched(res);
     res->gt_valid = false;
@@ -924,9 +961,14 @@ int wg_launch_gone(wahgpu_ctx* ctx, int op, wahgpu_bv* x, wahgpu_bv* y, uint32_t
 // words of both operands, 9.8 at 7 K, 12.3 at 63 K, 17 at 0.4M, 29 at 1.4M,
 // 72 at 4M.  The row index an operand lacks is charged to its first use; an
 // operand that comes back is taken to come again.  A merge tile set on the
-// context asks for the merge.
-static bool in_group_space(const wahgpu_ctx* ctx, wahgpu_bv* x, wahgpu_bv* y, uint32_t groups) {
+// context asks for the merge.  A captured call may not allocate: it takes
+// group space only where the call before it has left all that it needs.  And a
+// context's first few calls do not pay for a large scratch block (2^27 bits:
+// 0.6 ms to allocate, 30 us a call to gain).
+static bool in_group_space(wahgpu_ctx* ctx, wahgpu_bv* x, wahgpu_bv* y, uint32_t groups) {
     if (ctx->merge_tile) return false;
+    const bool fits = ctx->gop_bytes >= gop_bytes(groups);
+    if ((!x->rows_valid || (y && !y->rows_valid) || !fits) && wg_capturing(ctx)) return false;
     const double g = groups * 1e-6, n = (double)x->h.n + (y ? y->h.n : 0);
     double in_groups = 6.6 + (y ? 4.0 : 3.1) * g;
     for (wahgpu_bv* b : {x, y}) {
@@ -934,14 +976,35 @@ static bool in_group_space(const wahgpu_ctx* ctx, wahgpu_bv* x, wahgpu_bv* y, ui
         if (!b->rows_valid && !b->used) in_groups += 3.0 + 1.5 * g;
         b->used = true;
     }
-    return in_groups < 7.0 + 0.5 * std::log2(1.0 + n / 200.0) + (y ? 13e-6 : 10e-6) * n;
+    if (!(in_groups < 7.0 + 0.5 * std::log2(1.0 + n / 200.0) + (y ? 13e-6 : 10e-6) * n)) return false;
+    if (!fits && gop_bytes(groups) > (1u << 20) && ctx->gop_missed < 4) {
+        ctx->gop_missed++;
+        return false;
+    }
+    return true;
 }
 
+// Both fall back to the merge, which needs next to no scratch, where group
+// space does not find the memory.
+static int launch_fsm(wahgpu_ctx* ctx, int op, wahgpu_bv* x, wahgpu_bv* y, uint32_t groups, uint32_t anb, uint32_t aval,
+                      wahgpu_bv* res) {
+    int rc = bv_reserve(res, (uint64_t)x->h.n + y->h.n);
+    if (rc) return rc;
+    if (in_group_space(ctx, x, y, groups)) {
+        rc = wg_launch_gop(ctx, GK_FSM, op, x, y, groups, anb, aval, res);
+        if (rc != WAHGPU_ENOMEM) return rc;
+    }
+    return wg_launch_merge(ctx, op, true, false, false, x, y, groups, anb, aval, res);
+}
 // x, or its complement, as compress() leaves it.
 static int launch_copy(wahgpu_ctx* ctx, bool flip, wahgpu_bv* x, uint32_t groups, uint32_t anb, uint32_t aval,
                        wahgpu_bv* res) {
-    if (groups > 0 && x->h.n > 0 && in_group_space(ctx, x, nullptr, groups))
-        return wg_launch_gop(ctx, flip ? GK_FLIP : GK_COPY, 0, x, nullptr, groups, anb, aval, res);
+    int rc = bv_reserve(res, x->h.n);
+    if (rc) return rc;
+    if (groups > 0 && x->h.n > 0 && in_group_space(ctx, x, nullptr, groups)) {
+        rc = wg_launch_gop(ctx, flip ? GK_FLIP : GK_COPY, 0, x, nullptr, groups, anb, aval, res);
+        if (rc != WAHGPU_ENOMEM) return rc;
+    }
     return wg_launch_merge(ctx, 0, false, true, flip, x, nullptr, groups, anb, aval, res);
 }
 
@@ -1130,8 +1193,7 @@ extern "C" int wahgpu_bv_binop_into(wahgpu_ctx* ctx, int op, int inplace, wahgpu
     if (mb.n != b->h.n) { rc = collapsed_copy(ctx, b, &tmpb); if (rc) { if (tmpa) wahgpu_bv_free(tmpa); return rc; } cb = tmpb; }
     switch (p.kind) {
     case PK_MERGE_FSM:
-        if (in_group_space(ctx, ca, cb, G)) rc = wg_launch_gop(ctx, GK_FSM, op, ca, cb, G, anb, aval, res);
-        else rc = wg_launch_merge(ctx, op, true, false, false, ca, cb, G, anb, aval, res);
+        rc = launch_fsm(ctx, op, ca, cb, G, anb, aval, res);
         break;
     case PK_MERGE_CANON:
         // canonical result: the group-space kernel, or the word-space merge
