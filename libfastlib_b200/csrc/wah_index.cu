@@ -78,9 +78,11 @@ extern "C" int wahgpu_index_from_triple(wahgpu_ctx* ctx, int kind, uint64_t nrow
 // plus at most 2S edge bitmaps.  S is the smallest stride that keeps the rows
 // within CUM_BUDGET bytes (or the context's WAHGPU_TUNE_CUM_STRIDE): 1, a row
 // per bitmap, where that fits (a range is then its rows alone: no word of a
-// bitmap is read), else at least 8.  Indexes with fewer than two rows' worth
-// of bitmaps keep none.
-static constexpr uint64_t CUM_BUDGET = 2ull << 30;
+// bitmap is read), else at least 8.  Rows past CUM_FREELY are kept per bitmap
+// only while they take less than an eighth of the device memory that is free,
+// so that many indexes do not crowd out what a program holds besides.
+// Indexes with fewer than two rows' worth of bitmaps keep none.
+static constexpr uint64_t CUM_BUDGET = 2ull << 30, CUM_FREELY = 256ull << 20;
 static int cumulative_rows(wahgpu_index* x) {
     wahgpu_ctx* ctx = x->ctx;
     const uint32_t nobs = x->nobs;
@@ -89,7 +91,12 @@ static int cumulative_rows(wahgpu_index* x) {
     x->cum_k = 0; x->cum_stride = 0;
     if (ctx->cum_stride == 1 || gx == 0) return WAHGPU_OK;
     const uint64_t fit = (nobs * gx * 4 + CUM_BUDGET - 1) / CUM_BUDGET;
-    const uint64_t stride = ctx->cum_stride ? ctx->cum_stride : fit <= 1 ? 1 : std::max<uint64_t>(8, fit);
+    bool each = fit <= 1;
+    if (each && !ctx->cum_stride && nobs * gx * 4 > CUM_FREELY) {
+        size_t unused = 0, total = 0;
+        each = cudaMemGetInfo(&unused, &total) == cudaSuccess && nobs * gx * 4 < unused / 8;
+    }
+    const uint64_t stride = ctx->cum_stride ? ctx->cum_stride : each ? 1 : std::max<uint64_t>(8, fit);
     const uint64_t K = nobs / stride;
     if (K < 2 && stride > 1) return WAHGPU_OK;
     if (K == 0) return WAHGPU_OK;
@@ -594,9 +601,10 @@ static void launch_range_mode(const wahgpu_batch* B, const RangeArgs& a) {
 extern "C" int wahgpu_batch_run(wahgpu_batch* B) {
     if (!B) return WAHGPU_EINVAL;
     wahgpu_ctx* ctx = B->ctx;
-    if (B->etiles == 0) return WAHGPU_OK;
     // the counts start from those known beforehand (0 for most queries)
     CUDA_TRY(ctx, cudaMemcpyAsync(B->d_counts, B->d_init, B->out_bytes, cudaMemcpyDeviceToDevice, ctx->stream));
+    if (B->etiles == 0) return WAHGPU_OK;
+    B->captured |= wg_capturing(ctx);
     if (B->nedges) {
         EdgeArgs e;
         e.idx = B->d_idx; e.terms = B->d_terms;
@@ -766,8 +774,9 @@ extern "C" int64_t wahgpu_batch_min_bytes(wahgpu_batch* B) { return B ? (int64_t
 extern "C" int wahgpu_batch_free(wahgpu_batch* B) {
     if (!B) return WAHGPU_EINVAL;
     wahgpu_ctx* ctx = B->ctx;
-    // results that have been fetched leave nothing of the batch in flight
-    if (!B->h_valid) cudaStreamSynchronize(ctx->stream);
+    // results that have been fetched leave nothing of the batch in flight,
+    // but for the replays of a graph that holds it
+    if (!B->h_valid || B->captured) cudaStreamSynchronize(ctx->stream);
     wg_free(ctx, B->d_tab); wg_free(ctx, B->d_counts);
     wg_free(ctx, B->d_rids); wg_free(ctx, B->d_dense);
     wg_free(ctx, B->d_items); wg_free(ctx, B->d_scan_tmp);

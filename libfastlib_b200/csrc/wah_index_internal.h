@@ -71,6 +71,7 @@ struct wahgpu_batch {
     bool capped = false;              // row ids limited per query, each query in a region of its own
     std::vector<uint64_t> h_lim, h_base;
     bool h_valid = false;
+    bool captured = false;            // a graph may hold a run of it
     unsigned char* h_stage = nullptr;  // pinned staging of the uploaded tables
 };
 
