@@ -598,6 +598,8 @@ static void launch_range_mode(const wahgpu_batch* B, const RangeArgs& a) {
     else launch_range<RQUADS, MODE, false>(B->ctx, a);
 }
 
+static constexpr size_t SLOTS_AT_MOST = 64u << 20;  // scratch for the row ids a count pass keeps
+
 extern "C" int wahgpu_batch_run(wahgpu_batch* B) {
     if (!B) return WAHGPU_EINVAL;
     wahgpu_ctx* ctx = B->ctx;
@@ -629,13 +631,13 @@ extern "C" int wahgpu_batch_run(wahgpu_batch* B) {
     a.dense = B->d_dense;
     a.recs = nullptr; a.sync = nullptr; a.nitems = nitems; a.status = B->d_status;
     a.gx = (B->groups + (B->anb ? 1u : 0u) + 3u) & ~3u;
-    a.item_cnt = nullptr; a.item_off = nullptr; a.item_list = nullptr;
+    a.item_cnt = nullptr; a.item_off = nullptr; a.item_list = nullptr; a.slots = nullptr;
     a.capped = B->capped && B->d_rids ? 1u : 0u;
     // Row ids: order 0 asks for the look-back, order 2 for two passes (of
     // several queries); order 1 takes the look-back while every item has a
     // CTA of its own at once.  Past that a CTA would sit waiting for the
     // slowest of the items before its own: 1024 conjunctions over 10M rows,
-    // 256 ids each, take 4.3 ms so and 3.1 ms in two passes.
+    // 256 ids each, take 4.3 ms so and 2.6 ms in two passes.
     const bool ids = B->d_rids || B->d_dense;
     const bool two_pass = ids && ((ctx->range_order == 2 && B->nq > 1) ||
                                   (ctx->range_order == 1 && nitems > 4u * (uint32_t)ctx->sm_count));
@@ -651,8 +653,12 @@ extern "C" int wahgpu_batch_run(wahgpu_batch* B) {
                 B->d_items = nullptr; B->d_scan_tmp = nullptr;
                 return wg_fail(ctx, WAHGPU_ENOMEM, "two-pass item arrays: allocation failed");
             }
+            // without them every item with hits is evaluated again
+            if (!B->d_dense && (size_t)nitems * RSLOT * 4 <= SLOTS_AT_MOST)
+                B->d_slots = static_cast<uint32_t*>(wg_alloc(ctx, (size_t)nitems * RSLOT * 4));
         }
         if (B->d_dense) CUDA_TRY(ctx, cudaMemsetAsync(B->d_dense, 0, ((size_t)B->groups + 1) * 4, ctx->stream));
+        else a.slots = B->d_slots;
         CUDA_TRY(ctx, cudaMemsetAsync(B->d_items, 0, (size_t)nitems * 8, ctx->stream));
         a.item_cnt = B->d_items;
         launch_range_mode<RM_ITEMS>(B, a);
@@ -779,7 +785,7 @@ extern "C" int wahgpu_batch_free(wahgpu_batch* B) {
     if (!B->h_valid || B->captured) cudaStreamSynchronize(ctx->stream);
     wg_free(ctx, B->d_tab); wg_free(ctx, B->d_counts);
     wg_free(ctx, B->d_rids); wg_free(ctx, B->d_dense);
-    wg_free(ctx, B->d_items); wg_free(ctx, B->d_scan_tmp);
+    wg_free(ctx, B->d_items); wg_free(ctx, B->d_scan_tmp); wg_free(ctx, B->d_slots);
     wg_host_free(ctx, B->h_stage);
     wg_host_free(ctx, B->h_out);
     delete B;

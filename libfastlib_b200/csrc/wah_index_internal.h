@@ -63,6 +63,7 @@ struct wahgpu_batch {
     // two-pass order: per-item hits and first row-id slots (2 x nq*ntiles)
     // and the scan's temporary storage, allocated at the first such run
     unsigned long long* d_items = nullptr;
+    uint32_t* d_slots = nullptr;  // row ids the count pass keeps (RSLOT per item)
     void* d_scan_tmp = nullptr;
     size_t scan_tmp_bytes = 0;
     std::vector<unsigned long long> h_counts, h_start;

@@ -124,12 +124,24 @@ struct RangeArgs {
     // q*ntiles + k
     unsigned long long* item_cnt;
     const unsigned long long* item_off;
-    const uint2* item_list;      // capped: {item, ids before it within its query}, status->n of them
+    // capped: {item, ids before it within its query}: the items to evaluate
+    // from the front (status->n of them), those whose ids are in their slots
+    // from the back (status->groups)
+    const uint2* item_list;
+    uint32_t* slots;             // two passes: RSLOT row ids per item, in any order (or null)
     // 1: every query writes at most rid_lim row ids into its own region at
     // rid_base (one pass: offsets within the query by a segmented look-back;
     // two: a list of the items holding ids under their query's limit)
     uint32_t capped;
 };
+
+// Row ids kept by the count pass for an item with at most so many: the id
+// pass orders and copies them instead of evaluating the item again.  A
+// conjunction that needs many items to fill its limit has few hits in each.
+// 32: a lane each, 128 bytes of scratch per item.  1024 conjunctions over 10M
+// rows, 256 ids each: 3.06 -> 2.64 ms of kernels (with 4 terms 1.19 -> 0.90; one
+// term, many hits in every item, 0.35 -> 0.36).
+constexpr uint32_t RSLOT = 32;
 
 // 64-bit sums segmented at the first item of each query: {sum lo, sum hi,
 // -, head}; (f1, s1) + (f2, s2) = (f1 | f2, f2 ? s2 : s1 + s2) is
@@ -586,13 +598,27 @@ __device__ __forceinline__ uint4 dense_terms(const RangeArgs& A, const DevQuery&
     return acc;
 }
 
+// The ids of a slot (c of them, unique) in ascending order to ids off, off + 1,
+// ... of the query's region, those under lim (whole warp).
+__device__ __forceinline__ void copy_slot(const RangeArgs& A, uint32_t item, uint32_t c, const DevQuery& DQ, uint64_t off) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t rbase0 = A.capped ? DQ.rid_base : 0ull;
+    const uint64_t room = A.rid_cap > rbase0 ? A.rid_cap - rbase0 : 0ull;
+    const uint64_t lim = A.capped ? min(DQ.rid_lim, room) : room;
+    const uint32_t id = lane < c ? A.slots[(size_t)item * RSLOT + lane] : 0xFFFFFFFFu;
+    uint32_t rank = 0;
+    for (uint32_t j = 0; j < c; ++j) rank += __shfl_sync(0xffffffffu, id, j) < id ? 1u : 0u;
+    if (lane < c && off + rank < lim) A.rids[rbase0 + off + rank] = id;
+}
+
 // Q quads of groups per thread: tiles of 4 * Q * RTHREADS groups.  GEN: the
 // batch holds terms that are not dense (tiles of RT groups).  Dense terms are
 // bound by the rows' loads (16 KB per row and tile, shared in L2) and the
 // edge rows' gathers, the others by the block barriers between their steps.
 // One range over 1M rows of 100 values with its row ids: 17 us on 32 CTAs,
 // 93 us when 8 CTAs walked the edge bitmaps' words; 1024 conjunctions over
-// 10M rows: 3.1 ms against 7.7 ms (9 GB of rows from DRAM at 3.6 TB/s).
+// 10M rows: 2.6 ms against 7.7 ms.  (Asking the next item's rows into L2 ahead
+// made that 3.8: most rows of later terms are never needed.)
 template <int Q, int MODE, bool GEN>
 __global__ void __launch_bounds__(RTHREADS, 6) k_range(RangeArgs A) {
     static_assert(!GEN || Q == RQUADS, "the tile index is over RT groups");
@@ -614,6 +640,13 @@ __global__ void __launch_bounds__(RTHREADS, 6) k_range(RangeArgs A) {
     uint32_t par = 0;
     const bool listed = MODE == RM_IDS && A.capped;  // the items holding ids under their query's limit
     const uint32_t nitems = listed ? A.status->n : A.nitems;
+    if (listed && A.slots) {
+        const uint32_t ns = A.status->groups;
+        for (uint32_t i = blockIdx.x * RWARPS + warp; i < ns; i += gridDim.x * RWARPS) {
+            const uint2 li = A.item_list[A.nitems - 1u - i];
+            copy_slot(A, li.x, (uint32_t)A.item_cnt[li.x], A.queries[li.x / A.ntiles], li.y);
+        }
+    }
     for (uint32_t at = first; at < nitems; at += MODE == RM_LOOK ? nitems : gridDim.x) {
         const uint2 li = listed ? A.item_list[at] : make_uint2(at, 0u);
         const uint32_t item = li.x;
@@ -625,7 +658,12 @@ __global__ void __launch_bounds__(RTHREADS, 6) k_range(RangeArgs A) {
         const DevQuery DQ = A.queries[q];
         if (MODE == RM_IDS && !listed) {
             if (tid == 0 && k == 0) A.rid_start[q] = A.item_off[qi];
-            if (A.item_cnt[qi] == 0ull) continue;  // no hits
+            const unsigned long long c = A.item_cnt[qi];
+            if (c == 0ull) continue;  // no hits
+            if (A.slots && c <= RSLOT) {
+                if (warp == 0) copy_slot(A, qi, (uint32_t)c, DQ, A.item_off[qi]);
+                continue;
+            }
         }
         // the thread's quads: 32 Q consecutive ones per warp, neighbouring lanes on neighbouring quads
         const uint32_t ql = warp * (32u * Q) + lane;  // + 32 i
@@ -672,9 +710,40 @@ __global__ void __launch_bounds__(RTHREADS, 6) k_range(RangeArgs A) {
         for (int i = 0; i < Q; ++i) cnt += __popc(acc[i].x) + __popc(acc[i].y) + __popc(acc[i].z) + __popc(acc[i].w);
         cnt = __reduce_add_sync(0xffffffffu, cnt);  // the warp's hits
         if (MODE <= RM_ITEMS) {
-            if (lane == 0 && cnt) {
+            if (cnt == 0u) continue;
+            uint32_t o = 0;  // the item's hits counted before these
+            if (lane == 0) {
                 atomicAdd(&A.counts[DQ.q], (unsigned long long)cnt);
-                if (MODE == RM_ITEMS) atomicAdd(&A.item_cnt[qi], (unsigned long long)cnt);
+                if (MODE == RM_ITEMS) o = (uint32_t)atomicAdd(&A.item_cnt[qi], (unsigned long long)cnt);
+            }
+            if (MODE == RM_ITEMS && A.slots && cnt <= RSLOT) {
+                o = __shfl_sync(0xffffffffu, o, 0);
+                if (o + cnt <= RSLOT) {
+                    uint32_t c = 0;
+#pragma unroll
+                    for (int i = 0; i < Q; ++i) c += __popc(acc[i].x) + __popc(acc[i].y) + __popc(acc[i].z) + __popc(acc[i].w);
+                    uint32_t s = c;
+#pragma unroll
+                    for (int d = 1; d < 32; d <<= 1) {
+                        const uint32_t u = __shfl_up_sync(0xffffffffu, s, d);
+                        if (lane >= (uint32_t)d) s += u;
+                    }
+                    uint32_t* p = A.slots + (size_t)qi * RSLOT + (o + s - c);
+                    if (c) {
+#pragma unroll
+                        for (int i = 0; i < Q; ++i) {
+                            const uint32_t row = (g0 + 4u * (ql + 32u * i)) * 31u;
+                            const uint32_t v[4] = {acc[i].x, acc[i].y, acc[i].z, acc[i].w};
+#pragma unroll
+                            for (uint32_t e = 0; e < 4u; ++e)
+                                for (uint32_t bits = v[e]; bits;) {
+                                    const uint32_t hb = 31u - __clz(bits);
+                                    bits ^= 1u << hb;
+                                    *p++ = row + e * 31u + (30u - hb);
+                                }
+                        }
+                    }
+                }
             }
             continue;
         }
@@ -799,7 +868,8 @@ __global__ void __launch_bounds__(RTHREADS, 6) k_range(RangeArgs A) {
 // Capped queries, between the passes: a warp per query scans its items' hits
 // and lists those holding ids under the limit (in any order) with the ids
 // before them, so that the second pass visits no item only to skip it (0.9
-// ms without the list, 0.6 with it, of 81 K items).
+// ms without the list, 0.6 with it, of 81 K items).  Items of at most RSLOT
+// hits are listed apart, their ids are at hand.
 __global__ void __launch_bounds__(RTHREADS) k_cap_items(RangeArgs A, uint2* __restrict__ list) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t q = (blockIdx.x * RTHREADS + threadIdx.x) >> 5;
@@ -816,12 +886,14 @@ __global__ void __launch_bounds__(RTHREADS) k_cap_items(RangeArgs A, uint2* __re
             const uint32_t u = __shfl_up_sync(0xffffffffu, s, d);
             if (lane >= (uint32_t)d) s += u;
         }
-        const bool on = c != 0u && before + (s - c) < lim;
-        const uint32_t m = __ballot_sync(0xffffffffu, on);
-        uint32_t at = 0;
-        if (lane == 0 && m) at = atomicAdd(&A.status->n, __popc(m));
-        at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
-        if (on) list[at] = make_uint2(q * A.ntiles + k, (uint32_t)before + (s - c));
+        const bool on = c != 0u && before + (s - c) < lim, kept = A.slots && c <= RSLOT;
+        const uint32_t me = __ballot_sync(0xffffffffu, on && !kept), mk = __ballot_sync(0xffffffffu, on && kept);
+        uint32_t ae = 0, ak = 0;
+        if (lane == 0 && me) ae = atomicAdd(&A.status->n, __popc(me));
+        if (lane == 0 && mk) ak = atomicAdd(&A.status->groups, __popc(mk));
+        ae = __shfl_sync(0xffffffffu, ae, 0) + __popc(me & ((1u << lane) - 1u));
+        ak = __shfl_sync(0xffffffffu, ak, 0) + __popc(mk & ((1u << lane) - 1u));
+        if (on) list[kept ? A.nitems - 1u - ak : ae] = make_uint2(q * A.ntiles + k, (uint32_t)before + (s - c));
         before += __shfl_sync(0xffffffffu, s, 31);
     }
 }
