@@ -71,12 +71,12 @@ void* wg_alloc(wahgpu_ctx* ctx, size_t bytes) {
                 ctx->bytes_allocated -= kv.first;
             }
         ctx->pool.clear();
-        if (ctx->gop_scratch && !ctx->gop_captured) {
-            cudaFree(ctx->gop_scratch);
-            ctx->bytes_allocated -= ctx->gop_bytes;
-            ctx->sizes.erase(ctx->gop_scratch);
-            ctx->gop_scratch = nullptr;
-            ctx->gop_bytes = 0;
+        if (ctx->ws && !ctx->ws_captured) {
+            cudaFree(ctx->ws);
+            ctx->bytes_allocated -= ctx->ws_bytes;
+            ctx->sizes.erase(ctx->ws);
+            ctx->ws = nullptr;
+            ctx->ws_bytes = 0;
         }
         cudaGetLastError();
         if (cudaMalloc(&p, c) != cudaSuccess) { cudaGetLastError(); return nullptr; }
@@ -160,25 +160,26 @@ bool wg_capturing(const wahgpu_ctx* ctx) {
     if (cudaStreamIsCapturing(ctx->stream, &cs) != cudaSuccess) { cudaGetLastError(); return true; }
     return cs != cudaStreamCaptureStatusNone;
 }
-// Result patterns of the two-pass engine: one block of the context that grows
-// with its calls and is never handed to anything else, so a captured call's
-// replays write into no other object.  A block that captured calls hold is
-// kept beside the larger one that follows it (at least twice its size, so
-// these come to less than the last) until the context ends.
-static unsigned char* gop_scratch(wahgpu_ctx* ctx, size_t bytes, bool captured) {
-    if (ctx->gop_bytes < bytes) {
-        const size_t want = ctx->gop_captured ? std::max(bytes, 2 * ctx->gop_bytes) : bytes;
-        if (!ctx->gop_captured) wg_free(ctx, ctx->gop_scratch);
-        ctx->gop_scratch = nullptr;
-        ctx->gop_bytes = 0;
-        ctx->gop_captured = false;
-        ctx->gop_scratch = wg_alloc(ctx, want);
-        if (!ctx->gop_scratch) return nullptr;
+// Scratch of one call (the two-pass engine's result patterns, a batch's
+// items): one block of the context that grows with its calls and is never
+// handed to anything else, so a captured call's replays write into no other
+// object.  A block that captured calls hold is kept beside the larger one that
+// follows it (at least twice its size, so these come to less than the last)
+// until the context ends.
+unsigned char* wg_workspace(wahgpu_ctx* ctx, size_t bytes, bool captured) {
+    if (ctx->ws_bytes < bytes) {
+        const size_t want = std::max(bytes, ctx->ws_captured ? 2 * ctx->ws_bytes : ctx->ws_bytes + ctx->ws_bytes / 2);
+        if (!ctx->ws_captured) wg_free(ctx, ctx->ws);
+        ctx->ws = nullptr;
+        ctx->ws_bytes = 0;
+        ctx->ws_captured = false;
+        ctx->ws = wg_alloc(ctx, want);
+        if (!ctx->ws) return nullptr;
         std::lock_guard<std::mutex> g(ctx->mu);
-        ctx->gop_bytes = ctx->sizes[ctx->gop_scratch];
+        ctx->ws_bytes = ctx->sizes[ctx->ws];
     }
-    ctx->gop_captured |= captured;
-    return static_cast<unsigned char*>(ctx->gop_scratch);
+    ctx->ws_captured |= captured;
+    return static_cast<unsigned char*>(ctx->ws);
 }
 // The dense kernel's records, after the TileRec array of the scratch block.
 static uint4* wg_dense_recs(wahgpu_ctx* ctx, TileRec* recs) {
@@ -803,7 +804,7 @@ int wg_launch_gop(wahgpu_ctx* ctx, int kind, int op, wahgpu_bv* x, wahgpu_bv* y,
     // is at hand; else they are part of the scratch
     const bool keep = result_rows(res, groups);
     const size_t rb = (size_t)ntiles * PT * 4, hb = (size_t)ntiles * TROWS * sizeof(uint2);
-    unsigned char* scr = gop_scratch(ctx, gop_bytes(groups), wg_capturing(ctx));
+    unsigned char* scr = wg_workspace(ctx, gop_bytes(groups), wg_capturing(ctx));
     if (!scr) return wg_fail(ctx, WAHGPU_ENOMEM, "allocation of %u tiles of result patterns failed", ntiles);
     uint32_t* tot = reinterpret_cast<uint32_t*>(scr + rb + hb);
     GopArgs a;
@@ -967,7 +968,7 @@ int wg_launch_gone(wahgpu_ctx* ctx, int op, wahgpu_bv* x, wahgpu_bv* y, uint32_t
 // 0.6 ms to allocate, 30 us a call to gain).
 static bool in_group_space(wahgpu_ctx* ctx, wahgpu_bv* x, wahgpu_bv* y, uint32_t groups) {
     if (ctx->merge_tile) return false;
-    const bool fits = ctx->gop_bytes >= gop_bytes(groups);
+    const bool fits = ctx->ws_bytes >= gop_bytes(groups);
     if ((!x->rows_valid || (y && !y->rows_valid) || !fits) && wg_capturing(ctx)) return false;
     const double g = groups * 1e-6, n = (double)x->h.n + (y ? y->h.n : 0);
     double in_groups = 6.6 + (y ? 4.0 : 3.1) * g;

@@ -30,10 +30,10 @@ struct wahgpu_ctx {
     // reads those of every result launched since the last read
     std::vector<wah::DevMeta*> meta_blocks, meta_free;
     std::vector<struct wahgpu_bv*> pending;  // launched, metadata not read yet
-    void* gop_scratch = nullptr;   // two-pass engine's result patterns (gop_scratch())
-    size_t gop_bytes = 0;
-    uint32_t gop_missed = 0;       // calls that went without a larger one
-    bool gop_captured = false;     // a captured call writes to it
+    void* ws = nullptr;            // scratch of one call (wg_workspace())
+    size_t ws_bytes = 0;
+    bool ws_captured = false;      // a captured call writes to it
+    uint32_t gop_missed = 0;       // group-space calls that went without a larger one
     uint64_t launches = 0;
     uint32_t row_results = 0;           // results that could have kept a row index so far
     uint32_t dense_tile = 2048;         // WAHGPU_TUNE_DENSE_TILE
@@ -103,6 +103,7 @@ void wg_launch_pdl(void (*k)(Params...), uint32_t grid, uint32_t threads, size_t
 }
 int wg_fail(wahgpu_ctx* ctx, int code, const char* fmt, ...);
 bool wg_capturing(const wahgpu_ctx* ctx);
+unsigned char* wg_workspace(wahgpu_ctx* ctx, size_t bytes, bool captured);
 void* wg_alloc(wahgpu_ctx* ctx, size_t bytes);
 void wg_free(wahgpu_ctx* ctx, void* p);
 void* wg_host_alloc(wahgpu_ctx* ctx, size_t bytes);

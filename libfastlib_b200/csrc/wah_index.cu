@@ -643,35 +643,35 @@ extern "C" int wahgpu_batch_run(wahgpu_batch* B) {
                                   (ctx->range_order == 1 && nitems > 4u * (uint32_t)ctx->sm_count));
     a.tile_major = ((ctx->range_order != 0 && !ids) || two_pass) ? 1u : 0u;
     if (two_pass) {
-        if (!B->d_items) {
-            B->d_items = static_cast<unsigned long long*>(wg_alloc(ctx, (size_t)nitems * 16));
-            cub::DeviceScan::ExclusiveSum(nullptr, B->scan_tmp_bytes, B->d_items, B->d_items + nitems, (int)nitems,
-                                          ctx->stream);
-            B->d_scan_tmp = wg_alloc(ctx, std::max<size_t>(B->scan_tmp_bytes, 16));
-            if (!B->d_items || !B->d_scan_tmp) {
-                wg_free(ctx, B->d_items); wg_free(ctx, B->d_scan_tmp);
-                B->d_items = nullptr; B->d_scan_tmp = nullptr;
-                return wg_fail(ctx, WAHGPU_ENOMEM, "two-pass item arrays: allocation failed");
-            }
-            // without them every item with hits is evaluated again
-            if (!B->d_dense && (size_t)nitems * RSLOT * 4 <= SLOTS_AT_MOST)
-                B->d_slots = static_cast<uint32_t*>(wg_alloc(ctx, (size_t)nitems * RSLOT * 4));
-        }
+        // per item its hits, its first row-id slot or list entry, and the ids
+        // kept (without them every item with hits is evaluated again)
+        const bool cap = wg_capturing(ctx);
+        const size_t ib = (size_t)nitems * 16;
+        if (!a.capped && !B->scan_tmp_bytes)
+            cub::DeviceScan::ExclusiveSum(nullptr, B->scan_tmp_bytes, static_cast<unsigned long long*>(nullptr),
+                                          static_cast<unsigned long long*>(nullptr), (int)nitems, ctx->stream);
+        const size_t tb = a.capped ? 0 : (B->scan_tmp_bytes + 127) & ~(size_t)127;
+        size_t sb = !B->d_dense && (size_t)nitems * RSLOT * 4 <= SLOTS_AT_MOST ? (size_t)nitems * RSLOT * 4 : 0;
+        if (cap && ctx->ws_bytes < ib + tb + sb) sb = 0;
+        unsigned char* ws = wg_workspace(ctx, ib + tb + sb, cap);
+        if (!ws && sb) { sb = 0; ws = wg_workspace(ctx, ib + tb, cap); }
+        if (!ws) return wg_fail(ctx, WAHGPU_ENOMEM, "two-pass item arrays: allocation failed");
+        unsigned long long* items = reinterpret_cast<unsigned long long*>(ws);
+        unsigned long long* second = items + nitems;
         if (B->d_dense) CUDA_TRY(ctx, cudaMemsetAsync(B->d_dense, 0, ((size_t)B->groups + 1) * 4, ctx->stream));
-        else a.slots = B->d_slots;
-        CUDA_TRY(ctx, cudaMemsetAsync(B->d_items, 0, (size_t)nitems * 8, ctx->stream));
-        a.item_cnt = B->d_items;
+        if (sb) a.slots = reinterpret_cast<uint32_t*>(ws + ib + tb);
+        CUDA_TRY(ctx, cudaMemsetAsync(items, 0, (size_t)nitems * 8, ctx->stream));
+        a.item_cnt = items;
         launch_range_mode<RM_ITEMS>(B, a);
         CUDA_TRY(ctx, cudaGetLastError());
         if (a.capped) {
-            uint2* list = reinterpret_cast<uint2*>(B->d_items + nitems);
+            uint2* list = reinterpret_cast<uint2*>(second);
             k_cap_items<<<(B->nrange + RWARPS - 1) / RWARPS, RTHREADS, 0, ctx->stream>>>(a, list);
             CUDA_TRY(ctx, cudaGetLastError());
             a.item_list = list;
         } else {
-            CUDA_TRY(ctx, cub::DeviceScan::ExclusiveSum(B->d_scan_tmp, B->scan_tmp_bytes, B->d_items,
-                                                        B->d_items + nitems, (int)nitems, ctx->stream));
-            a.item_off = B->d_items + nitems;
+            CUDA_TRY(ctx, cub::DeviceScan::ExclusiveSum(ws + ib, B->scan_tmp_bytes, items, second, (int)nitems, ctx->stream));
+            a.item_off = second;
         }
         launch_range_mode<RM_IDS>(B, a);
         ctx->launches += 2;  // the count pass and the scan
@@ -785,7 +785,6 @@ extern "C" int wahgpu_batch_free(wahgpu_batch* B) {
     if (!B->h_valid || B->captured) cudaStreamSynchronize(ctx->stream);
     wg_free(ctx, B->d_tab); wg_free(ctx, B->d_counts);
     wg_free(ctx, B->d_rids); wg_free(ctx, B->d_dense);
-    wg_free(ctx, B->d_items); wg_free(ctx, B->d_scan_tmp); wg_free(ctx, B->d_slots);
     wg_host_free(ctx, B->h_stage);
     wg_host_free(ctx, B->h_out);
     delete B;

@@ -60,12 +60,7 @@ struct wahgpu_batch {
     uint32_t* d_rids = nullptr;
     uint64_t rid_cap = 0;
     uint32_t* d_dense = nullptr;
-    // two-pass order: per-item hits and first row-id slots (2 x nq*ntiles)
-    // and the scan's temporary storage, allocated at the first such run
-    unsigned long long* d_items = nullptr;
-    uint32_t* d_slots = nullptr;  // row ids the count pass keeps (RSLOT per item)
-    void* d_scan_tmp = nullptr;
-    size_t scan_tmp_bytes = 0;
+    size_t scan_tmp_bytes = 0;        // two-pass order, not capped: the scan's temporary storage
     std::vector<unsigned long long> h_counts, h_start;
     uint64_t bytes = 0;               // algorithmic bytes one run reads
     uint64_t min_bytes = 0;           // the bytes sumBins itself must read (covered set or complement)
