@@ -81,7 +81,9 @@ extern "C" int wahgpu_index_from_triple(wahgpu_ctx* ctx, int kind, uint64_t nrow
 // bitmap is read), else at least 8.  Rows past CUM_FREELY are kept per bitmap
 // only while they take less than an eighth of the device memory that is free,
 // so that many indexes do not crowd out what a program holds besides.
-// Indexes with fewer than two rows' worth of bitmaps keep none.
+// Indexes with fewer than two rows' worth of bitmaps keep none.  A row for the
+// bitmaps past the last whole stride comes after them: the last row is then
+// the OR of all bitmaps, whose 1 bits tell whether any two share a row.
 static constexpr uint64_t CUM_BUDGET = 2ull << 30, CUM_FREELY = 256ull << 20;
 static int cumulative_rows(wahgpu_index* x) {
     wahgpu_ctx* ctx = x->ctx;
@@ -100,9 +102,10 @@ static int cumulative_rows(wahgpu_index* x) {
     const uint64_t K = nobs / stride;
     if (K < 2 && stride > 1) return WAHGPU_OK;
     if (K == 0) return WAHGPU_OK;
-    x->d_cum = static_cast<uint32_t*>(wg_alloc(ctx, K * gx * 4));
+    const uint64_t bytes = (nobs + stride - 1) / stride * gx * 4;
+    x->d_cum = static_cast<uint32_t*>(wg_alloc(ctx, bytes));
     if (!x->d_cum) return WAHGPU_OK;  // no room: ranges use the bitmaps alone
-    CUDA_TRY(ctx, cudaMemsetAsync(x->d_cum, 0, K * gx * 4, ctx->stream));
+    CUDA_TRY(ctx, cudaMemsetAsync(x->d_cum, 0, bytes, ctx->stream));
     x->cum_k = (uint32_t)K;
     x->cum_stride = (uint32_t)stride;
     return WAHGPU_OK;
@@ -182,8 +185,14 @@ int wg_index_attach(wahgpu_index* x) {
         a.words = x->d_words; a.bm = x->d_bm; a.nobs = nobs; a.choff = d_choff; a.nchunks = nchunks; a.cstart = d_cg;
         a.ntiles = nt; a.tiles = x->d_tiles; a.touch = touch; a.tw = tw;
         a.gx = (x->groups + (x->anb ? 1u : 0u) + 3u) & ~3u;
-        a.cum = x->cum_k ? x->d_cum : nullptr;
-        a.cum_nb = x->cum_k * x->cum_stride; a.cum_stride = x->cum_stride;
+        // without rows, the OR of all bitmaps alone
+        a.cum = x->d_cum; a.cum_stride = x->cum_k ? x->cum_stride : nobs;
+        if (!a.cum) {
+            a.cum = tmp.get<uint32_t>(a.gx);
+            if (!a.cum) return wg_fail(ctx, WAHGPU_ENOMEM, "index allocation failed");
+            CUDA_TRY(ctx, cudaMemsetAsync(a.cum, 0, (size_t)a.gx * 4, ctx->stream));
+        }
+        const uint32_t nr = (nobs + a.cum_stride - 1) / a.cum_stride;
         k_chunk_place<<<blocks, ITHREADS, 0, ctx->stream>>>(a);
         const uint32_t nparts = (uint32_t)(((uint64_t)nt * tw + LTILE - 1) / LTILE);
         TileRec* recs; LaunchSync* sync;
@@ -193,15 +202,10 @@ int wg_index_attach(wahgpu_index* x) {
         ctx->launches += 2;
         unsigned long long* d_or = reinterpret_cast<unsigned long long*>(d_st + 1);  // 1 bits of all bitmaps OR'ed
         unsigned long long h_or = 0;
-        if (x->cum_k) {
-            k_cum_prefix<<<(a.gx + 255) / 256, 256, 0, ctx->stream>>>(x->d_cum, x->cum_k, a.gx);
-            ctx->launches++;
-            if (x->cum_stride == 1) {
-                k_row_ones<<<std::min<uint32_t>((a.gx + 255) / 256, 2u * (uint32_t)ctx->sm_count), 256, 0, ctx->stream>>>(
-                    x->d_cum + (size_t)(x->cum_k - 1) * a.gx, a.gx, d_or);
-                ctx->launches++;
-            }
-        }
+        if (nr > 1) k_cum_prefix<<<(a.gx + 255) / 256, 256, 0, ctx->stream>>>(a.cum, nr, a.gx);
+        k_row_ones<<<std::min<uint32_t>((a.gx + 255) / 256, 2u * (uint32_t)ctx->sm_count), 256, 0, ctx->stream>>>(
+            a.cum + (size_t)(nr - 1) * a.gx, a.gx, d_or);
+        ctx->launches += nr > 1 ? 2 : 1;
         CUDA_TRY(ctx, cudaGetLastError());
         CUDA_TRY(ctx, cudaMemcpyAsync(&st, d_st, sizeof(DevMeta), cudaMemcpyDeviceToHost, ctx->stream));
         CUDA_TRY(ctx, cudaMemcpyAsync(&h_or, d_or, sizeof h_or, cudaMemcpyDeviceToHost, ctx->stream));
@@ -210,7 +214,14 @@ int wg_index_attach(wahgpu_index* x) {
         // no row in two bitmaps: the OR holds as many 1 bits as all of them
         uint64_t ones = 0;
         for (uint32_t j = 0; j < nobs; ++j) ones += x->bones[j];
-        x->disjoint = x->cum_stride == 1 && h_or == ones;
+        x->disjoint = h_or == ones;
+        if (!x->disjoint) {
+            // rows tell a bitmap by C(j + 1) & ~C(j), which drops what it
+            // shares with an earlier one: such an index goes by its words
+            wg_free(ctx, x->d_cum);
+            x->d_cum = nullptr;
+            x->cum_k = x->cum_stride = 0;
+        }
     } else {
         CUDA_TRY(ctx, cudaMemsetAsync(x->d_tl_off, 0, ((size_t)nt + 1) * 4, ctx->stream));
     }
@@ -407,8 +418,9 @@ static int locate(wahgpu_ctx* ctx, const wahgpu_index* x, const wahgpu_term* t, 
     }
     // sumBins reads the complement when the range holds more than half the
     // index's words (src/index.cpp:6490); the bits are the same either way
+    // where no row is in two bitmaps
     const uint64_t in = x->cum_words[h1] - x->cum_words[h0], all = x->cum_words[x->nobs];
-    out.flip = (2 * in > all) ? 1u : 0u;
+    out.flip = (x->disjoint && 2 * in > all) ? 1u : 0u;
     return WAHGPU_OK;
 }
 

@@ -26,7 +26,7 @@ struct wahgpu_index {
     uint32_t* d_tl_bm = nullptr;
     uint32_t* d_cum = nullptr;        // cumulative dense rows (range spans in two reads)
     uint32_t cum_stride = 0, cum_k = 0;
-    bool disjoint = false;            // no row in two bitmaps (known with a cumulative row per bitmap)
+    bool disjoint = false;            // no row in two bitmaps
     void* d_values = nullptr;
     uint32_t vtype = 0;
     wah::DevIndex dev{};

@@ -1134,8 +1134,8 @@ struct PlaceArgs {
     uint32_t* tiles;      // per-bitmap tile index: nobs x (ntiles+1) x {word, its first group}
     uint32_t* touch;      // ntiles x tw words, bit b of row k: bitmap b holds a 1 bit in tile k (zeroed)
     uint32_t tw;
-    uint32_t* cum;        // block ORs for the cumulative rows (zeroed), or null
-    uint32_t cum_nb, cum_stride, gx;  // bitmaps b < cum_nb go into row b / cum_stride
+    uint32_t* cum;        // block ORs for the cumulative rows (zeroed)
+    uint32_t cum_stride, gx;  // bitmap b goes into row b / cum_stride
 };
 
 // Second pass over the words, from every chunk's first group: the word
@@ -1154,7 +1154,7 @@ __global__ void __launch_bounds__(ITHREADS) k_chunk_place(PlaceArgs A) {
     uint32_t* tix = A.tiles + (size_t)b * (A.ntiles + 1) * 2;
     uint32_t* tcol = A.touch + (b >> 5);  // + tile * tw
     const uint32_t tbit = 1u << (b & 31u);
-    uint32_t* row = A.cum && b < A.cum_nb ? A.cum + (size_t)(b / A.cum_stride) * A.gx : nullptr;
+    uint32_t* row = A.cum + (size_t)(b / A.cum_stride) * A.gx;
     uint32_t carry = (uint32_t)A.cstart[ch];
     uint32_t marked = 0xFFFFFFFFu;  // the last tile this chunk marked
     for (uint32_t base0 = i0; base0 < i1; base0 += 128) {
@@ -1200,16 +1200,14 @@ __global__ void __launch_bounds__(ITHREADS) k_chunk_place(PlaceArgs A) {
             if (bits)
                 for (uint32_t k = k0 == before ? k0 + 1u : k0; k <= k1; ++k) atomicOr(tcol + (size_t)k * A.tw, tbit);
             if (hb) marked = __shfl_sync(0xffffffffu, k1, 31u - __clz(hb));
-            if (row) {
-                if (bits && wd <= ALLONES) atomicOr(row + p, wd);
-                else if (bits && c <= 32u) for (uint32_t g = 0; g < c; ++g) row[p + g] = ALLONES;
-                uint32_t f = __ballot_sync(0xffffffffu, bits && wd >= HEADER1 && c > 32u);
-                while (f) {
-                    const uint32_t src = __ffs(f) - 1u;
-                    f &= f - 1u;
-                    const uint32_t fp = __shfl_sync(0xffffffffu, p, src), fc = __shfl_sync(0xffffffffu, c, src);
-                    for (uint32_t g = lane; g < fc; g += 32u) row[fp + g] = ALLONES;
-                }
+            if (bits && wd <= ALLONES) atomicOr(row + p, wd);
+            else if (bits && c <= 32u) for (uint32_t g = 0; g < c; ++g) row[p + g] = ALLONES;
+            uint32_t f = __ballot_sync(0xffffffffu, bits && wd >= HEADER1 && c > 32u);
+            while (f) {
+                const uint32_t src = __ffs(f) - 1u;
+                f &= f - 1u;
+                const uint32_t fp = __shfl_sync(0xffffffffu, p, src), fc = __shfl_sync(0xffffffffu, c, src);
+                for (uint32_t g = lane; g < fc; g += 32u) row[fp + g] = ALLONES;
             }
         }
     }
@@ -1221,7 +1219,7 @@ __global__ void __launch_bounds__(ITHREADS) k_chunk_place(PlaceArgs A) {
         const uint32_t pat = (m.aval & ((1u << m.anb) - 1u)) << (31u - m.anb);
         if (pat) {
             atomicOr(tcol + (size_t)(carry / RT) * A.tw, tbit);
-            if (row) atomicOr(row + carry, pat);
+            atomicOr(row + carry, pat);
         }
     }
 }
