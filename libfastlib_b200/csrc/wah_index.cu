@@ -215,6 +215,7 @@ int wg_index_attach(wahgpu_index* x) {
         uint64_t ones = 0;
         for (uint32_t j = 0; j < nobs; ++j) ones += x->bones[j];
         x->disjoint = h_or == ones;
+        x->partition = x->disjoint && h_or == x->nrows;
         if (!x->disjoint) {
             // rows tell a bitmap by C(j + 1) & ~C(j), which drops what it
             // shares with an earlier one: such an index goes by its words
@@ -418,9 +419,9 @@ static int locate(wahgpu_ctx* ctx, const wahgpu_index* x, const wahgpu_term* t, 
     }
     // sumBins reads the complement when the range holds more than half the
     // index's words (src/index.cpp:6490); the bits are the same either way
-    // where no row is in two bitmaps
+    // where every row is in one bitmap
     const uint64_t in = x->cum_words[h1] - x->cum_words[h0], all = x->cum_words[x->nobs];
-    out.flip = (x->disjoint && 2 * in > all) ? 1u : 0u;
+    out.flip = (x->partition && 2 * in > all) ? 1u : 0u;
     return WAHGPU_OK;
 }
 

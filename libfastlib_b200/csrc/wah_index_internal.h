@@ -27,6 +27,7 @@ struct wahgpu_index {
     uint32_t* d_cum = nullptr;        // cumulative dense rows (range spans in two reads)
     uint32_t cum_stride = 0, cum_k = 0;
     bool disjoint = false;            // no row in two bitmaps
+    bool partition = false;           // and every row in one
     void* d_values = nullptr;
     uint32_t vtype = 0;
     wah::DevIndex dev{};

@@ -1,4 +1,5 @@
-"""Ranges over bitmaps that share rows (every bitmap counts in whole), with
+"""Ranges over bitmaps that are no partition of the rows: rows in several
+bitmaps (every bitmap counts in whole) and rows in none (never a hit), with
 cumulative rows per bitmap, at a stride and none."""
 import numpy as np
 import pytest
@@ -42,7 +43,7 @@ def _check(L, ctx, idx, sets, spans):
 
 @pytest.mark.parametrize("stride", [0, 1, 2, 8])
 @pytest.mark.parametrize("rows", [62, 31 * 4096 + 5])
-@pytest.mark.parametrize("kind", ["equal", "some", "last"])
+@pytest.mark.parametrize("kind", ["equal", "some", "gaps", "last"])
 def test_ranges(gpu_ctx, kind, rows, stride):
     import libfastlib_b200 as L
     rng = np.random.default_rng(rows + stride)
@@ -51,7 +52,7 @@ def test_ranges(gpu_ctx, kind, rows, stride):
         sets = np.repeat(rng.random((1, rows)) < 0.5, 2, axis=0)
         sets[:, :31] = True
     else:
-        owner = rng.integers(0, n, rows)
+        owner = rng.integers(0, n + (1 if kind == "gaps" else 0), rows)
         sets = np.stack([owner == j for j in range(n)])
         if kind == "some":
             sets |= rng.random((n, rows)) < 0.02
