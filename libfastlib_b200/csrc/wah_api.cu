@@ -131,34 +131,45 @@ void wg_host_free(wahgpu_ctx* ctx, void* p) {
     ctx->hpool[it->second].push_back(p);
 }
 
+// The stream's calls are being captured: they run later, and perhaps often.
+bool wg_capturing(const wahgpu_ctx* ctx) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &cs) != cudaSuccess) { cudaGetLastError(); return true; }
+    return cs != cudaStreamCaptureStatusNone;
+}
 // Scratch for the look-back scans: tile records plus the launch sync words.
+// A captured call's replays go on using the block that the call was given: such
+// a block is kept beside the larger one that follows it (at least twice its
+// size, so these come to less than the last) until the context ends.  A
+// captured call takes what is there.
 int wg_scratch(wahgpu_ctx* ctx, uint32_t ntiles, TileRec** recs, LaunchSync** sync) {
+    const bool cap = wg_capturing(ctx);
     if (ntiles > ctx->scratch_tiles) {
-        uint32_t want = ntiles < 1024 ? 1024 : ntiles + ntiles / 2;
+        if (cap)
+            return wg_fail(ctx, WAHGPU_ECUDA, "a captured call needs scratch for %u tiles: make it once before the capture", ntiles);
+        const uint32_t want = std::max({ntiles + ntiles / 2, 1024u, ctx->scratch_captured ? 2 * ctx->scratch_tiles : 0u});
         CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-        if (ctx->scratch) cudaFree(ctx->scratch);
+        if (ctx->scratch_captured) ctx->scratch_kept.push_back(ctx->scratch);
+        else if (ctx->scratch) cudaFree(ctx->scratch);
         ctx->scratch = nullptr;
+        ctx->scratch_tiles = 0;
+        ctx->scratch_captured = false;
         // sync words, TileRec records, then the dense kernel's 16-byte
         // records and the single-pass kernel's (each format in a region of
         // its own, so a stale record of one is never read by the other)
         size_t bytes = sizeof(LaunchSync) * 2 + (size_t)want * (sizeof(TileRec) + 2 * sizeof(uint4));
         if (cudaMalloc(&ctx->scratch, bytes) != cudaSuccess) {
             cudaGetLastError();
-            ctx->scratch_tiles = 0;
+            ctx->scratch = nullptr;
             return wg_fail(ctx, WAHGPU_ENOMEM, "scratch allocation of %zu bytes failed", bytes);
         }
         CUDA_TRY(ctx, cudaMemsetAsync(ctx->scratch, 0, bytes, ctx->stream));
         ctx->scratch_tiles = want;
     }
+    ctx->scratch_captured |= cap;
     *sync = reinterpret_cast<LaunchSync*>(ctx->scratch);
     *recs = reinterpret_cast<TileRec*>(reinterpret_cast<char*>(ctx->scratch) + 2 * sizeof(LaunchSync));
     return WAHGPU_OK;
-}
-// The stream's calls are being captured: they run later, and perhaps often.
-bool wg_capturing(const wahgpu_ctx* ctx) {
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(ctx->stream, &cs) != cudaSuccess) { cudaGetLastError(); return true; }
-    return cs != cudaStreamCaptureStatusNone;
 }
 // Scratch of one call (the two-pass engine's result patterns, a batch's
 // items): one block of the context that grows with its calls and is never
@@ -231,6 +242,7 @@ extern "C" int wahgpu_ctx_destroy(wahgpu_ctx* ctx) {
     for (auto& kv : ctx->sizes) cudaFree(kv.first);
     for (auto& kv : ctx->hsizes) cudaFreeHost(kv.first);
     if (ctx->scratch) cudaFree(ctx->scratch);
+    for (void* p : ctx->scratch_kept) cudaFree(p);
     if (ctx->h_meta_stage) cudaFreeHost(ctx->h_meta_stage);
     cudaStreamDestroy(ctx->own_stream);
     delete ctx;

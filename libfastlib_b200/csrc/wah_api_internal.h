@@ -25,6 +25,8 @@ struct wahgpu_ctx {
     // look-back scratch: two LaunchSync words then TileRec records
     void* scratch = nullptr;
     uint32_t scratch_tiles = 0;
+    bool scratch_captured = false;      // a captured call uses it
+    std::vector<void*> scratch_kept;    // smaller ones that captured calls use
     void* h_meta_stage = nullptr;  // pinned staging for metadata reads
     // the bitvectors' metadata live in blocks of META_SLOTS, so that one copy
     // reads those of every result launched since the last read
