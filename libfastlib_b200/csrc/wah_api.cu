@@ -369,15 +369,16 @@ static void bv_unpend(wahgpu_bv* b) {  // ctx->mu held
     b->pend = -1;
 }
 // b's metadata have been launched on the context's stream: the host copy is
-// stale.  Work that is only being captured runs at some later time, so such a
-// result is read when it is asked for and not along with another one.
+// stale.  Work that is only being captured runs at some later time, and again
+// whenever its graph does, so a result that a captured call writes is read when
+// it is asked for and not along with another one, from then on.
 static void bv_launched(wahgpu_bv* b) {
     wahgpu_ctx* ctx = b->ctx;
     b->h_valid = false;
     b->told = false;
-    const bool later = wg_capturing(ctx);
+    b->replayed |= wg_capturing(ctx);
     std::lock_guard<std::mutex> g(ctx->mu);
-    if (later) { bv_unpend(b); return; }
+    if (b->replayed) { bv_unpend(b); return; }
     b->pend_stream = ctx->stream;
     if (b->pend < 0) {
         b->pend = (int32_t)ctx->pending.size();
@@ -683,7 +684,7 @@ static int wg_gtile(wahgpu_bv* b) {
     k_gtile<<<blocks, threads, 0, ctx->stream>>>(b->words, b->bpos, b->h.n, b->h.groups, nt, b->gt);
     ctx->launches++;
     CUDA_TRY(ctx, cudaGetLastError());
-    b->gt_valid = true;
+    b->gt_valid = !b->replayed && !wg_capturing(ctx);
     return WAHGPU_OK;
 }
 
@@ -755,16 +756,16 @@ static bool rows_reserve(wahgpu_bv* b, uint32_t groups, void* (*alloc)(wahgpu_ct
 }
 // Room for a result's row index: a cached block, or, once the context has
 // made a few such results, a new one (a fresh context's first calls do not
-// pay for blocks that may never be read).  A captured call keeps none: until
-// its replay the index would not be that of the words.
+// pay for blocks that may never be read).  A result that a captured call
+// writes keeps none: its replays change the words without the index.
 static bool result_rows(wahgpu_bv* res, uint32_t groups) {
-    if (wg_capturing(res->ctx)) return false;
+    if (res->replayed || wg_capturing(res->ctx)) return false;
     const bool fresh = res->ctx->row_results < 8;
     if (fresh) res->ctx->row_results++;
     return rows_reserve(res, groups, fresh ? wg_alloc_cached : wg_alloc);
 }
-// Row index of b (host metadata must be valid); built once, and by a captured
-// call on each of its replays.
+// Row index of b (host metadata must be valid); built once, by a captured
+// call on each of its replays, and for words that replays change on each use.
 static int wg_rows(wahgpu_bv* b) {
     wahgpu_ctx* ctx = b->ctx;
     // positions are taken from the words: none that the upload scan refused
@@ -775,7 +776,7 @@ static int wg_rows(wahgpu_bv* b) {
     k_rows<<<(ntiles + GW - 1) / GW, GCTA, 0, ctx->stream>>>(b->words, b->bpos, b->h.n, b->h.groups, ntiles, b->rows);
     ctx->launches++;
     CUDA_TRY(ctx, cudaGetLastError());
-    b->rows_valid = !wg_capturing(ctx);
+    b->rows_valid = !b->replayed && !wg_capturing(ctx);
     return WAHGPU_OK;
 }
 
@@ -986,7 +987,7 @@ static bool in_group_space(wahgpu_ctx* ctx, wahgpu_bv* x, wahgpu_bv* y, uint32_t
     double in_groups = 6.6 + (y ? 4.0 : 3.1) * g;
     for (wahgpu_bv* b : {x, y}) {
         if (!b) continue;
-        if (!b->rows_valid && !b->used) in_groups += 3.0 + 1.5 * g;
+        if (!b->rows_valid && (!b->used || b->replayed)) in_groups += 3.0 + 1.5 * g;
         b->used = true;
     }
     if (!(in_groups < 7.0 + 0.5 * std::log2(1.0 + n / 200.0) + (y ? 13e-6 : 10e-6) * n)) return false;
@@ -1279,6 +1280,7 @@ static void bv_take(wahgpu_bv* b, wahgpu_bv* tmp) {
     std::swap(b->rows_cap, tmp->rows_cap);
     std::swap(b->rows_valid, tmp->rows_valid);
     std::swap(b->used, tmp->used);
+    std::swap(b->replayed, tmp->replayed);
     b->compressed_form = tmp->compressed_form;
 }
 

@@ -64,6 +64,7 @@ struct wahgpu_bv {
     bool told = false;          // the device status in h has been reported
     int32_t pend = -1;          // its place in ctx->pending
     cudaStream_t pend_stream = nullptr;  // where it was launched
+    bool replayed = false;      // a captured call writes to it: its words may change at any time
     uint32_t* gt = nullptr;     // group-tile index (k_gtile), built on first use
     bool gt_valid = false;
     uint2* rows = nullptr;      // row index (k_rows), built on first use or with the result
