@@ -63,7 +63,11 @@ typedef struct {
 int wahgpu_ctx_create(int device, wahgpu_ctx** out);
 int wahgpu_ctx_destroy(wahgpu_ctx* ctx);
 /* Runs the context's work on `stream` (a cudaStream_t); NULL restores the
- * context's own stream. */
+ * context's own stream.  Metadata of a result launched on an earlier stream
+ * are waited for; work on its buffers is ordered between streams by the
+ * caller.  A captured call keeps the sizes and the row indexes that its
+ * operands have when it is captured: capture the call that writes an operand
+ * before the calls that read it. */
 int wahgpu_ctx_set_stream(wahgpu_ctx* ctx, void* stream);
 void* wahgpu_ctx_stream(wahgpu_ctx* ctx);
 /* Waits for all work queued on the context's stream. */

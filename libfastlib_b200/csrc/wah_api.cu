@@ -394,11 +394,16 @@ int wg_bv_meta(wahgpu_bv* b) {
     wahgpu_ctx* ctx = b->ctx;
     if (!b->h_valid) {
         const DevMeta* blk = nullptr;
+        bool elsewhere;
         {
             std::lock_guard<std::mutex> g(ctx->mu);
             for (const DevMeta* m : ctx->meta_blocks)
                 if (b->meta >= m && b->meta < m + META_SLOTS) blk = m;
+            elsewhere = b->pend >= 0 && b->pend_stream != ctx->stream;
         }
+        // launched before the context was given another stream: that one is
+        // waited for too, by the device, for it need not be there any more
+        if (elsewhere && !wg_capturing(ctx)) CUDA_TRY(ctx, cudaDeviceSynchronize());
         DevMeta* st = reinterpret_cast<DevMeta*>(ctx->h_meta_stage);
         CUDA_TRY(ctx, cudaMemcpyAsync(st, blk, META_SLOTS * sizeof(DevMeta), cudaMemcpyDeviceToHost, ctx->stream));
         CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
