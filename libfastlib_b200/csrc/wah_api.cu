@@ -657,6 +657,8 @@ int wg_launch_merge(wahgpu_ctx* ctx, int op, bool fsm, bool unary, bool flip,
     a.out = res->words; a.obp = res->bpos; a.meta = res->meta;
     a.recs = recs; a.sync = sync; a.ntiles = ntiles;
     a.aval = aval; a.anb = anb;
+    a.late = ctx->test_withhold;
+    ctx->test_withhold = 0xFFFFFFFFu;
     dim3 g(ntiles);
     if (tb == 16) launch_merge_tb<16>(ctx, op, fsm, unary, flip, g, ctx->stream, a);
     else if (tb == 32) launch_merge_tb<32>(ctx, op, fsm, unary, flip, g, ctx->stream, a);

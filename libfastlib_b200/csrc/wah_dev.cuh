@@ -37,6 +37,7 @@ struct LaunchSync {
     uint32_t epoch;
     uint32_t pad;
 };
+constexpr uint32_t DONE_ERROR = 0x80000000u;  // in `done`: a CTA of the launch gave up
 
 constexpr uint32_t REC_AGG = 1, REC_INCL = 2;
 constexpr uint32_t SPIN_LIMIT = 1u << 22;  // ~1 s worst case with backoff
@@ -90,11 +91,13 @@ __device__ __forceinline__ uint32_t claim_tile(LaunchSync* s) {
     return atomicAdd(&s->ticket, 1u);
 }
 // Called once per CTA at exit by thread 0; the last CTA of the launch resets
-// the ticket and advances the epoch.
-__device__ __forceinline__ void finish_tile(LaunchSync* s, uint32_t ntiles) {
+// the ticket and advances the epoch, and, where status is given, stores there
+// whether a CTA gave up (its thread 0 has set DONE_ERROR before coming here).
+__device__ __forceinline__ void finish_tile(LaunchSync* s, uint32_t ntiles, uint32_t* status = nullptr) {
     __threadfence();
     uint32_t d = atomicAdd(&s->done, 1u);
-    if (d == ntiles - 1) {
+    if ((d & ~DONE_ERROR) == ntiles - 1) {
+        if (status) *status = d & DONE_ERROR ? DEV_ERR_TIMEOUT : 0u;
         s->ticket = 0;
         s->done = 0;
         __threadfence();

@@ -63,6 +63,7 @@ struct MergeArgs {
     LaunchSync* sync;
     uint32_t ntiles;
     uint32_t aval, anb;   // result active word (already combined)
+    uint32_t late;        // test hook: this tile publishes once another gave up (UINT32_MAX: none)
 };
 
 // Look-back aggregate: heads, last head (position, class, count-1 flag), popcount.
@@ -539,13 +540,15 @@ __global__ void __launch_bounds__(MERGE_THREADS, TB == 64 ? 5 : 4) k_merge(Merge
         }
         // ---- decoupled look-back over the preceding tiles
         const uint32_t epoch = S.hdr[1];
+        if (t == A.late)
+            for (uint32_t it = 0; it < 2u * SPIN_LIMIT && !(ld_cg(&A.sync->done) & DONE_ERROR); ++it) __nanosleep(256);
         Agg prefix = agg_identity();
         if (t == 0) {
             if (lane == 0) {
                 // every other tile writes its metadata after this record has
-                // reached it
+                // reached it, or gives up, which the last CTA tells (a store
+                // of 0 here could come after an error)
                 A.meta->nfill = 0;
-                A.meta->status = 0;
                 publish(&A.recs[0], epoch, REC_INCL, agg_pack(tot));
             }
         } else {
@@ -553,7 +556,7 @@ __global__ void __launch_bounds__(MERGE_THREADS, TB == 64 ? 5 : 4) k_merge(Merge
             bool ok;
             prefix = agg_unpack(warp_lookback(A.recs, t, epoch, agg_pack(agg_identity()), AggComb(), &ok));
             if (lane == 0) {
-                if (!ok) atomicExch(&A.meta->status, DEV_ERR_TIMEOUT);
+                if (!ok) atomicOr(&A.sync->done, DONE_ERROR);
                 publish(&A.recs[t], epoch, REC_INCL, agg_pack(agg_combine(prefix, tot)));
             }
         }
@@ -614,7 +617,7 @@ __global__ void __launch_bounds__(MERGE_THREADS, TB == 64 ? 5 : 4) k_merge(Merge
     }
     if (wrote_fill) atomicOr(&A.meta->nfill, 1u);
     __syncthreads();
-    if (tid == 0) finish_tile(A.sync, A.ntiles);
+    if (tid == 0) finish_tile(A.sync, A.ntiles, &A.meta->status);
 }
 
 }  // namespace wah
