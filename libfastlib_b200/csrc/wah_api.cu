@@ -154,9 +154,10 @@ int wg_scratch(wahgpu_ctx* ctx, uint32_t ntiles, TileRec** recs, LaunchSync** sy
         ctx->scratch = nullptr;
         ctx->scratch_tiles = 0;
         ctx->scratch_captured = false;
-        // sync words, TileRec records, then the dense kernel's 16-byte
-        // records and the single-pass kernel's (each format in a region of
-        // its own, so a stale record of one is never read by the other)
+        // sync words (the second's ticket for the merge's claims), TileRec
+        // records, then the dense kernel's 16-byte records and the single-pass
+        // kernel's (each format in a region of its own, so a stale record of
+        // one is never read by the other)
         size_t bytes = sizeof(LaunchSync) * 2 + (size_t)want * (sizeof(TileRec) + 2 * sizeof(uint4));
         if (cudaMalloc(&ctx->scratch, bytes) != cudaSuccess) {
             cudaGetLastError();

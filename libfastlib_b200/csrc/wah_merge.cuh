@@ -20,15 +20,15 @@
 // written by the thread that meets the next run head (its length is only
 // known then); mixed literals are written at once.  Head counts, the last
 // head and popcounts are carried across tiles by a single-pass decoupled
-// look-back over TileRec records, in block order.  The walk's count-1 fills
+// look-back over TileRec records, in claim order.  The walk's count-1 fills
 // are told from the words meeting at a one-group run (single_flag), so no
 // state is carried for them.
 //
 // Bound by the chain of dependent steps of a tile (search, loads, scans,
-// look-back).  2^28 bits, d = 1e-3 / 1e-2: 14 / 29 us a call.  The form
+// look-back).  2^28 bits, d = 1e-3 / 1e-2: 14 / 30 us a call.  The form
 // that carried the walk's five step states as transfer functions through the
-// scans, claimed its tile by an atomic and had its metadata cleared by a
-// memset took 23.5 / 58.
+// scans, claimed its tile after the launch before it was done and had its
+// metadata cleared by a memset took 23.5 / 58.
 #ifndef WAH_MERGE_CUH
 #define WAH_MERGE_CUH
 #include "wah_dev.cuh"
@@ -293,12 +293,18 @@ __global__ void __launch_bounds__(MERGE_THREADS, TB == 64 ? 5 : 4) k_merge(Merge
     TileShared& S = *reinterpret_cast<TileShared*>(smem_raw);
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
 
-    // tile = block: blocks are dispatched in order, so a tile's predecessors
-    // are running or done (and every wait is bounded)
-    const uint32_t t = blockIdx.x;
+    // Tiles in claim order: a tile's predecessors are running or done,
+    // whatever order the blocks are dispatched in.  The claims of a launch
+    // have a word of their own, which its last claim sets back to 0; this
+    // launch begins when every block of the launch before it has made its
+    // claim, so they are made while that one drains.  (2^28 bits, d = 1e-2, 700
+    // tiles: 1.5 us a call over tile = block; claims after the wait, 3.)
+    if (tid == 0) S.hdr[0] = atomicInc(&A.sync[1].ticket, A.ntiles - 1u);
     const uint32_t G = A.groups;
     pdl_wait();
     pdl_launch();
+    __syncthreads();
+    const uint32_t t = S.hdr[0];
     // the launch epoch, read while the tile is found (it only changes after
     // the last CTA of the previous launch on this stream finished)
     if (tid == MERGE_THREADS - 1) S.hdr[1] = ld_cg(&A.sync->epoch);
