@@ -836,6 +836,8 @@ int wg_launch_gop(wahgpu_ctx* ctx, int kind, int op, wahgpu_bv* x, wahgpu_bv* y,
     a.out = res->words; a.obp = res->bpos; a.meta = res->meta;
     a.orow = keep ? res->rows : reinterpret_cast<uint2*>(scr + rb);
     a.aval = aval; a.anb = anb;
+    a.withhold = ctx->test_withhold;
+    ctx->test_withhold = 0xFFFFFFFFu;
     cudaStream_t s = ctx->stream;
     if (kind == GK_CANON) launch_gop_kind<GK_CANON>(ctx, op, ntiles, s, a);
     else if (kind == GK_FSM) launch_gop_kind<GK_FSM>(ctx, op, ntiles, s, a);

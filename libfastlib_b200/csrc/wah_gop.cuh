@@ -68,9 +68,11 @@ struct GopArgs {
     const uint32_t* yw; const uint2* yr; const uint32_t* ybp; uint32_t ny;
     uint32_t groups, ntiles;
     uint32_t* R;          // ntiles * PT result patterns; bit 31: as a run of one group it is a count-1 fill
-    uint32_t* heads; uint32_t* first; uint32_t* ones;  // per tile: heads, first head (GNONE: none), 1 bits
+    // per tile: heads (GNONE: the tile gave up), first head (GNONE: none), 1 bits
+    uint32_t* heads; uint32_t* first; uint32_t* ones;
     uint32_t* out; uint32_t* obp; uint2* orow; DevMeta* meta;
     uint32_t aval, anb;
+    uint32_t withhold;    // test hook: this tile's words are not staged (UINT32_MAX: none)
 };
 
 // Word range of one operand over the tile [g0, g1): words [wi0, wend), the
@@ -296,7 +298,8 @@ __global__ void __launch_bounds__(GCTA, 3) k_gop(const __grid_constant__ GopArgs
     // issues the copies of a tile's words: from the one covering the group
     // before it to the one after its last, 16-byte ends rounded outwards (the
     // word arrays are pool blocks: aligned and padded to 256 bytes)
-    auto stage = [&](uint2 row, uint32_t b) {
+    auto stage = [&](uint32_t u, uint2 row, uint32_t b) {
+        if (u == A.withhold) return;
         const uint32_t half = lane & 16u, n = half ? A.ny : A.nx;
         const uint32_t fst = __shfl_sync(0xffffffffu, row.y, half);
         const uint32_t lst = __shfl_sync(0xffffffffu, row.y + __popc(row.x), half + TROWS - 1u);
@@ -313,18 +316,20 @@ __global__ void __launch_bounds__(GCTA, 3) k_gop(const __grid_constant__ GopArgs
     };
 
     uint2 nrow = load_rows(t);
-    stage(nrow, 0);
+    stage(t, nrow, 0);
     if (t + GW < tend) nrow = load_rows(t + GW);
     for (uint32_t k = 0; t < tend; t += GW, ++k) {
         const uint32_t b = k & 1u;
         if (t + GW < tend) {
-            stage(nrow, b ^ 1u);
+            stage(t + GW, nrow, b ^ 1u);
             if (t + 2 * GW < tend) nrow = load_rows(t + 2 * GW);
         }
         if (!__all_sync(0xffffffffu, mbar_wait(&W.bar[b], (k >> 1) & 1u))) {
-            // gave up: nothing of the tile is written; leave once the copies
-            // in flight are done or have been waited for as long again
-            if (lane == 0) atomicExch(&A.meta->status, DEV_ERR_TIMEOUT);
+            // gave up: this tile and the warp's others say so, for k_gpack to
+            // write nothing by their counts; leave once the copies in flight
+            // are done or have been waited for as long again
+            if (lane == 0)
+                for (uint32_t u = t; u < tend; u += GW) A.heads[u] = GNONE;
             if (t + GW < tend) mbar_wait(&W.bar[b ^ 1u], ((k + 1u) >> 1) & 1u);
             return;
         }
@@ -495,7 +500,12 @@ __global__ void __launch_bounds__(GCTA) k_gpack(const __grid_constant__ GopArgs 
     // heads before the range; the last CTA also sums the 1 bits
     const bool last = tend == A.ntiles;
     uint32_t part = 0, ones = 0;
-    for (uint32_t i = threadIdx.x; i < tb; i += GCTA) part += A.heads[i];
+    bool gone = false;  // a tile up to the range's end gave up
+    for (uint32_t i = threadIdx.x; i < tb; i += GCTA) {
+        const uint32_t c = A.heads[i];
+        gone |= c == GNONE;
+        part += c;
+    }
     if (last) for (uint32_t i = threadIdx.x; i < A.ntiles; i += GCTA) ones += A.ones[i];
     part = __reduce_add_sync(0xffffffffu, part);
     ones = __reduce_add_sync(0xffffffffu, ones);
@@ -504,6 +514,7 @@ __global__ void __launch_bounds__(GCTA) k_gpack(const __grid_constant__ GopArgs 
         uint32_t carry = 0;
         for (uint32_t i = tb; i < tend; i += 32u) {
             const uint32_t c = i + lane < tend ? A.heads[i + lane] : 0u;
+            gone |= c == GNONE;
             uint32_t x = c;
 #pragma unroll
             for (int d = 1; d < 32; d <<= 1) {
@@ -515,7 +526,15 @@ __global__ void __launch_bounds__(GCTA) k_gpack(const __grid_constant__ GopArgs 
         }
         part = carry;  // warp 0: the range's heads
     }
-    __syncthreads();
+    if (__syncthreads_or(gone)) {
+        // no word has a place; the last CTA, which has seen every tile, says so
+        if (last && threadIdx.x == 0) {
+            A.meta->n = A.meta->groups = A.meta->nset = A.meta->anb = A.meta->aval = A.meta->w0 = 0;
+            atomicExch(&A.meta->status, DEV_ERR_TIMEOUT);
+        }
+        if (t < tend) mbar_wait(&W.bar[0], 0);
+        return;
+    }
     uint32_t base = 0;
 #pragma unroll
     for (uint32_t k = 0; k < (uint32_t)GW; ++k) base += sh[0][k];
