@@ -97,7 +97,7 @@ int64_t wahgpu_ctx_launches(wahgpu_ctx* ctx);
  * record, so the tile after it waits until its bounded wait gives up and
  * the call reports WAHGPU_ETIMEOUT (the hook then clears itself); in one on
  * the word-space merge, it publishes only once a wait for it has given up; in
- * one on the two-pass kernels, its words are not copied in and it gives up.
+ * one on the two-pass kernels, its wait for its words counts as given up.
  * WAHGPU_TEST_FAIL_ALLOC = n: the n-th device allocation from now fails as
  * if the device were out of memory (WAHGPU_ENOMEM), once. */
 #define WAHGPU_TEST_WITHHOLD_TILE 100

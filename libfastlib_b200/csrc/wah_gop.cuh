@@ -72,7 +72,7 @@ struct GopArgs {
     uint32_t* heads; uint32_t* first; uint32_t* ones;
     uint32_t* out; uint32_t* obp; uint2* orow; DevMeta* meta;
     uint32_t aval, anb;
-    uint32_t withhold;    // test hook: this tile's words are not staged (UINT32_MAX: none)
+    uint32_t withhold;    // test hook: this tile's wait counts as given up (UINT32_MAX: none)
 };
 
 // Word range of one operand over the tile [g0, g1): words [wi0, wend), the
@@ -298,8 +298,7 @@ __global__ void __launch_bounds__(GCTA, 3) k_gop(const __grid_constant__ GopArgs
     // issues the copies of a tile's words: from the one covering the group
     // before it to the one after its last, 16-byte ends rounded outwards (the
     // word arrays are pool blocks: aligned and padded to 256 bytes)
-    auto stage = [&](uint32_t u, uint2 row, uint32_t b) {
-        if (u == A.withhold) return;
+    auto stage = [&](uint2 row, uint32_t b) {
         const uint32_t half = lane & 16u, n = half ? A.ny : A.nx;
         const uint32_t fst = __shfl_sync(0xffffffffu, row.y, half);
         const uint32_t lst = __shfl_sync(0xffffffffu, row.y + __popc(row.x), half + TROWS - 1u);
@@ -316,15 +315,15 @@ __global__ void __launch_bounds__(GCTA, 3) k_gop(const __grid_constant__ GopArgs
     };
 
     uint2 nrow = load_rows(t);
-    stage(t, nrow, 0);
+    stage(nrow, 0);
     if (t + GW < tend) nrow = load_rows(t + GW);
     for (uint32_t k = 0; t < tend; t += GW, ++k) {
         const uint32_t b = k & 1u;
         if (t + GW < tend) {
-            stage(t + GW, nrow, b ^ 1u);
+            stage(nrow, b ^ 1u);
             if (t + 2 * GW < tend) nrow = load_rows(t + 2 * GW);
         }
-        if (!__all_sync(0xffffffffu, mbar_wait(&W.bar[b], (k >> 1) & 1u))) {
+        if (!__all_sync(0xffffffffu, mbar_wait(&W.bar[b], (k >> 1) & 1u)) || t == A.withhold) {
             // gave up: this tile and the warp's others say so, for k_gpack to
             // write nothing by their counts; leave once the copies in flight
             // are done or have been waited for as long again

@@ -1,7 +1,6 @@
-"""A tile of the two-pass kernels whose words never arrive (made on the device
-by WAHGPU_TEST_WITHHOLD_TILE, the wait bounded): the call reports
-WAHGPU_ETIMEOUT, nothing is written by the counts of tiles that gave up, and
-the next call is exact."""
+"""A tile of the two-pass kernels that gives up its wait for its words (made by
+WAHGPU_TEST_WITHHOLD_TILE): the call reports WAHGPU_ETIMEOUT, nothing is
+written by the counts of tiles that gave up, and the next call is exact."""
 import numpy as np
 import pytest
 
@@ -12,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("tile", [0, 1, 70, -1])
-def test_words_that_never_arrive(tile):
+def test_a_tile_that_gives_up(tile):
     import libfastlib_b200 as L
     ctx = L.Context(0)
     nbits = 31 * (512 * 101 + 7)  # 102 tiles
