@@ -788,16 +788,17 @@ static int wg_rows(wahgpu_bv* b) {
     return WAHGPU_OK;
 }
 
+static constexpr uint32_t GOP_CTAS_AT_MOST = 4096;  // room for their warps' first heads
 template <int OP, int KIND>
-static void launch_gop_op(const wahgpu_ctx* ctx, uint32_t ntiles, cudaStream_t s, const GopArgs& a) {
+static void launch_gop_op(const wahgpu_ctx* ctx, uint32_t ntiles, cudaStream_t s, GopArgs& a) {
     static PerDeviceSetup setup;
     const size_t sm = GW * sizeof(GopWarp<(KIND >= GK_COPY)>);
     const uint32_t per_sm = (uint32_t)wg_kernel_setup(setup, ctx->device, k_gop<OP, KIND>, GCTA, sm);
-    const uint32_t grid = std::min<uint32_t>((ntiles + GW - 1) / GW, per_sm * (uint32_t)ctx->sm_count);
-    wg_launch_pdl(k_gop<OP, KIND>, grid, GCTA, sm, s, a);
+    a.gop_ctas = std::min<uint32_t>({(ntiles + GW - 1) / GW, per_sm * (uint32_t)ctx->sm_count, GOP_CTAS_AT_MOST});
+    wg_launch_pdl(k_gop<OP, KIND>, a.gop_ctas, GCTA, sm, s, a);
 }
 template <int KIND>
-static void launch_gop_kind(const wahgpu_ctx* ctx, int op, uint32_t ntiles, cudaStream_t s, const GopArgs& a) {
+static void launch_gop_kind(const wahgpu_ctx* ctx, int op, uint32_t ntiles, cudaStream_t s, GopArgs& a) {
     switch (op) {
     case OP_AND: launch_gop_op<OP_AND, KIND>(ctx, ntiles, s, a); break;
     case OP_OR: launch_gop_op<OP_OR, KIND>(ctx, ntiles, s, a); break;
@@ -808,7 +809,7 @@ static void launch_gop_kind(const wahgpu_ctx* ctx, int op, uint32_t ntiles, cuda
 
 static size_t gop_bytes(uint32_t groups) {
     const size_t ntiles = ((uint64_t)groups + PT - 1) / PT;
-    return ntiles * (PT * 4 + TROWS * sizeof(uint2) + 12);
+    return ntiles * (PT * 4 + TROWS * sizeof(uint2) + 12) + std::min<size_t>((ntiles + GW - 1) / GW, GOP_CTAS_AT_MOST) * GW * 4;
 }
 
 // Two-pass group-space engine (wah_gop.cuh): the result patterns per group
@@ -833,6 +834,7 @@ int wg_launch_gop(wahgpu_ctx* ctx, int kind, int op, wahgpu_bv* x, wahgpu_bv* y,
     a.yw = y ? y->words : nullptr; a.yr = y ? y->rows : nullptr; a.ybp = y ? y->bpos : nullptr; a.ny = y ? y->h.n : 0;
     a.groups = groups; a.ntiles = ntiles;
     a.R = reinterpret_cast<uint32_t*>(scr); a.heads = tot; a.first = tot + ntiles; a.ones = tot + 2 * (size_t)ntiles;
+    a.wfirst = tot + 3 * (size_t)ntiles; a.gop_ctas = 0;
     a.out = res->words; a.obp = res->bpos; a.meta = res->meta;
     a.orow = keep ? res->rows : reinterpret_cast<uint2*>(scr + rb);
     a.aval = aval; a.anb = anb;

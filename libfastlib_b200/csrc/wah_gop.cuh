@@ -70,6 +70,8 @@ struct GopArgs {
     uint32_t* R;          // ntiles * PT result patterns; bit 31: as a run of one group it is a count-1 fill
     // per tile: heads (GNONE: the tile gave up), first head (GNONE: none), 1 bits
     uint32_t* heads; uint32_t* first; uint32_t* ones;
+    uint32_t* wfirst;     // first head of each warp of k_gop (GNONE: none)
+    uint32_t gop_ctas;    // CTAs of k_gop
     uint32_t* out; uint32_t* obp; uint2* orow; DevMeta* meta;
     uint32_t aval, anb;
     uint32_t withhold;    // test hook: this tile's wait counts as given up (UINT32_MAX: none)
@@ -271,6 +273,11 @@ struct GopWarp {
     uint64_t bar[2];
 };
 
+// A warp of k_gop marks tile t and its later ones as given up.
+__device__ __noinline__ void give_up(uint32_t* heads, uint32_t t, uint32_t tend) {
+    for (; t < tend; t += GW) heads[t] = GNONE;
+}
+
 template <int OP, int KIND>
 __global__ void __launch_bounds__(GCTA, 3) k_gop(const __grid_constant__ GopArgs A) {
     constexpr bool UNARY = KIND >= GK_COPY;
@@ -285,7 +292,11 @@ __global__ void __launch_bounds__(GCTA, 3) k_gop(const __grid_constant__ GopArgs
     pdl_wait();
     pdl_launch();
     if (blockIdx.x == 0 && threadIdx.x == 0) { A.meta->nfill = 0; A.meta->status = 0; }
-    if (t >= tend) return;
+    if (t >= tend) {
+        if (lane == 0) A.wfirst[blockIdx.x * GW + warp] = GNONE;
+        return;
+    }
+    uint32_t head0 = GNONE;  // the warp's first head
     const uint32_t le = (2u << lane) - 1u;  // lanes up to this one (lane 31: all)
     const uint32_t* __restrict__ xw = A.xw;
     const uint32_t* __restrict__ yw = A.yw;
@@ -327,8 +338,7 @@ __global__ void __launch_bounds__(GCTA, 3) k_gop(const __grid_constant__ GopArgs
             // gave up: this tile and the warp's others say so, for k_gpack to
             // write nothing by their counts; leave once the copies in flight
             // are done or have been waited for as long again
-            if (lane == 0)
-                for (uint32_t u = t; u < tend; u += GW) A.heads[u] = GNONE;
+            if (lane == 0) give_up(A.heads, t, tend);
             if (t + GW < tend) mbar_wait(&W.bar[b ^ 1u], ((k + 1u) >> 1) & 1u);
             return;
         }
@@ -461,8 +471,33 @@ __global__ void __launch_bounds__(GCTA, 3) k_gop(const __grid_constant__ GopArgs
         heads = __reduce_add_sync(0xffffffffu, heads);
         first = __reduce_min_sync(0xffffffffu, first);
         if (lane == 0) { A.heads[t] = heads; A.first[t] = first; A.ones[t] = ones; }
+        head0 = min(head0, first);
         __syncwarp();  // the buffer, the rows and the head masks are free again
     }
+    if (lane == 0) A.wfirst[blockIdx.x * GW + warp] = head0;
+}
+
+// The first head of the tiles from i on (whole warp): of the rest of tile
+// i - 1's k_gop CTA, else of the CTAs after it by their warps' first heads, 256
+// at a time.  (By the tiles alone a result of one run read them all: 2^28 bits,
+// 323 us a call with every tile looking, heads or not, 31 so.)
+__device__ __noinline__ uint32_t head_from(const uint32_t* __restrict__ first, const uint32_t* __restrict__ wfirst,
+                                           uint32_t ntiles, uint32_t gop_ctas, uint32_t i) {
+    const uint32_t lane = threadIdx.x & 31u;
+    if (i >= ntiles) return GNONE;
+    uint32_t lo, hi, h = GNONE;
+    const uint32_t cta = (i - 1u) / ((ntiles + gop_ctas - 1u) / gop_ctas);
+    gop_range_of(ntiles, cta, gop_ctas, lo, hi);
+    for (; h == GNONE && i < hi; i += 32u) h = __reduce_min_sync(0xffffffffu, i + lane < hi ? first[i + lane] : GNONE);
+    const uint32_t nw = gop_ctas * GW;
+    for (uint32_t s = (cta + 1u) * GW; h == GNONE && s < nw; s += 256u) {
+        uint32_t v = GNONE;
+#pragma unroll
+        for (uint32_t j = 0; j < 8u; ++j)
+            if (s + 32u * j + lane < nw) v = min(v, wfirst[s + 32u * j + lane]);
+        h = __reduce_min_sync(0xffffffffu, v);
+    }
+    return h;
 }
 
 struct PackWarp {
@@ -477,7 +512,7 @@ constexpr uint32_t GRANGE = 1024;  // tiles of a CTA at most
 __global__ void __launch_bounds__(GCTA) k_gpack(const __grid_constant__ GopArgs A) {
     extern __shared__ __align__(16) unsigned char gsm[];
     __shared__ uint32_t sh[2][GW];
-    __shared__ uint32_t pre[GRANGE];  // heads before each tile of the range, from its start
+    __shared__ uint32_t pre[GRANGE + 1];  // heads before each tile of the range, from its start, and in all of it
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     PackWarp& W = reinterpret_cast<PackWarp*>(gsm)[warp];
     uint32_t tb, tend;
@@ -499,10 +534,10 @@ __global__ void __launch_bounds__(GCTA) k_gpack(const __grid_constant__ GopArgs 
     // heads before the range; the last CTA also sums the 1 bits
     const bool last = tend == A.ntiles;
     uint32_t part = 0, ones = 0;
-    bool gone = false;  // a tile up to the range's end gave up
+    uint32_t gone = 0;  // GNONE among the counts: a tile up to the range's end gave up
     for (uint32_t i = threadIdx.x; i < tb; i += GCTA) {
         const uint32_t c = A.heads[i];
-        gone |= c == GNONE;
+        gone |= c;
         part += c;
     }
     if (last) for (uint32_t i = threadIdx.x; i < A.ntiles; i += GCTA) ones += A.ones[i];
@@ -513,7 +548,7 @@ __global__ void __launch_bounds__(GCTA) k_gpack(const __grid_constant__ GopArgs 
         uint32_t carry = 0;
         for (uint32_t i = tb; i < tend; i += 32u) {
             const uint32_t c = i + lane < tend ? A.heads[i + lane] : 0u;
-            gone |= c == GNONE;
+            gone |= c;
             uint32_t x = c;
 #pragma unroll
             for (int d = 1; d < 32; d <<= 1) {
@@ -523,9 +558,10 @@ __global__ void __launch_bounds__(GCTA) k_gpack(const __grid_constant__ GopArgs 
             if (i + lane < tend) pre[i + lane - tb] = carry + x - c;
             carry += __shfl_sync(0xffffffffu, x, 31);
         }
+        if (lane == 0) pre[tend - tb] = carry;
         part = carry;  // warp 0: the range's heads
     }
-    if (__syncthreads_or(gone)) {
+    if (__syncthreads_or(gone >> 31)) {
         // no word has a place; the last CTA, which has seen every tile, says so
         if (last && threadIdx.x == 0) {
             A.meta->n = A.meta->groups = A.meta->nset = A.meta->anb = A.meta->aval = A.meta->w0 = 0;
@@ -554,12 +590,15 @@ __global__ void __launch_bounds__(GCTA) k_gpack(const __grid_constant__ GopArgs 
     for (uint32_t k = 0; t < tend; t += GW, ++k) {
         const uint32_t b = k & 1u;
         if (t + GW < tend) stage(t + GW, b ^ 1u);
-        // the first head after the tile: of the tiles after it, 32 at a time
-        uint32_t later = GNONE;
-        for (uint32_t i = t + 1u; later == GNONE; i += 32u) {
-            const uint32_t v = i + lane < A.ntiles ? A.first[i + lane] : (i + lane == A.ntiles ? A.groups : GNONE);
-            later = __reduce_min_sync(0xffffffffu, v);
+        // the first head after the tile: nearly always of the 32 tiles after it
+        uint32_t later;
+        {
+            const uint32_t i = t + 1u + lane;
+            later = __reduce_min_sync(0xffffffffu, i < A.ntiles ? A.first[i] : (i == A.ntiles ? A.groups : GNONE));
         }
+        const uint32_t before = pre[t - tb];
+        if (later == GNONE && pre[t - tb + 1u] != before)
+            later = min(head_from(A.first, A.wfirst, A.ntiles, A.gop_ctas, t + 33u), A.groups);
         if (!__all_sync(0xffffffffu, mbar_wait(&W.bar[b], (k >> 1) & 1u))) {
             if (lane == 0) atomicExch(&A.meta->status, DEV_ERR_TIMEOUT);
             if (t + GW < tend) mbar_wait(&W.bar[b ^ 1u], ((k + 1u) >> 1) & 1u);
@@ -574,7 +613,7 @@ __global__ void __launch_bounds__(GCTA) k_gpack(const __grid_constant__ GopArgs 
             const uint32_t u = __shfl_up_sync(0xffffffffu, x, d);
             if (lane >= (uint32_t)d) x += u;
         }
-        x += base + pre[t - tb] - c;  // lane r: index of row r's first head
+        x += base + before - c;  // lane r: index of row r's first head
         const uint32_t fh = H ? g0 + 32u * lane + (__ffs(H) - 1u) : GNONE;
         uint32_t nx = __shfl_down_sync(0xffffffffu, fh, 1);
         if (lane >= TROWS - 1u) nx = later;
