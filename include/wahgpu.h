@@ -85,7 +85,8 @@ int64_t wahgpu_ctx_launches(wahgpu_ctx* ctx);
                                       4 single-pass group-space kernel over CTA tiles, \
                                       5 single-pass group-space kernel over warp tiles */
 #define WAHGPU_TUNE_RANGE_ORDER 2 /* batch work order: 0 query by query; 1 (default) tile by tile, row ids in one \
-                                     pass (query by query) for small batches, else as 2; 2 tile by tile, row ids \
+                                     pass (query by query), as 2 for large capped batches whose limits leave \
+                                     most tiles unvisited; 2 tile by tile, row ids \
                                      of several queries placed by a count pass and a scan (capped batches: the id \
                                      pass revisits only the tiles holding ids under each query's limit) */
 #define WAHGPU_TUNE_RANGE_CTAS 3  /* resident CTAs per SM of the persistent range launch: 0 (all that fit) .. 32 */
@@ -291,7 +292,7 @@ int64_t wahgpu_evaluate(wahgpu_ctx* ctx, const wahgpu_term* terms, uint32_t nter
 /* Batches: nq conjunctive queries, query q being terms
  * [query_offsets[q], query_offsets[q+1]); all indexes of a batch share one
  * row count.  The whole batch runs at once (wahgpu_batch_run: one or two
- * kernel launches, three with the row ids of a large batch; capturable in a
+ * kernel launches, three with the limited row ids of a large batch; capturable in a
  * CUDA graph after a first run); rid_cap > 0 keeps the row ids of all queries
  * back to back in device memory, rid_cap == 0 counts only. */
 int wahgpu_batch_create(wahgpu_ctx* ctx, const wahgpu_term* terms, const uint32_t* query_offsets,

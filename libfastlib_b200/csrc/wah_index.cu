@@ -454,6 +454,19 @@ extern "C" int wahgpu_batch_create_capped(wahgpu_ctx* ctx, const wahgpu_term* te
     return batch_create(ctx, terms, query_offsets, nq, tot, 0, LOC_HITS, rid_caps, out);
 }
 
+static constexpr size_t SLOTS_AT_MOST = 64u << 20;  // scratch for the row ids a count pass keeps
+
+// Does the second pass over a capped batch evaluate a quarter of its items at
+// most?  A query's items are visited from the first on until its limit is
+// reached, and not at all where the count pass keeps their ids.
+static bool few_ids(const std::vector<double>& hits, const std::vector<DevQuery>& q, uint32_t ntiles) {
+    const bool kept = q.size() * ntiles * RSLOT * 4 <= SLOTS_AT_MOST;
+    double share = 0;
+    for (size_t i = 0; i < q.size(); ++i)
+        if (!kept || hits[i] > (double)ntiles * (RSLOT / 2)) share += std::min(1.0, (double)q[i].rid_lim / std::max(1.0, hits[i]));
+    return 4 * share <= (double)q.size();
+}
+
 static int batch_create(wahgpu_ctx* ctx, const wahgpu_term* terms, const uint32_t* query_offsets,
                         uint32_t nq, uint64_t rid_cap, int dense_first, int mode, const uint64_t* caps,
                         wahgpu_batch** out) {
@@ -499,6 +512,7 @@ static int batch_create(wahgpu_ctx* ctx, const wahgpu_term* terms, const uint32_
     std::vector<uint64_t> base(nq, 0);  // counts known beforehand
     std::vector<uint32_t> edge_term, edge_q;  // {term, bitmap} and query of the edges counted alone
     const bool count_only = !rid_cap && !dense_first;
+    std::vector<double> hits;  // capped: expected per query
     uint64_t rid_base = 0;
     bool general = false;
     for (uint32_t q = 0; q < nq; ++q) {
@@ -523,6 +537,13 @@ static int batch_create(wahgpu_ctx* ctx, const wahgpu_term* terms, const uint32_
         d.rid_base = rid_base;
         d.rid_lim = caps ? caps[q] : 0;
         rid_base += caps ? caps[q] : 0;
+        if (caps) {
+            // hits expected, the terms taken as independent
+            double h = x0->nrows;
+            for (uint32_t i = d.t0; i < d.t1; ++i)
+                h *= std::min(1.0, (double)term_estimate(idx[dt[i].index], dt[i]) / std::max(1u, x0->nrows));
+            hits.push_back(h);
+        }
         std::stable_sort(dt.begin() + d.t0, dt.begin() + d.t1, [&](const DevTerm& a, const DevTerm& b) {
             if (a.dense != b.dense) return a.dense > b.dense;
             return term_estimate(idx[a.index], a) < term_estimate(idx[b.index], b);
@@ -549,6 +570,7 @@ static int batch_create(wahgpu_ctx* ctx, const wahgpu_term* terms, const uint32_
     }
     B->rid_cap = rid_cap;
     B->capped = caps != nullptr;
+    if (caps) B->few_ids = few_ids(hits, dq, B->ntiles);
     if (caps) {
         B->h_lim.assign(caps, caps + nq);
         B->h_base.resize(nq);
@@ -611,8 +633,6 @@ static void launch_range_mode(const wahgpu_batch* B, const RangeArgs& a) {
     else launch_range<RQUADS, MODE, false>(B->ctx, a);
 }
 
-static constexpr size_t SLOTS_AT_MOST = 64u << 20;  // scratch for the row ids a count pass keeps
-
 extern "C" int wahgpu_batch_run(wahgpu_batch* B) {
     if (!B) return WAHGPU_EINVAL;
     wahgpu_ctx* ctx = B->ctx;
@@ -647,13 +667,17 @@ extern "C" int wahgpu_batch_run(wahgpu_batch* B) {
     a.item_cnt = nullptr; a.item_off = nullptr; a.item_list = nullptr; a.slots = nullptr;
     a.capped = B->capped && B->d_rids ? 1u : 0u;
     // Row ids: order 0 asks for the look-back, order 2 for two passes (of
-    // several queries); order 1 takes the look-back while every item has a
-    // CTA of its own at once.  Past that a CTA would sit waiting for the
-    // slowest of the items before its own: 1024 conjunctions over 10M rows,
-    // 256 ids each, take 4.3 ms so and 2.05 ms in two passes.
+    // several queries); order 1 takes two passes for a capped batch of many
+    // items whose limits leave most of them unvisited by the second pass (few_ids()).
+    // Where all ids are wanted that pass evaluates the items again, and the
+    // look-back's waits cost less: ms by look-back / two passes, uncapped,
+    // 2048 items of ranges over 1M rows 0.172 / 0.198, 256 conjunctions over
+    // 50M rows 9.3 / 12.3; 256 ids each, 1264 items 0.113 / 0.130, 5056 0.311 /
+    // 0.260, 1024 conjunctions over 10M rows (80896) 4.3 / 2.3; 2^20 ids each,
+    // 256 conjunctions over 50M rows 8.4 / 10.5, 256 ranges over them 2.1 / 1.3.
     const bool ids = B->d_rids || B->d_dense;
     const bool two_pass = ids && ((ctx->range_order == 2 && B->nq > 1) ||
-                                  (ctx->range_order == 1 && nitems > 4u * (uint32_t)ctx->sm_count));
+                                  (ctx->range_order == 1 && B->few_ids && nitems > 16u * (uint32_t)ctx->sm_count));
     a.tile_major = ((ctx->range_order != 0 && !ids) || two_pass) ? 1u : 0u;
     // items are claimed one by one where CTAs take several; with about one each
     // the claims' round trips are only added (one query of 50M rows: 46 us

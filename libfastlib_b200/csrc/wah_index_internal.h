@@ -66,6 +66,7 @@ struct wahgpu_batch {
     uint64_t bytes = 0;               // algorithmic bytes one run reads
     uint64_t min_bytes = 0;           // the bytes sumBins itself must read (covered set or complement)
     bool capped = false;              // row ids limited per query, each query in a region of its own
+    bool few_ids = false;             // its limits leave most items unvisited by a second pass
     std::vector<uint64_t> h_lim, h_base;
     bool h_valid = false;
     bool captured = false;            // a graph may hold a run of it
