@@ -16,7 +16,6 @@
 #include <cstdarg>
 #include <cstring>
 #include <mutex>
-#include <map>
 #include <vector>
 #include <string>
 
@@ -42,94 +41,48 @@ int wg_fail(wahgpu_ctx* ctx, int code, const char* fmt, ...) {
     } while (0)
 
 // -------------------------------------------------------------- allocator
-static size_t size_class(size_t b) {
-    if (b < 256) return 256;
-    if (b <= (1u << 20)) { size_t c = 256; while (c < b) c <<= 1; return c; }
-    return (b + (1u << 20) - 1) & ~(size_t)((1u << 20) - 1);
-}
-void* wg_alloc(wahgpu_ctx* ctx, size_t bytes) {
-    size_t c = size_class(bytes);
-    {
-        std::lock_guard<std::mutex> g(ctx->mu);
-        if (ctx->test_fail_alloc > 0 && --ctx->test_fail_alloc == 0) return nullptr;  // test hook
-        auto it = ctx->pool.find(c);
-        if (it != ctx->pool.end() && !it->second.empty()) {
-            void* p = it->second.back();
-            it->second.pop_back();
-            return p;
-        }
-    }
+static void* driver_get(size_t bytes) {
     void* p = nullptr;
-    if (cudaMalloc(&p, c) != cudaSuccess) {
-        // release cached blocks and retry once
+    if (cudaMalloc(&p, bytes) == cudaSuccess) return p;
+    cudaGetLastError();
+    return nullptr;
+}
+static void driver_put(void* p) { cudaFree(p); }
+static void* driver_host_get(size_t bytes) {
+    void* p = nullptr;
+    if (cudaMallocHost(&p, bytes) == cudaSuccess) return p;
+    cudaGetLastError();
+    return nullptr;
+}
+static void driver_host_put(void* p) { cudaFreeHost(p); }
+// Slabs of 1, 8 and then 64 MB of device memory, 64 KB .. 16 MB of pinned memory.
+wahgpu_ctx::wahgpu_ctx()
+    : dev(driver_get, driver_put, (size_t)1 << 20, 8, (size_t)64 << 20),
+      host(driver_host_get, driver_host_put, (size_t)64 << 10, 2, (size_t)16 << 20) {}
+
+void* wg_alloc(wahgpu_ctx* ctx, size_t bytes) {
+    if (ctx->test_fail_alloc > 0 && --ctx->test_fail_alloc == 0) return nullptr;  // test hook
+    void* p = ctx->dev.take(bytes);
+    if (!p) {
+        // release cached memory and retry once
         cudaStreamSynchronize(ctx->stream);
-        std::lock_guard<std::mutex> g(ctx->mu);
-        for (auto& kv : ctx->pool)
-            for (void* q : kv.second) {
-                cudaFree(q);
-                ctx->sizes.erase(q);
-                ctx->bytes_allocated -= kv.first;
-            }
-        ctx->pool.clear();
         if (ctx->ws && !ctx->ws_captured) {
-            cudaFree(ctx->ws);
-            ctx->bytes_allocated -= ctx->ws_bytes;
-            ctx->sizes.erase(ctx->ws);
+            ctx->dev.give(ctx->ws);
             ctx->ws = nullptr;
             ctx->ws_bytes = 0;
         }
-        cudaGetLastError();
-        if (cudaMalloc(&p, c) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+        ctx->dev.trim();
+        p = ctx->dev.take(bytes);
     }
-    std::lock_guard<std::mutex> g(ctx->mu);
-    ctx->sizes[p] = c;
-    ctx->bytes_allocated += c;
     return p;
 }
-// A cached block of the pool, or null: for buffers that a call can do without.
-static void* wg_alloc_cached(wahgpu_ctx* ctx, size_t bytes) {
-    std::lock_guard<std::mutex> g(ctx->mu);
-    auto it = ctx->pool.find(size_class(bytes));
-    if (it == ctx->pool.end() || it->second.empty()) return nullptr;
-    void* p = it->second.back();
-    it->second.pop_back();
-    return p;
-}
-void wg_free(wahgpu_ctx* ctx, void* p) {
-    if (!p) return;
-    std::lock_guard<std::mutex> g(ctx->mu);
-    auto it = ctx->sizes.find(p);
-    if (it == ctx->sizes.end()) return;
-    ctx->pool[it->second].push_back(p);
-}
+void wg_free(wahgpu_ctx* ctx, void* p) { ctx->dev.give(p); }
 
-// Pinned host blocks, pooled by size class like the device blocks: staging
-// for copies that must not wait for the host (a block goes back to the pool
-// only once the copies reading it are known to be done).
-void* wg_host_alloc(wahgpu_ctx* ctx, size_t bytes) {
-    const size_t c = size_class(bytes);
-    {
-        std::lock_guard<std::mutex> g(ctx->mu);
-        auto it = ctx->hpool.find(c);
-        if (it != ctx->hpool.end() && !it->second.empty()) {
-            void* p = it->second.back();
-            it->second.pop_back();
-            return p;
-        }
-    }
-    void* p = nullptr;
-    if (cudaMallocHost(&p, c) != cudaSuccess) { cudaGetLastError(); return nullptr; }
-    std::lock_guard<std::mutex> g(ctx->mu);
-    ctx->hsizes[p] = c;
-    return p;
-}
-void wg_host_free(wahgpu_ctx* ctx, void* p) {
-    if (!p) return;
-    std::lock_guard<std::mutex> g(ctx->mu);
-    auto it = ctx->hsizes.find(p);
-    if (it == ctx->hsizes.end()) return;
-    ctx->hpool[it->second].push_back(p);
-}
+// Pinned host blocks: staging for copies that must not wait for the host (a
+// block goes back to the pool only once the copies reading it are known to be
+// done).
+void* wg_host_alloc(wahgpu_ctx* ctx, size_t bytes) { return ctx->host.take(bytes); }
+void wg_host_free(wahgpu_ctx* ctx, void* p) { ctx->host.give(p); }
 
 // The stream's calls are being captured: they run later, and perhaps often.
 bool wg_capturing(const wahgpu_ctx* ctx) {
@@ -149,8 +102,7 @@ int wg_scratch(wahgpu_ctx* ctx, uint32_t ntiles, TileRec** recs, LaunchSync** sy
             return wg_fail(ctx, WAHGPU_ECUDA, "a captured call needs scratch for %u tiles: make it once before the capture", ntiles);
         const uint32_t want = std::max({ntiles + ntiles / 2, 1024u, ctx->scratch_captured ? 2 * ctx->scratch_tiles : 0u});
         CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-        if (ctx->scratch_captured) ctx->scratch_kept.push_back(ctx->scratch);
-        else if (ctx->scratch) cudaFree(ctx->scratch);
+        if (!ctx->scratch_captured) wg_free(ctx, ctx->scratch);
         ctx->scratch = nullptr;
         ctx->scratch_tiles = 0;
         ctx->scratch_captured = false;
@@ -159,11 +111,8 @@ int wg_scratch(wahgpu_ctx* ctx, uint32_t ntiles, TileRec** recs, LaunchSync** sy
         // kernel's (each format in a region of its own, so a stale record of
         // one is never read by the other)
         size_t bytes = sizeof(LaunchSync) * 2 + (size_t)want * (sizeof(TileRec) + 2 * sizeof(uint4));
-        if (cudaMalloc(&ctx->scratch, bytes) != cudaSuccess) {
-            cudaGetLastError();
-            ctx->scratch = nullptr;
-            return wg_fail(ctx, WAHGPU_ENOMEM, "scratch allocation of %zu bytes failed", bytes);
-        }
+        ctx->scratch = wg_alloc(ctx, bytes);
+        if (!ctx->scratch) return wg_fail(ctx, WAHGPU_ENOMEM, "scratch allocation of %zu bytes failed", bytes);
         CUDA_TRY(ctx, cudaMemsetAsync(ctx->scratch, 0, bytes, ctx->stream));
         ctx->scratch_tiles = want;
     }
@@ -187,8 +136,7 @@ unsigned char* wg_workspace(wahgpu_ctx* ctx, size_t bytes, bool captured) {
         ctx->ws_captured = false;
         ctx->ws = wg_alloc(ctx, want);
         if (!ctx->ws) return nullptr;
-        std::lock_guard<std::mutex> g(ctx->mu);
-        ctx->ws_bytes = ctx->sizes[ctx->ws];
+        ctx->ws_bytes = ctx->dev.size(ctx->ws);
     }
     ctx->ws_captured |= captured;
     return static_cast<unsigned char*>(ctx->ws);
@@ -227,7 +175,8 @@ extern "C" int wahgpu_ctx_create(int device, wahgpu_ctx** out) {
         return wg_fail(nullptr, WAHGPU_ECUDA, "stream creation failed");
     }
     c->stream = c->own_stream;
-    if (cudaMallocHost(&c->h_meta_stage, sizeof(DevMeta) * (META_SLOTS + 4)) != cudaSuccess) {
+    c->h_meta_stage = wg_host_alloc(c, sizeof(DevMeta) * (META_SLOTS + 4));
+    if (!c->h_meta_stage) {
         cudaStreamDestroy(c->own_stream);
         delete c;
         return wg_fail(nullptr, WAHGPU_ENOMEM, "pinned staging allocation failed");
@@ -240,13 +189,8 @@ extern "C" int wahgpu_ctx_destroy(wahgpu_ctx* ctx) {
     if (!ctx) return WAHGPU_EINVAL;
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
-    for (auto& kv : ctx->sizes) cudaFree(kv.first);
-    for (auto& kv : ctx->hsizes) cudaFreeHost(kv.first);
-    if (ctx->scratch) cudaFree(ctx->scratch);
-    for (void* p : ctx->scratch_kept) cudaFree(p);
-    if (ctx->h_meta_stage) cudaFreeHost(ctx->h_meta_stage);
     cudaStreamDestroy(ctx->own_stream);
-    delete ctx;
+    delete ctx;  // and its memory with it
     return WAHGPU_OK;
 }
 
@@ -750,27 +694,22 @@ int wg_launch_dense(wahgpu_ctx* ctx, int op, wahgpu_bv* x, wahgpu_bv* y, uint32_
 }
 
 // Room for the row index of b over `groups` groups.
-static bool rows_reserve(wahgpu_bv* b, uint32_t groups, void* (*alloc)(wahgpu_ctx*, size_t)) {
+static bool rows_reserve(wahgpu_bv* b, uint32_t groups) {
     wahgpu_ctx* ctx = b->ctx;
     const uint32_t need = (uint32_t)(((uint64_t)groups + PT - 1) / PT) * TROWS;
     if (b->rows && b->rows_cap >= need) return true;
     wg_free(ctx, b->rows);
     b->rows_valid = false;
     b->rows_cap = 0;
-    b->rows = static_cast<uint2*>(alloc(ctx, (size_t)need * sizeof(uint2)));
+    b->rows = static_cast<uint2*>(wg_alloc(ctx, (size_t)need * sizeof(uint2)));
     if (!b->rows) return false;
     b->rows_cap = need;
     return true;
 }
-// Room for a result's row index: a cached block, or, once the context has
-// made a few such results, a new one (a fresh context's first calls do not
-// pay for blocks that may never be read).  A result that a captured call
-// writes keeps none: its replays change the words without the index.
+// Room for a result's row index.  A result that a captured call writes keeps
+// none: its replays change the words without the index.
 static bool result_rows(wahgpu_bv* res, uint32_t groups) {
-    if (res->replayed || wg_capturing(res->ctx)) return false;
-    const bool fresh = res->ctx->row_results < 8;
-    if (fresh) res->ctx->row_results++;
-    return rows_reserve(res, groups, fresh ? wg_alloc_cached : wg_alloc);
+    return !res->replayed && !wg_capturing(res->ctx) && rows_reserve(res, groups);
 }
 // Row index of b (host metadata must be valid); built once, by a captured
 // call on each of its replays, and for words that replays change on each use.
@@ -779,7 +718,7 @@ static int wg_rows(wahgpu_bv* b) {
     // positions are taken from the words: none that the upload scan refused
     if (b->h.status) return wg_fail(ctx, WAHGPU_EFORMAT, "the bitvector's words are malformed");
     if (b->rows_valid) return WAHGPU_OK;
-    if (!rows_reserve(b, b->h.groups, wg_alloc)) return wg_fail(ctx, WAHGPU_ENOMEM, "allocation failed");
+    if (!rows_reserve(b, b->h.groups)) return wg_fail(ctx, WAHGPU_ENOMEM, "allocation failed");
     const uint32_t ntiles = (b->h.groups + PT - 1) / PT;
     k_rows<<<(ntiles + GW - 1) / GW, GCTA, 0, ctx->stream>>>(b->words, b->bpos, b->h.n, b->h.groups, ntiles, b->rows);
     ctx->launches++;
@@ -988,9 +927,7 @@ int wg_launch_gone(wahgpu_ctx* ctx, int op, wahgpu_bv* x, wahgpu_bv* y, uint32_t
 // 72 at 4M.  The row index an operand lacks is charged to its first use; an
 // operand that comes back is taken to come again.  A merge tile set on the
 // context asks for the merge.  A captured call may not allocate: it takes
-// group space only where the call before it has left all that it needs.  And a
-// context's first few calls do not pay for a large scratch block (2^27 bits:
-// 0.6 ms to allocate, 30 us a call to gain).
+// group space only where the call before it has left all that it needs.
 static bool in_group_space(wahgpu_ctx* ctx, wahgpu_bv* x, wahgpu_bv* y, uint32_t groups) {
     if (ctx->merge_tile) return false;
     const bool fits = ctx->ws_bytes >= gop_bytes(groups);
@@ -1002,12 +939,7 @@ static bool in_group_space(wahgpu_ctx* ctx, wahgpu_bv* x, wahgpu_bv* y, uint32_t
         if (!b->rows_valid && (!b->used || b->replayed)) in_groups += 3.0 + 1.5 * g;
         b->used = true;
     }
-    if (!(in_groups < 7.0 + 0.5 * std::log2(1.0 + n / 200.0) + (y ? 13e-6 : 10e-6) * n)) return false;
-    if (!fits && gop_bytes(groups) > (1u << 20) && ctx->gop_missed < 4) {
-        ctx->gop_missed++;
-        return false;
-    }
-    return true;
+    return in_groups < 7.0 + 0.5 * std::log2(1.0 + n / 200.0) + (y ? 13e-6 : 10e-6) * n;
 }
 
 // Both fall back to the merge, which needs next to no scratch, where group

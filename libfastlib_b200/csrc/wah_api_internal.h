@@ -3,11 +3,11 @@
 #define WAH_API_INTERNAL_H
 #include <cuda_runtime.h>
 #include <atomic>
-#include <map>
 #include <mutex>
 #include <string>
 #include <vector>
 #include "wah_dev.cuh"
+#include "wah_pool.h"
 
 struct wahgpu_ctx {
     int device = 0;
@@ -16,17 +16,12 @@ struct wahgpu_ctx {
     cudaStream_t own_stream = nullptr;  // the context's own stream
     std::string err;
     std::mutex mu;
-    // caching device allocator: size class -> free blocks; block -> class
-    std::map<size_t, std::vector<void*>> pool;
-    std::map<void*, size_t> sizes;
-    std::map<size_t, std::vector<void*>> hpool;  // pinned host blocks by size class
-    std::map<void*, size_t> hsizes;
-    size_t bytes_allocated = 0;
+    wah::BlockPool dev, host;  // device and pinned memory
+    wahgpu_ctx();
     // look-back scratch: two LaunchSync words then TileRec records
     void* scratch = nullptr;
     uint32_t scratch_tiles = 0;
     bool scratch_captured = false;      // a captured call uses it
-    std::vector<void*> scratch_kept;    // smaller ones that captured calls use
     void* h_meta_stage = nullptr;  // pinned staging for metadata reads
     // the bitvectors' metadata live in blocks of META_SLOTS, so that one copy
     // reads those of every result launched since the last read
@@ -35,9 +30,7 @@ struct wahgpu_ctx {
     void* ws = nullptr;            // scratch of one call (wg_workspace())
     size_t ws_bytes = 0;
     bool ws_captured = false;      // a captured call writes to it
-    uint32_t gop_missed = 0;       // group-space calls that went without a larger one
     uint64_t launches = 0;
-    uint32_t row_results = 0;           // results that could have kept a row index so far
     uint32_t dense_tile = 2048;         // WAHGPU_TUNE_DENSE_TILE
     uint32_t dense_engine = 0;          // WAHGPU_TUNE_DENSE_ENGINE
     uint32_t range_order = 1;           // WAHGPU_TUNE_RANGE_ORDER
