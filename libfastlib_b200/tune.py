@@ -14,16 +14,28 @@ from . import TUNE_DENSE_ENGINE, TUNE_DENSE_TILE, TUNE_RANGE_CTAS, TUNE_RANGE_OR
 
 def _time(fn, reps: int) -> float:
     import torch
-    fn()  # warm-up (first-launch attribute setting, allocation)
-    torch.cuda.synchronize()
     s = torch.cuda.current_stream()
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-    e0.record(s)
-    for _ in range(reps):
-        fn()
-    e1.record(s)
+
+    def ms(n):
+        e0.record(s)
+        for _ in range(n):
+            fn()
+        e1.record(s)
+        torch.cuda.synchronize()
+        return e0.elapsed_time(e1) / n
+
+    # warm-up (first-launch attribute setting, allocation): until two calls
+    # take as long
+    fn()
     torch.cuda.synchronize()
-    return e0.elapsed_time(e1) / reps
+    last = ms(1)
+    for _ in range(8):
+        now = ms(1)
+        if abs(now - last) <= 0.1 * max(now, last):
+            break
+        last = now
+    return ms(reps)
 
 
 def tune_batch(ctx, batch, count_only: bool = True, ctas=(0, 1, 2, 4), reps: int = 2):
