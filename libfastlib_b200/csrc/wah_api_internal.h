@@ -8,6 +8,7 @@
 #include <vector>
 #include "wah_dev.cuh"
 #include "wah_pool.h"
+#include "wah_budget.h"
 
 struct wahgpu_ctx {
     int device = 0;
@@ -30,6 +31,7 @@ struct wahgpu_ctx {
     void* ws = nullptr;            // scratch of one call (wg_workspace())
     size_t ws_bytes = 0;
     bool ws_captured = false;      // a captured call writes to it
+    size_t kept_at_most = wah::KEPT_AT_MOST;  // row ids that a batch's count pass keeps, bytes
     uint64_t launches = 0;
     uint32_t dense_tile = 2048;         // WAHGPU_TUNE_DENSE_TILE
     uint32_t dense_engine = 0;          // WAHGPU_TUNE_DENSE_ENGINE

@@ -454,13 +454,11 @@ extern "C" int wahgpu_batch_create_capped(wahgpu_ctx* ctx, const wahgpu_term* te
     return batch_create(ctx, terms, query_offsets, nq, tot, 0, LOC_HITS, rid_caps, out);
 }
 
-static constexpr size_t SLOTS_AT_MOST = 64u << 20;  // scratch for the row ids a count pass keeps
-
 // Does the second pass over a capped batch evaluate a quarter of its items at
 // most?  A query's items are visited from the first on until its limit is
 // reached, and not at all where the count pass keeps their ids.
-static bool few_ids(const std::vector<double>& hits, const std::vector<DevQuery>& q, uint32_t ntiles) {
-    const bool kept = q.size() * ntiles * RSLOT * 4 <= SLOTS_AT_MOST;
+static bool few_ids(const std::vector<double>& hits, const std::vector<DevQuery>& q, uint32_t ntiles, size_t kept_at_most) {
+    const bool kept = kept_bytes(q.size() * ntiles, kept_at_most) != 0;
     double share = 0;
     for (size_t i = 0; i < q.size(); ++i)
         if (!kept || hits[i] > (double)ntiles * (RSLOT / 2)) share += std::min(1.0, (double)q[i].rid_lim / std::max(1.0, hits[i]));
@@ -570,7 +568,7 @@ static int batch_create(wahgpu_ctx* ctx, const wahgpu_term* terms, const uint32_
     }
     B->rid_cap = rid_cap;
     B->capped = caps != nullptr;
-    if (caps) B->few_ids = few_ids(hits, dq, B->ntiles);
+    if (caps) B->few_ids = few_ids(hits, dq, B->ntiles, ctx->kept_at_most);
     if (caps) {
         B->h_lim.assign(caps, caps + nq);
         B->h_base.resize(nq);
@@ -690,12 +688,12 @@ extern "C" int wahgpu_batch_run(wahgpu_batch* B) {
         // per item its hits, its first row-id slot or list entry, and the ids
         // kept (without them every item with hits is evaluated again)
         const bool cap = wg_capturing(ctx);
-        const size_t ib = (size_t)nitems * 16;
+        const size_t ib = (size_t)nitems * ITEM_BYTES;
         if (!a.capped && !B->scan_tmp_bytes)
             cub::DeviceScan::ExclusiveSum(nullptr, B->scan_tmp_bytes, static_cast<unsigned long long*>(nullptr),
                                           static_cast<unsigned long long*>(nullptr), (int)nitems, ctx->stream);
         const size_t tb = a.capped ? 0 : (B->scan_tmp_bytes + 127) & ~(size_t)127;
-        size_t sb = !B->d_dense && (size_t)nitems * RSLOT * 4 <= SLOTS_AT_MOST ? (size_t)nitems * RSLOT * 4 : 0;
+        size_t sb = B->d_dense ? 0 : kept_bytes(nitems, ctx->kept_at_most);
         if (cap && ctx->ws_bytes < ib + tb + sb) sb = 0;
         unsigned char* ws = wg_workspace(ctx, ib + tb + sb, cap);
         if (!ws && sb) { sb = 0; ws = wg_workspace(ctx, ib + tb, cap); }

@@ -43,6 +43,7 @@
 #define WAH_RANGE_CUH
 #include "wah_dev.cuh"
 #include "wah_keys.h"
+#include "wah_budget.h"
 
 namespace wah {
 
@@ -141,7 +142,9 @@ struct RangeArgs {
 // 32: a lane each, 128 bytes of scratch per item.  1024 conjunctions over 10M
 // rows, 256 ids each: 3.06 -> 2.64 ms of kernels (with 4 terms 1.19 -> 0.90; one
 // term, many hits in every item, 0.35 -> 0.36).
-constexpr uint32_t RSLOT = 32;
+constexpr uint32_t RSLOT = KEPT_IDS;
+static_assert(RSLOT == 32, "a lane each");
+static_assert(RECORD_BYTES == sizeof(TileRec), "what the server charges a tile");
 
 // 64-bit sums segmented at the first item of each query: {sum lo, sum hi,
 // -, head}; (f1, s1) + (f2, s2) = (f1 | f2, f2 ? s2 : s1 + s2) is

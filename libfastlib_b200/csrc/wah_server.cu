@@ -5,12 +5,14 @@
 // Requests enter a FIFO.  A worker thread owns `nslots` execution slots, each
 // a context of its own (stream, look-back scratch, memory pool).  Whenever a
 // slot is idle it takes the pending requests in arrival order, as many as
-// fit both the batch size and the scratch budget (the device memory their
-// evaluation needs: tile records, counts, row-id buffers), builds one batch
+// fit both the batch size and the scratch budget (the device memory that the
+// batches in flight use, wah_budget.h; a request that takes more than the slots'
+// share leaves runs while nothing else does), builds one batch
 // and launches it; requests that arrive meanwhile wait for the next idle
 // slot, so batches of consecutive arrivals run concurrently on the device.
 // A slot's batch is finished when its CUDA event has completed; its requests
-// are then answered and their scratch returns to the budget.
+// are then answered and their charge returns to the budget.  The memory itself
+// stays with the slot's context for its next batches.
 #include "../../include/wahgpu.h"
 #include "wah_api_internal.h"
 #define WAH_RANGE_TYPES_ONLY
@@ -60,6 +62,7 @@ struct wahgpu_server {
     std::vector<Slot> slots;
     uint32_t max_batch = 0;
     size_t budget = 0, in_use = 0;
+    size_t kept = 0;  // of the budget: the slots' kept row ids
     std::mutex mu;
     std::condition_variable cv_work, cv_done;
     std::deque<Request*> pending;
@@ -72,11 +75,9 @@ struct wahgpu_server {
 
 namespace {
 
-// Device memory one request needs while it is evaluated.
 size_t request_scratch(const wahgpu_term* terms, uint64_t rid_cap) {
     const wahgpu_index* x = terms[0].idx;
-    const size_t ntiles = x ? x->ntiles : 1;
-    return ntiles * sizeof(wah::TileRec) + 16 + (size_t)rid_cap * 4;
+    return wah::request_charge(x ? x->ntiles : 1, rid_cap);
 }
 
 void finish_slot(wahgpu_server* S, Slot& sl) {
@@ -176,7 +177,7 @@ void worker_loop(wahgpu_server* S) {
                 std::lock_guard<std::mutex> g(S->mu);
                 while (!S->pending.empty() && take.size() < S->max_batch) {
                     Request* r = S->pending.front();
-                    if (S->in_use + scr + r->scratch > S->budget) break;
+                    if (S->in_use + scr > 0 && S->in_use + scr + r->scratch > S->budget - S->kept) break;
                     scr += r->scratch;
                     take.push_back(r);
                     S->pending.pop_front();
@@ -226,6 +227,8 @@ extern "C" int wahgpu_server_create(wahgpu_ctx* ctx, uint32_t nslots, uint32_t m
             delete S;
             return wg_fail(ctx, rc, "wahgpu_server_create: slot context creation failed");
         }
+        sl.ctx->kept_at_most = wah::slot_kept(scratch_budget, nslots);
+        S->kept += sl.ctx->kept_at_most;
     }
     S->worker = std::thread(worker_loop, S);
     *out = S;
