@@ -12,7 +12,10 @@
 // slot, so batches of consecutive arrivals run concurrently on the device.
 // A slot's batch is finished when its CUDA event has completed; its requests
 // are then answered and their charge returns to the budget.  The memory itself
-// stays with the slot's context for its next batches.
+// stays with the slot's context for its next batches, and most of it is made
+// when the server is: an allocation, which now and then takes tens of ms, stalls
+// the worker, the requests that wait make larger batches, and these allocate
+// again (5,000 queries/s answered at 2,400-3,100 with a median of 0.3-0.6 s).
 #include "../../include/wahgpu.h"
 #include "wah_api_internal.h"
 #define WAH_RANGE_TYPES_ONLY
@@ -227,8 +230,13 @@ extern "C" int wahgpu_server_create(wahgpu_ctx* ctx, uint32_t nslots, uint32_t m
             delete S;
             return wg_fail(ctx, rc, "wahgpu_server_create: slot context creation failed");
         }
+        // the memory of its batches, as far as there is any now
+        const size_t share = scratch_budget / 4 / nslots;
         sl.ctx->kept_at_most = wah::slot_kept(scratch_budget, nslots);
         S->kept += sl.ctx->kept_at_most;
+        wg_workspace(sl.ctx, sl.ctx->kept_at_most + std::min(share, (size_t)16 << 20), false);
+        sl.ctx->dev.reserve(std::min(share, (size_t)64 << 20));
+        sl.ctx->host.reserve(std::min({share, (size_t)max_batch * 8192, (size_t)64 << 20}));
     }
     S->worker = std::thread(worker_loop, S);
     *out = S;
