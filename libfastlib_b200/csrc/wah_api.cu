@@ -61,7 +61,10 @@ wahgpu_ctx::wahgpu_ctx()
       host(driver_host_get, driver_host_put, (size_t)64 << 10, 2, (size_t)16 << 20) {}
 
 void* wg_alloc(wahgpu_ctx* ctx, size_t bytes) {
-    if (ctx->test_fail_alloc > 0 && --ctx->test_fail_alloc == 0) return nullptr;  // test hook
+    {
+        std::lock_guard<std::mutex> g(ctx->mu);
+        if (ctx->test_fail_alloc > 0 && --ctx->test_fail_alloc == 0) return nullptr;  // test hook
+    }
     void* p = ctx->dev.take(bytes);
     if (!p) {
         // release cached memory and retry once
@@ -1267,8 +1270,8 @@ extern "C" int wahgpu_bv_decompress(wahgpu_bv* b) {
     wahgpu_bv* r = wg_bv_new(ctx);
     if (!r) return wg_fail(ctx, WAHGPU_ENOMEM, "allocation failed");
     rc = bv_reserve(r, G);
-    if (!rc && b->h.n) rc = wg_rows(b);
-    if (!rc && b->h.n) {
+    if (!rc) rc = wg_rows(b);  // n > 0: words without groups would be as many
+    if (!rc) {
         // the groups are b's: only the words and their number change
         r->h = b->h;
         r->h.n = G;
@@ -1283,8 +1286,6 @@ extern "C" int wahgpu_bv_decompress(wahgpu_bv* b) {
         ctx->launches++;
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) rc = wg_fail(ctx, WAHGPU_ECUDA, "launch failed: %s", cudaGetErrorString(e));
-    } else if (!rc) {
-        rc = wg_scan_meta(r, G, b->h.anb, b->h.aval);
     }
     if (rc) { wahgpu_bv_free(r); return rc; }
     cudaStreamSynchronize(ctx->stream);
