@@ -302,8 +302,8 @@ __global__ void __launch_bounds__(MERGE_THREADS, TB == 64 ? 5 : 4) k_merge(Merge
     if (tid == 0) S.hdr[0] = atomicInc(&A.sync[1].ticket, A.ntiles - 1u);
     const uint32_t G = A.groups;
     pdl_wait();
+    __syncthreads();  // no thread lets the next launch begin before the claim is made
     pdl_launch();
-    __syncthreads();
     const uint32_t t = S.hdr[0];
     // the launch epoch, read while the tile is found (it only changes after
     // the last CTA of the previous launch on this stream finished)
