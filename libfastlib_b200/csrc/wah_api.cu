@@ -55,10 +55,10 @@ static void* driver_host_get(size_t bytes) {
     return nullptr;
 }
 static void driver_host_put(void* p) { cudaFreeHost(p); }
-// Slabs of 1, 8 and then 64 MB of device memory, 64 KB .. 16 MB of pinned memory.
+// Slabs of 1, 8 and then 64 MB of device memory, 64 KB .. 64 MB of pinned memory.
 wahgpu_ctx::wahgpu_ctx()
     : dev(driver_get, driver_put, (size_t)1 << 20, 8, (size_t)64 << 20),
-      host(driver_host_get, driver_host_put, (size_t)64 << 10, 2, (size_t)16 << 20) {}
+      host(driver_host_get, driver_host_put, (size_t)64 << 10, 2, (size_t)64 << 20) {}
 
 void* wg_alloc(wahgpu_ctx* ctx, size_t bytes) {
     {
@@ -125,11 +125,11 @@ int wg_scratch(wahgpu_ctx* ctx, uint32_t ntiles, TileRec** recs, LaunchSync** sy
     return WAHGPU_OK;
 }
 // Scratch of one call (the two-pass engine's result patterns, a batch's
-// items): one block of the context that grows with its calls and is never
-// handed to anything else, so a captured call's replays write into no other
-// object.  A block that captured calls hold is kept beside the larger one that
-// follows it (at least twice its size, so these come to less than the last)
-// until the context ends.
+// items): one block of the context that grows with its calls.  One that a
+// captured call has been given is handed to nothing else until the context
+// ends, so that replays write into no other object: it is kept beside the
+// larger one that follows it (at least twice its size, so these come to less
+// than the last).
 unsigned char* wg_workspace(wahgpu_ctx* ctx, size_t bytes, bool captured) {
     if (ctx->ws_bytes < bytes) {
         const size_t want = std::max(bytes, ctx->ws_captured ? 2 * ctx->ws_bytes : ctx->ws_bytes + ctx->ws_bytes / 2);

@@ -43,11 +43,11 @@ class BlockPool {
     }
 
     // A block of at least `bytes`, or null.  A block given back serves sizes of
-    // its class, one of several MB also smaller ones down to half its size.
+    // its class; one of several MB that shares a slab, sizes down to its half too.
     void* take(size_t bytes) {
-        const size_t c = size_class(bytes);
+        const size_t c = size_class(bytes), upto = c > ((size_t)1 << 20) && c <= most_ / 4 ? 2 * c : c;
         std::lock_guard<std::mutex> g(mu_);
-        for (auto it = free_.lower_bound(c); it != free_.end() && it->first <= (c > ((size_t)1 << 20) ? 2 * c : c); ++it) {
+        for (auto it = free_.lower_bound(c); it != free_.end() && it->first <= upto; ++it) {
             if (it->second.empty()) continue;
             void* p = it->second.back();
             it->second.pop_back();
