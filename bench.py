@@ -655,7 +655,7 @@ def main():
                                       "contexts with a stream each, one graph forking and joining them"},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak if achieved else None, "traffic": traffic, "peak_kind": peak_kind,
-                         "kernel": engine_kernels + " (+ the metadata memset), per-call CUDA events over the "
+                         "kernel": engine_kernels + ", per-call CUDA events over the "
                                    "dense-path calls " + ", ".join(dense_calls),
                          "traffic_source": f"profiles/{traffic_file} (ncu dram__bytes_read.sum + "
                                            "dram__bytes_write.sum per operator call), calls "

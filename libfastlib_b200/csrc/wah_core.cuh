@@ -19,12 +19,13 @@
 //   * a run of exactly one group is a count-1 fill word iff the walk emitted
 //     that group through append_counter or by copying a count-1 fill word
 //     verbatim, else the literal 0 / 0x7FFFFFFF.
-// The walk is sequential, but its step structure is a finite-state function
-// of local information at every boundary between the two streams' words:
-// each step lies inside one word of its "driver" operand, and whether a step
-// continues across a boundary depends only on the step type and the words
-// meeting there.  So the step state at every segment follows from a parallel
-// prefix over per-segment transfer functions (5 states, composed as tables).
+// The walk is sequential, but which of these happened follows from the words
+// of both operands that meet at the group, and over count-1 fills from the
+// nearest longer words before it: single_flag() below, which the kernels use.
+// The walk's step states as a finite-state function of the words at every
+// boundary (5 states, per-segment transfer functions composed as tables:
+// seg_transfer, fsm_*, seg_fill_flag) are the form that the CPU models check
+// it against.
 #ifndef WAH_CORE_CUH
 #define WAH_CORE_CUH
 #include <stdint.h>

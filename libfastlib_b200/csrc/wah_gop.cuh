@@ -26,16 +26,15 @@
 //  * k_gpack: a tile's R arrives the same way; each head's lane writes its
 //    word at the number of heads before it: the literal, or the run word
 //    whose length reaches the next head.
-// Bound by instruction issue (the integer pipe first) and the few warps that
-// two buffers per warp leave room for.  At 2^28 bits, both operands of d =
-// 0.1 / 0.5: 39 / 40 us a call against 79 / 65 for the form before it (a
-// word-start marker per word and warp max-scans over 128 groups, operands
-// staged without prefetch, four neighbouring groups per lane; ~2370 + 1060
-// instructions per tile against 715 + 720).  Tiles of 256 groups double the
-// resident warps and are slower (46 / 50 us: the per-tile work), and so is
-// packing a tile's words in k_gop with k_gpack a copy (45 / 48: the integer
-// pipe is busy 69 % of the time there); launching each kernel while the one
-// before it drains saves 3 us a call.
+// Bound by instruction issue (60-62 % of the slots, the integer pipe 57-61 %
+// busy) and the few warps that two buffers per warp leave room for.  At 2^28
+// bits, both operands of d = 0.1 / 0.5: 39 / 40 us a call against 79 / 65 for the
+// form before it (a word-start marker per word and warp max-scans over 128
+// groups, operands staged without prefetch, four neighbouring groups per lane;
+// ~2370 + 1060 instructions per tile against 720 + 775).  Tiles of 256 groups
+// double the resident warps and are slower (46 / 50 us: the per-tile work), and
+// so is packing a tile's words in k_gop with k_gpack a copy (45 / 48);
+// launching each kernel while the one before it drains saves 3 us a call.
 #ifndef WAH_GOP_CUH
 #define WAH_GOP_CUH
 #include <type_traits>

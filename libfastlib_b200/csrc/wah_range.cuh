@@ -36,9 +36,10 @@
 // A query's dense terms go first; an empty AND skips the rest.
 //
 // Counts run tile by tile (the queries of a batch share a tile's rows and
-// words in L2), items dealt to the CTAs in turn.  Row ids take two such
-// passes around a scan of the items' hits, or, when the items are few, one
-// pass with a decoupled look-back in query order.
+// words in L2); where the CTAs take several items each, these are claimed one
+// by one.  Row ids take one pass with a decoupled look-back in query order, or,
+// for limits that leave most items unvisited, two tile by tile around a list of
+// the others.
 #ifndef WAH_RANGE_CUH
 #define WAH_RANGE_CUH
 #include "wah_dev.cuh"
@@ -139,9 +140,10 @@ struct RangeArgs {
 // Row ids kept by the count pass for an item with at most so many: the id
 // pass orders and copies them instead of evaluating the item again.  A
 // conjunction that needs many items to fill its limit has few hits in each.
-// 32: a lane each, 128 bytes of scratch per item.  1024 conjunctions over 10M
-// rows, 256 ids each: 3.06 -> 2.64 ms of kernels (with 4 terms 1.19 -> 0.90; one
-// term, many hits in every item, 0.35 -> 0.36).
+// 32: a lane each, 128 bytes of scratch per item.  When added, before the items
+// were claimed: 1024 conjunctions over 10M rows, 256 ids each, 3.06 -> 2.64 ms of
+// kernels (with 4 terms 1.19 -> 0.90; one term, many hits in every item, 0.35 ->
+// 0.36).
 constexpr uint32_t RSLOT = KEPT_IDS;
 static_assert(RSLOT == 32, "a lane each");
 static_assert(RECORD_BYTES == sizeof(TileRec), "what the server charges a tile");
@@ -620,7 +622,7 @@ __device__ __forceinline__ void copy_slot(const RangeArgs& A, uint32_t item, uin
 // edge rows' gathers, the others by the block barriers between their steps.
 // One range over 1M rows of 100 values with its row ids: 17 us on 32 CTAs,
 // 93 us when 8 CTAs walked the edge bitmaps' words; 1024 conjunctions over
-// 10M rows: 2.05 ms against 7.7 ms.  (Asking the next item's rows into L2 ahead
+// 10M rows with 256 ids each: 2.2 ms against 7.7 ms.  (Asking the next item's rows into L2 ahead
 // made that 3.8: most rows of later terms are never needed.)
 template <int Q, int MODE, bool GEN>
 __global__ void __launch_bounds__(RTHREADS, 6) k_range(RangeArgs A) {
