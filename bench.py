@@ -467,8 +467,8 @@ def main():
         ctx.set_stream(None)
         return
 
-    # per-call device time of each operator call (its kernels and metadata
-    # memset): a graph of REPS back-to-back calls, timed by events.  The
+    # per-call device time of each operator call (its kernels): a graph of
+    # REPS back-to-back calls, timed by events.  The
     # roofline line is for the dense-path calls, which the reference's _d2
     # rule (|a|+|b|)*31 > nbits selects for the denser pairs and which take
     # most of the step: by default the two-pass group-space kernels (k_gop,

@@ -538,8 +538,9 @@ def estimate_count(ctx: Context, term) -> int:
 
 
 class Batch:
-    """Queries prepared once and run as one kernel launch (capturable in a
-    CUDA graph).  queries: list of lists of terms."""
+    """Queries prepared once and run at once, in one to three kernel launches
+    (capturable in a CUDA graph after a first run).  queries: list of lists of
+    terms."""
 
     def __init__(self, ctx: Context, queries, rid_cap: int = 0, caps=None):
         """rid_cap: room for the row ids of all queries, back to back; caps:
