@@ -298,8 +298,8 @@ __global__ void __launch_bounds__(MERGE_THREADS, TB == 64 ? 5 : 4) k_merge(Merge
     // have a word of their own, which its last claim sets back to 0; this
     // launch begins when every block of the launch before it has made its
     // claim, so they are made while that one drains.  (2^28 bits, d = 1e-2, 700
-    // tiles: 1.5 us a call over tile = block; claims after the wait, 3.)
-    if (tid == 0) S.hdr[0] = atomicInc(&A.sync[1].ticket, A.ntiles - 1u);
+    // tiles: 1.8 us a call over tile = block; claims after the wait, 3.5.)
+    if (tid == 0) S.hdr[0] = A.ntiles > 1u ? atomicInc(&A.sync[1].ticket, A.ntiles - 1u) : 0u;
     const uint32_t G = A.groups;
     pdl_wait();
     __syncthreads();  // no thread lets the next launch begin before the claim is made
