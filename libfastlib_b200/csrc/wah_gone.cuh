@@ -36,8 +36,29 @@
 
 namespace wah {
 
+constexpr int GT = DT;            // groups per tile, a warp's
+constexpr int GWARPS = 4;         // warps per CTA
+constexpr int GTHREADS = GWARPS * 32;
+constexpr int NCH = GT / 128;
 constexpr int GROWS = 8;          // 32-word rows of each operand in flight per lane
 constexpr uint32_t GSHORT = 8;    // fills up to this many groups of the tile are painted by their own lane
+
+// Word range of one operand over the tile [g0, g1): words [wi0, wend), the
+// first starting at group s0.  gt: the operand's group-tile index (entry
+// past the end = (n, G)).  Returns false for words the metadata scan would
+// have rejected (a tile word count that cannot be).
+__device__ __forceinline__ bool gop_range(const uint32_t* __restrict__ gt, uint32_t n, uint32_t g0, uint32_t g1,
+                                          uint32_t& wi0, uint32_t& s0, uint32_t& nw) {
+    const uint32_t e0 = g0 / DT, e1 = (g1 + DT - 1) / DT;
+    wi0 = __ldg(gt + 2 * e0); s0 = __ldg(gt + 2 * e0 + 1);
+    const uint32_t wi1 = __ldg(gt + 2 * e1), s1 = __ldg(gt + 2 * e1 + 1);
+    // the word covering g1 belongs to the tile when it starts before g1
+    const uint32_t wend = (wi1 < n && s1 < g1) ? wi1 + 1u : wi1;
+    nw = wend - wi0;
+    const bool ok = wi0 < n && wend <= n && wend > wi0 && nw <= (uint32_t)GT && !(g0 > 0 && s0 >= g0 && wi0 == 0);
+    if (!ok) nw = 0;
+    return ok;
+}
 
 // per warp: both operands' patterns over its tile (group g0 + i at index i)
 struct GoneWarp {

@@ -42,17 +42,12 @@
 
 namespace wah {
 
-constexpr int GT = DT;                    // groups per tile of the single-pass warp-tile engine (wah_gone.cuh)
 constexpr int PT = 512;                   // groups per tile of this engine, a warp's
 constexpr int TROWS = PT / 32;            // rows of 32 groups per tile
 constexpr int GW = 8;                     // warps per CTA of this engine
 constexpr int GBUF = PT + 8;              // staged words of a tile: its own, the ones either side, 16-byte ends
 constexpr int GCTA = GW * 32;
 constexpr uint32_t GNONE = 0xFFFFFFFFu;   // no head
-// the single-pass warp-tile engine's shape (wah_gone.cuh)
-constexpr int GWARPS = 4;
-constexpr int GTHREADS = GWARPS * 32;
-constexpr int NCH = GT / 128;
 static_assert(TROWS == 16, "a half warp holds a tile's rows");
 
 enum GopKind : int {
@@ -75,23 +70,6 @@ struct GopArgs {
     uint32_t aval, anb;
     uint32_t withhold;    // test hook: this tile's wait counts as given up (UINT32_MAX: none)
 };
-
-// Word range of one operand over the tile [g0, g1): words [wi0, wend), the
-// first starting at group s0.  gt: the operand's group-tile index (entry
-// past the end = (n, G)).  Returns false for words the metadata scan would
-// have rejected (a tile word count that cannot be).
-__device__ __forceinline__ bool gop_range(const uint32_t* __restrict__ gt, uint32_t n, uint32_t g0, uint32_t g1,
-                                          uint32_t& wi0, uint32_t& s0, uint32_t& nw) {
-    const uint32_t e0 = g0 / DT, e1 = (g1 + DT - 1) / DT;
-    wi0 = __ldg(gt + 2 * e0); s0 = __ldg(gt + 2 * e0 + 1);
-    const uint32_t wi1 = __ldg(gt + 2 * e1), s1 = __ldg(gt + 2 * e1 + 1);
-    // the word covering g1 belongs to the tile when it starts before g1
-    const uint32_t wend = (wi1 < n && s1 < g1) ? wi1 + 1u : wi1;
-    nw = wend - wi0;
-    const bool ok = wi0 < n && wend <= n && wend > wi0 && nw <= (uint32_t)GT && !(g0 > 0 && s0 >= g0 && wi0 == 0);
-    if (!ok) nw = 0;
-    return ok;
-}
 
 // The word covering group g < groups and its first group (whole warp): a
 // 32-way search of the block positions (bp[0] = 0, ascending), then a scan of
