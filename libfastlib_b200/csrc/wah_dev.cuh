@@ -97,11 +97,11 @@ __device__ __forceinline__ void finish_tile(LaunchSync* s, uint32_t ntiles, uint
     __threadfence();
     uint32_t d = atomicAdd(&s->done, 1u);
     if ((d & ~DONE_ERROR) == ntiles - 1) {
-        if (status) *status = d & DONE_ERROR ? DEV_ERR_TIMEOUT : 0u;
         s->ticket = 0;
         s->done = 0;
         __threadfence();
         atomicAdd(&s->epoch, 1u);
+        if (status) *status = d & DONE_ERROR ? DEV_ERR_TIMEOUT : 0u;
     }
 }
 
